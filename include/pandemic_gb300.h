@@ -190,10 +190,8 @@ typedef struct pt_tuning {
     int infect_blocks_per_sm;   /* infection grid, 256-thread blocks per SM: 1..32 */
     int radix_blocks_per_sm;    /* persistent blocks of a day's radix pass per SM: 1..4
                                    (3 at 80 registers a thread, 4 at 64) */
-    int sched_tf;               /* the schedule kernel's Threefry arithmetic (same results):
-                                   0 integer adds and funnel shifts; 1 the 64-bit adds as
-                                   multiply-adds with carry; 2 also the rotations as wide
-                                   multiplies (moves work from the ALU to the FMA pipe) */
+    int sched_tf;               /* 0..2, kept as given; every value runs the same Threefry
+                                   arithmetic, the one measured fastest */
     int dense_level;            /* days whose sort reads every schedule key directly instead
                                    of entries the schedule kernel appends: 0 none; 1, 2, 3
                                    when the instance's infected are at least a quarter of,

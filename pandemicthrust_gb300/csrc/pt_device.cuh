@@ -41,52 +41,56 @@ static __constant__ int c_weekend_assign[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}
 
 // ---------------------------------------------------------------- Threefry
 // Threefry-2x64-20 and 2x32-20 (Salmon et al., SC'11; the Random123 rotation
-// tables).  64-bit words are handled as 32-bit halves so each rotation is two
-// funnel shifts and each add an add/add-with-carry pair.
+// tables).  The integer (ALU) pipe bounds every kernel that draws many blocks: a
+// 64-bit rotation is two funnel shifts and an XOR two logic operations, 76 ALU
+// instructions a block, and each 64-bit add takes two more.  So the adds are kept off
+// that pipe where it can be done: the high word is a multiply-add with carry by a 1 the
+// compiler cannot see (FMA pipe), the first round's sum of the two key-added counter
+// words is 2 ctr + (k0 + k1), and each key injection of x0 is folded into the next
+// round's add (three operands).  Measured alone on a GB300: 110 ALU and 135
+// instructions a block, 239 cycles a warp, against 126 / 147 / 275 with plain
+// add / add-with-carry pairs, 257 with every add as a multiply-add, 300 and more with
+// rotations or low words as wide multiplies.
 struct u64h { uint32_t lo, hi; };
 
 __device__ __forceinline__ u64h mk(uint64_t v) { return {(uint32_t)v, (uint32_t)(v >> 32)}; }
+__device__ __forceinline__ uint64_t pack64(u64h v) { return ((uint64_t)v.hi << 32) | v.lo; }
 
-__device__ __forceinline__ u64h add64(u64h a, u64h b)
+static __constant__ uint32_t c_one = 1u;   // (not const: the compiler may not fold it)
+
+__device__ __forceinline__ uint64_t add64(uint64_t a, uint64_t b)
 {
+    const u64h x = mk(a), y = mk(b);
     u64h r;
-    asm("add.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, %5;"
-        : "=r"(r.lo), "=r"(r.hi) : "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi));
-    return r;
+    asm("add.cc.u32 %0, %2, %4;\n\tmadc.lo.u32 %1, %3, %6, %5;"
+        : "=r"(r.lo), "=r"(r.hi) : "r"(x.lo), "r"(x.hi), "r"(y.lo), "r"(y.hi), "r"(c_one));
+    return pack64(r);
 }
 
 template <int R>
-__device__ __forceinline__ u64h rotl64(u64h x)
+__device__ __forceinline__ uint64_t rotl64(uint64_t v)
 {
+    const u64h x = mk(v);
     if constexpr (R == 32) {
-        return {x.hi, x.lo};
+        return pack64({x.hi, x.lo});
     } else if constexpr (R < 32) {
-        return {__funnelshift_l(x.hi, x.lo, R), __funnelshift_l(x.lo, x.hi, R)};
+        return pack64({__funnelshift_l(x.hi, x.lo, R), __funnelshift_l(x.lo, x.hi, R)});
     } else {
-        return {__funnelshift_l(x.lo, x.hi, R - 32), __funnelshift_l(x.hi, x.lo, R - 32)};
+        return pack64({__funnelshift_l(x.lo, x.hi, R - 32), __funnelshift_l(x.hi, x.lo, R - 32)});
     }
 }
 
-template <int R>
-__device__ __forceinline__ void mix64(u64h &x0, u64h &x1)
-{
-    x0 = add64(x0, x1);
-    x1 = rotl64<R>(x1);
-    x1.lo ^= x0.lo;
-    x1.hi ^= x0.hi;
-}
-
 struct TfKey {
-    u64h k0, k1, k2;       // key schedule: k2 = parity ^ k0 ^ k1
+    uint64_t k0, k1, k2;   // key schedule: k2 = parity ^ k0 ^ k1
     uint32_t k32_0, k32_1, k32_2;
 };
 
 __device__ __forceinline__ TfKey make_key(const SimConst &c)
 {
     TfKey k;
-    k.k0 = mk(c.key0);
-    k.k1 = mk(c.key1);
-    k.k2 = mk(0x1BD11BDAA9FC1A22ULL ^ c.key0 ^ c.key1);
+    k.k0 = c.key0;
+    k.k1 = c.key1;
+    k.k2 = 0x1BD11BDAA9FC1A22ULL ^ c.key0 ^ c.key1;
     k.k32_0 = (uint32_t)c.key0;
     k.k32_1 = (uint32_t)c.key1;
     k.k32_2 = 0x1BD11BDAu ^ k.k32_0 ^ k.k32_1;
@@ -97,93 +101,23 @@ __device__ __forceinline__ TfKey make_key(const SimConst &c)
 // w[0] = lo(x0), w[1] = hi(x0), w[2] = lo(x1), w[3] = hi(x1).
 __device__ __forceinline__ void tf2x64(const TfKey &k, uint64_t ctr, uint32_t w[4])
 {
-    u64h c = mk(ctr);
-    u64h x0 = add64(c, k.k0);
-    u64h x1 = add64(c, k.k1);
-    const u64h ks[3] = {k.k0, k.k1, k.k2};
+    // x0 holds the sum of a round; x1 its rotated and XORed word
+    uint64_t x0 = 2 * ctr + (k.k0 + k.k1), x1 = ctr + k.k1;
+    const uint64_t ks[3] = {k.k0, k.k1, k.k2};
 #pragma unroll
     for (int blk = 0; blk < 5; blk++) {
-        if ((blk & 1) == 0) {
-            mix64<16>(x0, x1); mix64<42>(x0, x1); mix64<12>(x0, x1); mix64<31>(x0, x1);
-        } else {
-            mix64<16>(x0, x1); mix64<32>(x0, x1); mix64<24>(x0, x1); mix64<21>(x0, x1);
-        }
+        x1 = rotl64<16>(x1) ^ x0;
+        x0 = add64(x1, x0);
+        x1 = ((blk & 1) == 0 ? rotl64<42>(x1) : rotl64<32>(x1)) ^ x0;
+        x0 = add64(x1, x0);
+        x1 = ((blk & 1) == 0 ? rotl64<12>(x1) : rotl64<24>(x1)) ^ x0;
+        x0 = add64(x1, x0);
+        x1 = ((blk & 1) == 0 ? rotl64<31>(x1) : rotl64<21>(x1)) ^ x0;
         const int s = blk + 1;
-        x0 = add64(x0, ks[s % 3]);
-        x1 = add64(x1, add64(ks[(s + 1) % 3], u64h{(uint32_t)s, 0u}));
+        x1 += ks[(s + 1) % 3] + (uint64_t)s;
+        x0 += s < 5 ? ks[s % 3] + x1 : ks[s % 3];   // with the next round's add
     }
-    w[0] = x0.lo; w[1] = x0.hi; w[2] = x1.lo; w[3] = x1.hi;
-}
-
-// The same Threefry-2x64-20 with part of its integer work moved from the ALU pipe
-// (IADD3 / SHF / LOP3) to the multiply-add pipe.  `m` holds run-time constants (kernel
-// parameters, so the compiler cannot fold the multiplies back into adds and shifts):
-// m.one = 1 and m.pow[i] = 2^r for the rotation amounts r below 32.
-//   MODE 1: every 64-bit add is a multiply-add with carry, x * 1 + y.
-//   MODE 2: also every rotation: x * 2^r as a 32 x 32 -> 64 multiply gives both
-//           halves of x shifted by r; two of them and an OR rotate a 64-bit word, and
-//           the OR folds into the round's XOR.
-// Bit-identical to tf2x64 (integer arithmetic, exact in every form).
-struct TfMul {
-    uint32_t one;
-    uint32_t pow[6];   // 2^16, 2^10 (rotation 42 = swap + 10), 2^12, 2^31, 2^24, 2^21
-};
-
-__device__ __forceinline__ u64h add64m(u64h a, u64h b, uint32_t one)
-{
-    u64h r;
-    asm("mad.lo.cc.u32 %0, %2, %6, %4;\n\tmadc.lo.u32 %1, %3, %6, %5;"
-        : "=r"(r.lo), "=r"(r.hi) : "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(one));
-    return r;
-}
-
-// rotate left by r in (0, 32) with p = 2^r: the 64-bit products hold (x << r) in the
-// low word and (x >> (32 - r)) in the high word
-__device__ __forceinline__ u64h rotl64m(u64h x, uint32_t p)
-{
-    const unsigned long long t = (unsigned long long)x.lo * p, u = (unsigned long long)x.hi * p;
-    return {(uint32_t)t | (uint32_t)(u >> 32), (uint32_t)u | (uint32_t)(t >> 32)};
-}
-
-template <int MODE, int R, int PI>
-__device__ __forceinline__ void mix64m(u64h &x0, u64h &x1, const TfMul &m)
-{
-    x0 = MODE >= 1 ? add64m(x0, x1, m.one) : add64(x0, x1);
-    if constexpr (MODE >= 2 && R != 32) {
-        const u64h s = R > 32 ? u64h{x1.hi, x1.lo} : x1;
-        x1 = rotl64m(s, m.pow[PI]);
-    } else {
-        x1 = rotl64<R>(x1);
-    }
-    x1.lo ^= x0.lo;
-    x1.hi ^= x0.hi;
-}
-
-template <int MODE>
-__device__ __forceinline__ void tf2x64m(const TfKey &k, uint64_t ctr, uint32_t w[4], const TfMul &m)
-{
-    if constexpr (MODE == 0) {
-        tf2x64(k, ctr, w);
-    } else {
-        const u64h c = mk(ctr);
-        u64h x0 = add64m(c, k.k0, m.one);
-        u64h x1 = add64m(c, k.k1, m.one);
-        const u64h ks[3] = {k.k0, k.k1, k.k2};
-#pragma unroll
-        for (int blk = 0; blk < 5; blk++) {
-            if ((blk & 1) == 0) {
-                mix64m<MODE, 16, 0>(x0, x1, m); mix64m<MODE, 42, 1>(x0, x1, m);
-                mix64m<MODE, 12, 2>(x0, x1, m); mix64m<MODE, 31, 3>(x0, x1, m);
-            } else {
-                mix64m<MODE, 16, 0>(x0, x1, m); mix64m<MODE, 32, 0>(x0, x1, m);
-                mix64m<MODE, 24, 4>(x0, x1, m); mix64m<MODE, 21, 5>(x0, x1, m);
-            }
-            const int s = blk + 1;
-            x0 = add64m(x0, ks[s % 3], m.one);
-            x1 = add64m(x1, add64(ks[(s + 1) % 3], u64h{(uint32_t)s, 0u}), m.one);
-        }
-        w[0] = x0.lo; w[1] = x0.hi; w[2] = x1.lo; w[3] = x1.hi;
-    }
+    w[0] = (uint32_t)x0; w[1] = (uint32_t)(x0 >> 32); w[2] = (uint32_t)x1; w[3] = (uint32_t)(x1 >> 32);
 }
 
 template <int R>
@@ -320,6 +254,92 @@ __device__ __forceinline__ int errand_row_loop(float y, float &frac)
     return row;
 }
 
+// The schedule kernel's form of the same draw.  A destination is row i of an errand
+// table in shared memory (ErrandRow, built per instance and hour): rows 0-3 are the
+// errand types 9, 11, 12 and 13, row 4 the afterschool type 8 of weekday children.
+// Everything runs on the draw itself, w = (float)r, with every probability scaled by
+// 2^32: scaling by a power of two commutes with each rounding below, so row, quotient
+// and business number are those of errand_row.  Type 10 has probability 0 and a
+// remainder past type 9 is above 0, so the search never ends there and its
+// subtraction of 0 is left out.
+constexpr float kTwo32 = 4294967296.f;
+template <bool WEEKEND>
+struct ErrandPdf {
+    static constexpr float p9 = (WEEKEND ? 0.51493f : 0.61919f), p11 = (WEEKEND ? 0.25586f : 0.27812f),
+                           p12 = (WEEKEND ? 0.1162f : 0.06601f), p13 = (WEEKEND ? 0.113f : 0.03668f);
+};
+constexpr int kErrandRows = 5;
+
+struct __align__(32) ErrandRow {
+    float d, r;     // 2^32 x the type's probability and 2^-32 x its reciprocal rounded to nearest
+    float count;    // locations of the type
+    int first;      // bucket of the type's first location in this hour
+    int last;       // and of its last one
+};
+
+// Row i of the table of one hour.
+template <bool WEEKEND>
+__device__ __forceinline__ ErrandRow errand_table_row(const SimConst &c, int i, int hour_base, int lo)
+{
+    typedef ErrandPdf<WEEKEND> P;
+    const int type = i == 4 ? 8 : (i == 0 ? 9 : 10 + i);
+    ErrandRow e;
+    // children: the quotient is the draw itself, y = w 2^-32
+    e.d = i == 4 ? kTwo32 : kTwo32 * (i == 0 ? P::p9 : (i == 1 ? P::p11 : (i == 2 ? P::p12 : P::p13)));
+    e.r = (i == 4 ? 1.f : (i == 0 ? 1.0f / P::p9 : (i == 1 ? 1.0f / P::p11 : (i == 2 ? 1.0f / P::p12 : 1.0f / P::p13)))) /
+          kTwo32;
+    e.count = __int2float_rn(c.type_count[type]);
+    e.first = hour_base + c.type_offset[type] - lo;
+    e.last = e.first + c.type_count[type] - 1;
+    return e;
+}
+
+// 1 when x > 0, else 0, for |x| = 0 or >= 2^-60
+__device__ __forceinline__ float unit_step(float x)
+{
+    float t;
+    asm("mul.rn.sat.f32 %0, %1, 0f6F800000;" : "=f"(t) : "f"(x));   // x 2^96, clamped to [0, 1]
+    return t;
+}
+
+// The byte offset of draw w's row in a table (`base`: the offset of row 0, or of row 4
+// with `p9` above every draw, for a child) and the remainder x the quotient divides.
+// All on the floating-point pipe, which the Threefry blocks leave idle: the steps
+// t1 >= t2 >= t3 are 0 or 1 (differences of floats are 0 or far above 2^-60 here), x
+// takes the subtractions in the loop's order and rounding, and the offset is summed
+// in the bits of denormal floats, where adding is integer adding.
+constexpr float kNoRow = 0x1p100f;   // p9 of a child: no draw exceeds it
+template <bool WEEKEND>
+__device__ __forceinline__ int errand_step(float w, float p9, int base, float &x)
+{
+    typedef ErrandPdf<WEEKEND> P;
+    constexpr float p11 = kTwo32 * P::p11, p12 = kTwo32 * P::p12;
+    const float f1 = __fsub_rn(w, p9), f2 = __fsub_rn(f1, p11), f3 = __fsub_rn(f2, p12);
+    const float t1 = unit_step(f1), t2 = unit_step(f2), t3 = unit_step(f3);
+    x = __fmaf_rn(-t3, p12, __fmaf_rn(-t2, p11, __fmaf_rn(-t1, p9, w)));
+    constexpr int row = (int)sizeof(ErrandRow);
+    const float step = __int_as_float(row);
+    return __float_as_int(__fmaf_rn(t3, step, __fmaf_rn(t2, step, __fmaf_rn(t1, step, __int_as_float(base)))));
+}
+
+template <bool WEEKEND>
+__device__ __forceinline__ float errand_p9(bool adult) { return adult ? kTwo32 * ErrandPdf<WEEKEND>::p9 : kNoRow; }
+
+// x / d of a table row, rounded to nearest (div_rn_recip on the scaled values)
+__device__ __forceinline__ float errand_quotient(const ErrandRow &e, float x) { return div_rn_recip(x, e.d, e.r); }
+
+// The bucket draw r falls into: business_in_type's rounding and clamp on the table.
+template <bool WEEKEND>
+__device__ __forceinline__ int errand_bucket(const ErrandRow *rows, uint32_t r, float p9, int base)
+{
+    float x;
+    const int at = errand_step<WEEKEND>(__uint2float_rn(r), p9, base, x);
+    const ErrandRow &e = *reinterpret_cast<const ErrandRow *>(reinterpret_cast<const char *>(rows) + at);
+    const float4 q = *reinterpret_cast<const float4 *>(&e.d);   // d, r, count, first
+    const int b = __float2int_rz(__fmul_rn(div_rn_recip(x, q.x, q.y), q.z));
+    return min(__float_as_int(q.w) + b, e.last);
+}
+
 // device_fishAfterschoolOrErrandDestination_weekday, PandemicSim.cu:2909-2947
 // (unsigned business number, as the reference).  Children go to an afterschool
 // location (type 8); adults to an errand type drawn by errand_row.  Both are computed
@@ -351,23 +371,25 @@ __device__ __forceinline__ int fish_weekend_dest(const SimConst &c, uint32_t r)
 // weekend destinations all lie in [lo, L) (lo = first location of type 9), so the
 // bucket index used here is the order-preserving compact form hour * R + dest - lo,
 // R = L - lo.
-template <int MODE = 0>
+__device__ __forceinline__ void weekend_hours(const uint32_t w[3], int &h1, int &h2, int &h3)
+{
+    h1 = (int)(w[0] % 10u);
+    h2 = (int)(w[1] % 10u);
+    h3 = (int)(w[2] % 10u);
+    if (h2 == h1) h2 = h2 == 9 ? 0 : h2 + 1;
+    // h1 and h2 differ, so two steps pass both whichever comes first
+    if (h3 == h1 || h3 == h2) h3 = h3 == 9 ? 0 : h3 + 1;
+    if (h3 == h1 || h3 == h2) h3 = h3 == 9 ? 0 : h3 + 1;
+}
+
 __device__ __forceinline__ void weekend_errands(const SimConst &c, const TfKey &k, uint64_t ctr, int lo, int R,
-                                                int out[3], const TfMul *m = nullptr)
+                                                int out[3])
 {
     uint32_t w[8];
-    if constexpr (MODE == 0) {
-        tf2x64(k, ctr, w);
-        tf2x64(k, ctr + 1, w + 4);
-    } else {
-        tf2x64m<MODE>(k, ctr, w, *m);
-        tf2x64m<MODE>(k, ctr + 1, w + 4, *m);
-    }
-    int h1 = (int)(w[0] % 10u);
-    int h2 = (int)(w[1] % 10u);
-    if (h2 == h1) h2 = (h2 + 1) % 10;
-    int h3 = (int)(w[2] % 10u);
-    while (h3 == h1 || h3 == h2) h3 = (h3 + 1) % 10;
+    tf2x64(k, ctr, w);
+    tf2x64(k, ctr + 1, w + 4);
+    int h1, h2, h3;
+    weekend_hours(w, h1, h2, h3);
     out[0] = fish_weekend_dest(c, w[3]) - lo + h1 * R;
     out[1] = fish_weekend_dest(c, w[4]) - lo + h2 * R;
     out[2] = fish_weekend_dest(c, w[5]) - lo + h3 * R;

@@ -404,7 +404,8 @@ __global__ void __launch_bounds__(THREADS, MINB) k_radix_pass(const uint32_t *__
     if (skip && *(volatile const int *)skip) return;
     __shared__ int s_tile;
     // segment, tile within it, entry base, entry count; for a dense segment of a day's
-    // first pass: 1, the instance's persons, first person and first bucket
+    // first pass: 1, the instance's persons, first person and first bucket; for another
+    // segment of that pass: 0, -, the segment's last region
     __shared__ int s_seg[8];
     __shared__ unsigned s_epoch;
     __shared__ int s_hist[WARPS][256];
@@ -450,6 +451,8 @@ __global__ void __launch_bounds__(THREADS, MINB) k_radix_pass(const uint32_t *__
                     pb = sg.ic[k].pbase;
                     bb = sg.ic[k].bbase[sg.weekend];
                     scount = (sg.weekend ? 3 : 2) * nk;   // every schedule key of the instance
+                } else if (day0) {
+                    pb = sg.ic[k].pend / sg.region_persons - 1;   // the segment's last region
                 }
             }
             s_tile = t;
@@ -493,6 +496,33 @@ __global__ void __launch_bounds__(THREADS, MINB) k_radix_pass(const uint32_t *__
                 key[j] = (uint32_t)(kg - bb);
                 const bool marked = in && ((sg.mark[kg >> 5] >> (kg & 31)) & 1u);
                 val[j] = marked ? (uint32_t)(pb + (sg.weekend ? i / 3 : (i < nk ? i : i - nk))) : kDropped;
+            }
+        } else if (day0) {
+            // the schedule's entries, region after region: entry i of the segment is entry
+            // i - region_prefix[r] of its region r, whose slots start at 3 C r
+            const int c0 = stile * kRadixTile + warp * WARP_ITEMS;
+            const int rlast = s_seg[6];   // the segment's last region
+            int r = 0, at = 0, next = 0;
+            if (c0 < scount) {
+                const int4 c = sg.chunk_region[(sbase + c0) / kRegionChunk];
+                r = c.x;
+                at = c.y;
+                next = c.z;
+            }
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++) {
+                const int i = base + 32 * j;
+                const bool in = full || i < scount;
+                if (in) {
+                    while (i >= next) {   // ends: the last region's end is scount
+                        r++;
+                        at = next;
+                        next = r < rlast ? sg.region_prefix[r + 1] : scount;
+                    }
+                }
+                const size_t src = 3 * (size_t)r * sg.region_persons + (i - at);
+                key[j] = in ? keys_in[src] : 0u;
+                val[j] = in ? vals_in[src] : 0u;
             }
         } else {
 #pragma unroll
@@ -866,46 +896,6 @@ __device__ __forceinline__ uint32_t recover_word(uint32_t st, int d2r, bool &cha
     return out;
 }
 
-// A day kernel's person tile: its look-back ticket and the instance it belongs to.
-// Thread 0 takes the ticket; with a single instance the instance record is read in
-// parallel with the ticket's round trip instead of after it.
-struct TileInfo {
-    int tile;
-    unsigned epoch;
-    int inst, pbase, pend, first_person_after;  // first_person_after: pbase + N, or the tile start if not running
-};
-
-__device__ __forceinline__ void tile_begin(const LookBack &lb, const InstConst *ic, const InstState *is,
-                                           const int32_t *tile_inst, int K, int day, TileInfo &out)
-{
-    __shared__ TileInfo s_t;
-    if (threadIdx.x == 0) {
-        TileInfo t;
-        int N = 0, running = 0;
-        if (K == 1) {
-            t.inst = 0;
-            t.pbase = ic[0].pbase;
-            t.pend = ic[0].pend;
-            N = ic[0].c.N;
-            running = instance_running(ic[0], is[0], day);
-        }
-        t.tile = atomicAdd(&lb.ctl[0], 1);
-        t.epoch = (unsigned)(*(volatile int *)&lb.ctl[2]) & 0x3FFFFFFFu;
-        if (K != 1) {
-            const int k = tile_inst[t.tile];
-            t.inst = k;
-            t.pbase = ic[k].pbase;
-            t.pend = ic[k].pend;
-            N = ic[k].c.N;
-            running = instance_running(ic[k], is[k], day);
-        }
-        t.first_person_after = running ? t.pbase + N : t.tile * kPersonTile;
-        s_t = t;
-    }
-    __syncthreads();
-    out = s_t;
-}
-
 // The sweep: kernel_countInfectedStatusAndRecover (PandemicSim.cu:2097-2192), the
 // copy_if of the infected (:2207-2224) and runToCompletion's day bookkeeping
 // (:891-937) in three launches over every instance:
@@ -1188,16 +1178,6 @@ __global__ void __launch_bounds__(kEmitWarps * 32) k_sweep_emit(const int32_t *t
     }
 }
 
-// The look-back control block sits right after the tile words.
-static LookBack make_lb(const DevArrays &d)
-{
-    LookBack lb;
-    lb.tiles = d.tiles;
-    lb.ctl = (int *)(d.tiles + d.tiles_cap);
-    lb.error = &d.sc->error;
-    return lb;
-}
-
 cudaError_t launch_sweep(const DevArrays &d, int day, cudaStream_t s)
 {
     const int tiles = d.P / kSweepTile;
@@ -1245,7 +1225,11 @@ __device__ __forceinline__ void weekday_pair_keys(const SimConst &c, const uint3
     k2 = R + d2 - lo;
 }
 
-__device__ __forceinline__ bool is_marked(const uint32_t *mark, int b) { return (mark[b >> 5] >> (b & 31)) & 1u; }
+// mark word of bucket b, its bit shifted to bit 0 (the others follow)
+__device__ __forceinline__ uint32_t mark_bit(const uint32_t *mark, uint32_t b)
+{
+    return __funnelshift_r(mark[b >> 5], 0u, b);
+}
 
 // Fire-and-forget global updates (PTX red): the thread does not wait for the result.
 __device__ __forceinline__ void red_add(int *p, int v)
@@ -1259,27 +1243,6 @@ __device__ __forceinline__ void red_or(uint32_t *p, uint32_t v)
 }
 
 __device__ __forceinline__ void mark_bucket(uint32_t *mark, int b) { red_or(&mark[b >> 5], 1u << (b & 31)); }
-
-// Adds this lane's key b (when `on`) to the block's digit histograms of the radix
-// passes.  Called by all 32 lanes.  The lower digits are spread out and each lane
-// adds its own; the top digit of a tile's keys is often the same across the warp,
-// and then one lane adds the count.
-__device__ __forceinline__ void digit_count(int (*s_dh)[256], int passes, bool on, uint32_t b)
-{
-    const unsigned act = __ballot_sync(0xffffffffu, on);
-    if (!act) return;
-    if (on)
-        for (int p = 0; p < passes - 1; p++) atomicAdd(&s_dh[p][(b >> (8 * p)) & 255u], 1);
-    const int top = passes - 1;
-    const uint32_t d = (b >> (8 * top)) & 255u;
-    const int leader = __ffs(act) - 1;
-    const uint32_t d0 = __shfl_sync(0xffffffffu, d, leader);
-    if (__all_sync(0xffffffffu, !on || d == d0)) {
-        if ((int)(threadIdx.x & 31) == leader) atomicAdd(&s_dh[top][d0], __popc(act));
-    } else if (on) {
-        atomicAdd(&s_dh[top][d], 1);
-    }
-}
 
 // Marks the errand buckets today's contact draws will read: the only buckets that
 // must be materialised.  Destinations are regenerated from the schedule counter, as
@@ -1330,214 +1293,245 @@ __global__ void k_mark_buckets(const InstConst *ic, const InstState *is, const u
     }
 }
 
-// Schedule kernel, one person tile per block.  Warps own 512 consecutive persons and
-// walk them in rounds (weekday: 64 persons a round, a pair per lane, one Threefry
-// block per pair; weekend: 32 persons a round, one per lane), so key writes are
-// coalesced.  The kernel writes every person's keys, accumulates the radix digit
-// histograms of the entries of marked buckets in shared memory, and appends those
-// entries as (instance-local key, person) in ascending person order (warp scans +
-// block scan + decoupled look-back) to the instance's segment: the order the radix
-// sort needs for stability.  Per-round
-// marked counts of a lane are packed in one register between the two phases.  The
-// instance's constants are staged in shared memory.
-constexpr int kSchedThreads = 256, kSchedTile = kPersonTile, kSchedWarpPersons = 512;
+// Schedule kernel.  The persons are cut into regions of C consecutive ones (64 to 1024,
+// launch_schedule), each inside one instance.  A persistent block owns a run of regions
+// and its warps take them one by one; a warp walks its region in rounds (weekday: 64
+// persons a round, a pair per lane, one Threefry block per pair; weekend: 32 persons a
+// round, one per lane).  The kernel writes every person's keys and keeps the entries of
+// marked buckets, compacted in ascending person order, in the warp's part of shared
+// memory; full parts are added to the block's radix digit histograms and copied, as
+// (instance-local key, person), to the region's slots of the entry arrays (3C from 3C
+// times the region's number).  The sort's first pass reads the regions of an instance
+// one after another (k_day_digit_bases scans their counts): the order its stability needs.
+//
+// No warp waits for another within an instance.  A form that placed the entries of
+// all tiles contiguously by a decoupled look-back spent two thirds of its issue slots
+// waiting: at this rate of tiles (80 per microsecond) a look-back of 32 tiles per
+// round trip cannot keep up.  What is left is the integer pipe (62-71% busy) and
+// instruction issue, so the work around the Threefry blocks is kept small: a
+// destination is one table row found on the floating-point pipe (errand_bucket), marks
+// cost a ballot per bit of a lane's count, and the per-entry work runs over compacted
+// entries with all lanes busy.  At 50M persons: 400 us a weekday and 930 us a weekend day
+// with marking, 620 and 1,250 before (look-back, selects, add / add-with-carry Threefry).
+constexpr int kSchedThreads = 256, kSchedWarps = kSchedThreads / 32;
+constexpr int kSchedPart = 256;       // persons whose entries a warp's part holds (a person's place fits a byte)
+constexpr int kSchedBlocksPerSm = 5;  // 47 registers; 6 (40) and 7 (32, spills) cost 15% and 21% more on weekends
+                                      // and 5% and 55% more on weekdays at 50M persons
 
-template <bool WEEKEND, int TF>
-__global__ void __launch_bounds__(kSchedThreads, 8) k_sched(const InstConst *ic, InstState *is,
-                                                         const int32_t *tile_inst, int K, const uint8_t *age,
-                                                         const uint32_t *mark, int32_t *keys, int *digit_hist,
-                                                         int passes, uint32_t *ckeys, uint32_t *cvals, Scalars *sc,
-                                                         LookBack lb, int day, TfMul tm)
+// Adds the block's histograms to instance k's stripe of the day's digit histograms
+// and clears them.  Block-uniform; the caller separates it from other uses of s_dh by barriers.
+__device__ __forceinline__ void sched_flush_digits(int (*s_dh)[256], int passes, int *digit_hist, int k)
 {
-    if (*(volatile int *)&sc->done) return;
-    __shared__ int s_dh[kMaxRadixPasses][256];   // digit histograms of the marked entries
-    for (int i = threadIdx.x; i < kMaxRadixPasses * 256; i += kSchedThreads) (&s_dh[0][0])[i] = 0;
-    __shared__ SimConst s_c;
-    const int csz = (int)(sizeof(SimConst) / 4);
-    if (K == 1)  // the only instance: copy its constants while thread 0 takes the ticket
-        for (int i = threadIdx.x; i < csz; i += kSchedThreads)
-            reinterpret_cast<int *>(&s_c)[i] = reinterpret_cast<const int *>(&ic[0].c)[i];
-    TileInfo ti;
-    tile_begin(lb, ic, is, tile_inst, K, day, ti);
-    const int tile = ti.tile;
-    const unsigned epoch = ti.epoch;
-    const int inst = ti.inst;
-    if (K != 1)
-        for (int i = threadIdx.x; i < csz; i += kSchedThreads)
-            reinterpret_cast<int *>(&s_c)[i] = reinterpret_cast<const int *>(&ic[inst].c)[i];
-    const int pbase = ti.pbase;
-    const int N = ti.first_person_after - pbase;   // persons to schedule (0 when not running)
-    const int tbase = tile * kSchedTile - pbase;   // the tile's first person, instance numbering
-    const int valid = N - tbase < kSchedTile ? (N - tbase > 0 ? N - tbase : 0) : kSchedTile;
-    int32_t *kk = keys + ic[inst].kbase;   // the instance's key slots
-    const int NK = ic[inst].c.N;           // their layout: weekday hour 0 at [0, N), hour 1 at [N, 2N)
-    const uint8_t *tage = age + pbase + tbase;
-    __syncthreads();
-    const SimConst &c = s_c;
-    const TfKey key = make_key(c);
-    const int bb = ic[inst].bbase[WEEKEND ? 1 : 0];
-    const unsigned long long E0 = is[inst].errand_offset;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wl = warp * kSchedWarpPersons;      // the warp's first person, tile numbering
-    constexpr int kRounds = WEEKEND ? 16 : 8;
-    // which of the lane's entries are marked: bit 3j + k (weekend) / 4j + k (weekday) of
-    // round j, kept for the append phase
-    constexpr int kPer = WEEKEND ? 3 : 4;
-    unsigned long long mbits = 0;
-    int mine = 0;
-    if (WEEKEND) {
-        // kernel_assignWeekendErrands (PandemicSim.cu:2082-2094): counters E0 + 2p, E0 + 2p + 1
-        const int lo = c.type_offset[9], R = c.L - lo;
-#pragma unroll 1
-        for (int j = 0; j < kRounds; j++) {
-            const int i = wl + 32 * j + lane;
-            uint32_t kb[3] = {0u, 0u, 0u};
-            bool mk[3] = {false, false, false};
-            if (i < valid) {
-                int d[3];
-                weekend_errands<TF>(c, key, E0 + 2ull * (unsigned long long)(tbase + i), lo, R, d, &tm);
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    kb[k] = (uint32_t)(bb + d[k]);
-                    kk[3 * (size_t)(tbase + i) + k] = (int32_t)kb[k];
-                    mk[k] = is_marked(mark, (int)kb[k]);
-                }
-            }
-            const int cnt = (int)mk[0] + (int)mk[1] + (int)mk[2];
-#pragma unroll
-            for (int k = 0; k < 3; k++) digit_count(s_dh, passes, mk[k], kb[k] - (uint32_t)bb);
-            mbits |= (unsigned long long)((uint32_t)mk[0] | ((uint32_t)mk[1] << 1) | ((uint32_t)mk[2] << 2)) << (kPer * j);
-            mine += cnt;
-        }
-    } else {
-        const int lo = c.type_offset[8], R = c.L - lo;
-#pragma unroll 1
-        for (int j = 0; j < kRounds; j++) {
-            const int i = wl + 64 * j + 2 * lane;  // even: counter E0 + p/2 covers p, p+1
-            uint32_t kb[4] = {0u, 0u, 0u, 0u};
-            bool mk[4] = {false, false, false, false};
-            if (i < valid) {
-                uint32_t w[4];
-                tf2x64m<TF>(key, E0 + (uint64_t)((tbase + i) / 2), w, tm);
-#pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    if (i + k < valid) {
-                        int k1, k2;
-                        weekday_pair_keys(c, w, k, tage[i + k] == 5, lo, R, k1, k2);
-                        kb[2 * k] = (uint32_t)(k1 + bb);
-                        kb[2 * k + 1] = (uint32_t)(k2 + bb);
-                        kk[tbase + i + k] = (int32_t)kb[2 * k];
-                        kk[(size_t)NK + tbase + i + k] = (int32_t)kb[2 * k + 1];
-                        mk[2 * k] = is_marked(mark, (int)kb[2 * k]);
-                        mk[2 * k + 1] = is_marked(mark, (int)kb[2 * k + 1]);
-                    }
-                }
-            }
-            const int cnt = (int)mk[0] + (int)mk[1] + (int)mk[2] + (int)mk[3];
-#pragma unroll
-            for (int k = 0; k < 4; k++) digit_count(s_dh, passes, mk[k], kb[k] - (uint32_t)bb);
-            mbits |= (unsigned long long)((uint32_t)mk[0] | ((uint32_t)mk[1] << 1) | ((uint32_t)mk[2] << 2) |
-                                          ((uint32_t)mk[3] << 3)) << (kPer * j);
-            mine += cnt;
-        }
+    int *h = digit_hist + ((size_t)k * kDigitStripes + blockIdx.x % kDigitStripes) * kMaxRadixPasses * 256;
+    for (int p = 0; p < passes; p++) {
+        const int v = s_dh[p][threadIdx.x];
+        if (v) red_add(&h[p * 256 + threadIdx.x], v);
+        s_dh[p][threadIdx.x] = 0;
     }
-    // tile position: warp totals, block scan over warps, look-back
-    __shared__ int s_wtot[kSchedThreads / 32];
-    __shared__ int s_wbase[kSchedThreads / 32];
-    int wt = mine;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) wt += __shfl_xor_sync(0xffffffffu, wt, o);
-    if (lane == 0) s_wtot[warp] = wt;
-    __syncthreads();
-    // A dense instance (most of today's buckets are read): the sort's first pass reads
-    // the keys written above, so only the marked count is needed, not the entries.
-    const bool dense = is[inst].dense != 0;
-    if (dense) {
-        if (threadIdx.x == 0) {
-            int tot = 0;
-            for (int w = 0; w < kSchedThreads / 32; w++) tot += s_wtot[w];
-            if (tot) red_add(&is[inst].marked, tot);
-        }
-    } else if (warp == 0) {
-        // the instance's entries form their own segment: its first tile starts the scan
-        int tot = 0;
-        for (int w = 0; w < kSchedThreads / 32; w++) tot += s_wtot[w];
-        const unsigned prefix = lookback_publish_warp(lb, epoch, tile, (unsigned)tot, tbase == 0);
-        if (lane == 0) {
-            int run = (int)prefix;
-            for (int w = 0; w < kSchedThreads / 32; w++) {
-                s_wbase[w] = run;
-                run += s_wtot[w];
-            }
-            if (pbase + tbase + kSchedTile == ti.pend) is[inst].marked = run;
-        }
-    }
-    __syncthreads();
-    {
-        int *h = digit_hist + ((size_t)inst * kDigitStripes + blockIdx.x % kDigitStripes) * kMaxRadixPasses * 256;
-        for (int p = 0; p < passes; p++) {
-            const int v = s_dh[p][threadIdx.x];
-            if (v) red_add(&h[p * 256 + threadIdx.x], v);
-        }
-    }
-    if (dense) {
-        lookback_end(lb);
-        return;
-    }
-    ckeys += ic[inst].kbase;   // the instance's segment of the entry arrays
-    cvals += ic[inst].kbase;
-    // append the marked entries, rounds in order, lanes in order within a round
-    int run = s_wbase[warp];
-    const int gbase = pbase + tbase;   // global id of the tile's first person
-#pragma unroll 1
-    for (int j = 0; j < kRounds; j++) {
-        const uint32_t bits = (uint32_t)(mbits >> (kPer * j)) & ((1u << kPer) - 1u);
-        const int cnt = __popc(bits);
-        if (__ballot_sync(0xffffffffu, cnt > 0) == 0) continue;
-        const int incl = warp_inclusive_scan(cnt);
-        int pos = run + incl - cnt;
-        if (cnt > 0) {
-            if (WEEKEND) {
-                const int i = wl + 32 * j + lane;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    if ((bits >> k) & 1u) {
-                        ckeys[pos] = (uint32_t)kk[3 * (size_t)(tbase + i) + k] - (uint32_t)bb;
-                        cvals[pos] = (uint32_t)(gbase + i);
-                        pos++;
-                    }
-                }
-            } else {
-                // entry k of the round: person i + k / 2, hour k % 2
-                const int i = wl + 64 * j + 2 * lane;
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if ((bits >> k) & 1u) {
-                        ckeys[pos] = (uint32_t)kk[(size_t)(k & 1) * NK + tbase + i + (k >> 1)] - (uint32_t)bb;
-                        cvals[pos] = (uint32_t)(gbase + i + (k >> 1));
-                        pos++;
-                    }
-                }
-            }
-        }
-        run += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    lookback_end(lb);
 }
 
-// The run-time constants of tf2x64m: 1 and the powers of two of the rotations.
-static TfMul tf_multipliers()
+// The warp's part of `n` entries: into the digit histograms, and (unless the instance is
+// dense) to the entry arrays at ck / cv.
+__device__ __forceinline__ void sched_flush_entries(const uint32_t *my_key, const uint8_t *my_who, int n, int lane,
+                                                    uint32_t bb, uint32_t first, int (*s_dh)[256], int passes,
+                                                    bool dense, uint32_t *ck, uint32_t *cv)
 {
-    TfMul m;
-    m.one = 1u;
-    const int r[6] = {16, 10, 12, 31, 24, 21};
-    for (int i = 0; i < 6; i++) m.pow[i] = 1u << r[i];
-    return m;
+    __syncwarp();
+    for (int e = lane; e < n; e += 32) {
+        const uint32_t b = my_key[e] - bb;
+#pragma unroll
+        for (int p = 0; p < kMaxRadixPasses; p++)
+            if (p < passes) atomicAdd(&s_dh[p][(b >> (8 * p)) & 255u], 1);
+        if (!dense) {
+            ck[e] = b;
+            cv[e] = first + my_who[e];
+        }
+    }
+    __syncwarp();
+}
+
+template <bool WEEKEND>
+__global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
+    k_sched(const InstConst *ic, InstState *is, const int32_t *tile_inst, int regions, int C, const uint8_t *age,
+            const uint32_t *mark, int32_t *keys, int *digit_hist, int passes, uint32_t *ckeys, uint32_t *cvals,
+            int32_t *region_count, const Scalars *sc, int day)
+{
+    if (*(volatile const int *)&sc->done) return;
+    static_assert(kSchedThreads == 256, "one thread per digit in sched_flush_digits");
+    constexpr int kPer = WEEKEND ? 3 : 2;                       // keys per person
+    constexpr int kCap = kPer * kSchedPart;                     // entries of a warp's part at most
+    constexpr int kRound = WEEKEND ? 32 : 64;                   // persons per round
+    __shared__ __align__(16) uint32_t s_key[kSchedWarps][kCap]; // marked keys of the warp's persons (global buckets)
+    __shared__ uint8_t s_who[kSchedWarps][kCap];                // their persons, numbered within the part
+    __shared__ int s_dh[kMaxRadixPasses][256];                  // digit histograms of the current instance's entries
+    __shared__ ErrandRow s_row[2 * kErrandRows];                // errand tables (weekday: hour 0, hour 1)
+    __shared__ int s_next;                                      // next region of the block's run
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    uint32_t *const my_key = s_key[warp];
+    uint8_t *const my_who = s_who[warp];
+    for (int i = threadIdx.x; i < kMaxRadixPasses * 256; i += kSchedThreads) (&s_dh[0][0])[i] = 0;
+    const int r1 = (int)((long long)regions * (blockIdx.x + 1) / gridDim.x);
+    for (int r = (int)((long long)regions * blockIdx.x / gridDim.x); r < r1;) {
+        // the block's regions of one instance: [r, end)
+        const int inst = tile_inst[(long long)r * C / kPersonTile];
+        const InstConst &ik = ic[inst];
+        const int end = min(r1, ik.pend / C);
+        if (!instance_running(ik, is[inst], day)) {
+            r = end;
+            continue;
+        }
+        const TfKey key = make_key(ik.c);
+        const int pbase = ik.pbase, N = ik.c.N;
+        const int bb = ik.bbase[WEEKEND ? 1 : 0];
+        const int lo = ik.c.type_offset[WEEKEND ? 9 : 8], R = ik.c.L - lo;
+        int32_t *const kk = keys + ik.kbase;   // the instance's key slots: weekday hour 0 at [0, N), hour 1 at [N, 2N)
+        const bool dense = is[inst].dense != 0;
+        const unsigned long long E0 = is[inst].errand_offset;
+        if (threadIdx.x < 2 * kErrandRows) {
+            const int hour = threadIdx.x / kErrandRows;
+            s_row[threadIdx.x] = errand_table_row<WEEKEND>(ik.c, threadIdx.x % kErrandRows, bb + hour * R, lo);
+        }
+        if (threadIdx.x == 0) s_next = r;
+        __syncthreads();
+        for (;;) {
+            int q = 0;
+            if (lane == 0) q = atomicAdd(&s_next, 1);
+            q = __shfl_sync(0xffffffffu, q, 0);
+            if (q >= end) break;
+            const int rp = q * C - pbase;                       // the region's first person, instance numbering
+            const int rend = min(rp + C, N);                    // (below rp when the region is all padding)
+            uint32_t *const ck = ckeys + 3 * (size_t)q * C, *const cv = cvals + 3 * (size_t)q * C;
+            int run = 0, part = rp, written = 0;                // entries in the part, its first person, entries flushed
+#pragma unroll 1
+            for (int p0 = rp; p0 < rend; p0 += kRound) {
+                if (p0 - part >= kSchedPart) {
+                    sched_flush_entries(my_key, my_who, run, lane, (uint32_t)bb, (uint32_t)(pbase + part), s_dh, passes,
+                                        dense, ck + written, cv + written);
+                    written += run;
+                    run = 0;
+                    part = p0;
+                }
+                if (WEEKEND) {
+                    // kernel_assignWeekendErrands (PandemicSim.cu:2082-2094): counters E0 + 2p, E0 + 2p + 1
+                    const int p = p0 + lane;
+                    uint32_t w[8];
+                    tf2x64(key, E0 + 2ull * (unsigned long long)p, w);
+                    tf2x64(key, E0 + 2ull * (unsigned long long)p + 1ull, w + 4);
+                    int h[3];
+                    weekend_hours(w, h[0], h[1], h[2]);
+                    uint32_t kb[3];
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                        kb[k] = (uint32_t)(errand_bucket<true>(s_row, w[3 + k], errand_p9<true>(true), 0) + h[k] * R);
+                    // the round's 96 key slots, written in whole 16-byte pieces through the
+                    // unused end of the warp's part (run <= 3 (p0 - part))
+                    uint32_t *const stage = my_key + 3 * (p0 - part);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) stage[3 * lane + k] = kb[k];
+                    __syncwarp();
+                    if (p0 + 32 <= N) {
+                        if (lane < 24)
+                            *reinterpret_cast<uint4 *>(kk + 3 * (size_t)p0 + 4 * lane) =
+                                *reinterpret_cast<const uint4 *>(stage + 4 * lane);
+                    } else {
+                        for (int i = lane; i < 3 * (N - p0); i += 32) kk[3 * (size_t)p0 + i] = (int32_t)stage[i];
+                    }
+                    const uint32_t in = p < N ? 1u : 0u;
+                    uint32_t mk[3];
+#pragma unroll
+                    for (int k = 0; k < 3; k++) mk[k] = mark_bit(mark, kb[k]) & in;
+                    const uint32_t cnt = mk[0] + mk[1] + mk[2];
+                    const unsigned b0 = __ballot_sync(0xffffffffu, cnt & 1u), b1 = __ballot_sync(0xffffffffu, cnt & 2u);
+                    __syncwarp();   // the stage is read before the entries below reach it
+                    if ((b0 | b1) == 0) continue;
+                    int pos = run + __popc(b0 & lt) + 2 * __popc(b1 & lt);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        if (mk[k]) {
+                            my_key[pos] = kb[k];
+                            my_who[pos] = (uint8_t)(p - part);
+                        }
+                        pos += (int)mk[k];
+                    }
+                    run += __popc(b0) + 2 * __popc(b1);
+                } else {
+                    // kernel_assignWeekdayAfterschoolAndErrands (PandemicSim.cu:2972-3022): counter E0 + p / 2
+                    const int p = p0 + 2 * lane;
+                    uint32_t w[4];
+                    const uchar2 ag = *reinterpret_cast<const uchar2 *>(age + pbase + p);
+                    tf2x64(key, E0 + (uint64_t)(p / 2), w);
+                    const bool ad[2] = {ag.x == 5, ag.y == 5};
+                    // a child's second draw is its first (one afterschool place)
+                    w[1] = ad[0] ? w[1] : w[0];
+                    w[3] = ad[1] ? w[3] : w[2];
+                    constexpr int kChild = (kErrandRows - 1) * (int)sizeof(ErrandRow);
+                    const float p9[2] = {errand_p9<false>(ad[0]), errand_p9<false>(ad[1])};
+                    const int base[2] = {ad[0] ? 0 : kChild, ad[1] ? 0 : kChild};
+                    uint32_t kb[4];   // [person][hour]
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        kb[k] = (uint32_t)errand_bucket<false>(s_row + (k & 1) * kErrandRows, w[k], p9[k >> 1], base[k >> 1]);
+                    const uint32_t in[2] = {p < N ? 1u : 0u, p + 1 < N ? 1u : 0u};
+                    uint32_t mk[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) mk[k] = mark_bit(mark, kb[k]) & in[k >> 1];
+                    if (p + 1 < N) {
+                        *reinterpret_cast<int2 *>(kk + p) = make_int2((int)kb[0], (int)kb[2]);
+                        if ((N & 1) == 0) {   // hour 1's slots start 8-byte aligned
+                            *reinterpret_cast<int2 *>(kk + (size_t)N + p) = make_int2((int)kb[1], (int)kb[3]);
+                        } else {
+                            kk[(size_t)N + p] = (int)kb[1];
+                            kk[(size_t)N + p + 1] = (int)kb[3];
+                        }
+                    } else if (p < N) {
+                        kk[p] = (int)kb[0];
+                        kk[(size_t)N + p] = (int)kb[1];
+                    }
+                    const uint32_t cnt = mk[0] + mk[1] + mk[2] + mk[3];
+                    const unsigned b0 = __ballot_sync(0xffffffffu, cnt & 1u), b1 = __ballot_sync(0xffffffffu, cnt & 2u),
+                                   b2 = __ballot_sync(0xffffffffu, cnt & 4u);
+                    if ((b0 | b1 | b2) == 0) continue;
+                    int pos = run + __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (mk[k]) {
+                            my_key[pos] = kb[k];
+                            my_who[pos] = (uint8_t)(p + (k >> 1) - part);
+                        }
+                        pos += (int)mk[k];
+                    }
+                    run += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+                }
+            }
+            sched_flush_entries(my_key, my_who, run, lane, (uint32_t)bb, (uint32_t)(pbase + part), s_dh, passes, dense,
+                                ck + written, cv + written);
+            written += run;
+            if (lane == 0) {
+                region_count[q] = written;
+                if (written) red_add(&is[inst].marked, written);
+            }
+        }
+        __syncthreads();
+        sched_flush_digits(s_dh, passes, digit_hist, inst);
+        __syncthreads();
+        r = end;
+    }
 }
 
 int day_buckets(const SimConst &c, bool weekend)
 {
     return weekend ? 10 * (c.L - c.type_offset[9]) : 2 * (c.L - c.type_offset[8]);
+}
+
+// Persons per region of the schedule kernel: the largest power of two that still
+// leaves four regions for every resident warp (small simulations spread over the SMs,
+// large ones have fewer counts to scan and longer runs of entries per region).
+static int sched_region_persons(long long P)
+{
+    int C = kSchedMaxRegion;
+    while (C > kSchedMinRegion && P / C < 4ll * kSchedWarps * kSchedBlocksPerSm * sm_count()) C /= 2;
+    return C;
 }
 
 // mark (or mark everything for complete tables), then the schedule kernel
@@ -1553,23 +1547,14 @@ cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, bool full
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    const int blocks = d.P / kSchedTile;
-    const LookBack lb = make_lb(d);
+    const int C = sched_region_persons(d.P), regions = d.P / C;
+    const int blocks = std::min(div_up(regions, kSchedWarps), kSchedBlocksPerSm * sm_count());
     const int passes = radix_passes(d.bucket_max[weekend ? 1 : 0]);
-    const TfMul tm = tf_multipliers();
-#define PT_SCHED(W, T)                                                                                              \
-    k_sched<W, T><<<blocks, kSchedThreads, 0, s>>>(d.ic, d.is, d.tile_inst, d.K, d.age, d.mark, d.keys, d.digit_hist, \
-                                                    passes, d.rk1, d.rv1, d.sc, lb, day, tm)
-    const int tf = d.tune.sched_tf;
-    if (weekend) {
-        if (tf == 2) PT_SCHED(true, 2);
-        else if (tf == 1) PT_SCHED(true, 1);
-        else PT_SCHED(true, 0);
-    } else {
-        if (tf == 2) PT_SCHED(false, 2);
-        else if (tf == 1) PT_SCHED(false, 1);
-        else PT_SCHED(false, 0);
-    }
+#define PT_SCHED(W)                                                                                              \
+    k_sched<W><<<blocks, kSchedThreads, 0, s>>>(d.ic, d.is, d.tile_inst, regions, C, d.age, d.mark, d.keys,       \
+                                                d.digit_hist, passes, d.rk1, d.rv1, d.region_count, d.sc, day)
+    if (weekend) PT_SCHED(true);
+    else PT_SCHED(false);
 #undef PT_SCHED
     count_launch();
     return cudaGetLastError();
@@ -1597,6 +1582,9 @@ static RadixArgs day_radix_args(const DevArrays &d, bool weekend)
     r.seg.ic = d.ic;
     r.seg.is = d.is;
     r.seg.segments = d.K;
+    r.seg.region_prefix = d.region_prefix;
+    r.seg.chunk_region = d.chunk_region;
+    r.seg.region_persons = sched_region_persons(d.P);
     r.seg.day_keys = d.keys;
     r.seg.tile_prefix0 = d.tile_prefix0;
     r.seg.mark = d.mark;
@@ -1611,48 +1599,89 @@ static RadixArgs day_radix_args(const DevArrays &d, bool weekend)
     return r;
 }
 
-// One block per instance: the digit bases of its segment from the digit histograms
-// the schedule kernel accumulated (summing the stripes, clearing them).  Block 0
-// also numbers the segments' radix tiles (tile_prefix) and adds the day's
-// materialised entries to the running total.
-__global__ void k_day_digit_bases(int *digit_hist, int *digit_base, int passes, const InstConst *ic,
-                                  const InstState *is, int K, int weekend, int32_t *tile_prefix,
-                                  int32_t *tile_prefix0, Scalars *sc)
+// The day's sort tables, a row of blocks per instance (blockIdx.y).
+//  * Block 0 of the row: the digit bases of the instance's segment from the digit
+//    histograms the schedule kernel accumulated (summing the stripes, clearing them).
+//  * Every block: its 4096 regions of the instance.  Their place in the segment is an
+//    exclusive scan of the regions' entry counts; a block sums the counts before its
+//    own itself (at most a few hundred KB from L2) rather than wait for the others.
+//    Output: region_prefix, and for every kRegionChunk entries of the segment the region
+//    the first of them lies in, with its prefix and its end (chunk_region).
+//  * The first block also numbers the segments' radix tiles (tile_prefix) and adds the
+//    day's materialised entries to the running total.
+constexpr int kBasesThreads = 1024, kBasesRegions = 4 * kBasesThreads;
+
+__global__ void __launch_bounds__(kBasesThreads) k_day_digit_bases(int *digit_hist, int *digit_base, int passes,
+                                                                   const InstConst *ic, const InstState *is, int K,
+                                                                   int weekend, int C, const int32_t *region_count,
+                                                                   int32_t *region_prefix, int4 *chunk_region,
+                                                                   int32_t *tile_prefix, int32_t *tile_prefix0,
+                                                                   Scalars *sc)
 {
     if (*(volatile const int *)&sc->done) return;
-    const int k = blockIdx.x;
+    const int k = blockIdx.y, t = threadIdx.x;
+    // regions of the block (an instance starts on a person tile, and 4 C persons divide one)
+    const int r0 = ic[k].pbase / C, r1 = ic[k].pend / C, rb = r0 + (int)blockIdx.x * kBasesRegions;
+    if (rb < r1 && is[k].marked > 0 && !is[k].dense) {
+        int before = 0;
+        for (int r = r0 + 4 * t; r < rb; r += kBasesRegions) {
+            const int4 c = *reinterpret_cast<const int4 *>(region_count + r);
+            before += c.x + c.y + c.z + c.w;
+        }
+        int4 c = make_int4(0, 0, 0, 0);
+        const int r = rb + 4 * t;
+        if (r < r1) c = *reinterpret_cast<const int4 *>(region_count + r);
+        int carry, total;
+        block_exclusive_scan<kBasesThreads, int>(before, carry);
+        int at = carry + block_exclusive_scan<kBasesThreads, int>(c.x + c.y + c.z + c.w, total);
+        if (r < r1) {
+            int4 *const chunks = chunk_region + ic[k].kbase / kRegionChunk;
+            const int n[4] = {c.x, c.y, c.z, c.w};
+            int pre[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                pre[j] = at;
+                at += n[j];
+                for (int m = (pre[j] + kRegionChunk - 1) / kRegionChunk; m * kRegionChunk < at; m++)
+                    chunks[m] = make_int4(r + j, pre[j], at, 0);
+            }
+            *reinterpret_cast<int4 *>(region_prefix + r) = make_int4(pre[0], pre[1], pre[2], pre[3]);
+        }
+    }
+    if (blockIdx.x != 0) return;
     for (int p = 0; p < passes; p++) {
         int v = 0;
-        for (int st = 0; st < kDigitStripes; st++) {
-            int *h = &digit_hist[(((size_t)k * kDigitStripes + st) * kMaxRadixPasses + p) * 256 + threadIdx.x];
-            v += *h;
-            *h = 0;
-        }
+        if (t < 256)
+            for (int st = 0; st < kDigitStripes; st++) {
+                int *h = &digit_hist[(((size_t)k * kDigitStripes + st) * kMaxRadixPasses + p) * 256 + t];
+                v += *h;
+                *h = 0;
+            }
         int total;
-        const int excl = block_exclusive_scan<256, int>(v, total);
-        digit_base[((size_t)k * passes + p) * 256 + threadIdx.x] = excl;
+        const int excl = block_exclusive_scan<kBasesThreads, int>(v, total);
+        if (t < 256) digit_base[((size_t)k * passes + p) * 256 + t] = excl;
     }
     if (k != 0) return;
     int carry = 0, carry0 = 0;
     unsigned long long entries = 0;
-    for (int b = 0; b < K; b += 256) {
-        const int i = b + (int)threadIdx.x;
+    for (int b = 0; b < K; b += kBasesThreads) {
+        const int i = b + t;
         const int m = i < K ? is[i].marked : 0;
         // the first pass reads every key of a dense instance, the appended entries otherwise
         const int m0 = (i < K && is[i].dense) ? (weekend ? 3 : 2) * ic[i].c.N : m;
         int total;
-        const int excl = block_exclusive_scan<256, int>((m + kRadixTile - 1) / kRadixTile, total);
+        const int excl = block_exclusive_scan<kBasesThreads, int>((m + kRadixTile - 1) / kRadixTile, total);
         if (i < K) tile_prefix[i] = carry + excl;
         carry += total;
         int total0;
-        const int excl0 = block_exclusive_scan<256, int>((m0 + kRadixTile - 1) / kRadixTile, total0);
+        const int excl0 = block_exclusive_scan<kBasesThreads, int>((m0 + kRadixTile - 1) / kRadixTile, total0);
         if (i < K) tile_prefix0[i] = carry0 + excl0;
         carry0 += total0;
         int msum;
-        block_exclusive_scan<256, int>(m, msum);
+        block_exclusive_scan<kBasesThreads, int>(m, msum);
         entries += (unsigned long long)msum;
     }
-    if (threadIdx.x == 0) {
+    if (t == 0) {
         tile_prefix[K] = carry;
         tile_prefix0[K] = carry0;
         sc->materialised_sum += entries;
@@ -1662,8 +1691,11 @@ __global__ void k_day_digit_bases(int *digit_hist, int *digit_base, int passes, 
 cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s)
 {
     const int P = radix_passes(d.bucket_max[weekend ? 1 : 0]);
-    k_day_digit_bases<<<d.K, 256, 0, s>>>(d.digit_hist, d.digit_base, P, d.ic, d.is, d.K, weekend ? 1 : 0,
-                                          d.tile_prefix, d.tile_prefix0, d.sc);
+    const int C = sched_region_persons(d.P);
+    const dim3 grid(std::max(1, div_up(d.persons_max / C, kBasesRegions)), d.K);
+    k_day_digit_bases<<<grid, kBasesThreads, 0, s>>>(d.digit_hist, d.digit_base, P, d.ic, d.is, d.K, weekend ? 1 : 0,
+                                                    C, d.region_count, d.region_prefix,
+                                                    d.chunk_region, d.tile_prefix, d.tile_prefix0, d.sc);
     count_launch();
     return cudaGetLastError();
 }
@@ -2238,8 +2270,37 @@ long long max_spin_limit() { return kSpinLimit; }
 // differs from __fdiv_rn(x, pdf[r]).  (Below about 2^-100 the correction step's
 // remainder underflows and the two can differ; no draw gets there.)  counts[3]:
 // reciprocal table entries that differ from __frcp_rn of their probability.
+// The schedule kernel's table form (errand_step and the scaled quotient) against the
+// same loop; `rows` holds the errand table of the day type.
+template <bool WEEKEND>
+__device__ bool errand_table_differs(uint32_t r, const ErrandRow *rows)
+{
+    constexpr int kRow = (int)sizeof(ErrandRow);
+    float x, want;
+    const int at = errand_step<WEEKEND>(__uint2float_rn(r), errand_p9<WEEKEND>(true), 0, x);
+    const int row = errand_row_loop<WEEKEND>(to_unit(r), want);
+    bool bad = at % kRow != 0 || at < 0 || at > 3 * kRow;
+    if (bad) return true;
+    const ErrandRow &e = rows[at / kRow];
+    bad = (at == 0 ? 9 : 10 + at / kRow) != row || __float_as_uint(div_rn_recip(x, e.d, e.r)) != __float_as_uint(want);
+    if (!WEEKEND) {
+        // a child's row: the quotient is the draw
+        const int c = errand_step<false>(__uint2float_rn(r), errand_p9<false>(false), 4 * kRow, x);
+        bad |= c != 4 * kRow || __float_as_uint(div_rn_recip(x, rows[4].d, rows[4].r)) != __float_as_uint(to_unit(r));
+    }
+    return bad;
+}
+
 __global__ void k_errand_selftest(unsigned long long *counts)
 {
+    __shared__ SimConst s_none;   // the tables' locations do not matter here
+    __shared__ ErrandRow rows[2 * kErrandRows];
+    for (int i = threadIdx.x; i < (int)(sizeof(SimConst) / 4); i += blockDim.x) reinterpret_cast<int *>(&s_none)[i] = 0;
+    __syncthreads();
+    if (threadIdx.x < 2 * kErrandRows)
+        rows[threadIdx.x] = threadIdx.x < kErrandRows ? errand_table_row<false>(s_none, threadIdx.x, 0, 0)
+                                                      : errand_table_row<true>(s_none, threadIdx.x - kErrandRows, 0, 0);
+    __syncthreads();
     unsigned long long bad_wd = 0, bad_we = 0, bad_div = 0;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < (1ull << 32);
@@ -2251,6 +2312,8 @@ __global__ void k_errand_selftest(unsigned long long *counts)
         ra = errand_row<true>(y, a);
         rb = errand_row_loop<true>(y, b);
         bad_we += (ra != rb || __float_as_uint(a) != __float_as_uint(b)) ? 1 : 0;
+        bad_wd += errand_table_differs<false>((uint32_t)i, rows) ? 1 : 0;
+        bad_we += errand_table_differs<true>((uint32_t)i, rows + kErrandRows) ? 1 : 0;
         if (i == 0 || (i >= 0x2F800000ull && i <= 0x3F800000ull)) {   // 0 and [2^-32, 1]
             const float x = __uint_as_float((uint32_t)i);
             const int rows[4] = {9, 11, 12, 13};

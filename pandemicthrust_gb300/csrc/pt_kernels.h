@@ -13,6 +13,8 @@ constexpr int kMaxDays = 256;
 constexpr int kPersonTile = 4096;  // persons per sweep / schedule tile
 constexpr int kRadixTileEntries = 4096;  // entries per radix-pass tile (256 look-back words each)
 constexpr int kScanTileEntries = 4096;   // values per scan tile (one look-back word each)
+constexpr int kSchedMinRegion = 64, kSchedMaxRegion = 1024;   // persons per region of the schedule kernel
+constexpr int kRegionChunk = 256;  // entries per chunk_region word (a radix warp's entries are whole chunks)
 constexpr int kDigitStripes = 16;  // copies of the day's radix digit histograms (spreads the updates)
 
 // Constants of one simulation (setup kernels take them by value; the day kernels
@@ -90,8 +92,8 @@ struct Tuning {
     int infect_blocks_per_sm = 8;   // infection grid: 256-thread blocks per SM (twice as
                                     // many 128-thread blocks for the thread-per-infector kernels)
     int radix_blocks_per_sm = 4;    // persistent blocks of a day's radix pass per SM (1..4)
-    int sched_tf = 0;               // schedule kernel's Threefry arithmetic: 0 ALU adds and
-                                    // shifts, 1 multiply-add adds, 2 also multiply rotations
+    int sched_tf = 0;               // accepted (0..2) and kept, without effect: one form of the
+                                    // Threefry arithmetic is the fastest everywhere (tf2x64)
     int dense_level = 0;            // when a day's sort reads the schedule keys directly:
                                     // 0 never; 1, 2, 3: infected >= buckets / 4, x 1, x 2
     int radix_threads = 256;        // threads per block of a day's radix passes: 256 or 512
@@ -121,6 +123,9 @@ struct DevArrays {
     int *digit_base;          // K x 4 x 256
     int32_t *tile_prefix;     // K + 1: radix tiles of the instances' segments
     int32_t *tile_prefix0;    // K + 1: the same for the first pass (a dense segment's input is all its keys)
+    int32_t *region_count;    // P / kSchedMinRegion: entries the schedule kernel wrote in each region
+    int32_t *region_prefix;   // P / kSchedMinRegion: their exclusive prefix within the instance
+    int4 *chunk_region;       // 3P / kRegionChunk: region of every kRegionChunk-th entry of a segment, its prefix and end
     uint32_t *mark;           // bitmap over today's buckets: 1 = materialise
     int32_t *infected;        // P ascending infected ids
     int32_t *infected_inst;   // P: instance of each infected list position
@@ -135,6 +140,7 @@ struct DevArrays {
     const int32_t *tile_inst; // P / kPersonTile: instance of each person tile
     int K;
     int P;                    // persons including padding, a multiple of kPersonTile
+    int persons_max;          // of the largest instance, including padding
     int buckets[2];           // weekday / weekend bucket slots over all instances
     int bucket_max[2];        // largest weekday / weekend bucket count of one instance
     int locations;            // locations over all instances
@@ -185,6 +191,14 @@ struct RadixSegments {
     const InstConst *ic = nullptr;
     const InstState *is = nullptr;
     int segments = 0;
+    // The first pass of a day's sort reads the entries the schedule kernel wrote region by
+    // region (see k_sched): region r's at 3 region_persons r, its first one entry
+    // region_prefix[r] of the segment; chunk_region[(kbase + i) / kRegionChunk] is the
+    // region of entry i (a multiple of kRegionChunk) of the segment at kbase, with that
+    // region's prefix and its end.
+    const int32_t *region_prefix = nullptr;
+    const int4 *chunk_region = nullptr;
+    int region_persons = 0;
     // The day's sort: in its first pass a segment whose instance is dense today reads
     // its entries straight from the schedule keys (global bucket ids at
     // day_keys[kbase ...], 2N weekday hour-major / 3N weekend person-major, persons

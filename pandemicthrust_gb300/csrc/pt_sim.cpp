@@ -320,7 +320,7 @@ static pt_status engine_setup(Engine *s)
             return fail(s, PT_ERR_ARG, "batch too large for 32-bit ids");
     }
     const long long Bday = std::max(B0, B1), Bmax = std::max(Bday, LT + 1);
-    const long long tiles_cap = std::max({maxP, Bmax + 1, HS + 1}) / ptk::kScanTileEntries + 4;
+    const long long tiles_cap = std::max(Bmax + 1, HS + 1) / ptk::kScanTileEntries + 4;
 
     // small block: scalars, look-back tiles and control words, instance records and
     // state, generation histograms, household offsets, setup counters
@@ -401,6 +401,8 @@ static pt_status engine_setup(Engine *s)
        "instance records");
     d.K = K;
     d.P = (int)P;
+    d.persons_max = 0;
+    for (int k = 0; k < K; k++) d.persons_max = std::max(d.persons_max, s->ic[k].pend - s->ic[k].pbase);
     d.buckets[0] = (int)B0;
     d.buckets[1] = (int)B1;
     d.locations = (int)LT;
@@ -428,6 +430,8 @@ static pt_status engine_setup(Engine *s)
     bytes += round256(8 * 4);                                                      // radix ctl
     bytes += round256((size_t)K * ptk::kDigitStripes * 4 * 256 * 4);               // digit histograms
     bytes += round256((size_t)K * 4 * 256 * 4) + 2 * round256(((size_t)K + 1) * 4);  // digit bases, tile prefixes
+    const size_t nregions = n / ptk::kSchedMinRegion, nchunks = 3 * n / ptk::kRegionChunk + 1;
+    bytes += 2 * round256(nregions * 4) + round256(nchunks * sizeof(int4));   // schedule regions
     bytes += round256(((size_t)Bday / 32 + 1) * 4);        // bucket mark bitmap
     bytes += round256(n * 4) * 2;               // infected, infected_inst
     bytes += round256(n / 16 * 2) + round256((ntiles + 1) * 4);  // sweep masks, sweep tile counts
@@ -461,6 +465,9 @@ static pt_status engine_setup(Engine *s)
     d.digit_base = a.take<int>((size_t)K * 4 * 256);
     d.tile_prefix = a.take<int32_t>((size_t)K + 1);
     d.tile_prefix0 = a.take<int32_t>((size_t)K + 1);
+    d.region_count = a.take<int32_t>(nregions);
+    d.region_prefix = a.take<int32_t>(nregions);
+    d.chunk_region = a.take<int4>(nchunks);
     d.mark = a.take<uint32_t>((size_t)Bday / 32 + 1);
     d.infected = a.take<int32_t>(n);
     d.infected_inst = a.take<int32_t>(n);
@@ -933,7 +940,7 @@ static std::vector<long long> tune_key(const Engine *s)
 
 // The tuner.  The infection, radix and schedule stages are timed separately (per-stage
 // CUDA events around every day), so one run measures one candidate of each: run i
-// uses infection candidate i, radix candidate i % 3 and Threefry form (i + 1) % 3.
+// uses infection candidate i and radix candidate i % 3.
 // Two more runs then try the dense-day sort levels 2 and 3 with the shapes chosen.
 static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
 {
@@ -956,9 +963,8 @@ static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
     // radix passes: (blocks per SM, threads per block)
     const int radix[] = {3, 4, 2};
     const int radix_threads[] = {256, 256, 512};
-    const int tfs[] = {0, 1, 2};
     const int runs = (int)(sizeof(infect) / sizeof(infect[0]));
-    float best_inf = 1e30f, best_rad[3] = {1e30f, 1e30f, 1e30f}, best_tf[3] = {1e30f, 1e30f, 1e30f};
+    float best_inf = 1e30f, best_rad[3] = {1e30f, 1e30f, 1e30f}, best_sched = 1e30f;
     int best_i = 0;
     const int saved_max = s->max_days;
     const int trial = days > 0 ? std::min(days, saved_max) : saved_max;
@@ -968,7 +974,7 @@ static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
         t.infect_blocks_per_sm = infect[i].bps;
         t.radix_blocks_per_sm = radix[i % 3];
         t.radix_threads = radix_threads[i % 3];
-        t.sched_tf = tfs[(i + 1) % 3];
+        t.sched_tf = 0;
         t.dense_level = 0;
         pt_status st = engine_set_tuning(s, &t);
         if (st == PT_OK) st = engine_reset(s);
@@ -983,28 +989,26 @@ static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
         const float inf = ms[kStInfect] + ms[8 + kStInfect];
         const float rad = ms[kStRadix] + ms[8 + kStRadix];
         const float sch = ms[kStSchedule] + ms[8 + kStSchedule];
-        best_tf[(i + 1) % 3] = std::min(best_tf[(i + 1) % 3], sch);
+        best_sched = std::min(best_sched, sch);
         if (inf < best_inf) {
             best_inf = inf;
             best_i = i;
         }
         best_rad[i % 3] = std::min(best_rad[i % 3], rad);
     }
-    int rbest = 0, tbest = 0;
-    for (int r = 1; r < 3; r++) {
+    int rbest = 0;
+    for (int r = 1; r < 3; r++)
         if (best_rad[r] < best_rad[rbest]) rbest = r;
-        if (best_tf[r] < best_tf[tbest]) tbest = r;
-    }
     pt_tuning t;
     t.infect_coop = infect[best_i].coop;
     t.infect_blocks_per_sm = infect[best_i].bps;
     t.radix_blocks_per_sm = radix[rbest];
     t.radix_threads = radix_threads[rbest];
-    t.sched_tf = tfs[tbest];
+    t.sched_tf = 0;
     t.dense_level = 0;
     // the dense-day sort changes both the schedule and the sort stage: its levels are
     // timed after the others are chosen, against their schedule + sort time
-    float best_dense = best_rad[rbest] + best_tf[tbest];
+    float best_dense = best_rad[rbest] + best_sched;
     for (int lv = 2; lv <= 3; lv++) {
         pt_tuning c = t;
         c.dense_level = lv;
