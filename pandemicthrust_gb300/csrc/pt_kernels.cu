@@ -1242,7 +1242,15 @@ __device__ __forceinline__ void red_or(uint32_t *p, uint32_t v)
     asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Sets bucket b's bit.
 __device__ __forceinline__ void mark_bucket(uint32_t *mark, int b) { red_or(&mark[b >> 5], 1u << (b & 31)); }
+
+// The same into a block's copy of the bitmap (s_mark), which is merged at the end.
+__device__ __forceinline__ void mark_bucket_shared(uint32_t *s_mark, int b)
+{
+    const uint32_t bit = 1u << (b & 31);
+    if (!(*(volatile uint32_t *)&s_mark[b >> 5] & bit)) atomicOr(&s_mark[b >> 5], bit);
+}
 
 // Marks the errand buckets today's contact draws will read: the only buckets that
 // must be materialised.  Destinations are regenerated from the schedule counter, as
@@ -1252,11 +1260,28 @@ __device__ __forceinline__ void mark_bucket(uint32_t *mark, int b) { red_or(&mar
 // the same Threefry block, :3697-3702; children use the afterschool profile), and on
 // weekends the two errand slots picked by word 3 of the infection counter's block
 // (:1892, :1909, :1929).
-__global__ void k_mark_buckets(const InstConst *ic, const InstState *is, const uint8_t *age, const int32_t *infected,
-                               const int32_t *infected_inst, int weekend, uint32_t *mark, const Scalars *sc)
+//
+// On a dense day the infected far outnumber the bitmap's words, and updates of one
+// word are served one after another: 2M infected over 640 words took 400 us.  So when
+// the bitmap fits a block's shared memory (kMarkSharedWords) and the infected are at
+// least kMarkSharedPerWord to a word, each block marks a copy of its own and merges the
+// words it set.  Below that the merge (a word per block) would cost more than it saves.
+constexpr int kMarkSharedWords = 8192, kMarkSharedPerWord = 64;
+constexpr int kMarkThreads = 256, kMarkBlocksPerSm = 4;
+
+__global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *ic, const InstState *is,
+                                                               const uint8_t *age, const int32_t *infected,
+                                                               const int32_t *infected_inst, int weekend,
+                                                               uint32_t *mark, int words, const Scalars *sc)
 {
     if (sc->done) return;
     const int I = sc->infected;
+    __shared__ uint32_t s_mark[kMarkSharedWords];
+    const bool shared = words <= kMarkSharedWords && I >= kMarkSharedPerWord * words;
+    if (shared) {
+        for (int i = threadIdx.x; i < words; i += blockDim.x) s_mark[i] = 0u;
+        __syncthreads();
+    }
     for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < I; pos += gridDim.x * blockDim.x) {
         const int k = infected_inst[pos];
         const InstConst &ik = ic[k];
@@ -1274,7 +1299,9 @@ __global__ void k_mark_buckets(const InstConst *ic, const InstState *is, const u
             const int prof = (int)(w[3] % 6u);
 #pragma unroll
             for (int j = 0; j < 2; j++) {
-                mark_bucket(mark, ik.bbase[1] + d[c_weekend_assign[prof][j]]);
+                const int b = ik.bbase[1] + d[c_weekend_assign[prof][j]];
+                if (shared) mark_bucket_shared(s_mark, b);
+                else mark_bucket(mark, b);
             }
         } else {
             const int lo = c.type_offset[8], R = c.L - lo;
@@ -1287,8 +1314,23 @@ __global__ void k_mark_buckets(const InstConst *ic, const InstState *is, const u
             k1 += ik.bbase[0];
             k2 += ik.bbase[0];
             const int prof = adult ? (int)((w[slot] ^ w[slot + 1]) % 3u) : 3;
-            if (c_weekday_assign[prof][0] > 0) mark_bucket(mark, k1);
-            if (c_weekday_assign[prof][1] > 0) mark_bucket(mark, k2);
+            if (c_weekday_assign[prof][0] > 0) {
+                if (shared) mark_bucket_shared(s_mark, k1);
+                else mark_bucket(mark, k1);
+            }
+            if (c_weekday_assign[prof][1] > 0) {
+                if (shared) mark_bucket_shared(s_mark, k2);
+                else mark_bucket(mark, k2);
+            }
+        }
+    }
+    if (shared) {
+        __syncthreads();
+        // blocks start at different words, so they do not queue at the same one
+        const int first = (int)((long long)words * blockIdx.x / gridDim.x);
+        for (int i = threadIdx.x; i < words; i += blockDim.x) {
+            const int w = first + i < words ? first + i : first + i - words;
+            if (s_mark[w]) red_or(&mark[w], s_mark[w]);
         }
     }
 }
@@ -1541,8 +1583,8 @@ cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, bool full
     cudaError_t e = cudaMemsetAsync(d.mark, full_tables ? 0xFF : 0, ((size_t)B / 32 + 1) * 4, s);
     if (e != cudaSuccess) return e;
     if (!full_tables) {
-        k_mark_buckets<<<sm_count() * 4, 128, 0, s>>>(d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0,
-                                                      d.mark, d.sc);
+        k_mark_buckets<<<sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, s>>>(
+            d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.mark, B / 32 + 1, d.sc);
         count_launch();
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
