@@ -189,15 +189,15 @@ typedef struct pt_tuning {
     int infect_coop;            /* 0: one thread per infector; 1: eight lanes per infector */
     int infect_blocks_per_sm;   /* infection grid, 256-thread blocks per SM: 1..32 */
     int radix_blocks_per_sm;    /* persistent blocks of a day's radix pass per SM: 1..4
-                                   (3 at 80 registers a thread, 4 at 64) */
+                                   (three fit; 4 runs as 3) */
     int sched_tf;               /* 0..2, kept as given; every value runs the same Threefry
                                    arithmetic, the one measured fastest */
     int dense_level;            /* days whose sort reads every schedule key directly instead
                                    of entries the schedule kernel appends: 0 none; 1, 2, 3
                                    when the instance's infected are at least a quarter of,
                                    as many as, twice its buckets */
-    int radix_threads;          /* threads per block of a day's radix passes: 256 (16 entries
-                                   each) or 512 (8 each; radix_blocks_per_sm at most 2) */
+    int radix_threads;          /* 256, or 512 with radix_blocks_per_sm at most 2; kept as
+                                   given, every value runs 256-thread blocks */
 } pt_tuning;
 
 /* Sets / reads the launch shapes of sim (allowed before or after pt_setup). */
@@ -206,8 +206,8 @@ pt_status pt_get_tuning(const pt_sim *sim, pt_tuning *t);
 
 /* The tuner: after pt_setup, runs the first `days` days (0: all of max_days) once
  * per candidate launch shape with per-stage CUDA events, keeps the fastest shape for
- * the infection stage and for the radix stage (each is timed on its own stage), sets
- * it, and resets the epidemic.  Results of later runs do not depend on the choice.
+ * the infection stage and the fastest dense_level for the schedule and radix stages,
+ * sets it, and resets the epidemic.  Results of later runs do not depend on the choice.
  * A shape found for an engine of the same size (instances, persons, bucket counts,
  * SM count) earlier in the process is reused without timing.  chosen may be NULL. */
 pt_status pt_autotune(pt_sim *sim, int days, pt_tuning *chosen);

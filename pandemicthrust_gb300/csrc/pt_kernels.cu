@@ -6,8 +6,9 @@
 //   sweep   recover + 16 status bins + ordered infected list, one pass
 //           (kernel_countInfectedStatusAndRecover :2097-2192 + copy_if :2207-2224)
 //   sched   schedule keys + bucket histogram          (:2972-3022 / :2082-2094)
-//   bucket  scan of the histogram (bucket offsets) and a stable LSD radix sort of
-//           the (key, person) entries (CUB sort + lower_bound, :1212-1248, :1313-1354)
+//   bucket  a stable LSD radix sort of the (key, person) entries, whose last pass also
+//           writes each bucket's start and size (CUB sort + lower_bound, :1212-1248,
+//           :1313-1354)
 //   infect  contacts and infection draws; the first attempt in (position, slot)
 //           order claims each (victim, strain)        (:3236-3379)
 //   apply   winners write status, day, generation     (:3048-3067)
@@ -89,16 +90,15 @@ cudaError_t launch_household_types(const SimConst &c, uint8_t *types, int32_t *s
 // Generic exclusive scan (single pass, decoupled look-back): out[i] = sum in[0..i),
 // out[n] = total.  With clear_in the input is zeroed after it is read.  With
 // passes > 0, in[] is a histogram over keys 0..n-1 and the scan also accumulates,
-// for each radix pass p, the histogram of the key's 8-bit digit p weighted by the
-// count (digit_hist[p][256]), from which the radix sort takes its digit bases.
+// for each radix pass p, the histogram of the key's digit p (dbits bits) weighted by
+// the count (digit_hist[p][256]), from which the radix sort takes its digit bases.
 constexpr int kScanThreads = 256, kScanItems = 16, kScanTile = kScanThreads * kScanItems;
 static_assert(kScanTile == kScanTileEntries, "the host sizes the scan look-back words by kScanTileEntries");
 constexpr int kMaxRadixPasses = 4;
 
 __global__ void __launch_bounds__(kScanThreads) k_scan(const int32_t *in, int32_t *out, int n, int clear_in,
-                                                       LookBack lb, const int *skip, int passes, int *digit_hist,
-                                                       const uint32_t *mark, int *total_out,
-                                                       unsigned long long *total_accum)
+                                                       LookBack lb, const int *skip, int passes, int dbits,
+                                                       int *digit_hist)
 {
     if (skip && *(volatile const int *)skip) return;
     __shared__ int s_dh[kMaxRadixPasses][256];
@@ -115,8 +115,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int32_t *in, int32_
     for (int k = 0; k < kScanItems; k++) {
         long long i = base + k;
         v[k] = i < n ? in[i] : 0;
-        // with a mark filter only marked buckets keep their entries
-        if (mark && i < n && !((mark[i >> 5] >> (i & 31)) & 1u)) v[k] = 0;
         sum += v[k];
     }
     if (clear_in) {
@@ -131,7 +129,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int32_t *in, int32_
         for (int k = 0; k < kScanItems; k++) {
             if (v[k] > 0) {
                 unsigned key = (unsigned)(base + k);
-                for (int p = 0; p < passes; p++) atomicAdd(&s_dh[p][(key >> (8 * p)) & 255u], v[k]);
+                for (int p = 0; p < passes; p++)
+                    atomicAdd(&s_dh[p][(key >> (dbits * p)) & ((1u << dbits) - 1u)], v[k]);
             }
         }
     }
@@ -150,11 +149,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int32_t *in, int32_
         if (i < n) out[i] = run;
         run += v[k];
     }
-    if (tile == (int)gridDim.x - 1 && threadIdx.x == 0) {
-        out[n] = (int)s_prefix + total;
-        if (total_out) *total_out = (int)s_prefix + total;
-        if (total_accum) *total_accum += (unsigned long long)((int)s_prefix + total);
-    }
+    if (tile == (int)gridDim.x - 1 && threadIdx.x == 0) out[n] = (int)s_prefix + total;
     if (passes > 0) {
         for (int p = 0; p < passes; p++) {
             int c = s_dh[p][threadIdx.x];
@@ -166,16 +161,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int32_t *in, int32_
 
 cudaError_t launch_scan_exclusive(const int32_t *in, int32_t *out, int n, int clear_in,
                                   unsigned long long *tiles, int *ctl, int *error,
-                                  const int *skip, int passes, int *digit_hist, cudaStream_t s,
-                                  const uint32_t *mark, int *total_out, unsigned long long *total_accum)
+                                  const int *skip, int passes, int dbits, int *digit_hist, cudaStream_t s)
 {
     int blocks = std::max(1, div_up(n, kScanTile));
     LookBack lb;
     lb.tiles = tiles;
     lb.ctl = ctl;
     lb.error = error;
-    k_scan<<<blocks, kScanThreads, 0, s>>>(in, out, n, clear_in, lb, skip, passes, digit_hist, mark, total_out,
-                                                           total_accum);
+    k_scan<<<blocks, kScanThreads, 0, s>>>(in, out, n, clear_in, lb, skip, passes, dbits, digit_hist);
     count_launch();
     return cudaGetLastError();
 }
@@ -315,70 +308,95 @@ cudaError_t launch_count_keys(const int32_t *keys, int n, int32_t *count, cudaSt
 // Bucket tables: the reference sorts (key, person) pairs stably by key and takes
 // lower bounds (CUB radix sort + thrust::lower_bound, PandemicSim.cu:1212-1248,
 // :3835-3862), so every bucket lists its persons in ascending id order.  This stable
-// LSD radix sort over 8-bit digits gives the same table.  Entries enter the first
-// pass in ascending person order; each pass ranks a tile of 4096 entries by digit
-// (warp-blocked, so the rank is stable), finds the tile's global position per digit
-// by a decoupled look-back over earlier tiles (one thread per digit), and writes.
-constexpr int kRadixThreads = 256, kRadixItems = 16;   // the default block: 256 threads x 16 entries
-constexpr int kRadixTile = kRadixThreads * kRadixItems;
+// LSD radix sort gives the same table: the fewest passes of at most 8 bits, the key's
+// bits spread evenly over them.  Entries enter the first pass in ascending person
+// order; each pass ranks a tile of 4096 (key, value) pairs by digit (warp-blocked, so
+// the rank is stable), places the tile in shared memory in digit order, finds the
+// tile's global position per digit by a decoupled look-back over earlier tiles (one
+// thread per digit) and writes each digit's run with consecutive threads.
+//
+// What bounds it (24M pairs on a GB300, each part left out in turn): reading and
+// writing 16 bytes an entry 64 us, ranking 50, look-back one tile a step 45, scattered
+// instead of linear writes 12.  So the look-back reads four predecessors a step, and
+// after the tile is placed, when more of them are ready (143 us instead of 171); and
+// three blocks of 256 threads an SM (80 registers) do better than four (64, 163 us),
+// 16 x 384 or 512 threads (154, 170) or 12 entries a thread (187).  Ranking by ballots
+// (160), match (208) or one warp barrier a round with three word sets (160) is slower.
+constexpr int kRadixThreads = 256, kRadixItems = 16, kRadixWarps = kRadixThreads / 32;
+constexpr int kRadixBlocksPerSm = 3;
+constexpr int kRadixTile = kRadixThreads * kRadixItems, kRadixWarpItems = kRadixItems * 32;
 static_assert(kRadixTile == kRadixTileEntries, "the host sizes the radix look-back words by kRadixTileEntries");
+static_assert(kRadixWarpItems % kRegionChunk == 0, "a warp's entries start at a chunk_region word");
+constexpr int kLookBackStep = 4;
 
-enum RadixMode { kRadixFirst = 0, kRadixMiddle = 1, kRadixLast = 2, kRadixOnly = 3 };
+// What a pass reads: plain keys with implicit values (entry i is person i); a day's first
+// pass (the schedule's regions, or the schedule keys of a dense instance); pairs.
+enum RadixIn { kInKeys = 0, kInDay = 1, kInPairs = 2 };
+// What it writes: pairs; the values only (the last pass); those and the bucket table
+// (a day's last pass).
+enum RadixOut { kOutPairs = 0, kOutValues = 1, kOutTable = 2 };
 constexpr uint32_t kDropped = 0xFFFFFFFFu;   // value of an entry a pass leaves out (no person id is this)
 
-// Person id of schedule entry i: the setup table is the identity, weekday entries
-// are hour-major (i < N hour 0, else hour 1), weekend entries person-major (3 per person).
-__device__ __forceinline__ uint32_t entry_person(long long i, int N, int person_mode)
-{
-    if (person_mode == 0) return (uint32_t)i;
-    if (person_mode == 1) return (uint32_t)(i < N ? i : i - N);
-    return (uint32_t)(i / 3);
-}
+struct RadixPass {
+    const uint32_t *keys;
+    const uint2 *in;
+    uint2 *out_pairs;
+    uint32_t *out_values;
+    uint2 *table;
+    int E, pass, passes, dbits;
+    const int *digit_base;
+    RadixSegments sg;
+    unsigned long long *status;
+    int *ctl, *error;
+    const int *skip;
+};
 
-// Lanes of the warp holding the same digit as this lane (among lanes in `valid`),
-// from one ballot per digit bit: constant cost, unlike a match over 256 values.
-__device__ __forceinline__ unsigned digit_peers(unsigned d, int nbits, unsigned valid)
+// The tile a block works on: its ticket, its segment and what it reads there.
+struct RadixTile {
+    int tile, seg, stile;   // ticket, segment, tile within the segment
+    int base, count;        // the segment's first entry slot and entries
+    int dense;              // day's first pass: the segment reads the schedule keys
+    int nk, pb, bb;         // dense: the instance's persons, first person; bb: its first bucket
+    int rlast;              // day's first pass: the segment's last region
+};
+
+// Exclusive prefix of the tile's digit d over the segment's earlier tiles: words of
+// kLookBackStep predecessors a step, in order, up to the nearest inclusive one.
+__device__ __forceinline__ int radix_look_back(volatile unsigned long long *st, unsigned epoch, int tile, int first,
+                                               int d, int *error)
 {
-    unsigned peers = valid;
+    int excl = 0, t = tile - 1;
+    long long spins = 0;
+    for (;;) {
+        unsigned long long w[kLookBackStep];
 #pragma unroll
-    for (int b = 0; b < 8; b++) {
-        if (b < nbits) {
-            const unsigned bit = (d >> b) & 1u;
-            const unsigned bal = __ballot_sync(0xffffffffu, bit);
-            peers &= bit ? bal : ~bal;
+        for (int q = 0; q < kLookBackStep; q++)
+            w[q] = t - q >= first ? st[(size_t)(t - q) * 256 + d] : lb_word(epoch, 2, 0u);
+        int took = 0;
+#pragma unroll
+        for (int q = 0; q < kLookBackStep; q++) {
+            const unsigned flag = (unsigned)(w[q] >> 32) & 3u;
+            if (took == q && (unsigned)(w[q] >> 34) == epoch && flag != 0) {
+                excl += (int)(unsigned)w[q];
+                if (flag == 2) return excl;
+                took = q + 1;
+            }
+        }
+        t -= took;
+        if (took == 0) {
+            if (++spins > kSpinLimit) {
+                atomicExch(error, 2);
+                return excl;
+            }
+            __nanosleep(32);
         }
     }
-    return peers;
 }
 
-// Per-item record kept between the two phases of a pass: bits 0-7 digit, 8-16 the
-// entry's place among the warp's entries of that digit (earlier rounds, then lanes),
-// bit 17 valid.
-__device__ __forceinline__ uint32_t pack_place(unsigned d, unsigned place, bool ok)
-{
-    return d | (place << 8) | ((unsigned)ok << 17);
-}
-
-// The warp's entries of digit d before this round (s_hist[warp][d]) for every lane of
-// the round: the lowest lane of each digit group advances the count and broadcasts the
-// old value to its group.  Rounds are separated by __syncwarp, so each sees the last.
-__device__ __forceinline__ unsigned warp_digit_before(int *hist_d, unsigned peers, unsigned rank, unsigned cnt,
-                                                      bool ok, int lane)
-{
-    int before = 0;
-    if (ok && rank == 0) {
-        before = *hist_d;
-        *hist_d = before + (int)cnt;
-    }
-    before = __shfl_sync(0xffffffffu, before, ok ? __ffs(peers) - 1 : lane);
-    return (unsigned)before;
-}
-
-// One stable radix pass over 8 bits of the keys.  FILTER (first pass only) drops
-// entries whose bucket is not set in `mark`; passes whose input count lives on the
-// device read it from *count_dev.  Persistent blocks take tiles from a ticket in
-// order until the entries run out, so a short input costs no idle blocks.  Look-back
-// words carry the launch epoch (see lb_word), so they need no reset between passes.
+// One stable pass over dbits bits of the keys.  Persistent blocks take tiles from a
+// ticket in order until the entries run out, so a short input costs no idle blocks.
+// Look-back words carry the launch epoch (see lb_word), so they need no reset between
+// passes.
 //
 // Segmented sorts (sg.tile_prefix set): segment k's entries lie at
 // [ic[k].kbase, ic[k].kbase + is[k].marked) and are ordered within the segment only,
@@ -386,278 +404,240 @@ __device__ __forceinline__ unsigned warp_digit_before(int *hist_d, unsigned peer
 // segments' tiles are numbered consecutively (segment k owns tiles
 // [tile_prefix[k], tile_prefix[k + 1])), and the look-back of a segment's first tile
 // starts from zero.  Unsegmented sorts are one segment [0, E).
-template <int MODE, int THREADS, int MINB>
-__global__ void __launch_bounds__(THREADS, MINB) k_radix_pass(const uint32_t *__restrict__ keys_in,
-                                                                 const uint32_t *__restrict__ vals_in,
-                                                                 uint32_t *__restrict__ keys_out,
-                                                                 uint32_t *__restrict__ vals_out, int E_arg,
-                                                                 const int *count_dev, const uint32_t *mark,
-                                                                 int pass, int passes, int nbits, int N,
-                                                                 int person_mode, const int *__restrict__ digit_base,
-                                                                 RadixSegments sg, unsigned long long *status,
-                                                                 int *ctl, int *error, const int *skip)
+template <int IN, int OUT>
+__global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass(RadixPass a)
 {
-    // a tile of kRadixTile entries: THREADS threads, ITEMS entries each
-    constexpr int WARPS = THREADS / 32, ITEMS = kRadixTile / THREADS, WARP_ITEMS = ITEMS * 32;
-    static_assert(THREADS >= 256 && ITEMS * THREADS == kRadixTile, "one thread per digit and whole tiles");
-    static_assert(WARP_ITEMS <= 512, "an entry's place in its warp's digit run fits 9 bits (pack_place)");
-    if (skip && *(volatile const int *)skip) return;
-    __shared__ int s_tile;
-    // segment, tile within it, entry base, entry count; for a dense segment of a day's
-    // first pass: 1, the instance's persons, first person and first bucket; for another
-    // segment of that pass: 0, -, the segment's last region
-    __shared__ int s_seg[8];
-    __shared__ unsigned s_epoch;
-    __shared__ int s_hist[WARPS][256];
+    if (a.skip && *(volatile const int *)a.skip) return;
+    extern __shared__ __align__(16) uint8_t radix_smem[];
+    uint2 *const s_pair = reinterpret_cast<uint2 *>(radix_smem);                              // kRadixTile
+    unsigned *const s_peers = reinterpret_cast<unsigned *>(radix_smem + kRadixTile * 8);      // kRadixWarps x 256
+    // counts and places within the tile (at most 4096) fit 16 bits
+    uint16_t (*const s_hist)[256] = reinterpret_cast<uint16_t (*)[256]>(radix_smem + kRadixTile * 8 + kRadixWarps * 1024);
+    __shared__ RadixTile s_t;
     __shared__ int s_base[256];   // global position of digit d's entries, less its tile-local start
-    __shared__ uint32_t s_key[kRadixTile];
-    __shared__ uint32_t s_val[kRadixTile];
-    const int shift = 8 * pass;
-    // first pass of a day's sort (explicit values: the setup sorts' implicit modes never are)
-    const bool day0 = (MODE == kRadixMiddle || MODE == kRadixLast) && sg.day_keys != nullptr && pass == 0;
-    const int *tprefix = day0 ? sg.tile_prefix0 : sg.tile_prefix;
-    int E = 0, tiles;
-    if (sg.tile_prefix) {
-        tiles = *(volatile const int *)&tprefix[sg.segments];
-    } else {
-        E = count_dev ? *(volatile const int *)count_dev : E_arg;
-        tiles = (E + kRadixTile - 1) / kRadixTile;
-    }
+    const RadixSegments &sg = a.sg;
+    const int *const tprefix = IN == kInDay ? sg.tile_prefix0 : sg.tile_prefix;
+    const int tiles = sg.tile_prefix ? *(volatile const int *)&tprefix[sg.segments] : (a.E + kRadixTile - 1) / kRadixTile;
     // only as many blocks as there are tiles take part (ticket, finish count)
-    const int active = tiles < (int)gridDim.x ? tiles : (int)gridDim.x;
+    const int active = min(tiles, (int)gridDim.x);
     if ((int)blockIdx.x >= active) return;
-    if (threadIdx.x == 0) s_epoch = (unsigned)(*(volatile int *)&ctl[2]) & 0x3FFFFFFFu;
+    const unsigned epoch = (unsigned)(*(volatile int *)&a.ctl[2]) & 0x3FFFFFFFu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned lt = (1u << lane) - 1u;
+    const unsigned bit = 1u << lane, lt = bit - 1u, dmask = (1u << a.dbits) - 1u;
+    const int shift = a.dbits * a.pass;
+    uint16_t *const hist = s_hist[warp];
+    unsigned *const peer = s_peers + warp * 256;   // the lanes of a round holding each digit; zero between rounds
+    for (int i = threadIdx.x; i < kRadixWarps * 256; i += kRadixThreads) {
+        (&s_hist[0][0])[i] = 0;
+        s_peers[i] = 0u;
+    }
     for (;;) {
-        if (threadIdx.x == 0) {
-            const int t = atomicAdd(&ctl[0], 1);
-            int k = 0, j = t, sbase = 0, scount = E, dense = 0, nk = 0, pb = 0, bb = 0;
+        if (warp == 0) {
+            int t = 0;
+            if (lane == 0) t = atomicAdd(&a.ctl[0], 1);
+            t = __shfl_sync(0xffffffffu, t, 0);
+            RadixTile r = {t, 0, t, 0, a.E, 0, 0, 0, 0, 0};
             if (sg.tile_prefix && t < tiles) {
-                // the segment owning tile t: the last k with tprefix[k] <= t
-                int lo = 0, hi = sg.segments - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (tprefix[mid] <= t) lo = mid;
-                    else hi = mid - 1;
+                // the segment owning tile t: the last k with tprefix[k] <= t, 32 probes a step
+                int lo = 0, hi = sg.segments;   // in [lo, hi)
+                while (hi - lo > 1) {
+                    const int step = (hi - lo + 31) / 32, i = lo + lane * step;
+                    const unsigned below = __ballot_sync(0xffffffffu, i < hi && tprefix[i] <= t);
+                    lo += (31 - __clz(below)) * step;   // lane 0's probe always holds
+                    hi = min(hi, lo + step);
                 }
-                k = lo;
-                j = t - tprefix[k];
-                sbase = (int)sg.ic[k].kbase;
-                scount = sg.is[k].marked;
-                if (day0 && sg.is[k].dense) {
-                    dense = 1;
-                    nk = sg.ic[k].c.N;
-                    pb = sg.ic[k].pbase;
-                    bb = sg.ic[k].bbase[sg.weekend];
-                    scount = (sg.weekend ? 3 : 2) * nk;   // every schedule key of the instance
-                } else if (day0) {
-                    pb = sg.ic[k].pend / sg.region_persons - 1;   // the segment's last region
+                const InstConst &k = sg.ic[lo];
+                r.seg = lo;
+                r.stile = t - tprefix[lo];
+                r.base = (int)k.kbase;
+                r.count = sg.is[lo].marked;
+                if (IN == kInDay || OUT == kOutTable) r.bb = k.bbase[sg.weekend];
+                if (IN == kInDay) {
+                    r.rlast = k.pend / sg.region_persons - 1;
+                    if (sg.is[lo].dense) {
+                        r.dense = 1;
+                        r.nk = k.c.N;
+                        r.pb = k.pbase;
+                        r.count = (sg.weekend ? 3 : 2) * r.nk;   // every schedule key of the instance
+                    }
                 }
             }
-            s_tile = t;
-            s_seg[0] = k;
-            s_seg[1] = j;
-            s_seg[2] = sbase;
-            s_seg[3] = scount;
-            s_seg[4] = dense;
-            s_seg[5] = nk;
-            s_seg[6] = pb;
-            s_seg[7] = bb;
+            if (lane == 0) s_t = r;
         }
-        __syncthreads();
-        const int tile = s_tile;
-        const unsigned epoch = s_epoch;
+        __syncthreads();   // (also ends the last tile's use of shared memory)
+        const int tile = s_t.tile, stile = s_t.stile, sbase = s_t.base, scount = s_t.count, table_base = s_t.bb;
+        const int rlast = s_t.rlast;
         if (tile >= tiles) break;
-        const int seg = s_seg[0], stile = s_seg[1], sbase = s_seg[2], scount = s_seg[3];
-        const bool dense = s_seg[4] != 0;
-        // the peer words of phase A alias the first WARPS * 256 words of s_key, which
-        // phase B only writes after the barrier that ends phase A
-        unsigned *const s_peer = s_key + warp * 256;
-        for (int i = threadIdx.x; i < WARPS * 256; i += THREADS) {
-            (&s_hist[0][0])[i] = 0;
-            s_key[i] = 0u;
-        }
-        __syncthreads();
-        const int base = stile * kRadixTile + warp * WARP_ITEMS + lane;  // index within the segment
+        const int first = stile * kRadixTile + warp * kRadixWarpItems + lane;   // index within the segment
         const bool full = (stile + 1) * kRadixTile <= scount;
-        uint32_t key[ITEMS], val[ITEMS], info[ITEMS];
-        if (dense) {
+        bool whole = full;   // every entry of the tile takes part
+        uint2 kv[kRadixItems];
+        if (IN == kInDay && s_t.dense) {
             // the instance's schedule keys, persons implicit (weekday hour-major: entry
             // i < N is person i's hour-0 key, i >= N person i - N's hour-1 key; weekend
             // person-major, three per person), instance-local bucket keys; an entry of
             // an unmarked bucket gets the value kDropped and is left out
-            const int nk = s_seg[5], pb = s_seg[6], bb = s_seg[7];
+            const int nk = s_t.nk, pb = s_t.pb, bb = s_t.bb;
+            whole = false;
 #pragma unroll
-            for (int j = 0; j < ITEMS; j++) {
-                const int i = base + 32 * j;
+            for (int j = 0; j < kRadixItems; j++) {
+                const int i = first + 32 * j;
                 const bool in = full || i < scount;
                 const int kg = in ? sg.day_keys[sbase + i] : bb;
-                key[j] = (uint32_t)(kg - bb);
                 const bool marked = in && ((sg.mark[kg >> 5] >> (kg & 31)) & 1u);
-                val[j] = marked ? (uint32_t)(pb + (sg.weekend ? i / 3 : (i < nk ? i : i - nk))) : kDropped;
+                kv[j].x = (uint32_t)(kg - bb);
+                kv[j].y = marked ? (uint32_t)(pb + (sg.weekend ? i / 3 : (i < nk ? i : i - nk))) : kDropped;
             }
-        } else if (day0) {
+        } else if (IN == kInDay) {
             // the schedule's entries, region after region: entry i of the segment is entry
-            // i - region_prefix[r] of its region r, whose slots start at 3 C r
-            const int c0 = stile * kRadixTile + warp * WARP_ITEMS;
-            const int rlast = s_seg[6];   // the segment's last region
-            int r = 0, at = 0, next = 0;
-            if (c0 < scount) {
-                const int4 c = sg.chunk_region[(sbase + c0) / kRegionChunk];
-                r = c.x;
-                at = c.y;
-                next = c.z;
-            }
+            // i - region_prefix[r] of its region r, whose slots start at 3 C r.  The record
+            // of a chunk names the region of its first entry, that region's prefix and the
+            // ends of it and of the next one; the records of the warp's chunks are read
+            // together, and only entries past those two regions look further.
+            constexpr int kChunks = kRadixWarpItems / kRegionChunk, kPer = kRadixItems / kChunks;
+            const int c0 = stile * kRadixTile + warp * kRadixWarpItems;
+            int4 rec[kChunks];
 #pragma unroll
-            for (int j = 0; j < ITEMS; j++) {
-                const int i = base + 32 * j;
-                const bool in = full || i < scount;
-                if (in) {
-                    while (i >= next) {   // ends: the last region's end is scount
+            for (int q = 0; q < kChunks; q++)
+                rec[q] = c0 + q * kRegionChunk < scount ? sg.chunk_region[(sbase + c0) / kRegionChunk + q]
+                                                        : make_int4(0, 0, INT_MAX, INT_MAX);
+#pragma unroll
+            for (int j = 0; j < kRadixItems; j++) {
+                const int i = first + 32 * j;
+                kv[j] = make_uint2(0u, kDropped);
+                if (full || i < scount) {
+                    const int4 c = rec[j / kPer];
+                    int r = c.x, at = c.y;
+                    if (i >= c.z) {
                         r++;
-                        at = next;
-                        next = r < rlast ? sg.region_prefix[r + 1] : scount;
-                    }
-                }
-                const size_t src = 3 * (size_t)r * sg.region_persons + (i - at);
-                key[j] = in ? keys_in[src] : 0u;
-                val[j] = in ? vals_in[src] : 0u;
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < ITEMS; j++) {
-                const int i = base + 32 * j;
-                const bool in = full || i < scount;
-                key[j] = in ? keys_in[sbase + i] : 0u;
-                if (MODE == kRadixFirst || MODE == kRadixOnly) {
-                    const uint32_t u = (uint32_t)i;
-                    val[j] = person_mode == 0 ? u : (person_mode == 1 ? (u < (uint32_t)N ? u : u - (uint32_t)N) : u / 3u);
-                } else {
-                    val[j] = in ? vals_in[sbase + i] : 0u;
-                }
-            }
-        }
-        // phase A: rank within the warp round, per-warp digit counts.  The lanes holding
-        // the same digit come from one ballot per digit bit for narrow digits, and for
-        // wider ones from a shared word per digit that each lane ORs its bit into (the
-        // leader clears it again); both give the same set.  The leader also advances the
-        // warp's count of the digit (warp_digit_before), so each entry leaves with its
-        // place among the warp's entries of its digit: earlier rounds, then lanes.
-        if (nbits <= 4) {
-#pragma unroll
-            for (int j = 0; j < ITEMS; j++) {
-                const int i = base + 32 * j;
-                bool ok = (full || i < scount) && val[j] != kDropped;
-                if ((MODE == kRadixFirst || MODE == kRadixOnly) && mark && ok)
-                    ok = (mark[key[j] >> 5] >> (key[j] & 31u)) & 1u;
-                const unsigned d = (key[j] >> shift) & 255u;
-                const unsigned peers = digit_peers(d, nbits, __ballot_sync(0xffffffffu, ok));
-                const unsigned rank = __popc(peers & lt), cnt = __popc(peers);
-                const unsigned before = warp_digit_before(&s_hist[warp][d], peers, rank, cnt, ok, lane);
-                __syncwarp();
-                info[j] = pack_place(d, before + rank, ok);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < ITEMS; j++) {
-                const int i = base + 32 * j;
-                bool ok = (full || i < scount) && val[j] != kDropped;
-                if ((MODE == kRadixFirst || MODE == kRadixOnly) && mark && ok)
-                    ok = (mark[key[j] >> 5] >> (key[j] & 31u)) & 1u;
-                const unsigned d = (key[j] >> shift) & 255u;
-                if (ok) atomicOr(&s_peer[d], 1u << lane);
-                __syncwarp();
-                const unsigned peers = ok ? s_peer[d] : 0u;
-                __syncwarp();
-                const unsigned rank = __popc(peers & lt), cnt = __popc(peers);
-                if (ok && rank == 0) s_peer[d] = 0u;
-                const unsigned before = warp_digit_before(&s_hist[warp][d], peers, rank, cnt, ok, lane);
-                __syncwarp();
-                info[j] = pack_place(d, before + rank, ok);
-            }
-        }
-        __syncthreads();
-        {
-            // thread d < 256: exclusive bases of the warps for digit d, then the look-back
-            const int d = threadIdx.x;
-            int run = 0, gbase = 0;
-            if (d < 256) {
-#pragma unroll
-                for (int w = 0; w < WARPS; w++) {
-                    int c = s_hist[w][d];
-                    s_hist[w][d] = run;
-                    run += c;
-                }
-                volatile unsigned long long *st = status;
-                int excl = 0;
-                if (stile == 0) {
-                    st[(size_t)tile * 256 + d] = lb_word(epoch, 2, (unsigned)run);
-                } else {
-                    st[(size_t)tile * 256 + d] = lb_word(epoch, 1, (unsigned)run);
-                    int t = tile - 1;
-                    long long spins = 0;
-                    while (t >= 0) {
-                        const unsigned long long w = st[(size_t)t * 256 + d];
-                        const unsigned flag = (unsigned)(w >> 32) & 3u;
-                        if ((unsigned)(w >> 34) != epoch || flag == 0) {
-                            if (++spins > kSpinLimit) {
-                                atomicExch(error, 2);
-                                break;
-                            }
-                            __nanosleep(32);
-                            continue;
+                        at = c.z;
+                        if (i >= c.w) {
+                            int next = c.w;
+                            do {   // ends: the last region's end is scount
+                                r++;
+                                at = next;
+                                next = r < rlast ? sg.region_prefix[r + 1] : scount;
+                            } while (i >= next);
                         }
-                        excl += (int)(unsigned)w;
-                        if (flag == 2) break;
-                        t--;
                     }
-                    st[(size_t)tile * 256 + d] = lb_word(epoch, 2, (unsigned)(excl + run));
+                    kv[j] = a.in[3 * (size_t)r * sg.region_persons + (i - at)];
                 }
-                gbase = sbase + digit_base[((size_t)seg * passes + pass) * 256 + d] + excl;
             }
-            // tile-local start of digit d (entries of the tile ordered by digit)
-            int tile_total;
-            const int toff = block_exclusive_scan<THREADS, int>(run, tile_total);
-            if (d < 256) {
-                s_base[d] = gbase - toff;
-                // each warp's first place of digit d in the tile's digit order
+        } else {
 #pragma unroll
-                for (int w = 0; w < WARPS; w++) s_hist[w][d] += toff;
+            for (int j = 0; j < kRadixItems; j++) {
+                const int i = first + 32 * j;
+                kv[j] = make_uint2(0u, kDropped);
+                if (full || i < scount) kv[j] = IN == kInKeys ? make_uint2(a.keys[sbase + i], (uint32_t)i) : a.in[sbase + i];
             }
-            if (d == 0) s_tile = tile_total;  // reuse: valid entries of this tile
         }
-        __syncthreads();
-        // phase B: place each entry in shared memory in digit order (stable): the warp's
-        // first place of its digit plus its place among the warp's entries of that digit ...
+        // Rank: each entry's place among the warp's entries of its digit (earlier rounds,
+        // then lanes).  The lanes of a round that hold a digit meet in its shared word; the
+        // lowest of them clears the word, advances the warp's count of the digit and
+        // broadcasts the count before it.
+        unsigned place[kRadixItems];
+        if (whole) {
 #pragma unroll
-        for (int j = 0; j < ITEMS; j++) {
-            const uint32_t r = info[j];
-            if ((r >> 17) & 1u) {
-                const int lpos = s_hist[warp][r & 255u] + (int)((r >> 8) & 511u);
-                s_key[lpos] = key[j];
-                s_val[lpos] = val[j];
+            for (int j = 0; j < kRadixItems; j++) {
+                const unsigned d = (kv[j].x >> shift) & dmask;
+                atomicOr(&peer[d], bit);
+                __syncwarp();
+                const unsigned peers = *(volatile unsigned *)&peer[d];
+                const unsigned rank = __popc(peers & lt);
+                int before = 0;
+                if (rank == 0) before = hist[d];
+                __syncwarp();
+                if (rank == 0) {
+                    peer[d] = 0u;
+                    hist[d] = (uint16_t)(before + __popc(peers));
+                }
+                before = __shfl_sync(0xffffffffu, before, __ffs(peers) - 1);
+                __syncwarp();
+                place[j] = (unsigned)before + rank;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < kRadixItems; j++) {
+                const bool ok = kv[j].y != kDropped;
+                const unsigned d = (kv[j].x >> shift) & dmask;
+                if (ok) atomicOr(&peer[d], bit);
+                __syncwarp();
+                const unsigned peers = ok ? *(volatile unsigned *)&peer[d] : bit;
+                const unsigned rank = __popc(peers & lt);
+                int before = 0;
+                if (ok && rank == 0) before = hist[d];
+                __syncwarp();
+                if (ok && rank == 0) {
+                    peer[d] = 0u;
+                    hist[d] = (uint16_t)(before + __popc(peers));
+                }
+                before = __shfl_sync(0xffffffffu, before, __ffs(peers) - 1);
+                __syncwarp();
+                place[j] = (unsigned)before + rank;
             }
         }
         __syncthreads();
-        // ... then write each digit's run with consecutive threads (coalesced)
-        const int valid = s_tile;
-        for (int i = threadIdx.x; i < valid; i += THREADS) {
-            const uint32_t k = s_key[i];
-            const unsigned d = (k >> shift) & 255u;
-            const int pos = s_base[d] + i;
-            if (MODE == kRadixFirst || MODE == kRadixMiddle || keys_out) keys_out[pos] = k;
-            vals_out[pos] = s_val[i];
+        // thread d: the warps' counts of digit d become their first places in the tile's
+        // digit order; the tile's count is published for the look-backs of later tiles
+        const int d = threadIdx.x;
+        int c[kRadixWarps], run = 0;
+#pragma unroll
+        for (int w = 0; w < kRadixWarps; w++) {
+            c[w] = run;
+            run += s_hist[w][d];
         }
+        volatile unsigned long long *const st = a.status;
+        st[(size_t)tile * 256 + d] = lb_word(epoch, stile == 0 ? 2 : 1, (unsigned)run);
+        int valid;
+        const int toff = block_exclusive_scan<kRadixThreads, int>(run, valid);
+#pragma unroll
+        for (int w = 0; w < kRadixWarps; w++) s_hist[w][d] = (uint16_t)(c[w] + toff);
         __syncthreads();
+        // the tile in shared memory in digit order (stable)
+#pragma unroll
+        for (int j = 0; j < kRadixItems; j++)
+            if (whole || kv[j].y != kDropped) s_pair[hist[(kv[j].x >> shift) & dmask] + place[j]] = kv[j];
+        int excl = 0;
+        if (stile != 0) {
+            excl = radix_look_back(st, epoch, tile, tile - stile, d, a.error);
+            st[(size_t)tile * 256 + d] = lb_word(epoch, 2, (unsigned)(excl + run));
+        }
+        s_base[d] = sbase + a.digit_base[((size_t)s_t.seg * a.passes + a.pass) * 256 + d] + excl - toff;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kRadixWarps; w++) s_hist[w][d] = 0;   // for the next tile (whose barrier follows)
+        // each digit's run with consecutive threads (coalesced)
+        auto write = [&](int i) {
+            const uint2 p = s_pair[i];
+            const int pos = s_base[(p.x >> shift) & dmask] + i;
+            if (OUT == kOutPairs) a.out_pairs[pos] = p;
+            else a.out_values[pos] = p.y;
+            if (OUT == kOutTable) {
+                // The tile's entries of a digit are in key order, so a bucket's entries here
+                // are one run: its first entry offers the bucket's start, first and last
+                // together add its length (see BucketSlot).
+                uint2 *const slot = a.table + table_base + p.x;
+                if (i == 0 || s_pair[i - 1].x != p.x) {
+                    atomicMax(&slot->x, kMaxStart - (uint32_t)pos);
+                    atomicAdd(&slot->y, (uint32_t)-i);
+                }
+                if (i == valid - 1 || s_pair[i + 1].x != p.x) atomicAdd(&slot->y, (uint32_t)(i + 1));
+            }
+        };
+        if (valid == kRadixTile) {
+#pragma unroll
+            for (int j = 0; j < kRadixItems; j++) write(d + j * kRadixThreads);
+        } else {
+            for (int i = d; i < valid; i += kRadixThreads) write(i);
+        }
     }
     if (threadIdx.x == 0) {
         __threadfence();
-        const int fin = atomicAdd(&ctl[1], 1);
+        const int fin = atomicAdd(&a.ctl[1], 1);
         if (fin == active - 1) {
-            ctl[0] = 0;
-            ctl[1] = 0;
-            atomicAdd(&ctl[2], 1);
+            a.ctl[0] = 0;
+            a.ctl[1] = 0;
+            atomicAdd(&a.ctl[2], 1);
             __threadfence();
         }
     }
@@ -672,56 +652,56 @@ static int key_bits(int buckets)
 
 int radix_passes(int buckets) { return std::max(1, (key_bits(buckets) + 7) / 8); }
 
+// The key's bits spread evenly over the passes: fewer digits mean longer runs to write
+// and no pass with only a few digits, whose shared words all lanes would meet at.
+int radix_digit_bits(int buckets)
+{
+    const int P = radix_passes(buckets);
+    return std::max(1, (key_bits(buckets) + P - 1) / P);
+}
+
+constexpr int kRadixSmem = kRadixTile * 8 + kRadixWarps * 256 * (4 + 2);
+
+template <int IN, int OUT>
+static cudaError_t radix_launch(const RadixPass &a, int grid, cudaStream_t s)
+{
+    static_assert(kRadixSmem <= 46 * 1024, "with the static part, no more than a launch may ask for without opt-in");
+    k_radix_pass<IN, OUT><<<grid, kRadixThreads, kRadixSmem, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
 cudaError_t launch_radix_sort(const RadixArgs &r, cudaStream_t s)
 {
     const int P = radix_passes(r.buckets);
-    const int bits = key_bits(r.buckets);
     const int tiles = std::max(1, div_up(r.E, kRadixTile));
-    const bool wide = r.threads == 512;   // 512 threads x 8 entries per tile, at most 2 blocks per SM
-    // 256 threads: 3 blocks per SM at 80 registers, or 4 at 64 (the passes with explicit
-    // values only; the implicit-value first pass keeps 3)
-    const int bps = std::max(1, std::min(wide ? 2 : 4, r.blocks_per_sm));
-    const bool four = !wide && bps == 4;
-    const int grid = std::max(1, std::min(tiles, bps * sm_count()));  // persistent blocks
-    const int grid3 = std::max(1, std::min(tiles, std::min(bps, 3) * sm_count()));
-    const uint32_t *kin = r.keys;
-    const uint32_t *vin = r.vals;   // nullptr: implicit values (entry index -> person)
-    const bool implicit = r.vals == nullptr;
+    const int grid = std::max(1, std::min(tiles, std::min(r.blocks_per_sm, kRadixBlocksPerSm) * sm_count()));
+    RadixPass a;
+    a.keys = r.keys;
+    a.in = r.in;
+    a.out_values = r.out;
+    a.table = r.table;
+    a.E = r.E;
+    a.passes = P;
+    a.dbits = radix_digit_bits(r.buckets);
+    a.digit_base = r.digit_base;
+    a.sg = r.seg;
+    a.status = r.status;
+    a.ctl = r.ctl;
+    a.error = r.error;
+    a.skip = r.skip;
+    const bool day = r.table != nullptr;
     for (int p = 0; p < P; p++) {
+        const bool first = p == 0, last = p == P - 1;
+        a.pass = p;
+        a.out_pairs = (p & 1) ? r.p1 : r.p0;
         cudaError_t e;
-        uint32_t *kout = (p & 1) ? r.k1 : r.k0;
-        // the last pass writes keys only when asked to (RadixArgs::keep_keys)
-        if (p == P - 1 && !r.keep_keys) kout = nullptr;
-        uint32_t *vout = (p == P - 1) ? r.out : ((p & 1) ? r.v1 : r.v0);
-        const int nbits = std::max(1, std::min(8, bits - 8 * p));
-        // the first pass of an implicit-value sort reads all E entries (and may
-        // filter); every other pass reads the count on the device, if any
-        const int *cnt = (p == 0 && implicit) ? nullptr : r.count_dev;
-        const uint32_t *mk = (p == 0) ? r.mark : nullptr;
-#define PT_RADIX_ARGS kin, vin, kout, vout, r.E, cnt, mk, p, P, nbits, r.N, r.person_mode, r.digit_base, r.seg, r.status, \
-                      r.ctl, r.error, r.skip
-        if (P == 1 && implicit)
-            k_radix_pass<kRadixOnly, kRadixThreads, 3><<<grid3, kRadixThreads, 0, s>>>(PT_RADIX_ARGS);
-        else if (p == 0 && implicit)
-            k_radix_pass<kRadixFirst, kRadixThreads, 3><<<grid3, kRadixThreads, 0, s>>>(PT_RADIX_ARGS);
-        else if (p == P - 1 && wide)
-            k_radix_pass<kRadixLast, 512, 2><<<grid, 512, 0, s>>>(PT_RADIX_ARGS);
-        else if (p == P - 1 && four)
-            k_radix_pass<kRadixLast, kRadixThreads, 4><<<grid, kRadixThreads, 0, s>>>(PT_RADIX_ARGS);
-        else if (p == P - 1)
-            k_radix_pass<kRadixLast, kRadixThreads, 3><<<grid, kRadixThreads, 0, s>>>(PT_RADIX_ARGS);
-        else if (wide)
-            k_radix_pass<kRadixMiddle, 512, 2><<<grid, 512, 0, s>>>(PT_RADIX_ARGS);
-        else if (four)
-            k_radix_pass<kRadixMiddle, kRadixThreads, 4><<<grid, kRadixThreads, 0, s>>>(PT_RADIX_ARGS);
-        else
-            k_radix_pass<kRadixMiddle, kRadixThreads, 3><<<grid, kRadixThreads, 0, s>>>(PT_RADIX_ARGS);
-#undef PT_RADIX_ARGS
-        count_launch();
-        e = cudaGetLastError();
+        if (first && day) e = last ? radix_launch<kInDay, kOutTable>(a, grid, s) : radix_launch<kInDay, kOutPairs>(a, grid, s);
+        else if (first) e = last ? radix_launch<kInKeys, kOutValues>(a, grid, s) : radix_launch<kInKeys, kOutPairs>(a, grid, s);
+        else if (!last) e = radix_launch<kInPairs, kOutPairs>(a, grid, s);
+        else e = day ? radix_launch<kInPairs, kOutTable>(a, grid, s) : radix_launch<kInPairs, kOutValues>(a, grid, s);
         if (e != cudaSuccess) return e;
-        kin = kout;
-        vin = vout;
+        a.in = a.out_pairs;
     }
     return cudaSuccess;
 }
@@ -737,7 +717,7 @@ cudaError_t launch_bucket_table(const RadixArgs &r, int32_t *counts, bool count_
         if (e != cudaSuccess) return e;
     }
     cudaError_t e = launch_scan_exclusive(counts, offset, r.buckets, 1, tiles, lb_ctl, r.error, r.skip, P,
-                                          digit_hist, s, nullptr, nullptr);
+                                          radix_digit_bits(r.buckets), digit_hist, s);
     if (e != cudaSuccess) return e;
     k_digit_bases<<<1, 256, 0, s>>>(digit_hist, (int *)r.digit_base, P, 1, r.skip);
     count_launch();
@@ -1342,7 +1322,7 @@ __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *
 // round, one per lane).  The kernel writes every person's keys and keeps the entries of
 // marked buckets, compacted in ascending person order, in the warp's part of shared
 // memory; full parts are added to the block's radix digit histograms and copied, as
-// (instance-local key, person), to the region's slots of the entry arrays (3C from 3C
+// (instance-local key, person), to the region's slots of the entry array (3C from 3C
 // times the region's number).  The sort's first pass reads the regions of an instance
 // one after another (k_day_digit_bases scans their counts): the order its stability needs.
 //
@@ -1373,21 +1353,19 @@ __device__ __forceinline__ void sched_flush_digits(int (*s_dh)[256], int passes,
 }
 
 // The warp's part of `n` entries: into the digit histograms, and (unless the instance is
-// dense) to the entry arrays at ck / cv.
+// dense) to `entries`.
 __device__ __forceinline__ void sched_flush_entries(const uint32_t *my_key, const uint8_t *my_who, int n, int lane,
                                                     uint32_t bb, uint32_t first, int (*s_dh)[256], int passes,
-                                                    bool dense, uint32_t *ck, uint32_t *cv)
+                                                    int dbits, bool dense, uint2 *entries)
 {
+    const uint32_t dmask = (1u << dbits) - 1u;
     __syncwarp();
     for (int e = lane; e < n; e += 32) {
         const uint32_t b = my_key[e] - bb;
 #pragma unroll
         for (int p = 0; p < kMaxRadixPasses; p++)
-            if (p < passes) atomicAdd(&s_dh[p][(b >> (8 * p)) & 255u], 1);
-        if (!dense) {
-            ck[e] = b;
-            cv[e] = first + my_who[e];
-        }
+            if (p < passes) atomicAdd(&s_dh[p][(b >> (dbits * p)) & dmask], 1);
+        if (!dense) entries[e] = make_uint2(b, first + my_who[e]);
     }
     __syncwarp();
 }
@@ -1395,7 +1373,7 @@ __device__ __forceinline__ void sched_flush_entries(const uint32_t *my_key, cons
 template <bool WEEKEND>
 __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
     k_sched(const InstConst *ic, InstState *is, const int32_t *tile_inst, int regions, int C, const uint8_t *age,
-            const uint32_t *mark, int32_t *keys, int *digit_hist, int passes, uint32_t *ckeys, uint32_t *cvals,
+            const uint32_t *mark, int32_t *keys, int *digit_hist, int passes, int dbits, uint2 *entries,
             int32_t *region_count, const Scalars *sc, int day)
 {
     if (*(volatile const int *)&sc->done) return;
@@ -1443,13 +1421,13 @@ __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
             if (q >= end) break;
             const int rp = q * C - pbase;                       // the region's first person, instance numbering
             const int rend = min(rp + C, N);                    // (below rp when the region is all padding)
-            uint32_t *const ck = ckeys + 3 * (size_t)q * C, *const cv = cvals + 3 * (size_t)q * C;
+            uint2 *const mine = entries + 3 * (size_t)q * C;    // the region's slots
             int run = 0, part = rp, written = 0;                // entries in the part, its first person, entries flushed
 #pragma unroll 1
             for (int p0 = rp; p0 < rend; p0 += kRound) {
                 if (p0 - part >= kSchedPart) {
                     sched_flush_entries(my_key, my_who, run, lane, (uint32_t)bb, (uint32_t)(pbase + part), s_dh, passes,
-                                        dense, ck + written, cv + written);
+                                        dbits, dense, mine + written);
                     written += run;
                     run = 0;
                     part = p0;
@@ -1546,8 +1524,8 @@ __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
                     run += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
                 }
             }
-            sched_flush_entries(my_key, my_who, run, lane, (uint32_t)bb, (uint32_t)(pbase + part), s_dh, passes, dense,
-                                ck + written, cv + written);
+            sched_flush_entries(my_key, my_who, run, lane, (uint32_t)bb, (uint32_t)(pbase + part), s_dh, passes, dbits,
+                                dense, mine + written);
             written += run;
             if (lane == 0) {
                 region_count[q] = written;
@@ -1580,7 +1558,10 @@ static int sched_region_persons(long long P)
 cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, bool full_tables, cudaStream_t s)
 {
     const int B = d.buckets[weekend ? 1 : 0];
-    cudaError_t e = cudaMemsetAsync(d.mark, full_tables ? 0xFF : 0, ((size_t)B / 32 + 1) * 4, s);
+    // the marks and, behind them, the day's bucket slots: one clear
+    cudaError_t e = cudaMemsetAsync(d.mark, 0, (size_t)(reinterpret_cast<char *>(d.bkt + B) -
+                                                        reinterpret_cast<char *>(d.mark)), s);
+    if (e == cudaSuccess && full_tables) e = cudaMemsetAsync(d.mark, 0xFF, ((size_t)B / 32 + 1) * 4, s);
     if (e != cudaSuccess) return e;
     if (!full_tables) {
         k_mark_buckets<<<sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, s>>>(
@@ -1591,10 +1572,10 @@ cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, bool full
     }
     const int C = sched_region_persons(d.P), regions = d.P / C;
     const int blocks = std::min(div_up(regions, kSchedWarps), kSchedBlocksPerSm * sm_count());
-    const int passes = radix_passes(d.bucket_max[weekend ? 1 : 0]);
+    const int passes = radix_passes(d.bucket_max[weekend ? 1 : 0]), dbits = radix_digit_bits(d.bucket_max[weekend ? 1 : 0]);
 #define PT_SCHED(W)                                                                                              \
     k_sched<W><<<blocks, kSchedThreads, 0, s>>>(d.ic, d.is, d.tile_inst, regions, C, d.age, d.mark, d.keys,       \
-                                                d.digit_hist, passes, d.rk1, d.rv1, d.region_count, d.sc, day)
+                                                d.digit_hist, passes, dbits, d.rp1, d.region_count, d.sc, day)
     if (weekend) PT_SCHED(true);
     else PT_SCHED(false);
 #undef PT_SCHED
@@ -1604,21 +1585,20 @@ cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, bool full
 
 // The day's radix sort: one sorted segment per instance, keys local to the instance,
 // so the passes cover the largest instance's buckets only.  A segment's first pass
-// reads the marked entries the schedule appended to the instance's part of (rk1, rv1)
+// reads the marked entries the schedule wrote region by region to the instance's part of rp1
 // in person order, or, for an instance dense today, every schedule key (keeping the
 // marked ones).  Equal keys come from one hour, in person order, in both inputs, so
 // the sorted tables are the same.
 static RadixArgs day_radix_args(const DevArrays &d, bool weekend)
 {
     RadixArgs r;
-    r.keys = d.rk1;
-    r.vals = d.rv1;
+    r.in = d.rp1;
     r.E = 3 * d.P;   // at most (sizes the persistent grid)
     r.buckets = d.bucket_max[weekend ? 1 : 0];
-    r.N = d.P;
-    r.person_mode = weekend ? 2 : 1;
-    r.k0 = d.rk0; r.v0 = d.rv0; r.k1 = d.rk1; r.v1 = d.rv1;
+    r.p0 = d.rp0;
+    r.p1 = d.rp1;
     r.out = (uint32_t *)d.bkt_people;
+    r.table = d.bkt;
     r.digit_base = d.digit_base;
     r.seg.tile_prefix = d.tile_prefix;
     r.seg.ic = d.ic;
@@ -1635,9 +1615,7 @@ static RadixArgs day_radix_args(const DevArrays &d, bool weekend)
     r.ctl = d.radix_ctl;
     r.error = &d.sc->error;
     r.skip = &d.sc->done;
-    r.keep_keys = true;  // the bucket offsets come from the sorted keys
     r.blocks_per_sm = d.tune.radix_blocks_per_sm;
-    r.threads = d.tune.radix_threads;
     return r;
 }
 
@@ -1648,7 +1626,7 @@ static RadixArgs day_radix_args(const DevArrays &d, bool weekend)
 //    exclusive scan of the regions' entry counts; a block sums the counts before its
 //    own itself (at most a few hundred KB from L2) rather than wait for the others.
 //    Output: region_prefix, and for every kRegionChunk entries of the segment the region
-//    the first of them lies in, with its prefix and its end (chunk_region).
+//    the first of them lies in, its prefix, its end and the next one's (chunk_region).
 //  * The first block also numbers the segments' radix tiles (tile_prefix) and adds the
 //    day's materialised entries to the running total.
 constexpr int kBasesThreads = 1024, kBasesRegions = 4 * kBasesThreads;
@@ -1678,14 +1656,14 @@ __global__ void __launch_bounds__(kBasesThreads) k_day_digit_bases(int *digit_hi
         int at = carry + block_exclusive_scan<kBasesThreads, int>(c.x + c.y + c.z + c.w, total);
         if (r < r1) {
             int4 *const chunks = chunk_region + ic[k].kbase / kRegionChunk;
-            const int n[4] = {c.x, c.y, c.z, c.w};
+            const int n[5] = {c.x, c.y, c.z, c.w, r + 4 < r1 ? region_count[r + 4] : 0};
             int pre[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 pre[j] = at;
                 at += n[j];
                 for (int m = (pre[j] + kRegionChunk - 1) / kRegionChunk; m * kRegionChunk < at; m++)
-                    chunks[m] = make_int4(r + j, pre[j], at, 0);
+                    chunks[m] = make_int4(r + j, pre[j], at, at + n[j + 1]);
             }
             *reinterpret_cast<int4 *>(region_prefix + r) = make_int4(pre[0], pre[1], pre[2], pre[3]);
         }
@@ -1742,60 +1720,9 @@ cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// Bucket offsets from the sorted keys of each instance's segment: entry i starts
-// bucket keys[i] when that differs from keys[i-1] (thrust::lower_bound in the
-// reference, PandemicSim.cu:1240-1248).  Lazy tables write only the offsets the
-// infection kernels read: the start of each bucket with entries and the end of the
-// bucket before it.  Every bucket an infected person reads holds that person, so it
-// has entries.  Complete tables write every offset, empty buckets included.  Offsets
-// are positions in the batch's bucketed person array; each instance's last offset
-// goes to its own end slot.
-__global__ void k_bucket_offsets(const uint32_t *keys, RadixSegments sg, int weekend, int full, int32_t *offset,
-                                 const int *skip)
-{
-    if (*(volatile const int *)skip) return;
-    const int tiles = sg.tile_prefix[sg.segments];
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-        int lo = 0, hi = sg.segments - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (sg.tile_prefix[mid] <= t) lo = mid;
-            else hi = mid - 1;
-        }
-        const InstConst &c = sg.ic[lo];
-        const int m = sg.is[lo].marked;
-        const int sbase = (int)c.kbase, bb = c.bbase[weekend], B = c.bcount[weekend];
-        const int first = (t - sg.tile_prefix[lo]) * kRadixTile;
-        int last = first + kRadixTile < m ? first + kRadixTile : m;
-        if (last == m) last = m + 1;  // the segment's last tile also writes the end offset
-        for (int i = first + (int)threadIdx.x; i < last; i += blockDim.x) {
-            const int prev = i == 0 ? -1 : (int)keys[sbase + i - 1];
-            const int cur = i == m ? B : (int)keys[sbase + i];
-            if (prev == cur) continue;
-            if (full) {
-                for (int b = prev + 1; b <= cur; b++) offset[bb + b] = sbase + i;
-            } else {
-                offset[bb + prev + 1] = sbase + i;
-                offset[bb + cur] = sbase + i;
-            }
-        }
-    }
-}
-
 cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, cudaStream_t s)
 {
     return launch_radix_sort(day_radix_args(d, weekend), s);
-}
-
-cudaError_t launch_bucket_offsets(const DevArrays &d, bool weekend, bool full_tables, cudaStream_t s)
-{
-    const RadixArgs r = day_radix_args(d, weekend);
-    const int P = radix_passes(r.buckets);
-    const uint32_t *sorted = ((P - 1) & 1) ? r.k1 : r.k0;  // where the last pass wrote the keys
-    k_bucket_offsets<<<sm_count() * 8, 256, 0, s>>>(sorted, r.seg, weekend ? 1 : 0, full_tables ? 1 : 0,
-                                                    d.bkt_offset, r.skip);
-    count_launch();
-    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------ infection
@@ -1939,7 +1866,8 @@ struct InfectArgs {
     const uint8_t *gen_p, *gen_s, *age;
     const uint4 *prec;
     const int32_t *wp_people;
-    const int32_t *keys, *bkt_offset, *bkt_people, *infected, *infected_inst;
+    const uint2 *bkt;
+    const int32_t *keys, *bkt_people, *infected, *infected_inst;
     unsigned long long *claim;
     int32_t *new_list;
     Scalars *sc;
@@ -2036,7 +1964,8 @@ __global__ void __launch_bounds__(128) k_infect_weekday(InfectArgs a, int day)
 #pragma unroll
         for (int hour = 0; hour < 2; hour++) {
             int want = c_weekday_assign[prof][hour];
-            const int eoff = a.bkt_offset[dest[hour]], ecnt = a.bkt_offset[dest[hour] + 1] - eoff;
+            const uint2 slot = a.bkt[dest[hour]];
+            const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
 #pragma unroll
             for (int j = 3; j < 8; j++) {
                 if (j == made && want > 0) {
@@ -2098,7 +2027,8 @@ __global__ void __launch_bounds__(128) k_infect_weekend(InfectArgs a, int day)
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             const int loc = k3[c_weekend_assign[prof][j]];
-            const int eoff = a.bkt_offset[loc], ecnt = a.bkt_offset[loc + 1] - eoff;
+            const uint2 slot = a.bkt[loc];
+            const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
             kv[3 + j] = select_victim(me, eoff, ecnt, v2[j], false, a.bkt_people, victims[3 + j]);
             ksum += kv[3 + j];
         }
@@ -2226,7 +2156,8 @@ __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
                 kv = select_victim(me, hoff, hcnt, wc, true, nullptr, victim);
             } else if (j < 5) {
                 const int loc = a.keys[ik.kbase + 3 * (size_t)lme + c_weekend_assign[prof][j - 3]];
-                const int eoff = a.bkt_offset[loc], ecnt = a.bkt_offset[loc + 1] - eoff;
+                const uint2 slot = a.bkt[loc];
+                const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
                 kv = select_victim(me, eoff, ecnt, j == 3 ? v0 : v1, false, a.bkt_people, victim);
             }
         } else {
@@ -2245,7 +2176,8 @@ __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
                 const int hour = e < want0 ? 0 : (e < want0 + want1 ? 1 : -1);
                 if (hour >= 0) {
                     const int dest = a.keys[ik.kbase + (size_t)hour * c.N + lme];
-                    const int eoff = a.bkt_offset[dest], ecnt = a.bkt_offset[dest + 1] - eoff;
+                    const uint2 slot = a.bkt[dest];
+                    const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
                     kv = select_victim(me, eoff, ecnt, wc, false, a.bkt_people, victim);
                 }
             }
@@ -2284,7 +2216,7 @@ cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_
     a.state = d.state; a.gen_p = d.gen_p; a.gen_s = d.gen_s; a.age = d.age;
     a.prec = d.prec;
     a.wp_people = d.wp_people; a.keys = d.keys;
-    a.bkt_offset = d.bkt_offset; a.bkt_people = d.bkt_people; a.infected = d.infected;
+    a.bkt = d.bkt; a.bkt_people = d.bkt_people; a.infected = d.infected;
     a.infected_inst = d.infected_inst;
     a.claim = d.claim; a.new_list = d.new_list; a.sc = d.sc;
     const Tuning &t = d.tune;

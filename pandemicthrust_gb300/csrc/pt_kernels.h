@@ -91,12 +91,13 @@ struct Tuning {
     int infect_coop = 0;            // 1: warp-cooperative contacts (8 lanes per infector)
     int infect_blocks_per_sm = 8;   // infection grid: 256-thread blocks per SM (twice as
                                     // many 128-thread blocks for the thread-per-infector kernels)
-    int radix_blocks_per_sm = 4;    // persistent blocks of a day's radix pass per SM (1..4)
+    int radix_blocks_per_sm = 4;    // persistent blocks of a day's radix pass per SM (1..4;
+                                    // three fit, more act as three)
     int sched_tf = 0;               // accepted (0..2) and kept, without effect: one form of the
                                     // Threefry arithmetic is the fastest everywhere (tf2x64)
     int dense_level = 0;            // when a day's sort reads the schedule keys directly:
                                     // 0 never; 1, 2, 3: infected >= buckets / 4, x 1, x 2
-    int radix_threads = 256;        // threads per block of a day's radix passes: 256 or 512
+    int radix_threads = 256;        // accepted (256, 512) and kept, without effect
 };
 
 // Device pointers of a batch of simulations (one simulation is a batch of one).
@@ -113,10 +114,10 @@ struct DevArrays {
     int32_t *wp_offset;       // locations + 2
     uint4 *prec;              // P packed per-person records for the contact draws (see PersonRec)
     int32_t *keys;            // 3P schedule keys (global bucket indices)
-    int32_t *bkt_offset;      // buckets (each instance's buckets and its end slot)
-    int32_t *bkt_count;       // buckets histogram, zero between uses
+    uint2 *bkt;               // today's buckets: start and size (BucketSlot below)
+    int32_t *bkt_count;       // the workplace histogram of the setup, zero between uses
     int32_t *bkt_people;      // 3P person ids bucket by bucket, ascending in each
-    uint32_t *rk0, *rv0, *rk1, *rv1;  // 3P each: radix ping-pong keys/values
+    uint2 *rp0, *rp1;         // 3P each: radix ping-pong (key, value) pairs
     unsigned long long *radix_status;  // ceil(3P/4096) x 256 epoch-tagged look-back words
     int *radix_ctl;           // ticket, finished
     int *digit_hist;          // K x kDigitStripes x 4 x 256 (the first 4 x 256 also serve the setup sorts)
@@ -125,7 +126,7 @@ struct DevArrays {
     int32_t *tile_prefix0;    // K + 1: the same for the first pass (a dense segment's input is all its keys)
     int32_t *region_count;    // P / kSchedMinRegion: entries the schedule kernel wrote in each region
     int32_t *region_prefix;   // P / kSchedMinRegion: their exclusive prefix within the instance
-    int4 *chunk_region;       // 3P / kRegionChunk: region of every kRegionChunk-th entry of a segment, its prefix and end
+    int4 *chunk_region;       // 3P / kRegionChunk: region of every kRegionChunk-th entry of a segment (RadixSegments)
     uint32_t *mark;           // bitmap over today's buckets: 1 = materialise
     int32_t *infected;        // P ascending infected ids
     int32_t *infected_inst;   // P: instance of each infected list position
@@ -147,6 +148,14 @@ struct DevArrays {
     Scalars *sc;
     Tuning tune;
 };
+
+// BucketSlot: a bucket of the day's errand table, one 8-byte load.  x: kMaxStart less the
+// place of its first person in bkt_people (0: no entries); y: its persons.  Cleared to
+// zero each day; the sort's last pass raises x to the largest offer (the smallest
+// place) and adds up y.
+constexpr uint32_t kMaxStart = 0x7FFFFFFFu;   // above every place, so a bucket with entries has x > 0
+__host__ __device__ inline int bucket_start(uint2 slot) { return (int)(kMaxStart - slot.x); }
+__host__ __device__ inline int bucket_count(uint2 slot) { return (int)slot.y; }
 
 // The static part of a person that the contact draws read, packed in 16 bytes so an
 // infector's own data is one 128-bit load (built once at setup, after the workplace
@@ -170,9 +179,7 @@ cudaError_t launch_household_types(const SimConst &c, uint8_t *types, int32_t *s
                                    int *persons, cudaStream_t s);
 cudaError_t launch_scan_exclusive(const int32_t *in, int32_t *out, int n, int clear_in,
                                   unsigned long long *tiles, int *ctl, int *error,
-                                  const int *skip, int passes, int *digit_hist, cudaStream_t s,
-                                  const uint32_t *mark = nullptr, int *total_out = nullptr,
-                                  unsigned long long *total_accum = nullptr);
+                                  const int *skip, int passes, int dbits, int *digit_hist, cudaStream_t s);
 cudaError_t launch_generate_households(const uint8_t *types, const int32_t *hh_offset, int slots,
                                        int32_t *household, uint8_t *age, cudaStream_t s);
 cudaError_t launch_assign_workplaces(const SimConst &c, uint8_t *age, int32_t *workplace, int loc_base,
@@ -194,8 +201,8 @@ struct RadixSegments {
     // The first pass of a day's sort reads the entries the schedule kernel wrote region by
     // region (see k_sched): region r's at 3 region_persons r, its first one entry
     // region_prefix[r] of the segment; chunk_region[(kbase + i) / kRegionChunk] is the
-    // region of entry i (a multiple of kRegionChunk) of the segment at kbase, with that
-    // region's prefix and its end.
+    // region of entry i (a multiple of kRegionChunk) of the segment at kbase, that region's
+    // prefix, its end and the end of the next one.
     const int32_t *region_prefix = nullptr;
     const int4 *chunk_region = nullptr;
     int region_persons = 0;
@@ -210,27 +217,26 @@ struct RadixSegments {
     int weekend = 0;
 };
 
-// Stable LSD radix sort of E keys in [0, buckets) with implicit person values
-// (person_mode 0: entry i is person i; 1: weekday hour-major; 2: weekend 3 per person).
+// Stable LSD radix sort of E keys in [0, buckets).  Without `table`: plain keys, entry i
+// has the value i.  With it, a day's sort (seg): see RadixSegments; the sorted persons
+// go to `out`, the buckets' starts and sizes to `table`.
 struct RadixArgs {
-    const uint32_t *keys;
-    int E, buckets, N, person_mode;
-    const uint32_t *vals = nullptr;   // explicit input values (nullptr: implicit)
-    const uint32_t *mark = nullptr;   // optional bucket filter of the first pass
-    const int *count_dev = nullptr;   // entry count after the filter (device)
-    uint32_t *k0, *v0, *k1, *v1, *out;
-    bool keep_keys = false;       // the last pass also writes the sorted keys (to k0 / k1 by pass parity)
+    const uint32_t *keys = nullptr;
+    const uint2 *in = nullptr;    // a day's entries (key, person), in the schedule's regions
+    int E, buckets;
+    uint2 *p0, *p1;               // ping-pong pairs, E each (in may be p1)
+    uint32_t *out;
+    uint2 *table = nullptr;
     const int *digit_base;        // [segment][pass][256]
     RadixSegments seg;
     unsigned long long *status;   // look-back words, ceil(E/4096) x 256, epoch-tagged
     int *ctl;                     // ticket, finished, epoch
     int *error;
     const int *skip;
-    int blocks_per_sm = 3;        // persistent blocks per SM (1..4; 4 only for 256 threads)
-    int threads = 256;            // threads per block of the explicit-value passes: 256 (16 entries
-                                  // each, up to 4 blocks per SM) or 512 (8 each, up to 2 blocks)
+    int blocks_per_sm = 4;        // persistent blocks per SM, at most what fits
 };
 int radix_passes(int buckets);
+int radix_digit_bits(int buckets);   // bits of a pass's digit
 cudaError_t launch_radix_sort(const RadixArgs &r, cudaStream_t s);
 // count (optional) + scan + digit bases + radix passes: a complete bucket table
 cudaError_t launch_bucket_table(const RadixArgs &r, int32_t *counts, bool count_keys, int32_t *offset,
@@ -254,7 +260,6 @@ cudaError_t launch_infected_list(const DevArrays &d, cudaStream_t s);           
 cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, bool full_tables, cudaStream_t s);
 cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s);
 cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, cudaStream_t s);
-cudaError_t launch_bucket_offsets(const DevArrays &d, bool weekend, bool full_tables, cudaStream_t s);
 cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_t s);
 cudaError_t launch_apply(const DevArrays &d, int day, cudaStream_t s);
 // weekday / weekend buckets of one instance (compact keys hour * R + dest - lo)

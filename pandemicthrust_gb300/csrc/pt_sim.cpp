@@ -408,7 +408,7 @@ static pt_status engine_setup(Engine *s)
     d.locations = (int)LT;
     // padding slots, then one scan of all household slots: offsets and person bases
     CK(ptk::launch_batch_padding(d, types, sizes, 0, false, s->stream), "padding slots");
-    CK(ptk::launch_scan_exclusive(sizes, d.hh_offset, (int)HS, 0, d.tiles, ctl, &d.sc->error, nullptr, 0, nullptr,
+    CK(ptk::launch_scan_exclusive(sizes, d.hh_offset, (int)HS, 0, d.tiles, ctl, &d.sc->error, nullptr, 0, 8, nullptr,
                                   s->stream), "household scan");
 
     // arena of per-person and per-location arrays
@@ -423,8 +423,8 @@ static pt_status engine_setup(Engine *s)
     bytes += round256(n * 4) * 3;               // household, workplace, wp_people
     bytes += round256(n * 16);                  // packed person records
     bytes += round256(((size_t)LT + 2) * 4);    // wp_offset
-    bytes += round256(3 * n * 4) * 6;           // keys, bkt_people, radix k0/v0/k1/v1
-    bytes += round256(((size_t)Bday + 1) * 4);  // bkt_offset
+    bytes += round256(3 * n * 4) * 2;           // keys, bkt_people
+    bytes += round256(3 * n * 8) * 2;           // radix pairs p0, p1
     bytes += round256((size_t)Bmax * 4);        // bkt_count (also the workplace histogram)
     bytes += round256(radix_tiles * 256 * 8);   // radix look-back words
     bytes += round256(8 * 4);                                                      // radix ctl
@@ -432,7 +432,8 @@ static pt_status engine_setup(Engine *s)
     bytes += round256((size_t)K * 4 * 256 * 4) + 2 * round256(((size_t)K + 1) * 4);  // digit bases, tile prefixes
     const size_t nregions = n / ptk::kSchedMinRegion, nchunks = 3 * n / ptk::kRegionChunk + 1;
     bytes += 2 * round256(nregions * 4) + round256(nchunks * sizeof(int4));   // schedule regions
-    bytes += round256(((size_t)Bday / 32 + 1) * 4);        // bucket mark bitmap
+    // the mark bitmap and, right behind it, the bucket slots of a day (cleared together)
+    bytes += round256(((size_t)Bday + 1) * sizeof(uint2)) + round256(((size_t)Bday / 32 + 1) * 4);
     bytes += round256(n * 4) * 2;               // infected, infected_inst
     bytes += round256(n / 16 * 2) + round256((ntiles + 1) * 4);  // sweep masks, sweep tile counts
     bytes += round256(2 * n * 8);               // claim
@@ -453,11 +454,8 @@ static pt_status engine_setup(Engine *s)
     d.prec = a.take<uint4>(n);
     d.keys = a.take<int32_t>(3 * n);
     d.bkt_people = a.take<int32_t>(3 * n);
-    d.rk0 = a.take<uint32_t>(3 * n);
-    d.rv0 = a.take<uint32_t>(3 * n);
-    d.rk1 = a.take<uint32_t>(3 * n);
-    d.rv1 = a.take<uint32_t>(3 * n);
-    d.bkt_offset = a.take<int32_t>((size_t)Bday + 1);
+    d.rp0 = a.take<uint2>(3 * n);
+    d.rp1 = a.take<uint2>(3 * n);
     d.bkt_count = a.take<int32_t>((size_t)Bmax);
     d.radix_status = a.take<unsigned long long>(radix_tiles * 256);
     d.radix_ctl = a.take<int>(8);
@@ -469,6 +467,7 @@ static pt_status engine_setup(Engine *s)
     d.region_prefix = a.take<int32_t>(nregions);
     d.chunk_region = a.take<int4>(nchunks);
     d.mark = a.take<uint32_t>((size_t)Bday / 32 + 1);
+    d.bkt = a.take<uint2>((size_t)Bday + 1);
     d.infected = a.take<int32_t>(n);
     d.infected_inst = a.take<int32_t>(n);
     d.sweep_flags = a.take<uint16_t>(n / 16);
@@ -507,9 +506,8 @@ static pt_status engine_setup(Engine *s)
         r.keys = (const uint32_t *)d.workplace;
         r.E = (int)P;
         r.buckets = (int)LT + 1;
-        r.N = (int)P;
-        r.person_mode = 0;
-        r.k0 = d.rk0; r.v0 = d.rv0; r.k1 = d.rk1; r.v1 = d.rv1;
+        r.p0 = d.rp0;
+        r.p1 = d.rp1;
         r.out = (uint32_t *)d.wp_people;
         r.digit_base = d.digit_base;
         r.status = d.radix_status;
@@ -597,8 +595,8 @@ static pt_status enqueue_day(Engine *s, int day)
     CK(ptk::launch_bucket_scan(d, weekend, st), "digit bases");
     if (t) cudaEventRecord(stage_event(s, day, kStRadix), st);
     CK(ptk::launch_bucket_sort(d, weekend, st), "bucket sort");
+    // (the sort's last pass writes the bucket slots: the offsets stage is empty)
     if (t) cudaEventRecord(stage_event(s, day, kStOffsets), st);
-    CK(ptk::launch_bucket_offsets(d, weekend, s->full_tables, st), "bucket offsets");
     if (t) cudaEventRecord(stage_event(s, day, kStInfect), st);
     CK(ptk::launch_infect(d, weekend, day, st), "infect");
     if (t) cudaEventRecord(stage_event(s, day, kStApply), st);
@@ -939,8 +937,7 @@ static std::vector<long long> tune_key(const Engine *s)
 }
 
 // The tuner.  The infection, radix and schedule stages are timed separately (per-stage
-// CUDA events around every day), so one run measures one candidate of each: run i
-// uses infection candidate i and radix candidate i % 3.
+// CUDA events around every day): run i uses infection candidate i.
 // Two more runs then try the dense-day sort levels 2 and 3 with the shapes chosen.
 static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
 {
@@ -960,11 +957,8 @@ static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
     // thread-per-infector kernel: 9 resident 128-thread blocks per SM at 56 registers;
     // warp-cooperative kernel: 6 resident 256-thread blocks per SM at 40 registers
     const Cand infect[] = {{0, 8}, {0, 4}, {1, 6}, {1, 12}, {1, 3}, {0, 16}};
-    // radix passes: (blocks per SM, threads per block)
-    const int radix[] = {3, 4, 2};
-    const int radix_threads[] = {256, 256, 512};
     const int runs = (int)(sizeof(infect) / sizeof(infect[0]));
-    float best_inf = 1e30f, best_rad[3] = {1e30f, 1e30f, 1e30f}, best_sched = 1e30f;
+    float best_inf = 1e30f, best_rad = 1e30f, best_sched = 1e30f;
     int best_i = 0;
     const int saved_max = s->max_days;
     const int trial = days > 0 ? std::min(days, saved_max) : saved_max;
@@ -972,8 +966,8 @@ static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
         pt_tuning t;
         t.infect_coop = infect[i].coop;
         t.infect_blocks_per_sm = infect[i].bps;
-        t.radix_blocks_per_sm = radix[i % 3];
-        t.radix_threads = radix_threads[i % 3];
+        t.radix_blocks_per_sm = 3;
+        t.radix_threads = 256;
         t.sched_tf = 0;
         t.dense_level = 0;
         pt_status st = engine_set_tuning(s, &t);
@@ -994,21 +988,18 @@ static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
             best_inf = inf;
             best_i = i;
         }
-        best_rad[i % 3] = std::min(best_rad[i % 3], rad);
+        best_rad = std::min(best_rad, rad);
     }
-    int rbest = 0;
-    for (int r = 1; r < 3; r++)
-        if (best_rad[r] < best_rad[rbest]) rbest = r;
     pt_tuning t;
     t.infect_coop = infect[best_i].coop;
     t.infect_blocks_per_sm = infect[best_i].bps;
-    t.radix_blocks_per_sm = radix[rbest];
-    t.radix_threads = radix_threads[rbest];
+    t.radix_blocks_per_sm = 3;
+    t.radix_threads = 256;
     t.sched_tf = 0;
     t.dense_level = 0;
     // the dense-day sort changes both the schedule and the sort stage: its levels are
     // timed after the others are chosen, against their schedule + sort time
-    float best_dense = best_rad[rbest] + best_sched;
+    float best_dense = best_rad + best_sched;
     for (int lv = 2; lv <= 3; lv++) {
         pt_tuning c = t;
         c.dense_level = lv;
@@ -1159,8 +1150,14 @@ pt_status pt_get_day_tables(pt_sim *s, int32_t *infected, int32_t *keys, int32_t
     }
     if (people) CK(pt_memcpy_sync(s, people, s->d.bkt_people, (size_t)E * 4, cudaMemcpyDeviceToHost), "copy");
     if (offsets) {
+        // starts of the buckets with entries; an empty one starts where the next one does
+        std::vector<uint2> slots((size_t)Bc);
+        CK(pt_memcpy_sync(s, slots.data(), s->d.bkt, (size_t)Bc * sizeof(uint2), cudaMemcpyDeviceToHost), "copy");
+        int marked = 0;
+        CK(pt_memcpy_sync(s, &marked, &s->d.is[0].marked, sizeof(int), cudaMemcpyDeviceToHost), "marked");
         std::vector<int32_t> co((size_t)Bc + 1);
-        CK(pt_memcpy_sync(s, co.data(), s->d.bkt_offset, ((size_t)Bc + 1) * 4, cudaMemcpyDeviceToHost), "copy");
+        co[Bc] = marked;
+        for (int b = Bc - 1; b >= 0; b--) co[b] = ptk::bucket_count(slots[b]) > 0 ? ptk::bucket_start(slots[b]) : co[b + 1];
         for (int h = 0; h < hours; h++)
             for (int loc = 0; loc < L; loc++)
                 offsets[(size_t)h * L + loc] = loc < lo ? co[(size_t)h * R] : co[(size_t)h * R + loc - lo];

@@ -41,11 +41,9 @@ constexpr size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Scratch layout (byte offsets into the static array)
 constexpr size_t kOffCounts = 0;                                                  // int[kMaxBuckets], zero between calls
-constexpr size_t kOffK0 = kOffCounts + align256((size_t)kMaxBuckets * 4);         // radix ping-pong buffers
-constexpr size_t kOffV0 = kOffK0 + align256((size_t)kMaxEntries * 4);
-constexpr size_t kOffK1 = kOffV0 + align256((size_t)kMaxEntries * 4);
-constexpr size_t kOffV1 = kOffK1 + align256((size_t)kMaxEntries * 4);
-constexpr size_t kOffStatus = kOffV1 + align256((size_t)kMaxEntries * 4);         // radix look-back words
+constexpr size_t kOffP0 = kOffCounts + align256((size_t)kMaxBuckets * 4);         // radix ping-pong pairs
+constexpr size_t kOffP1 = kOffP0 + align256((size_t)kMaxEntries * 8);
+constexpr size_t kOffStatus = kOffP1 + align256((size_t)kMaxEntries * 8);         // radix look-back words
 constexpr size_t kOffScanTiles = kOffStatus + align256((size_t)kRadixTiles * 256 * 8);  // scan look-back words + control
 constexpr size_t kOffRadixCtl = kOffScanTiles + align256((size_t)(kScanTiles + 4) * 8);
 constexpr size_t kOffDigitHist = kOffRadixCtl + 256;
@@ -121,12 +119,8 @@ extern "C" pt_status pt_bucket_table_static(const int32_t *keys, int n, int buck
     r.keys = (const uint32_t *)keys;
     r.E = n;
     r.buckets = buckets;
-    r.N = n;
-    r.person_mode = 0;  // entry i is item i
-    r.k0 = (uint32_t *)(base + kOffK0);
-    r.v0 = (uint32_t *)(base + kOffV0);
-    r.k1 = (uint32_t *)(base + kOffK1);
-    r.v1 = (uint32_t *)(base + kOffV1);
+    r.p0 = (uint2 *)(base + kOffP0);   // (plain keys: entry i is item i)
+    r.p1 = (uint2 *)(base + kOffP1);
     r.out = (uint32_t *)table;
     r.digit_base = (const int *)(base + kOffDigitBase);
     r.status = (unsigned long long *)(base + kOffStatus);
