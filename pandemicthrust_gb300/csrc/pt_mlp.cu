@@ -8,9 +8,7 @@
 //
 // Training GEMMs are small (a minibatch of a few hundred rows by 256) and need
 // transposed operands, so they run on the warp-level tensor-core instruction mma.sync
-// m16n8k16 (BF16 in, FP32 accumulate): one kernel with strided operands serves the
-// forward product X W^T, the data gradient dZ W and the weight gradient dZ^T X.
-// Inference over large batches runs every layer on tcgen05.mma (k_umma_layer below).
+// (k_gemm below).  Inference over large batches runs every layer on tcgen05.mma.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -29,34 +27,6 @@
 namespace {
 
 typedef __nv_bfloat16 bf16;
-
-constexpr int kTile = 64;   // block tile (M and N)
-constexpr int kTileK = 16;  // reduction step (one mma k-step)
-
-enum { kStoreF32 = 0, kForward = 1, kBackward = 2 };
-
-// C(i, j) = sum_r A(i, r) B(r, j) with A(i, r) = A[i*sa_i + r*sa_r] and
-// B(r, j) = B[r*sb_r + j*sb_j]; M x N outputs, R terms; any sizes (tiles zero-fill).
-struct GemmArgs {
-    const bf16 *A;
-    long long sa_i, sa_r;
-    const bf16 *B;
-    long long sb_r, sb_j;
-    int M, N, R;
-    int mode;
-    // kStoreF32: C[i*ldc + j] = acc
-    float *C;
-    long long ldc;
-    // kForward: z = acc + bias[j]; Z = z (FP32), H = act(z) (BF16); act = GELU if gelu
-    const float *bias;
-    float *Z;
-    bf16 *H;
-    int gelu;
-    // kBackward: dz = acc * GELU'(Zprev); dZf = dz (FP32), dZb = dz (BF16)
-    const float *Zprev;
-    float *dZf;
-    bf16 *dZb;
-};
 
 // The activation: GELU in its tanh form (Hendrycks and Gimpel, arXiv:1606.08415),
 // 0.5 z (1 + tanh(u)), u = sqrt(2/pi) (z + 0.044715 z^3), with the hardware tanh
@@ -89,96 +59,283 @@ __device__ __forceinline__ float gelu_grad(float z)
     return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * (kGeluC0 + 3.f * kGeluC1 * z2);
 }
 
-__device__ __forceinline__ uint32_t pack2(bf16 lo, bf16 hi)
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// ---------------------------------------------------------------- training GEMMs
+// A training step is a chain of small GEMMs (a batch of a few hundred rows by a few
+// hundred columns, a microsecond of work each), so what counts is how many launches
+// the chain has, how long one takes from its first load to its last store, and that
+// every SM has a part.  Hence: 32 x 32 output tiles (128 blocks for 512 x 256), the
+// whole reduction of 256 in flight at once (four cp.async stages of 64), operands read
+// by ldmatrix in either order, everything elementwise in the epilogues (bias, GELU and
+// its derivative, the loss, Adam; their inputs are read before the products start), and
+// independent GEMMs of a step in one launch.  A step of the 11-4x256-222 network at
+// batch 512 is 10 launches instead of 23 and takes 82 us on a GB300 instead of 640
+// (100 with programmatic dependent launches: the next launch's blocks get in the way).
+//
+// Products run on mma.sync m16n8k16 (BF16 in, FP32 accumulate), the reduction in
+// ascending steps of 16 into one accumulator, whatever the tiling.
+constexpr int kGemmThreads = 128, kGemmTile = 32, kGemmK = 64, kGemmStages = 4;
+constexpr int kGemmPitchK = (kGemmK + 8) * 2, kGemmPitchN = (kGemmTile + 8) * 2;   // bytes; odd multiples of 16
+constexpr int kGemmOperand = kGemmK * kGemmPitchN;   // one stage of one operand in either order (>= 32 x pitch K)
+static_assert(kGemmTile * kGemmPitchK <= kGemmOperand, "a stage holds an operand tile in both orders");
+constexpr int kGemmSmem = kGemmStages * 2 * kGemmOperand;
+constexpr int kBiasCols = 16, kBiasRows = 512;   // a bias block: columns, rows staged at once
+static_assert(kBiasCols * kBiasRows * 4 <= kGemmSmem, "the bias sums stage their rows in the same shared memory");
+
+// Adam's state of a layer's parameters, for the updates in the epilogues.
+struct AdamArgs {
+    float *w, *m, *v;   // FP32 parameters and moments, all layers
+    float lr, c1, c2;   // c1, c2: the bias corrections of the step
+};
+
+// Adam (Kingma and Ba, 2015) for parameter i with gradient gr and its values before the
+// step (w, m, v): stores the new ones, returns the new parameter.
+__device__ __forceinline__ float adam_step(const AdamArgs &a, long long i, float gr, float w, float m, float v)
 {
-    return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+    constexpr float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    const float mi = b1 * m + (1.f - b1) * gr;
+    const float vi = b2 * v + (1.f - b2) * gr * gr;
+    a.m[i] = mi;
+    a.v[i] = vi;
+    const float wi = w - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + eps);
+    a.w[i] = wi;
+    return wi;
 }
 
-__device__ __forceinline__ void mma_bf16(float d[4], const uint32_t a[4], const uint32_t b[2])
+enum GemmKind {
+    kOpNone = 0,
+    kOpForward,   // z = H W^T + b; Z = z, next H = act(z) (BF16)
+    kOpOutput,    // z = H W^T + b; Z = z
+    kOpLoss,      // z = H W^T + b; dz = 2 (z - y) / (rows x columns), the loss summed
+    kOpBackward,  // dz' = (dZ W) GELU'(Z')
+    kOpWeights,   // g = dZ^T H: the gradient, or Adam's update with it
+    kOpBias       // g = column sums of dZ: likewise
+};
+
+// One GEMM (or bias sum) of a launch.  A, B: BF16, row strides lda / ldb multiples of 16,
+// columns from the true width to the stride zero.
+struct GemmOp {
+    int kind, blocks;     // thread blocks of the op
+    int M, N, R;          // output rows and columns, terms of the reduction
+    const bf16 *A, *B;
+    int lda, ldb;
+    int Brows;            // rows of B in memory (weights: padded with zero rows)
+    const float *bias;
+    float *Z;             // forward: pre-activations out; backward: those of the layer before, in
+    int ldz;
+    bf16 *H;              // forward: next activations, row stride ldh
+    int ldh;
+    float *dZf;           // dz in FP32 (row stride ldd) and BF16
+    bf16 *dZb;
+    int ldd;
+    const float *Y;       // loss: targets, rows by `rows` (nullptr: in order)
+    const int *rows;
+    float *loss;
+    long long param;      // weights / bias: index of the first parameter
+    float *grad;          // the gradient array, or nullptr: update the parameters
+    bf16 *wpk;            // padded BF16 weights (row stride ldw) refreshed by the update
+    int ldw;
+};
+
+constexpr int kMaxOps = 4;
+struct GemmLaunch {
+    GemmOp op[kMaxOps];
+    AdamArgs adam;
+};
+
+__device__ __forceinline__ void mma_bf16(float d[4], const uint32_t a[4], uint32_t b0, uint32_t b1)
 {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                  "{%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// 128 threads: four warps, each a 32 x 32 part of the 64 x 64 block tile (2 x 4 mma
-// tiles of 16 x 8).  Fragment layout of m16n8k16 (g = lane / 4, t = lane % 4):
-// A rows g / g+8, columns 2t, 2t+1 / 2t+8, 2t+9; B rows 2t, 2t+1 / 2t+8, 2t+9, column g;
-// C rows g / g+8, columns 2t, 2t+1.
-__global__ void __launch_bounds__(128) k_gemm(GemmArgs g)
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(uint32_t r[4], uint32_t addr)
 {
-    __shared__ bf16 As[kTile][kTileK + 8];
-    __shared__ bf16 Bs[kTileK][kTile + 8];
+    if (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+// 16 bytes to shared memory, or zeros
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+// A stage of an operand.  KMAJOR: rows mn0 .. mn0 + 31 of the matrix, columns k0 .. k0 + 63
+// (the reduction runs along rows); else rows k0 .. k0 + 63, columns mn0 .. mn0 + 31.  Rows from
+// `rows` on and columns from `ld` on read as zeros.
+template <bool KMAJOR>
+__device__ __forceinline__ void load_operand(uint32_t dst, const bf16 *src, int ld, int rows, int mn0, int k0)
+{
+    constexpr int kChunks = (KMAJOR ? kGemmK : kGemmTile) / 8;   // 16-byte pieces of a row
+#pragma unroll
+    for (int i = 0; i < kGemmTile * kGemmK / 8 / kGemmThreads; i++) {
+        const int e = (int)threadIdx.x + i * kGemmThreads, r = e / kChunks, c = (e % kChunks) * 8;
+        const int row = (KMAJOR ? mn0 : k0) + r, col = (KMAJOR ? k0 : mn0) + c;
+        const bool ok = row < rows && col < ld;
+        cp_async16(dst + r * (KMAJOR ? kGemmPitchK : kGemmPitchN) + c * 2, ok ? src + (long long)row * ld + col : src, ok);
+    }
+}
+
+// acc(i, j) of the block's 32 x 32 tile at (bm, bn); warp w has rows 16 (w / 2), columns
+// 16 (w % 2) of it: acc[0] columns 0-7, acc[1] columns 8-15.
+template <bool A_KMAJOR, bool B_KMAJOR>
+__device__ __forceinline__ void gemm_tile(const GemmOp &g, int a_rows, int b_rows, int bm, int bn, uint32_t smem,
+                                          float acc[2][4])
+{
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gq = lane >> 2, tq = lane & 3;
-    const int bm = blockIdx.y * kTile, bn = blockIdx.x * kTile;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    float acc[2][4][4];
+    const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16;
+    const int steps = (g.R + 15) / 16, chunks = (g.R + kGemmK - 1) / kGemmK;
 #pragma unroll
-    for (int a = 0; a < 2; a++)
+    for (int q = 0; q < 4; q++) acc[0][q] = acc[1][q] = 0.f;
+    auto load = [&](int c) {
+        const uint32_t d = smem + (c % kGemmStages) * 2 * kGemmOperand;
+        load_operand<A_KMAJOR>(d, g.A, g.lda, a_rows, bm, c * kGemmK);
+        load_operand<B_KMAJOR>(d + kGemmOperand, g.B, g.ldb, b_rows, bn, c * kGemmK);
+    };
+    // one commit group a chunk (empty past the end), so the waits below count alike
 #pragma unroll
-        for (int b = 0; b < 4; b++)
+    for (int c = 0; c < kGemmStages - 1; c++) {
+        if (c < chunks) load(c);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const int l7 = lane & 7, l8 = (lane >> 3) & 1, l16 = lane >> 4;
+    for (int c = 0; c < chunks; c++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kGemmStages - 2) : "memory");
+        __syncthreads();   // chunk c has landed for every thread, and chunk c - 1 is used up
+        if (c + kGemmStages - 1 < chunks) load(c + kGemmStages - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const uint32_t sa = smem + (c % kGemmStages) * 2 * kGemmOperand, sb = sa + kGemmOperand;
+        const int n = min(kGemmK / 16, steps - c * (kGemmK / 16));
 #pragma unroll
-            for (int q = 0; q < 4; q++) acc[a][b][q] = 0.f;
-    const bf16 zero = __float2bfloat16(0.f);
-    for (int r0 = 0; r0 < g.R; r0 += kTileK) {
-        // consecutive threads read consecutive addresses: the index with stride 1 varies fastest
-        for (int e = threadIdx.x; e < kTile * kTileK; e += 128) {
-            const bool r_fast = g.sa_r == 1;
-            const int i = r_fast ? e / kTileK : e % kTile, r = r_fast ? e % kTileK : e / kTile;
-            const int gi = bm + i, gr = r0 + r;
-            As[i][r] = (gi < g.M && gr < g.R) ? g.A[gi * g.sa_i + gr * g.sa_r] : zero;
-        }
-        for (int e = threadIdx.x; e < kTileK * kTile; e += 128) {
-            const bool j_fast = g.sb_j == 1;
-            const int r = j_fast ? e / kTile : e % kTileK, j = j_fast ? e % kTile : e / kTileK;
-            const int gr = r0 + r, gj = bn + j;
-            Bs[r][j] = (gr < g.R && gj < g.N) ? g.B[gr * g.sb_r + gj * g.sb_j] : zero;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++) {
-            const int row = wm + mt * 16;
-            uint32_t a[4];
-            a[0] = pack2(As[row + gq][2 * tq], As[row + gq][2 * tq + 1]);
-            a[1] = pack2(As[row + gq + 8][2 * tq], As[row + gq + 8][2 * tq + 1]);
-            a[2] = pack2(As[row + gq][2 * tq + 8], As[row + gq][2 * tq + 9]);
-            a[3] = pack2(As[row + gq + 8][2 * tq + 8], As[row + gq + 8][2 * tq + 9]);
-#pragma unroll
-            for (int nt = 0; nt < 4; nt++) {
-                const int col = wn + nt * 8;
-                uint32_t b[2];
-                b[0] = pack2(Bs[2 * tq][col + gq], Bs[2 * tq + 1][col + gq]);
-                b[1] = pack2(Bs[2 * tq + 8][col + gq], Bs[2 * tq + 9][col + gq]);
-                mma_bf16(acc[mt][nt], a, b);
+        for (int k = 0; k < kGemmK / 16; k++) {
+            if (k < n) {
+                uint32_t a[4], b[4];
+                if (A_KMAJOR) ldmatrix4<false>(a, sa + (wm + l7 + 8 * l8) * kGemmPitchK + (16 * k + 8 * l16) * 2);
+                else ldmatrix4<true>(a, sa + (16 * k + l7 + 8 * l16) * kGemmPitchN + (wm + 8 * l8) * 2);
+                if (B_KMAJOR) ldmatrix4<false>(b, sb + (wn + l7 + 8 * l16) * kGemmPitchK + (16 * k + 8 * l8) * 2);
+                else ldmatrix4<true>(b, sb + (16 * k + l7 + 8 * l8) * kGemmPitchN + (wn + 8 * l16) * 2);
+                mma_bf16(acc[0], a, b[0], b[1]);
+                mma_bf16(acc[1], a, b[2], b[3]);
             }
+        }
+    }
+}
+
+// Column sums of dZ in row order: the block's rows staged in shared memory, then one
+// thread a column adds them.
+__device__ __forceinline__ void bias_block(const GemmOp &g, const AdamArgs &adam, int block, float *stage)
+{
+    const int j0 = block * kBiasCols, t = threadIdx.x;
+    const bool mine = t < kBiasCols && j0 + t < g.N;
+    const long long p = g.param + j0 + t;
+    float s = 0.f, w = 0.f, mm = 0.f, v = 0.f;
+    if (mine && !g.grad) {
+        w = adam.w[p];
+        mm = adam.m[p];
+        v = adam.v[p];
+    }
+    for (int i0 = 0; i0 < g.M; i0 += kBiasRows) {
+        const int rows = min(kBiasRows, g.M - i0);
+        for (int e = t; e < rows * (kBiasCols / 4); e += kGemmThreads) {
+            const int r = e / (kBiasCols / 4), c = e % (kBiasCols / 4) * 4;
+            cp_async16(smem_u32(stage + r * kBiasCols + c), g.dZf + (long long)(i0 + r) * g.ldd + j0 + c, true);
+        }
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (t < kBiasCols) {
+#pragma unroll 32
+            for (int r = 0; r < rows; r++) s += stage[r * kBiasCols + t];
         }
         __syncthreads();
     }
+    if (mine) {
+        if (g.grad) g.grad[p] = s;
+        else adam_step(adam, p, s, w, mm, v);
+    }
+}
+
+__global__ void __launch_bounds__(kGemmThreads) k_gemm(const __grid_constant__ GemmLaunch l)
+{
+    __shared__ __align__(16) uint8_t smem[kGemmSmem];
+    int block = blockIdx.x, o = 0;
+    while (block >= l.op[o].blocks) block -= l.op[o++].blocks;
+    const GemmOp &g = l.op[o];
+    if (g.kind == kOpBias) {
+        bias_block(g, l.adam, block, reinterpret_cast<float *>(smem));
+        return;
+    }
+    const int nb = (g.N + kGemmTile - 1) / kGemmTile;
+    const int bm = block / nb * kGemmTile, bn = block % nb * kGemmTile;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i0 = bm + (warp >> 1) * 16 + (lane >> 2), j0 = bn + (warp & 1) * 16 + 2 * (lane & 3);
+    // what the epilogue reads of its eight outputs, on its way while the products run
+    // (output e: row i0 + 8 ((e / 2) % 2), column j0 + 8 (e / 4) + e % 2)
+    float x0[8], x1[8], x2[8];
 #pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int i = bm + wm + mt * 16 + gq + (q >= 2 ? 8 : 0);
-                const int j = bn + wn + nt * 8 + 2 * tq + (q & 1);
-                if (i >= g.M || j >= g.N) continue;
-                const float v = acc[mt][nt][q];
-                const long long o = (long long)i * g.N + j;
-                if (g.mode == kStoreF32) {
-                    g.C[(long long)i * g.ldc + j] = v;
-                } else if (g.mode == kForward) {
-                    const float z = v + g.bias[j];
-                    g.Z[o] = z;
-                    g.H[o] = __float2bfloat16(g.gelu ? gelu(z) : z);
-                } else {
-                    const float dz = v * gelu_grad(g.Zprev[o]);
-                    g.dZf[o] = dz;
-                    g.dZb[o] = __float2bfloat16(dz);
-                }
+    for (int e = 0; e < 8; e++) {
+        const int i = i0 + 8 * ((e >> 1) & 1), j = j0 + 8 * (e >> 2) + (e & 1);
+        x0[e] = x1[e] = x2[e] = 0.f;
+        if (i >= g.M || j >= g.N) continue;
+        if (g.kind == kOpBackward) {
+            x0[e] = g.Z[(long long)i * g.ldz + j];
+        } else if (g.kind == kOpWeights) {
+            if (!g.grad) {
+                const long long p = g.param + (long long)i * g.N + j;
+                x0[e] = l.adam.w[p];
+                x1[e] = l.adam.m[p];
+                x2[e] = l.adam.v[p];
             }
+        } else {
+            x0[e] = g.bias[j];
+            if (g.kind == kOpLoss) x1[e] = g.Y[(g.rows ? (long long)g.rows[i] : i) * g.N + j];
+        }
+    }
+    float acc[2][4];
+    if (g.kind == kOpWeights) gemm_tile<false, false>(g, g.R, g.R, bm, bn, smem_u32(smem), acc);
+    else if (g.kind == kOpBackward) gemm_tile<true, false>(g, g.M, g.Brows, bm, bn, smem_u32(smem), acc);
+    else gemm_tile<true, true>(g, g.M, g.Brows, bm, bn, smem_u32(smem), acc);
+    const float scale = 2.f / (float)((long long)g.M * g.N);
+    float part = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const int i = i0 + 8 * ((e >> 1) & 1), j = j0 + 8 * (e >> 2) + (e & 1);
+        if (i >= g.M || j >= g.N) continue;
+        const float v = acc[e >> 2][e & 3];
+        if (g.kind == kOpForward) {
+            const float z = v + x0[e];
+            g.Z[(long long)i * g.ldz + j] = z;
+            g.H[(long long)i * g.ldh + j] = __float2bfloat16(gelu(z));
+        } else if (g.kind == kOpOutput) {
+            g.Z[(long long)i * g.ldz + j] = v + x0[e];
+        } else if (g.kind == kOpLoss) {
+            const float d = v + x0[e] - x1[e];
+            part += d * d;
+            g.dZf[(long long)i * g.ldd + j] = scale * d;
+            g.dZb[(long long)i * g.ldd + j] = __float2bfloat16(scale * d);
+        } else if (g.kind == kOpBackward) {
+            const float dz = v * gelu_grad(x0[e]);
+            g.dZf[(long long)i * g.ldd + j] = dz;
+            g.dZb[(long long)i * g.ldd + j] = __float2bfloat16(dz);
+        } else {
+            const long long p = g.param + (long long)i * g.N + j;
+            if (g.grad) g.grad[p] = v;
+            else g.wpk[(long long)i * g.ldw + j] = __float2bfloat16(adam_step(l.adam, p, v, x0[e], x1[e], x2[e]));
+        }
+    }
+    if (g.kind == kOpLoss) {
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o2);
+        if (lane == 0) atomicAdd(g.loss, part / (float)((long long)g.M * g.N));
+    }
 }
 
 // ---------------------------------------------------------------- tcgen05 inference
@@ -223,8 +380,6 @@ constexpr int kUmmaSmem = kUmmaBarBytes + kUmmaBiasBytes + kUmmaMaxN * kUmmaMaxK
 constexpr int kUmmaEpiWarps = 8;               // epilogue warps: two per lane quarter
 constexpr long long kUmmaSpin = 1ll << 22;     // polls of an mbarrier before a wait gives up
 static_assert(kUmmaSmem <= 227 * 1024, "the tcgen05 layer needs more shared memory than a CTA has");
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // two FP32 lanes in one 64-bit register, for the paired FP32 instructions (f32x2)
 __device__ __forceinline__ uint64_t f2(float lo, float hi)
@@ -799,15 +954,13 @@ __global__ void k_bias_sum(const float *const *b, int members, int n, float *out
     }
 }
 
-// Zero-padded BF16 copies for the tcgen05 path: src rows x cols (row stride cols) ->
-// dst prow x pcol.
-__global__ void k_pad_bf16(const bf16 *src, int rows, int cols, bf16 *dst, int prow, int pcol)
+// FP32 rows x cols (from src, contiguous rows) -> BF16 at dst, row stride ld (round to
+// nearest even); the rest of a row is left as it is.
+__global__ void k_weights_bf16(const float *src, int rows, int cols, bf16 *dst, int ld)
 {
-    const long long n = (long long)prow * pcol;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(i / pcol), c = (int)(i % pcol);
-        dst[i] = (r < rows && c < cols) ? src[(long long)r * cols + c] : __float2bfloat16(0.f);
-    }
+    const long long n = (long long)rows * cols;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        dst[i / cols * ld + i % cols] = __float2bfloat16(src[i]);
 }
 
 // The tcgen05 path's input: rows x din FP32 -> rows x kp BF16 (round to nearest even,
@@ -842,77 +995,28 @@ __global__ void k_compact_rows(const float *src, long long lds, float *dst, int 
     }
 }
 
-// rows of the data set -> a BF16 input batch and an FP32 target batch
-__global__ void k_gather(const float *X, const float *Y, const int *idx, int B, int din, int dout, bf16 *Hb,
-                         float *Yb)
+// rows of x in the order idx (nullptr: as they are) -> BF16 rows of stride ld, zeros
+// past din
+__global__ void k_gather(const float *X, const int *idx, int B, int din, bf16 *Hb, int ld)
 {
-    const int row = blockIdx.x;
-    if (row >= B) return;
-    const long long src = idx ? idx[row] : row;
-    for (int c = threadIdx.x; c < din; c += blockDim.x) Hb[(long long)row * din + c] = __float2bfloat16(X[src * din + c]);
-    if (Yb)
-        for (int c = threadIdx.x; c < dout; c += blockDim.x) Yb[(long long)row * dout + c] = Y[src * dout + c];
+    const long long n = (long long)B * ld;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const int row = (int)(i / ld), c = (int)(i % ld);
+        Hb[i] = __float2bfloat16(c < din ? X[(long long)(idx ? idx[row] : row) * din + c] : 0.f);
+    }
 }
 
-// acc = scale z (first) or acc + scale z over rows x cols (row strides lda, cols), the
+// acc = scale z (first) or acc + scale z over rows x cols (row strides lda, ldz), the
 // arithmetic of the tcgen05 layer's accumulating epilogue
-__global__ void k_accumulate(float *acc, long long lda, const float *z, int rows, int cols, float scale, int first)
+__global__ void k_accumulate(float *acc, long long lda, const float *z, int ldz, int rows, int cols, float scale, int first)
 {
     const long long n = (long long)rows * cols;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         float *a = acc + (i / cols) * lda + i % cols;
-        *a = first ? scale * z[i] : fmaf(scale, z[i], *a);
+        const float v = z[i / cols * ldz + i % cols];
+        *a = first ? scale * v : fmaf(scale, v, *a);
     }
-}
-
-// mean squared error over B x dout; gradient of the output layer
-__global__ void k_mse(const float *Z, const float *Y, int B, int dout, float *dZf, bf16 *dZb, float *loss)
-{
-    const long long n = (long long)B * dout;
-    const float scale = 2.f / (float)n;
-    float part = 0.f;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const float d = Z[e] - Y[e];
-        part += d * d;
-        dZf[e] = scale * d;
-        dZb[e] = __float2bfloat16(scale * d);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, part / (float)n);
-}
-
-// db[j] = sum_i dZ[i][j]
-__global__ void k_bias_grad(const float *dZf, int B, int N, float *db)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
-    float s = 0.f;
-    for (int i = 0; i < B; i++) s += dZf[(long long)i * N + j];
-    db[j] = s;
-}
-
-// Adam (Kingma and Ba, 2015) on the FP32 master parameters; refreshes the BF16 copy.
-__global__ void k_adam(float *w, float *m, float *v, const float *grad, bf16 *wb, long long n, float lr, float b1,
-                       float b2, float eps, float c1, float c2)
-{
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float gr = grad[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gr;
-        const float vi = b2 * v[i] + (1.f - b2) * gr * gr;
-        m[i] = mi;
-        v[i] = vi;
-        const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        w[i] = wi;
-        wb[i] = __float2bfloat16(wi);
-    }
-}
-
-__global__ void k_to_bf16(const float *src, bf16 *dst, long long n)
-{
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        dst[i] = __float2bfloat16(src[i]);
 }
 
 thread_local std::string g_mlp_create_error;
@@ -928,24 +1032,23 @@ struct pt_mlp {
     cudaStream_t stream = nullptr;
     // device
     float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;
-    bf16 *wb = nullptr;
+    std::vector<int> ld;        // width[l] to a multiple of 16: the row stride of H, Z and dZ
+    std::vector<bf16 *> wpk;    // BF16 weights of each layer, ld[l + 1] x ld[l], zero outside width[l + 1] x width[l]
     std::vector<bf16 *> H;      // H[0] = input batch, H[l+1] = layer l output (BF16)
     std::vector<float *> Z;     // Z[l] = layer l pre-activation (FP32)
     std::vector<float *> dZf;   // dZ[l] (FP32)
     std::vector<bf16 *> dZb;    // dZ[l] (BF16)
-    float *Ybatch = nullptr, *loss = nullptr;
+    float *loss = nullptr;              // of each step of an epoch (loss_cap)
+    int loss_cap = 0;
     float *X = nullptr, *Y = nullptr;   // data set
+    bf16 *Xe = nullptr;                 // its inputs in the epoch's order, BF16, row stride ld[0]
     int *perm = nullptr;
     int n = 0;
     long long step = 0;
     std::string err;
     std::vector<void *> allocs;
-    // tcgen05 inference: zero-padded BF16 copies of the weights (rows and columns to
-    // multiples of 16), the padded input batch, and a wait error word
+    // tcgen05 inference: the padded input batch and a wait error word
     int use_umma = 1;
-    bool packed_stale = true;
-    std::vector<bf16 *> wpk;
-    std::vector<int> kpad, npad;
     bf16 *h0p = nullptr;
     int *umma_err = nullptr;
     // inference input (FP32 rows copied from the host) and output (the last layer's
@@ -984,92 +1087,136 @@ static cudaError_t dalloc(pt_mlp *m, T **p, size_t count)
     return e;
 }
 
-static cudaError_t gemm(pt_mlp *m, const GemmArgs &g)
+// One launch of up to kMaxOps independent GEMMs.
+static cudaError_t gemm(pt_mlp *m, GemmLaunch &l, int ops)
 {
-    dim3 grid((g.N + kTile - 1) / kTile, (g.M + kTile - 1) / kTile);
-    k_gemm<<<grid, 128, 0, m->stream>>>(g);
+    unsigned blocks = 0;
+    for (int o = 0; o < ops; o++) {
+        GemmOp &g = l.op[o];
+        g.blocks = g.kind == kOpBias ? (g.N + kBiasCols - 1) / kBiasCols
+                                     : ((g.M + kGemmTile - 1) / kGemmTile) * ((g.N + kGemmTile - 1) / kGemmTile);
+        blocks += (unsigned)g.blocks;
+    }
+    if (blocks == 0) return cudaSuccess;
+    k_gemm<<<blocks, kGemmThreads, 0, m->stream>>>(l);
     return cudaGetLastError();
 }
 
-// forward pass over the B rows already in H[0]
-static cudaError_t forward(pt_mlp *m, int B)
+// forward pass over the B rows at h0 (BF16, row stride ld[0]).  With Y, the last layer forms
+// the loss (added to *loss) and its gradient dZ against the targets, rows by `rows`;
+// without, it leaves its outputs in Z.
+static cudaError_t forward(pt_mlp *m, int B, const bf16 *h0, const float *Y = nullptr, const int *rows = nullptr,
+                           float *loss = nullptr)
 {
     for (int l = 0; l < m->L; l++) {
-        const int din = m->width[l], dout = m->width[l + 1];
-        GemmArgs g{};
-        g.A = m->H[l];
-        g.sa_i = din;
-        g.sa_r = 1;
-        g.B = m->wb + m->woff[l];   // B(r, j) = W_l[j][r]
-        g.sb_r = 1;
-        g.sb_j = din;
+        const bool last = l + 1 == m->L;
+        GemmLaunch gl = {};
+        GemmOp &g = gl.op[0];
+        g.kind = !last ? kOpForward : (Y ? kOpLoss : kOpOutput);
+        g.A = l == 0 ? h0 : m->H[l];
+        g.lda = m->ld[l];
+        g.B = m->wpk[l];   // B(r, j) = W_l[j][r]
+        g.ldb = m->ld[l];
+        g.Brows = m->ld[l + 1];
         g.M = B;
-        g.N = dout;
-        g.R = din;
-        g.mode = kForward;
+        g.N = m->width[l + 1];
+        g.R = m->width[l];
         g.bias = m->w + m->boff[l];
         g.Z = m->Z[l];
+        g.ldz = m->ld[l + 1];
         g.H = m->H[l + 1];
-        g.gelu = l + 1 < m->L;
-        cudaError_t e = gemm(m, g);
+        g.ldh = m->ld[l + 1];
+        g.dZf = m->dZf[l];
+        g.dZb = m->dZb[l];
+        g.ldd = m->ld[l + 1];
+        g.Y = Y;
+        g.rows = rows;
+        g.loss = loss;
+        cudaError_t e = gemm(m, gl, 1);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
-// loss and gradients of every parameter for the B rows in H[0] / Ybatch
-static cudaError_t backward(pt_mlp *m, int B)
+// gradients of every parameter for the B rows at h0 whose forward pass has run: into
+// `grad`, or (nullptr) straight into Adam's update.  Layer l's weights are updated one
+// launch after the last product that reads them.
+static cudaError_t backward(pt_mlp *m, int B, const bf16 *h0, float *grad, const AdamArgs &adam)
 {
-    const int Lz = m->L - 1;
-    cudaError_t e = cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream);
-    if (e != cudaSuccess) return e;
-    k_mse<<<std::min(1024, (B * m->width[m->L] + 255) / 256), 256, 0, m->stream>>>(
-        m->Z[Lz], m->Ybatch, B, m->width[m->L], m->dZf[Lz], m->dZb[Lz], m->loss);
-    for (int l = Lz; l >= 0; l--) {
-        const int din = m->width[l], dout = m->width[l + 1];
-        // dW_l[j][k] = sum_i dZ_l[i][j] H_l[i][k]
-        GemmArgs gw{};
-        gw.A = m->dZb[l];
-        gw.sa_i = 1;
-        gw.sa_r = dout;
-        gw.B = m->H[l];
-        gw.sb_r = din;
-        gw.sb_j = 1;
-        gw.M = dout;
-        gw.N = din;
-        gw.R = B;
-        gw.mode = kStoreF32;
-        gw.C = m->grad + m->woff[l];
-        gw.ldc = din;
-        e = gemm(m, gw);
-        if (e != cudaSuccess) return e;
-        k_bias_grad<<<(dout + 127) / 128, 128, 0, m->stream>>>(m->dZf[l], B, dout, m->grad + m->boff[l]);
-        if (l > 0) {
-            // dZ_{l-1}[i][k] = (sum_j dZ_l[i][j] W_l[j][k]) GELU'(Z_{l-1}[i][k])
-            GemmArgs gd{};
-            gd.A = m->dZb[l];
-            gd.sa_i = dout;
-            gd.sa_r = 1;
-            gd.B = m->wb + m->woff[l];
-            gd.sb_r = din;
-            gd.sb_j = 1;
-            gd.M = B;
-            gd.N = din;
-            gd.R = dout;
-            gd.mode = kBackward;
-            gd.Zprev = m->Z[l - 1];
-            gd.dZf = m->dZf[l - 1];
-            gd.dZb = m->dZb[l - 1];
-            e = gemm(m, gd);
-            if (e != cudaSuccess) return e;
+    auto weights = [&](GemmOp &g, int l) {   // dW_l[j][k] = sum_i dZ_l[i][j] H_l[i][k]
+        g = GemmOp{};
+        g.kind = kOpWeights;
+        g.A = m->dZb[l];
+        g.lda = m->ld[l + 1];
+        g.B = l == 0 ? h0 : m->H[l];
+        g.ldb = m->ld[l];
+        g.M = m->width[l + 1];
+        g.N = m->width[l];
+        g.R = B;
+        g.param = m->woff[l];
+        g.grad = grad;
+        g.wpk = m->wpk[l];
+        g.ldw = m->ld[l];
+    };
+    auto bias = [&](GemmOp &g, int l) {      // db_l[j] = sum_i dZ_l[i][j]
+        g = GemmOp{};
+        g.kind = kOpBias;
+        g.M = B;
+        g.N = m->width[l + 1];
+        g.dZf = m->dZf[l];
+        g.ldd = m->ld[l + 1];
+        g.param = m->boff[l];
+        g.grad = grad;
+    };
+    GemmLaunch gl = {};
+    gl.adam = adam;
+    const int last = m->L - 1;
+    for (int l = last; l >= 1; l--) {
+        // dZ_{l-1}[i][k] = (sum_j dZ_l[i][j] W_l[j][k]) GELU'(Z_{l-1}[i][k])
+        GemmOp &g = gl.op[0];
+        g = GemmOp{};
+        g.kind = kOpBackward;
+        g.A = m->dZb[l];
+        g.lda = m->ld[l + 1];
+        g.B = m->wpk[l];
+        g.ldb = m->ld[l];
+        g.Brows = m->ld[l + 1];
+        g.M = B;
+        g.N = m->width[l];
+        g.R = m->width[l + 1];
+        g.Z = m->Z[l - 1];
+        g.ldz = m->ld[l];
+        g.dZf = m->dZf[l - 1];
+        g.dZb = m->dZb[l - 1];
+        g.ldd = m->ld[l];
+        int ops = 1;
+        if (l < last) {
+            weights(gl.op[ops++], l + 1);
+            bias(gl.op[ops++], l + 1);
         }
+        cudaError_t e = gemm(m, gl, ops);
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    int ops = 0;
+    for (int l = std::min(1, last); l >= 0; l--) {
+        weights(gl.op[ops++], l);
+        bias(gl.op[ops++], l);
+    }
+    return gemm(m, gl, ops);
 }
 
 static int grid_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 4096); }
 
 static int pad16(int x) { return (x + 15) / 16 * 16; }
+
+// the BF16 weights from the FP32 parameters
+static cudaError_t refresh_weights(pt_mlp *m)
+{
+    for (int l = 0; l < m->L; l++)
+        k_weights_bf16<<<grid_for((long long)m->width[l + 1] * m->width[l]), 256, 0, m->stream>>>(
+            m->w + m->woff[l], m->width[l + 1], m->width[l], m->wpk[l], m->ld[l]);
+    return cudaGetLastError();
+}
 
 // The tcgen05 path takes every layer whose padded sizes fit the kernel: inputs and
 // outputs at most 256 wide, hidden widths a multiple of 32.
@@ -1165,12 +1312,11 @@ static cudaError_t ensure_zout(pt_mlp *m)
 // layer accumulates in its epilogue), else forward() and k_accumulate.  *x0 caches the
 // zero-padded BF16 copy of x that the tcgen05 layers read: the first network of an
 // ensemble makes it (into its h0p), the others reuse it.
-// The tcgen05 path's per-network state: padded BF16 weights (re-padded after a
-// parameter change), the padded input buffer and the wait error word.
+// The tcgen05 path's per-network state: the padded input buffer and the wait error word.
 static cudaError_t umma_prepare(pt_mlp *m)
 {
     cudaError_t e = cudaSuccess;
-    if (m->wpk.empty()) {
+    if (!m->h0p) {
         static const cudaError_t attr = [] {
             cudaError_t a = cudaFuncSetAttribute(k_umma_layer<kUmmaEpiWarps>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaSmem);
@@ -1180,26 +1326,11 @@ static cudaError_t umma_prepare(pt_mlp *m)
             return a;
         }();
         if (attr != cudaSuccess) return attr;
-        for (int l = 0; l < m->L; l++) {
-            m->kpad.push_back(pad16(m->width[l]));
-            m->npad.push_back(pad16(m->width[l + 1]));
-            bf16 *p = nullptr;
-            e = dalloc(m, &p, (size_t)m->kpad[l] * m->npad[l]);
-            if (e != cudaSuccess) return e;
-            m->wpk.push_back(p);
+        if (!m->umma_err) {
+            e = dalloc(m, &m->umma_err, 1);
+            if (e == cudaSuccess) e = cudaMemsetAsync(m->umma_err, 0, sizeof(int), m->stream);
         }
-        e = dalloc(m, &m->h0p, (size_t)m->max_batch * m->kpad[0]);
-        if (e == cudaSuccess) e = dalloc(m, &m->umma_err, 1);
-        if (e == cudaSuccess) e = cudaMemsetAsync(m->umma_err, 0, sizeof(int), m->stream);
-        if (e != cudaSuccess) return e;
-        m->packed_stale = true;
-    }
-    if (m->packed_stale) {
-        for (int l = 0; l < m->L; l++)
-            k_pad_bf16<<<grid_for((long long)m->npad[l] * m->kpad[l]), 256, 0, m->stream>>>(
-                m->wb + m->woff[l], m->width[l + 1], m->width[l], m->wpk[l], m->npad[l], m->kpad[l]);
-        m->packed_stale = false;
-        e = cudaGetLastError();
+        if (e == cudaSuccess) e = dalloc(m, &m->h0p, (size_t)m->max_batch * m->ld[0]);
     }
     return e;
 }
@@ -1210,32 +1341,33 @@ static cudaError_t forward_infer(pt_mlp *m, int B, const float *x, const bf16 **
                                  float scale, bool first, bool hidden_only = false)
 {
     if (!m->use_umma || !umma_fits(m)) {
-        k_gather<<<B, 128, 0, m->stream>>>(x, nullptr, nullptr, B, m->width[0], m->width[m->L], m->H[0], nullptr);
-        cudaError_t e = forward(m, B);
-        if (e != cudaSuccess || B == 0) return e;
+        if (B == 0) return cudaSuccess;
+        k_gather<<<grid_for((long long)B * m->ld[0]), 256, 0, m->stream>>>(x, nullptr, B, m->width[0], m->H[0], m->ld[0]);
+        cudaError_t e = forward(m, B, m->H[0]);
+        if (e != cudaSuccess) return e;
         const long long total = (long long)B * m->width[m->L];
         k_accumulate<<<(int)std::min<long long>((total + 255) / 256, 4096), 256, 0, m->stream>>>(
-            y, ldy, m->Z[m->L - 1], B, m->width[m->L], scale, first ? 1 : 0);
+            y, ldy, m->Z[m->L - 1], m->ld[m->L], B, m->width[m->L], scale, first ? 1 : 0);
         return cudaGetLastError();
     }
     cudaError_t e = umma_prepare(m);
     if (e != cudaSuccess) return e;
     if (!*x0) {
-        k_input_bf16<<<grid_for((long long)B * m->kpad[0] / 8), 256, 0, m->stream>>>(x, B, m->width[0], m->h0p,
-                                                                                    m->kpad[0]);
+        k_input_bf16<<<grid_for((long long)B * m->ld[0] / 8), 256, 0, m->stream>>>(x, B, m->width[0], m->h0p,
+                                                                                    m->ld[0]);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         *x0 = m->h0p;
     }
     const int tiles = (B + kUmmaM - 1) / kUmmaM;
     for (int l = 0; l < (hidden_only ? m->L - 1 : m->L); l++) {
-        const int Kp = m->kpad[l], Np = m->npad[l];
+        const int Kp = m->ld[l], Np = m->ld[l + 1];
         const bool last = l + 1 == m->L;
         // one CTA per SM: the full shared-memory request keeps a second one off the SM,
         // so the 512 tensor-memory columns a CTA allocates are always free
         const int grid = std::max(1, std::min(tiles, sm_count_mlp()));
         const bf16 *A = l == 0 ? *x0 : m->H[l];
-        const long long lda = l == 0 ? m->kpad[0] : m->width[l];
+        const long long lda = m->ld[l];
         const bool sw = Kp % 64 == 0;   // the 128-byte swizzled layout: whole 128-byte box rows
         CUtensorMap ma, mw;
         if (!operand_map(&ma, A, B, Kp, lda, kUmmaM, sw) || !operand_map(&mw, m->wpk[l], Np, Kp, Kp, Np, sw))
@@ -1272,7 +1404,7 @@ static bool mean_layer_fits(pt_mlp *const *members, int count)
 static cudaError_t mean_layer(pt_mlp *const *members, int count, int B, float *y, int ldy, cudaStream_t s)
 {
     pt_mlp *m = members[0];
-    const int L = m->L, kh = m->width[L - 1], N = m->width[L], np = pad16(N);
+    const int L = m->L, kh = m->width[L - 1], N = m->width[L], np = m->ld[L];
     const size_t need = (size_t)np * kh * count;
     cudaError_t e = cudaSuccess;
     if (!m->mean_ptrs) e = dalloc(m, &m->mean_ptrs, 2 * kMeanMaxMembers);
@@ -1356,6 +1488,7 @@ pt_status pt_mlp_create(int layers, const int *widths, int max_batch, uint64_t s
     m->width.assign(widths, widths + layers + 1);
     m->max_batch = max_batch;
     m->stream = (cudaStream_t)cuda_stream;
+    for (int l = 0; l <= layers; l++) m->ld.push_back(pad16(widths[l]));
     for (int l = 0; l < layers; l++) {
         m->woff.push_back(m->nparam);
         m->nparam += (long long)widths[l + 1] * widths[l];
@@ -1372,19 +1505,26 @@ pt_status pt_mlp_create(int layers, const int *widths, int max_batch, uint64_t s
     const size_t P = (size_t)m->nparam;
     if (bad(dalloc(m, &m->w, P), "parameters") || bad(dalloc(m, &m->m, P), "adam m") ||
         bad(dalloc(m, &m->v, P), "adam v") || bad(dalloc(m, &m->grad, P), "gradients") ||
-        bad(dalloc(m, &m->wb, P), "bf16 weights") || bad(dalloc(m, &m->loss, 1), "loss") ||
-        bad(dalloc(m, &m->Ybatch, (size_t)max_batch * widths[layers]), "targets"))
+        bad(dalloc(m, &m->loss, 1), "loss"))
         return PT_ERR_CUDA;
+    m->loss_cap = 1;
+    // The BF16 buffers' padding columns (and the weights' padding rows) stay zero: they
+    // are cleared here and never written.
+    m->wpk.resize(layers);
     m->H.resize(layers + 1);
     m->Z.resize(layers);
     m->dZf.resize(layers);
     m->dZb.resize(layers);
+    auto zeroed = [&](bf16 **p, size_t n, const char *what) {
+        return bad(dalloc(m, p, n), what) || bad(cudaMemsetAsync(*p, 0, n * sizeof(bf16), m->stream), what);
+    };
     for (int l = 0; l <= layers; l++)
-        if (bad(dalloc(m, &m->H[l], (size_t)max_batch * widths[l]), "activations")) return PT_ERR_CUDA;
+        if (zeroed(&m->H[l], (size_t)max_batch * m->ld[l], "activations")) return PT_ERR_CUDA;
     for (int l = 0; l < layers; l++) {
-        const size_t n = (size_t)max_batch * widths[l + 1];
+        const size_t n = (size_t)max_batch * m->ld[l + 1];
         if (bad(dalloc(m, &m->Z[l], n), "pre-activations") || bad(dalloc(m, &m->dZf[l], n), "gradients") ||
-            bad(dalloc(m, &m->dZb[l], n), "gradients"))
+            zeroed(&m->dZb[l], n, "gradients") ||
+            zeroed(&m->wpk[l], (size_t)m->ld[l + 1] * m->ld[l], "bf16 weights"))
             return PT_ERR_CUDA;
     }
     // He-uniform weights (bound sqrt(6 / fan_in)), zero biases, from a seeded generator
@@ -1413,11 +1553,9 @@ pt_status pt_mlp_set_params(pt_mlp *m, const float *params)
     MCK(cudaMemcpyAsync(m->w, params, bytes, cudaMemcpyHostToDevice, m->stream), "parameters");
     MCK(cudaMemsetAsync(m->m, 0, bytes, m->stream), "adam m");
     MCK(cudaMemsetAsync(m->v, 0, bytes, m->stream), "adam v");
-    k_to_bf16<<<grid_for(m->nparam), 256, 0, m->stream>>>(m->w, m->wb, m->nparam);
-    MCK(cudaGetLastError(), "bf16 weights");
+    MCK(refresh_weights(m), "bf16 weights");
     MCK(cudaStreamSynchronize(m->stream), "sync");
     m->step = 0;
-    m->packed_stale = true;
     return PT_OK;
 }
 
@@ -1432,16 +1570,18 @@ pt_status pt_mlp_get_params(pt_mlp *m, float *params)
 pt_status pt_mlp_set_data(pt_mlp *m, const float *X, const float *Y, int n)
 {
     if (!m || !X || !Y || n < 1) return PT_ERR_ARG;
-    for (void *p : {(void *)m->X, (void *)m->Y, (void *)m->perm}) {
+    for (void *p : {(void *)m->X, (void *)m->Y, (void *)m->Xe, (void *)m->perm}) {
         if (!p) continue;
         cudaFree(p);
         m->allocs.erase(std::remove(m->allocs.begin(), m->allocs.end(), p), m->allocs.end());
     }
     m->X = m->Y = nullptr;
+    m->Xe = nullptr;
     m->perm = nullptr;
     const int din = m->width[0], dout = m->width[m->L];
     MCK(dalloc(m, &m->X, (size_t)n * din), "data");
     MCK(dalloc(m, &m->Y, (size_t)n * dout), "data");
+    MCK(dalloc(m, &m->Xe, (size_t)n * m->ld[0]), "data");
     MCK(dalloc(m, &m->perm, (size_t)n), "data");
     MCK(cudaMemcpyAsync(m->X, X, (size_t)n * din * sizeof(float), cudaMemcpyHostToDevice, m->stream), "data");
     MCK(cudaMemcpyAsync(m->Y, Y, (size_t)n * dout * sizeof(float), cudaMemcpyHostToDevice, m->stream), "data");
@@ -1454,40 +1594,46 @@ pt_status pt_mlp_train(pt_mlp *m, int epochs, int batch, float lr, uint64_t shuf
 {
     if (!m || epochs < 1 || batch < 1 || batch > m->max_batch || !(lr > 0.f)) return PT_ERR_ARG;
     if (!m->X) return mfail(m, PT_ERR_STATE, "pt_mlp_train before pt_mlp_set_data");
-    const int din = m->width[0], dout = m->width[m->L];
+    const int din = m->width[0], steps = (m->n + batch - 1) / batch;
+    if (steps > m->loss_cap) {
+        float *p = nullptr;
+        MCK(dalloc(m, &p, (size_t)steps), "losses");
+        m->loss = p;   // (the smaller one is freed with the network)
+        m->loss_cap = steps;
+    }
     std::vector<int> perm(m->n);
     std::mt19937_64 rng(shuffle_seed);
-    float last = 0.f;
     for (int ep = 0; ep < epochs; ep++) {
         std::iota(perm.begin(), perm.end(), 0);
         std::shuffle(perm.begin(), perm.end(), rng);
         MCK(cudaMemcpyAsync(m->perm, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice, m->stream),
             "permutation");
-        double sum = 0.0;
-        int steps = 0;
-        for (int s0 = 0; s0 < m->n; s0 += batch) {
-            const int B = std::min(batch, m->n - s0);
-            k_gather<<<B, 128, 0, m->stream>>>(m->X, m->Y, m->perm + s0, B, din, dout, m->H[0], m->Ybatch);
-            MCK(forward(m, B), "forward");
-            MCK(backward(m, B), "backward");
+        // the epoch's inputs in its order, and a loss word a step
+        k_gather<<<grid_for((long long)m->n * m->ld[0]), 256, 0, m->stream>>>(m->X, m->perm, m->n, din, m->Xe, m->ld[0]);
+        MCK(cudaGetLastError(), "gather");
+        MCK(cudaMemsetAsync(m->loss, 0, (size_t)steps * sizeof(float), m->stream), "losses");
+        for (int s = 0; s < steps; s++) {
+            const int s0 = s * batch, B = std::min(batch, m->n - s0);
+            const bf16 *h0 = m->Xe + (size_t)s0 * m->ld[0];
+            MCK(forward(m, B, h0, m->Y, m->perm + s0, m->loss + s), "forward");
             m->step++;
-            m->packed_stale = true;
-            const float c1 = 1.f - std::pow(0.9f, (float)m->step), c2 = 1.f - std::pow(0.999f, (float)m->step);
-            k_adam<<<grid_for(m->nparam), 256, 0, m->stream>>>(m->w, m->m, m->v, m->grad, m->wb, m->nparam, lr, 0.9f,
-                                                               0.999f, 1e-8f, c1, c2);
-            MCK(cudaGetLastError(), "adam");
-            if (ep == epochs - 1) {
-                float l = 0.f;
-                MCK(cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream), "loss");
-                MCK(cudaStreamSynchronize(m->stream), "sync");
-                sum += l * B;
-                steps += B;
-            }
+            AdamArgs a;
+            a.w = m->w;
+            a.m = m->m;
+            a.v = m->v;
+            a.lr = lr;
+            a.c1 = 1.f - std::pow(0.9f, (float)m->step);
+            a.c2 = 1.f - std::pow(0.999f, (float)m->step);
+            MCK(backward(m, B, h0, nullptr, a), "backward");
         }
-        if (ep == epochs - 1) last = (float)(sum / std::max(steps, 1));
     }
+    // the last epoch's losses
+    std::vector<float> l(steps);
+    MCK(cudaMemcpyAsync(l.data(), m->loss, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost, m->stream), "losses");
     MCK(cudaStreamSynchronize(m->stream), "sync");
-    if (epoch_loss) *epoch_loss = last;
+    double sum = 0.0;
+    for (int s = 0; s < steps; s++) sum += l[s] * std::min(batch, m->n - s * batch);
+    if (epoch_loss) *epoch_loss = (float)(sum / m->n);
     return PT_OK;
 }
 
@@ -1501,11 +1647,12 @@ pt_status pt_mlp_gradients(pt_mlp *m, const float *X, const float *Y, int n, flo
     if (e == cudaSuccess) e = cudaMemcpyAsync(dX, X, (size_t)n * din * sizeof(float), cudaMemcpyHostToDevice, m->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dY, Y, (size_t)n * dout * sizeof(float), cudaMemcpyHostToDevice, m->stream);
     if (e == cudaSuccess) {
-        k_gather<<<n, 128, 0, m->stream>>>(dX, dY, nullptr, n, din, dout, m->H[0], m->Ybatch);
+        k_gather<<<grid_for((long long)n * m->ld[0]), 256, 0, m->stream>>>(dX, nullptr, n, din, m->H[0], m->ld[0]);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = forward(m, n);
-    if (e == cudaSuccess) e = backward(m, n);
+    if (e == cudaSuccess) e = cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream);
+    if (e == cudaSuccess) e = forward(m, n, m->H[0], dY, nullptr, m->loss);
+    if (e == cudaSuccess) e = backward(m, n, m->H[0], m->grad, AdamArgs{});
     float l = 0.f;
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(grads, m->grad, (size_t)m->nparam * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
