@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -468,10 +469,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const v
     return false;
 }
 
+// (error: host memory, read after the stream has been synchronised)
 __device__ __forceinline__ void umma_fail(volatile int *fail, int *error)
 {
     *fail = 1;
-    atomicExch(error, 1);
+    *(volatile int *)error = 1;
+    __threadfence_system();
 }
 
 // TMA: the box at element coordinates (x, y) of the map into shared memory at dst,
@@ -483,6 +486,26 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
             dst),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
         : "memory");
+}
+
+// One lane of the (whole) warp.  The MMA warps run their loops with every lane and issue
+// under this for a few instructions at a time: the compiler then knows that one thread
+// issues.  Under a plain lane == 0 an MMA takes 140 issue cycles and a commit 410,
+// whatever the MMA's size; this way a 128 x 256 x 16 MMA with a commit every second one
+// takes the 128 it needs.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+
+// A plain bulk copy of `bytes` (a multiple of 16, both ends 16-byte aligned).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
 }
 
 __device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, bool accumulate)
@@ -502,8 +525,8 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 // tcgen05 shared-memory matrix descriptor: start >> 4 (bits 0-13), leading byte offset
 // >> 4 (16-29), stride byte offset >> 4 (32-45), the fixed 0b001 (46-48), base offset 0
 // (49-51, the operands are 1024-byte aligned), the swizzle mode (61-63: 0 none,
-// 2 128-byte).
-constexpr uint32_t kSwizzleNone = 0, kSwizzle128B = 2;
+// 2 128-byte, 4 64-byte).
+constexpr uint32_t kSwizzleNone = 0, kSwizzle128B = 2, kSwizzle64B = 4;
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo, uint32_t swizzle)
 {
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
@@ -544,6 +567,18 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t v[32])
                    "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
                  :
                  : "memory");
+}
+
+// 16 columns, complete on return.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
 }
 
 // The epilogue of one 32-column chunk of a tile row (v: its accumulator values): bias,
@@ -702,29 +737,25 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MMA issuer
-            bool ok = mbar_wait(b_w, 0, fail);
+        // MMA issuer (every lane; elect_one issues)
+        bool ok = mbar_wait(b_w, 0, fail);
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t idesc = umma_idesc(kUmmaM, Np);
+        int it = 0, tc = 0;
+        for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, tc++) {
+            const int b = tc & 1, use = tc >> 1;
+            ok = __all_sync(0xffffffffu, ok && (use == 0 || mbar_wait(b_acce + 8 * b, (use - 1) & 1, fail)));
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t idesc = umma_idesc(kUmmaM, Np);
-            int it = 0, tc = 0;
-            for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, tc++) {
-                const int b = tc & 1, use = tc >> 1;
-                if (use > 0 && !mbar_wait(b_acce + 8 * b, (use - 1) & 1, fail)) {
-                    ok = false;
-                    break;
-                }
+            const uint32_t d = tmem + 256u * b;
+            for (int ks = 0; ks < nks; ks++, it++) {
+                const int s = it % kUmmaStages, u = it / kUmmaStages;
+                ok = __all_sync(0xffffffffu, mbar_wait(b_full + 8 * s, u & 1, fail));
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                const uint32_t d = tmem + 256u * b;
-                for (int ks = 0; ks < nks; ks++, it++) {
-                    const int s = it % kUmmaStages, u = it / kUmmaStages;
-                    if (!mbar_wait(b_full + 8 * s, u & 1, fail)) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;");
-                    const int k0 = ks * KS, kc = min(KS, Kp - k0);
-                    const uint32_t a0 = sA_u + s * kUmmaStageBytes;
+                const int k0 = ks * KS, kc = min(KS, Kp - k0);
+                const uint32_t a0 = sA_u + s * kUmmaStageBytes;
+                if (elect_one()) {
                     for (int j = 0; j < kc / 16; j++) {
                         const int g = k0 / 16 + j;   // the MMA step within K
                         uint64_t ad, wd;
@@ -738,15 +769,16 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
                         umma_bf16(d, ad, wd, idesc, (ks | j) != 0);
                     }
                     umma_commit(b_empty + 8 * s);   // the stage is free once these MMAs complete
+                    if (ks == nks - 1) umma_commit(b_accf + 8 * b);
                 }
-                if (!ok) break;
-                umma_commit(b_accf + 8 * b);
+                __syncwarp();
             }
-            if (!ok) umma_fail(fail, error);
-            // every MMA issued completes before the tensor memory is freed
-            umma_commit(b_drain);
-            mbar_wait(b_drain, 0, nullptr);
         }
+        if (!ok && lane == 0) umma_fail(fail, error);
+        // every MMA issued completes before the tensor memory is freed
+        if (elect_one()) umma_commit(b_drain);
+        __syncwarp();
+        mbar_wait(b_drain, 0, nullptr);
         __syncwarp();
     } else {
         // epilogue: lanes (tile rows) 32 q .. 32 q + 31, 32-column chunks part, part + EPI / 4, ...
@@ -781,33 +813,333 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
 
+// ---------------------------------------------------------------- fused hidden layers
+// All hidden layers of one or more networks of a shape, activations kept on chip.  A
+// layer-by-layer launch writes and reads 0.5 KB of activations per row and layer, which
+// bounds it by DRAM (50 us a layer of 262,144 rows against 40 for the copies alone); here
+// a row's activations leave the SM once, after the last hidden layer.  A persistent CTA
+// takes items (a network and a tile of 128 rows) two at a time, X and Y, each with its
+// activations in shared memory (64 KB, the MMA's A operand) and a 128 x 256 FP32
+// accumulator in tensor memory, and works through X's layer 0, Y's layer 0, X's layer 1
+// and so on: a layer's MMAs need the whole epilogue before it, so Y's MMAs run beside X's
+// epilogue and the other way round.
+//   warp 0      producer: an item's inputs and, for each step (a layer of X or Y), the layer's
+//               weight slices of 32 K columns (16 KB) from L2 through a ring of kNetStages
+//   warp 1      MMA issuer
+//   warps 2-17  epilogue: bias, GELU, the next layer's activations (to shared memory in
+//               the operand layout; the last layer's to global memory)
+// Barriers: full / empty per stage; per item slot (X, Y) x: the inputs have landed, acc: the
+// layer's MMAs are done, a: its epilogue is (activations stored, accumulator drained).
+// Every wait is bounded, as in k_umma_layer.  The order of the MMAs into an accumulator is
+// that of k_umma_layer, and so are the results, bit for bit.  262,144 rows through 11-256-
+// 256-256-222 take 764 us with it, 607 of them here, against 1,031 layer by layer (GB300);
+// 32 rows 65 us instead of 220.  Bound by the weight slices, 27 bytes a clock and SM from
+// L2 with every SM reading, and then by the epilogue's GELUs.
+constexpr int kNetStages = 6, kNetK = 32, kNetStageBytes = kUmmaMaxN * kNetK * 2, kNetTileBytes = kUmmaM * kUmmaMaxK * 2;
+constexpr int kNetBarBytes = 1024;
+constexpr int kNetSmem = kNetBarBytes + 2 * kNetTileBytes + kNetStages * kNetStageBytes;
+constexpr int kNetEpiWarps = 16, kNetThreads = 32 * (2 + kNetEpiWarps);
+constexpr int kNetMaxMembers = 8;
+static_assert(kNetSmem <= 227 * 1024, "the fused layers need more shared memory than a CTA has");
+
+struct NetShape {
+    int M, kp0, hid, layers, members;   // rows, padded inputs, hidden width, hidden layers, networks
+    int sw0;                            // the input layer's operands are swizzled (kp0 a multiple of 64)
+    int slots;                          // items a CTA takes at a time: 1 or 2
+    const bf16 *w0, *w;                 // the networks' weight slices (PackArgs)
+    const float *bias;                  // members x layers x hid
+    bf16 *out[kNetMaxMembers];          // each network's last hidden activations, M x hid
+    int *error;
+};
+
+__global__ void __launch_bounds__(kNetThreads, 1)
+    k_umma_hidden(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ NetShape n)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const uint32_t b_full = smem_u32(smem), b_empty = b_full + 8 * kNetStages, b_x = b_empty + 8 * kNetStages,
+                   b_acc = b_x + 16, b_a = b_acc + 16, b_drain = b_a + 16;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 512);
+    volatile int *fail = reinterpret_cast<volatile int *>(smem + 576);
+    const uint32_t sA_u = smem_u32(smem + kNetBarBytes), sW_u = sA_u + 2 * kNetTileBytes;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (threadIdx.x == 32) {
+        for (int i = 0; i < kNetStages; i++) {
+            mbar_init(b_full + 8 * i, 1);
+            mbar_init(b_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(b_x + 8 * i, 1);
+            mbar_init(b_acc + 8 * i, 1);
+            mbar_init(b_a + 8 * i, kNetEpiWarps);
+        }
+        mbar_init(b_drain, 1);
+        *fail = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = *tmem_slot;
+    const int items = (n.M + kUmmaM - 1) / kUmmaM * n.members;   // item i: row tile i / members of network i % members
+    const int step = (int)gridDim.x * n.slots;
+    if (warp == 0) {
+        if (lane == 0) {
+            bool ok = true;
+            int it = 0, seen[2] = {0, 0};   // stage fills; items of each slot
+            for (int i0 = blockIdx.x * n.slots; ok && i0 < items; i0 += step) {
+                const int here = min(n.slots, items - i0);
+                for (int l = 0; ok && l < n.layers; l++)
+                    for (int t = 0; ok && t < here; t++) {
+                        const int m = (i0 + t) % n.members;
+                        if (l == 0) {
+                            // the slot's buffer is free once its last item's last MMAs have read it
+                            if (seen[t] > 0 && !mbar_wait(b_acc + 8 * t, (seen[t] * n.layers - 1) & 1, fail)) {
+                                ok = false;
+                                break;
+                            }
+                            seen[t]++;
+                            const int bw = n.sw0 ? 64 : 8, row = (i0 + t) / n.members * kUmmaM;
+                            mbar_expect_tx(b_x + 8 * t, (uint32_t)(kUmmaM * n.kp0 * 2));
+                            for (int c = 0; c < n.kp0 / bw; c++)
+                                tma_load_2d(sA_u + t * kNetTileBytes + c * kUmmaM * bw * 2, &tmX, bw * c, row, b_x + 8 * t);
+                        }
+                        // the layer's slices lie in memory as they do in a stage
+                        const int K = l == 0 ? n.kp0 : n.hid;
+                        const bf16 *src = l == 0 ? n.w0 + (size_t)m * n.kp0 * n.hid
+                                                 : n.w + (size_t)(m * (n.layers - 1) + l - 1) * n.hid * n.hid;
+                        for (int k0 = 0; k0 < K; k0 += kNetK, it++) {
+                            const int st = it % kNetStages, use = it / kNetStages;
+                            if (use > 0 && !mbar_wait(b_empty + 8 * st, (use - 1) & 1, fail)) {
+                                ok = false;
+                                break;
+                            }
+                            const uint32_t bytes = (uint32_t)(min(kNetK, K - k0) * n.hid * 2);
+                            mbar_expect_tx(b_full + 8 * st, bytes);
+                            bulk_load(sW_u + st * kNetStageBytes, src + (size_t)k0 * n.hid, bytes, b_full + 8 * st);
+                        }
+                    }
+            }
+            if (!ok) umma_fail(fail, n.error);
+            // every copy lands before the CTA ends: the last fill of each stage, the last inputs
+            for (int st = 0; st < kNetStages; st++) {
+                const int uses = it / kNetStages + (st < it % kNetStages ? 1 : 0);
+                if (uses > 0) mbar_wait(b_full + 8 * st, (uses - 1) & 1, nullptr);
+            }
+            for (int t = 0; t < 2; t++)
+                if (seen[t] > 0) mbar_wait(b_x + 8 * t, (seen[t] - 1) & 1, nullptr);
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // (every lane; elect_one issues)
+        bool ok = true;
+        const uint32_t idesc = umma_idesc(kUmmaM, n.hid);
+        int it = 0, seen[2] = {0, 0}, done[2] = {0, 0};   // stages; items and layers of each slot
+        for (int i0 = blockIdx.x * n.slots; ok && i0 < items; i0 += step) {
+            const int here = min(n.slots, items - i0);
+            for (int l = 0; ok && l < n.layers; l++)
+                for (int t = 0; ok && t < here; t++) {
+                    // the layer's activations (or inputs), and a drained accumulator
+                    ok = __all_sync(0xffffffffu, (done[t] == 0 || mbar_wait(b_a + 8 * t, (done[t] - 1) & 1, fail)) &&
+                                                     (l > 0 || mbar_wait(b_x + 8 * t, seen[t] & 1, fail)));
+                    if (!ok) break;
+                    done[t]++;
+                    if (l == 0) seen[t]++;
+                    const int K = l == 0 ? n.kp0 : n.hid;
+                    const uint32_t a0 = sA_u + t * kNetTileBytes, d = tmem + 256u * t;
+                    for (int k0 = 0; k0 < K; k0 += kNetK, it++) {
+                        const int st = it % kNetStages;
+                        ok = __all_sync(0xffffffffu, mbar_wait(b_full + 8 * st, (it / kNetStages) & 1, fail));
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;");
+                        const uint32_t w0 = sW_u + st * kNetStageBytes;
+                        if (elect_one()) {
+#pragma unroll
+                            for (int j = 0; j < kNetK / 16; j++) {
+                                if (k0 + 16 * j >= K) break;
+                                const int g = k0 / 16 + j;   // the MMA step within K
+                                uint64_t ad, wd;
+                                if (l > 0 || n.sw0) {
+                                    ad = umma_desc(a0 + (g >> 2) * kUmmaM * 128 + 32 * (g & 3), 16, 1024, kSwizzle128B);
+                                    wd = umma_desc(w0 + 32 * j, 16, 512, kSwizzle64B);
+                                } else {
+                                    ad = umma_desc(a0 + g * 32 * kUmmaM, 16 * kUmmaM, 128, kSwizzleNone);
+                                    wd = umma_desc(w0 + j * 32 * n.hid, 16 * n.hid, 128, kSwizzleNone);
+                                }
+                                umma_bf16(d, ad, wd, idesc, g != 0);
+                            }
+                            umma_commit(b_empty + 8 * st);   // the stage is free once these MMAs complete
+                            if (k0 + kNetK >= K) umma_commit(b_acc + 8 * t);
+                        }
+                        __syncwarp();
+                    }
+                }
+        }
+        if (!ok && lane == 0) umma_fail(fail, n.error);
+        // every MMA issued completes before the tensor memory is freed
+        if (elect_one()) umma_commit(b_drain);
+        __syncwarp();
+        mbar_wait(b_drain, 0, nullptr);
+        __syncwarp();
+    } else {
+        // epilogue: rows 32 q .. 32 q + 31, columns c0 .. c0 + cw - 1
+        const int part = (warp - 2) >> 2, q = warp & 3;
+        const int cw = n.hid / 4, c0 = part * cw;   // 16 to 64, a multiple of 16
+        const int r = 32 * q + lane;
+        int done[2] = {0, 0};
+        bool ok = true;
+        for (int i0 = blockIdx.x * n.slots; ok && i0 < items; i0 += step) {
+            const int here = min(n.slots, items - i0);
+            for (int l = 0; ok && l < n.layers; l++)
+                for (int t = 0; t < here; t++) {
+                    const int m = (i0 + t) % n.members, row = (i0 + t) / n.members * kUmmaM + r;
+                    const float *bias = n.bias + (size_t)(m * n.layers + l) * n.hid + c0;
+                    const bool last = l + 1 == n.layers;
+                    const uint32_t tb = tmem + 256u * t + ((uint32_t)(32 * q) << 16) + c0;
+                    const uint32_t arow = sA_u + t * kNetTileBytes + r * 128;
+                    if (!__all_sync(0xffffffffu, mbar_wait(b_acc + 8 * t, done[t] & 1, fail))) {
+                        ok = false;
+                        break;
+                    }
+                    done[t]++;
+                    asm volatile("tcgen05.fence::after_thread_sync;");
+                    for (int c = 0; c < cw; c += 16) {
+                        float4 bb[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) bb[j] = __ldg(reinterpret_cast<const float4 *>(bias + c) + j);
+                        uint32_t v[16];
+                        __syncwarp();   // tcgen05.ld and its wait are warp-collective
+                        tmem_ld16(tb + (uint32_t)c, v);
+                        uint32_t p[8];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const uint32_t *w = v + 4 * j;
+                            p[2 * j] = gelu_bf16x2(f2_add(f2(__uint_as_float(w[0]), __uint_as_float(w[1])), f2(bb[j].x, bb[j].y)));
+                            p[2 * j + 1] =
+                                gelu_bf16x2(f2_add(f2(__uint_as_float(w[2]), __uint_as_float(w[3])), f2(bb[j].z, bb[j].w)));
+                        }
+                        const int k0 = c0 + c;
+                        if (!last) {
+                            // two 16-byte pieces of the row, where the 128-byte swizzle has them
+                            const uint32_t blk = arow + (uint32_t)(k0 >> 6) * (kUmmaM * 128);
+#pragma unroll
+                            for (int k = 0; k < 2; k++) {
+                                const uint32_t a = blk + (uint32_t)(((((k0 & 63) >> 3) + k) ^ (r & 7)) << 4);
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(p[4 * k]),
+                                             "r"(p[4 * k + 1]), "r"(p[4 * k + 2]), "r"(p[4 * k + 3]) : "memory");
+                            }
+                        } else if (row < n.M) {
+                            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
+                                             n.out[m] + (size_t)row * n.hid + k0),
+                                         "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]), "r"(p[4]), "r"(p[5]), "r"(p[6]),
+                                         "r"(p[7])
+                                         : "memory");
+                        }
+                    }
+                    asm volatile("tcgen05.fence::before_thread_sync;");
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(b_a + 8 * t);
+                }
+        }
+        if (!ok && lane == 0) umma_fail(fail, n.error);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
+// The members' weights side by side: for the mean layer wc (np x members * hid: member
+// m's last weights in columns [m hid, (m + 1) hid)) and the summed last biases; for
+// k_umma_hidden (w0 set) the input layers' weights w0 (members x kp0 hid), the later hidden
+// ones' w (members x (layers - 1) x hid hid) and their biases (members x layers x hid).  The
+// hidden weights lie in slices of 32 K columns, each in the operand layout of its stage, so
+// a slice is one bulk copy of 16 KB: with the 64-byte swizzle row n has 64 bytes, its four 16-byte
+// pieces permuted by n / 2 % 4; without (input widths that are no multiple of 64) groups of
+// eight columns follow each other, 16 bytes a row.
+struct PackArgs {
+    const bf16 *wpk[kNetMaxMembers][16];
+    const float *bias[kNetMaxMembers][16];
+    int members, layers, kp0, hid, np, nout;
+    bf16 *w0, *w, *wc;
+    float *hbias, *bsum;
+};
+
+__global__ void k_pack_members(const __grid_constant__ PackArgs a)
+{
+    const long long stride = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long n0 = (long long)a.hid * a.kp0, nh = (long long)a.hid * a.hid, nc = (long long)a.np * a.hid;
+    if (a.w0) {
+        // element i of a layer with K columns: its row r and column c
+        auto place = [&](int i, int K, bool swizzled) {
+            const int s = i / (kNetK * a.hid), e = i % (kNetK * a.hid);   // slice, element of it
+            const int kc = min(kNetK, K - kNetK * s);
+            int r, c;
+            if (swizzled) {
+                r = e / kNetK;
+                c = ((e % kNetK / 8) ^ (r >> 1 & 3)) * 8 + e % 8;
+            } else {
+                r = e / 8 % a.hid;
+                c = e / (8 * a.hid) * 8 + e % 8;
+            }
+            return (long long)r * K + kNetK * s + min(c, kc - 1);
+        };
+        const bool sw0 = a.kp0 % 64 == 0;
+        for (long long i = first; i < n0 * a.members; i += stride)
+            a.w0[i] = a.wpk[i / n0][0][place((int)(i % n0), a.kp0, sw0)];
+        for (long long i = first; i < nh * a.members * (a.layers - 1); i += stride) {
+            const int k = (int)(i / nh);
+            a.w[i] = a.wpk[k / (a.layers - 1)][1 + k % (a.layers - 1)][place((int)(i % nh), a.hid, true)];
+        }
+        for (long long i = first; i < (long long)a.hid * a.layers * a.members; i += stride) {
+            const int k = (int)(i / a.hid);
+            a.hbias[i] = a.bias[k / a.layers][k % a.layers][i % a.hid];
+        }
+    }
+    for (long long i = first; i < nc * a.members; i += stride) {
+        const long long r = i / ((long long)a.hid * a.members);
+        const int c = (int)(i % ((long long)a.hid * a.members));
+        a.wc[i] = a.wpk[c / a.hid][a.layers][r * a.hid + c % a.hid];
+    }
+    for (long long i = first; i < a.nout; i += stride) {
+        float s = 0.f;
+        for (int m = 0; m < a.members; m++) s += a.bias[m][a.layers][i];
+        a.bsum[i] = s;
+    }
+}
+
 // ---------------------------------------------------------------- ensemble mean layer
 // The members' last layers in one GEMM: y = inv * (sum_m W_m h_m + sum_m b_m), the
-// mean of the members' outputs.  The members' last hidden activations h_m (M x Kh BF16
-// each) are one operand concatenated along K, their weights W_m (Np x Kh) side by
-// side in Wc (Np x members * Kh), so the tensor cores sum over members in the
-// accumulator and the outputs are written once (instead of a read-modify-write of an
-// FP32 accumulator per member).  Wc is too large for shared memory, so every stage of
+// mean of the members' outputs (one member: its outputs).  The members' last hidden
+// activations h_m (M x Kh BF16 each) are one operand concatenated along K, their weights
+// W_m (Np x Kh) side by side in Wc (Np x members * Kh), so the tensor cores sum over
+// members in the accumulator and the outputs are written once, to their rows of N
+// columns: a warp turns its 32 x 32 piece in shared memory, so that each store is 128
+// consecutive bytes.  (Written to padded rows and compacted by a second kernel, 262,144 x
+// 222 outputs cost 70 us more.)  Wc is too large for shared memory, so every stage of
 // the ring carries a 64-column slice of both operands (128-byte swizzled boxes); the
-// roles, accumulators, waits and epilogue are those of k_umma_layer.
-constexpr int kMeanMaxMembers = 8;
-constexpr int kMeanStages = 4;
+// roles, accumulators and waits are those of k_umma_layer.
+constexpr int kMeanStages = 4, kMeanEpiWarps = 8;
 constexpr int kMeanAStage = kUmmaM * 64 * 2;        // 16 KB
 constexpr int kMeanWStage = kUmmaMaxN * 64 * 2;     // 32 KB
-constexpr int kMeanSmem = kUmmaBarBytes + kUmmaBiasBytes + kMeanStages * (kMeanAStage + kMeanWStage);
+constexpr int kMeanTurn = 32 * 32 * 4;              // a warp's piece
+constexpr int kMeanSmem = kUmmaBarBytes + kUmmaBiasBytes + kMeanStages * (kMeanAStage + kMeanWStage) +
+                          kMeanEpiWarps * kMeanTurn;
 static_assert(kMeanSmem <= 227 * 1024, "the ensemble layer needs more shared memory than a CTA has");
 
 struct MeanMaps {
-    CUtensorMap a[kMeanMaxMembers];   // member m's hidden activations, box 64 x kUmmaM, 128-byte swizzle
+    CUtensorMap a[kNetMaxMembers];   // member m's hidden activations, box 64 x kUmmaM, 128-byte swizzle
 };
 
-template <int EPI>
-__global__ void __launch_bounds__(32 * (2 + EPI), 1)
+__global__ void __launch_bounds__(32 * (2 + kMeanEpiWarps), 1)
     k_umma_mean_layer(const __grid_constant__ MeanMaps maps, const __grid_constant__ CUtensorMap tmW, int M, int Kh,
-                      int members, int Np, int N, const float *bias_sum, float inv, float *Y, long long ldy, int vec,
-                      int *error)
+                      int members, int Np, int N, const float *bias_sum, float inv, float *Y, int *error)
 {
-    static_assert(EPI % 4 == 0, "each of the four lane quarters needs the same number of epilogue warps");
+    constexpr int EPI = kMeanEpiWarps;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t b_full = smem_u32(smem), b_empty = b_full + 8 * kMeanStages, b_accf = b_empty + 8 * kMeanStages,
                    b_acce = b_accf + 16, b_drain = b_acce + 16;
@@ -867,44 +1199,44 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MMA issuer: 4 MMAs (K = 16) per 64-column slice
-            bool ok = true;
-            const uint32_t idesc = umma_idesc(kUmmaM, Np);
-            int it = 0, tc = 0;
-            for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, tc++) {
-                const int b = tc & 1, use = tc >> 1;
-                if (use > 0 && !mbar_wait(b_acce + 8 * b, (use - 1) & 1, fail)) {
-                    ok = false;
-                    break;
-                }
+        // MMA issuer (every lane; elect_one issues): 4 MMAs (K = 16) per 64-column slice
+        bool ok = true;
+        const uint32_t idesc = umma_idesc(kUmmaM, Np);
+        int it = 0, tc = 0;
+        for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, tc++) {
+            const int b = tc & 1, use = tc >> 1;
+            ok = __all_sync(0xffffffffu, use == 0 || mbar_wait(b_acce + 8 * b, (use - 1) & 1, fail));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint32_t d = tmem + 256u * b;
+            for (int j = 0; j < nks; j++, it++) {
+                const int s = it % kMeanStages, u = it / kMeanStages;
+                ok = __all_sync(0xffffffffu, mbar_wait(b_full + 8 * s, u & 1, fail));
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                const uint32_t d = tmem + 256u * b;
-                for (int j = 0; j < nks; j++, it++) {
-                    const int s = it % kMeanStages, u = it / kMeanStages;
-                    if (!mbar_wait(b_full + 8 * s, u & 1, fail)) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t a = sA_u + s * stage_bytes, w = a + kMeanAStage;
+                const uint32_t a = sA_u + s * stage_bytes, w = a + kMeanAStage;
+                if (elect_one()) {
+#pragma unroll
                     for (int q = 0; q < 4; q++)
                         umma_bf16(d, umma_desc(a + 32 * q, 16, 1024, kSwizzle128B),
                                   umma_desc(w + 32 * q, 16, 1024, kSwizzle128B), idesc, (j | q) != 0);
                     umma_commit(b_empty + 8 * s);
+                    if (j == nks - 1) umma_commit(b_accf + 8 * b);
                 }
-                if (!ok) break;
-                umma_commit(b_accf + 8 * b);
+                __syncwarp();
             }
-            if (!ok) umma_fail(fail, error);
-            umma_commit(b_drain);
-            mbar_wait(b_drain, 0, nullptr);
         }
+        if (!ok && lane == 0) umma_fail(fail, error);
+        if (elect_one()) umma_commit(b_drain);
+        __syncwarp();
+        mbar_wait(b_drain, 0, nullptr);
         __syncwarp();
     } else {
         // epilogue: y = inv * (acc + sum of the biases), written once
         const int q = warp & 3, part = (warp - 2) >> 2;
         constexpr int parts = EPI / 4;
+        float *const turn = reinterpret_cast<float *>(smem + kUmmaBarBytes + kUmmaBiasBytes +
+                                                      kMeanStages * (kMeanAStage + kMeanWStage) + (warp - 2) * kMeanTurn);
         int tc = 0;
         for (int t = blockIdx.x; t < tiles; t += gridDim.x, tc++) {
             const int b = tc & 1, use = tc >> 1;
@@ -913,14 +1245,24 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
-            const int row = t * kUmmaM + 32 * q + lane;
+            const int row0 = t * kUmmaM + 32 * q;
             const uint32_t tb = tmem + ((uint32_t)(32 * q) << 16) + 256u * b;
             for (int c0 = 32 * part; c0 < Np; c0 += 32 * parts) {
                 uint32_t v[32];
-                __syncwarp();
+                __syncwarp();   // (also: the last piece has been written)
                 tmem_ld32_issue(tb + c0, v);
                 tmem_ld_wait(v);
-                if (row < M) epilogue_chunk(v, c0, row, s_bias, N, 0, nullptr, 0, Y, ldy, inv, 1, vec);
+                // element (row l, column j) of the piece at word 32 l + (j ^ l): no bank conflicts either way
+#pragma unroll
+                for (int j = 0; j < 32; j++)
+                    turn[32 * lane + (j ^ lane)] = inv * (__uint_as_float(v[j]) + s_bias[c0 + j]);
+                __syncwarp();
+                if (c0 + lane < N) {
+                    float *y = Y + (long long)row0 * N + c0 + lane;
+#pragma unroll 8
+                    for (int i = 0; i < 32; i++)
+                        if (row0 + i < M) y[(long long)i * N] = turn[32 * i + (lane ^ i)];
+                }
             }
             asm volatile("tcgen05.fence::before_thread_sync;");
             __syncwarp();
@@ -931,27 +1273,6 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
-}
-
-// Wc (np x members * kh): member m's padded last-layer weights in columns [m kh, (m+1) kh)
-__global__ void k_concat_weights(const bf16 *const *w, int members, int np, int kh, bf16 *wc)
-{
-    const long long n = (long long)np * kh * members;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / ((long long)kh * members);
-        const int c = (int)(i % ((long long)kh * members));
-        wc[i] = w[c / kh][r * kh + c % kh];
-    }
-}
-
-// sum over members of the last layer's biases (n outputs)
-__global__ void k_bias_sum(const float *const *b, int members, int n, float *out)
-{
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int m = 0; m < members; m++) s += b[m][c];
-        out[c] = s;
-    }
 }
 
 // FP32 rows x cols (from src, contiguous rows) -> BF16 at dst, row stride ld (round to
@@ -1047,22 +1368,26 @@ struct pt_mlp {
     long long step = 0;
     std::string err;
     std::vector<void *> allocs;
-    // tcgen05 inference: the padded input batch and a wait error word
+    uint64_t version = 0;       // of the weights: another number after every change, in any network
+    // tcgen05 inference: the padded input batch and a wait error word (host memory the
+    // device writes)
     int use_umma = 1;
     bf16 *h0p = nullptr;
     int *umma_err = nullptr;
-    // inference input (FP32 rows copied from the host) and output (the last layer's
-    // outputs, rows padded to a multiple of 32), max_batch rows each
+    // inference input (FP32 rows copied from the host), and the accumulator of last layers
+    // that run one by one (rows padded to a multiple of 32), max_batch rows each
     float *xin = nullptr;
     float *zout = nullptr;
     int ldz = 0;
-    // the ensemble mean layer (held by an ensemble's first network): the members' last
-    // weights side by side, their summed biases, and device copies of the pointers
-    bf16 *wcat = nullptr;
-    float *bsum = nullptr;
-    void **mean_ptrs = nullptr;   // kMeanMaxMembers weight pointers, then as many bias pointers
-    size_t wcat_elems = 0;
+    // the members' weights side by side (held by an ensemble's first network), the
+    // versions they were packed from and the capacity in members
+    PackArgs pack{};
+    bool pack_always = false;   // a call of this network has been captured
+    std::vector<uint64_t> packed;
+    int pack_cap = 0;
 };
+
+static std::atomic<uint64_t> g_weights_version{0};
 
 static pt_status mfail(pt_mlp *m, pt_status st, const std::string &msg)
 {
@@ -1263,45 +1588,29 @@ static EncodeTiledFn encode_tiled()
 }
 
 // A map over a rows x cols BF16 matrix (row stride ld elements, a multiple of 8) whose
-// box is box_rows rows by 64 columns with the 128-byte swizzle (sw; cols a multiple of
-// 64) or by 8 columns without: the TMA boxes of a tcgen05 operand in the kernel's two
+// box is box_rows rows by box_cols columns: 64 with the 128-byte swizzle, 8 without (cols a
+// multiple of box_cols): the TMA boxes of a tcgen05 operand in the kernels' two
 // shared-memory layouts.  Rows past `rows` read as zeros.
-static bool operand_map(CUtensorMap *map, const bf16 *base, int rows, int cols, long long ld, int box_rows, bool sw)
+static bool operand_map(CUtensorMap *map, const bf16 *base, int rows, int cols, long long ld, int box_rows, int box_cols)
 {
     const EncodeTiledFn fn = encode_tiled();
-    if (!fn || ld % 8 != 0 || cols % (sw ? 64 : 8) != 0) return false;
+    if (!fn || ld % 8 != 0 || cols % box_cols != 0) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {sw ? 64u : 8u, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1u, 1u};
+    const CUtensorMapSwizzle swizzle = box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE;
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16 *>(base), dims, strides, box, elem,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, sw ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 static int pad32(int x) { return (x + 31) / 32 * 32; }
 
-// rows x cols outputs from the padded accumulator (row stride lds) to dst (contiguous
-// rows): on the device straight into dst, for the host through the contiguous device
-// buffer `staging` and one copy.
-static cudaError_t copy_out(const float *src, int lds, float *staging, int rows, int cols, float *dst,
-                            cudaMemcpyKind kind, cudaStream_t s)
-{
-    if (rows == 0) return cudaSuccess;
-    float *to = kind == cudaMemcpyDeviceToDevice ? dst : staging;
-    k_compact_rows<<<std::min((rows + 7) / 8, 8192), 256, 0, s>>>(src, lds, to, rows, cols);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && kind != cudaMemcpyDeviceToDevice)
-        e = cudaMemcpyAsync(dst, staging, (size_t)rows * cols * sizeof(float), kind, s);
-    return e;
-}
-
-// The inference input and padded output buffers of a network, kept between calls.
+// The padded accumulator of a network, kept between calls.
 static cudaError_t ensure_zout(pt_mlp *m)
 {
     if (m->zout) return cudaSuccess;
-    cudaError_t e = dalloc(m, &m->xin, (size_t)m->max_batch * m->width[0]);
-    if (e != cudaSuccess) return e;
     m->ldz = pad32(m->width[m->L]);
     return dalloc(m, &m->zout, (size_t)m->max_batch * m->ldz);
 }
@@ -1315,24 +1624,23 @@ static cudaError_t ensure_zout(pt_mlp *m)
 // The tcgen05 path's per-network state: the padded input buffer and the wait error word.
 static cudaError_t umma_prepare(pt_mlp *m)
 {
-    cudaError_t e = cudaSuccess;
-    if (!m->h0p) {
-        static const cudaError_t attr = [] {
-            cudaError_t a = cudaFuncSetAttribute(k_umma_layer<kUmmaEpiWarps>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaSmem);
-            if (a == cudaSuccess)
-                a = cudaFuncSetAttribute(k_umma_mean_layer<kUmmaEpiWarps>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kMeanSmem);
-            return a;
-        }();
-        if (attr != cudaSuccess) return attr;
-        if (!m->umma_err) {
-            e = dalloc(m, &m->umma_err, 1);
-            if (e == cudaSuccess) e = cudaMemsetAsync(m->umma_err, 0, sizeof(int), m->stream);
-        }
-        if (e == cudaSuccess) e = dalloc(m, &m->h0p, (size_t)m->max_batch * m->ld[0]);
+    if (m->h0p) return cudaSuccess;
+    static const cudaError_t attr = [] {
+        cudaError_t a = cudaFuncSetAttribute(k_umma_layer<kUmmaEpiWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             kUmmaSmem);
+        if (a == cudaSuccess)
+            a = cudaFuncSetAttribute(k_umma_mean_layer, cudaFuncAttributeMaxDynamicSharedMemorySize, kMeanSmem);
+        if (a == cudaSuccess)
+            a = cudaFuncSetAttribute(k_umma_hidden, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmem);
+        return a;
+    }();
+    if (attr != cudaSuccess) return attr;
+    if (!m->umma_err) {
+        cudaError_t e = cudaHostAlloc((void **)&m->umma_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+        if (e != cudaSuccess) return e;
+        *m->umma_err = 0;
     }
-    return e;
+    return dalloc(m, &m->h0p, (size_t)m->max_batch * m->ld[0]);
 }
 
 // With hidden_only, the tcgen05 path stops after the last hidden layer (H[L-1] holds
@@ -1370,7 +1678,8 @@ static cudaError_t forward_infer(pt_mlp *m, int B, const float *x, const bf16 **
         const long long lda = m->ld[l];
         const bool sw = Kp % 64 == 0;   // the 128-byte swizzled layout: whole 128-byte box rows
         CUtensorMap ma, mw;
-        if (!operand_map(&ma, A, B, Kp, lda, kUmmaM, sw) || !operand_map(&mw, m->wpk[l], Np, Kp, Kp, Np, sw))
+        if (!operand_map(&ma, A, B, Kp, lda, kUmmaM, sw ? 64 : 8) ||
+            !operand_map(&mw, m->wpk[l], Np, Kp, Kp, Np, sw ? 64 : 8))
             return cudaErrorNotSupported;
         const int N = m->width[l + 1];
         const float *bias = m->w + m->boff[l];
@@ -1387,90 +1696,189 @@ static cudaError_t forward_infer(pt_mlp *m, int B, const float *x, const bf16 **
     return cudaSuccess;
 }
 
-// Whether an ensemble runs its last layers as one GEMM (k_umma_mean_layer): 2 to
-// kMeanMaxMembers members, all on the tcgen05 path, the last layer's input a
-// multiple of 64 wide and its output at most kUmmaMaxN.
+// Whether the networks' hidden layers run fused (k_umma_hidden): all on the tcgen05 path,
+// at least one hidden layer, every one as wide, 64 to 256 in steps of 64.
+static bool net_fits(pt_mlp *const *members, int count)
+{
+    const pt_mlp *m = members[0];
+    if (count > kNetMaxMembers || m->L < 2 || m->L > 15) return false;
+    const int hid = m->width[1];
+    if (hid % 64 != 0) return false;
+    for (int l = 2; l < m->L; l++)
+        if (m->width[l] != hid) return false;
+    for (int j = 0; j < count; j++)
+        if (!members[j]->use_umma || !umma_fits(members[j])) return false;
+    return true;
+}
+
+// Whether an ensemble runs its last layers as one GEMM (k_umma_mean_layer): up to
+// kNetMaxMembers members, all on the tcgen05 path, the last layer's input a multiple of
+// 64 wide and its output at most kUmmaMaxN.  A single network does when its hidden layers
+// are fused: that saves the pass that compacts padded outputs.
 static bool mean_layer_fits(pt_mlp *const *members, int count)
 {
-    if (count < 2 || count > kMeanMaxMembers) return false;
+    if (net_fits(members, count)) return true;
+    if (count < 2 || count > kNetMaxMembers) return false;
     for (int j = 0; j < count; j++)
         if (!members[j]->use_umma || !umma_fits(members[j])) return false;
     const pt_mlp *m = members[0];
-    return m->L >= 2 && m->width[m->L - 1] % 64 == 0 && pad16(m->width[m->L]) <= kUmmaMaxN;
+    return m->L >= 2 && m->L <= 15 && m->width[m->L - 1] % 64 == 0;
 }
 
-// The mean of the members' last layers over B rows into y (row stride ldy), after
-// every member's hidden layers have run (H[L-1] of each holds its activations).
-static cudaError_t mean_layer(pt_mlp *const *members, int count, int B, float *y, int ldy, cudaStream_t s)
+// The members' weights side by side in the first one's buffers, packed again when any of
+// them has changed (versions are never used twice, so equal versions are equal weights).
+// A captured call packs whenever its graph runs, so that it has the weights of that time;
+// from then on every call does, for a replay may have left another ensemble's there.
+static cudaError_t pack_members(pt_mlp *const *members, int count, bool hidden, cudaStream_t s)
 {
     pt_mlp *m = members[0];
-    const int L = m->L, kh = m->width[L - 1], N = m->width[L], np = m->ld[L];
-    const size_t need = (size_t)np * kh * count;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!m->pack_always) {
+        const cudaError_t q = cudaStreamIsCapturing(s, &capture);
+        if (q != cudaSuccess) return q;
+        m->pack_always = capture != cudaStreamCaptureStatusNone;
+        if (m->pack_always) m->packed.clear();
+    }
+    std::vector<uint64_t> v(1, hidden ? 1 : 0);
+    for (int j = 0; j < count; j++) v.push_back(members[j]->version);
+    if (v == m->packed) return cudaSuccess;
+    m->packed.clear();
+    PackArgs &a = m->pack;
+    const int L = m->L;
+    a.members = count;
+    a.layers = L - 1;
+    a.kp0 = m->ld[0];
+    a.hid = m->width[L - 1];
+    a.np = m->ld[L];
+    a.nout = m->width[L];
     cudaError_t e = cudaSuccess;
-    if (!m->mean_ptrs) e = dalloc(m, &m->mean_ptrs, 2 * kMeanMaxMembers);
-    if (e == cudaSuccess && !m->bsum) e = dalloc(m, &m->bsum, kUmmaMaxN);
-    if (e == cudaSuccess && m->wcat_elems < need) {
-        e = dalloc(m, &m->wcat, need);
-        if (e == cudaSuccess) m->wcat_elems = need;
+    if (m->pack_cap < count) {   // (smaller buffers are freed with the network)
+        m->pack_cap = 0;
+        const size_t c = (size_t)count;
+        e = dalloc(m, &a.wc, c * a.np * a.hid);
+        if (e == cudaSuccess) e = dalloc(m, &a.bsum, kUmmaMaxN);
+        if (e == cudaSuccess) e = dalloc(m, &a.w0, c * a.hid * a.kp0);
+        if (e == cudaSuccess) e = dalloc(m, &a.w, c * std::max(1, a.layers - 1) * a.hid * a.hid);
+        if (e == cudaSuccess) e = dalloc(m, &a.hbias, c * a.layers * a.hid);
+        if (e != cudaSuccess) return e;
+        m->pack_cap = count;
     }
+    for (int j = 0; j < count; j++)
+        for (int l = 0; l < L; l++) {
+            a.wpk[j][l] = members[j]->wpk[l];
+            a.bias[j][l] = members[j]->w + members[j]->boff[l];
+        }
+    PackArgs args = a;
+    if (!hidden) args.w0 = nullptr;
+    k_pack_members<<<2 * sm_count_mlp(), 256, 0, s>>>(args);
+    e = cudaGetLastError();
+    if (e == cudaSuccess && !m->pack_always) m->packed = v;
+    return e;
+}
+
+// Every member's hidden layers over the B rows of x, fused: H[L-1] of each holds its last
+// activations.
+static cudaError_t hidden_fused(pt_mlp *const *members, int count, int B, const float *x, cudaStream_t s)
+{
+    pt_mlp *m = members[0];
+    cudaError_t e = umma_prepare(m);
     if (e != cudaSuccess) return e;
-    void *h[2 * kMeanMaxMembers] = {};
-    for (int j = 0; j < count; j++) {
-        h[j] = members[j]->wpk[L - 1];
-        h[kMeanMaxMembers + j] = members[j]->w + members[j]->boff[L - 1];
-    }
-    e = cudaMemcpyAsync(m->mean_ptrs, h, sizeof(h), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return e;
-    k_concat_weights<<<grid_for((long long)need), 256, 0, s>>>((const bf16 *const *)m->mean_ptrs, count, np, kh,
-                                                               m->wcat);
-    k_bias_sum<<<1, 256, 0, s>>>((const float *const *)(m->mean_ptrs + kMeanMaxMembers), count, N, m->bsum);
+    const int kp0 = m->ld[0], hid = m->width[1], layers = m->L - 1;
+    k_input_bf16<<<grid_for((long long)B * kp0 / 8), 256, 0, s>>>(x, B, m->width[0], m->h0p, kp0);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    MeanMaps maps;
-    memset(&maps, 0, sizeof(maps));
-    for (int j = 0; j < count; j++)
-        if (!operand_map(&maps.a[j], members[j]->H[L - 1], B, kh, kh, kUmmaM, true)) return cudaErrorNotSupported;
-    CUtensorMap mw;
-    if (!operand_map(&mw, m->wcat, np, kh * count, (long long)kh * count, np, true)) return cudaErrorNotSupported;
-    const int vec = ldy % 32 == 0 && ldy >= pad32(N) && reinterpret_cast<uintptr_t>(y) % 32 == 0;
-    const int tiles = (B + kUmmaM - 1) / kUmmaM;
-    const int grid = std::max(1, std::min(tiles, sm_count_mlp()));
-    k_umma_mean_layer<kUmmaEpiWarps><<<grid, 32 * (2 + kUmmaEpiWarps), kMeanSmem, s>>>(
-        maps, mw, B, kh, count, np, N, m->bsum, 1.0f / (float)count, y, ldy, vec, m->umma_err);
+    NetShape n = {};
+    n.M = B;
+    n.kp0 = kp0;
+    n.hid = hid;
+    n.layers = layers;
+    n.members = count;
+    n.sw0 = kp0 % 64 == 0;
+    n.bias = m->pack.hbias;
+    for (int j = 0; j < count; j++) n.out[j] = members[j]->H[m->L - 1];
+    n.error = m->umma_err;
+    n.w0 = m->pack.w0;
+    n.w = m->pack.w;
+    CUtensorMap mx;
+    if (!operand_map(&mx, m->h0p, B, kp0, kp0, kUmmaM, n.sw0 ? 64 : 8)) return cudaErrorNotSupported;
+    // two items a CTA once every SM has one
+    const int items = (B + kUmmaM - 1) / kUmmaM * count;
+    n.slots = items > sm_count_mlp() ? 2 : 1;
+    const int grid = std::min((items + n.slots - 1) / n.slots, sm_count_mlp());
+    k_umma_hidden<<<grid, kNetThreads, kNetSmem, s>>>(mx, n);
     return cudaGetLastError();
 }
 
-// One chunk of B rows of x (device) through every member, their mean into acc (row
-// stride ldacc): the members' hidden layers, then one mean layer when it fits, else
-// each member's last layer accumulating in its epilogue.
-static cudaError_t ensemble_chunk(pt_mlp *const *members, int count, int B, const float *x, float *acc, int ldacc,
-                                  cudaStream_t s)
+// The mean of the members' last layers over B rows into y (contiguous rows), after every
+// member's hidden layers have run (H[L-1] of each holds its activations).
+static cudaError_t mean_layer(pt_mlp *const *members, int count, int B, float *y, cudaStream_t s)
 {
-    const bool fused = mean_layer_fits(members, count);
+    pt_mlp *m = members[0];
+    const int L = m->L, kh = m->width[L - 1], N = m->width[L], np = m->ld[L];
+    MeanMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    for (int j = 0; j < count; j++)
+        if (!operand_map(&maps.a[j], members[j]->H[L - 1], B, kh, kh, kUmmaM, 64)) return cudaErrorNotSupported;
+    CUtensorMap mw;
+    if (!operand_map(&mw, m->pack.wc, np, kh * count, (long long)kh * count, np, 64)) return cudaErrorNotSupported;
+    const int tiles = (B + kUmmaM - 1) / kUmmaM;
+    const int grid = std::max(1, std::min(tiles, sm_count_mlp()));
+    k_umma_mean_layer<<<grid, 32 * (2 + kMeanEpiWarps), kMeanSmem, s>>>(maps, mw, B, kh, count, np, N, m->pack.bsum,
+                                                                        1.0f / (float)count, y, m->umma_err);
+    return cudaGetLastError();
+}
+
+// One chunk of B rows of x (device) through every member, their mean to the contiguous
+// rows of `out`: the members' hidden layers (fused where they fit), then one mean layer
+// when it fits, else each member's last layer accumulating in its epilogue.
+static cudaError_t ensemble_chunk(pt_mlp *const *members, int count, int B, const float *x, float *out, cudaStream_t s)
+{
+    if (B == 0) return cudaSuccess;
+    pt_mlp *m = members[0];
+    const bool net = net_fits(members, count), mean = mean_layer_fits(members, count);
+    cudaError_t e = mean ? pack_members(members, count, net, s) : ensure_zout(m);
+    if (e == cudaSuccess && net) e = hidden_fused(members, count, B, x, s);
     const bf16 *x0 = nullptr;
-    cudaError_t e = cudaSuccess;
-    for (int j = 0; j < count && e == cudaSuccess; j++) {
+    for (int j = 0; j < count && e == cudaSuccess && !net; j++) {
         pt_mlp *q = members[j];
         const cudaStream_t own = q->stream;
         q->stream = s;
-        e = forward_infer(q, B, x, &x0, acc, ldacc, 1.0f / (float)count, j == 0, fused);
+        e = forward_infer(q, B, x, &x0, m->zout, m->ldz, 1.0f / (float)count, j == 0, mean);
         q->stream = own;
     }
-    if (e != cudaSuccess || !fused || B == 0) return e;
-    return mean_layer(members, count, B, acc, ldacc, s);
+    if (e != cudaSuccess) return e;
+    if (mean) return mean_layer(members, count, B, out, s);
+    k_compact_rows<<<std::min((B + 7) / 8, 8192), 256, 0, s>>>(m->zout, m->ldz, out, B, m->width[m->L]);
+    return cudaGetLastError();
 }
 
-// A device wait of the tcgen05 path that gave up: reported once, then cleared.
+// A device wait of the tcgen05 path that gave up: reported once, then cleared.  The
+// stream has been synchronised.
 static pt_status umma_check(pt_mlp *m)
 {
-    if (!m->umma_err) return PT_OK;
-    int h = 0;
-    MCK(cudaMemcpyAsync(&h, m->umma_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream), "tcgen05 error word");
-    MCK(cudaStreamSynchronize(m->stream), "sync");
-    if (h) {
-        cudaMemsetAsync(m->umma_err, 0, sizeof(int), m->stream);
-        return mfail(m, PT_ERR_TIMEOUT, "a tcgen05 MMA completion wait gave up");
+    if (!m->umma_err || *(volatile int *)m->umma_err == 0) return PT_OK;
+    *(volatile int *)m->umma_err = 0;
+    return mfail(m, PT_ERR_TIMEOUT, "a tcgen05 MMA completion wait gave up");
+}
+
+// The checks of an ensemble call; the rows its networks take at a time.
+static pt_status ensemble_check(pt_mlp *const *members, int count, int *chunk)
+{
+    pt_mlp *m = members[0];
+    if (!m) return PT_ERR_ARG;
+    *chunk = m->max_batch;
+    for (int j = 0; j < count; j++) {
+        pt_mlp *q = members[j];
+        if (!q) return PT_ERR_ARG;
+        if (q->L != m->L) return mfail(m, PT_ERR_ARG, "ensemble members differ in depth");
+        for (int l = 0; l <= m->L; l++)
+            if (q->width[l] != m->width[l]) return mfail(m, PT_ERR_ARG, "ensemble members differ in widths");
+        *chunk = std::min(*chunk, q->max_batch);
     }
+    // every member runs on the first member's stream: finish what is queued on its own
+    for (int j = 1; j < count; j++)
+        if (members[j]->stream != m->stream)
+            MCK(cudaStreamSynchronize(members[j]->stream), "ensemble member stream");
     return PT_OK;
 }
 
@@ -1556,6 +1964,7 @@ pt_status pt_mlp_set_params(pt_mlp *m, const float *params)
     MCK(refresh_weights(m), "bf16 weights");
     MCK(cudaStreamSynchronize(m->stream), "sync");
     m->step = 0;
+    m->version = ++g_weights_version;
     return PT_OK;
 }
 
@@ -1594,6 +2003,7 @@ pt_status pt_mlp_train(pt_mlp *m, int epochs, int batch, float lr, uint64_t shuf
 {
     if (!m || epochs < 1 || batch < 1 || batch > m->max_batch || !(lr > 0.f)) return PT_ERR_ARG;
     if (!m->X) return mfail(m, PT_ERR_STATE, "pt_mlp_train before pt_mlp_set_data");
+    m->version = ++g_weights_version;
     const int din = m->width[0], steps = (m->n + batch - 1) / batch;
     if (steps > m->loss_cap) {
         float *p = nullptr;
@@ -1668,25 +2078,7 @@ pt_status pt_mlp_gradients(pt_mlp *m, const float *X, const float *Y, int n, flo
 pt_status pt_mlp_predict(pt_mlp *m, const float *X, int n, float *Y)
 {
     if (!m || !X || !Y || n < 0) return PT_ERR_ARG;
-    const int din = m->width[0], dout = m->width[m->L];
-    const int chunk = m->max_batch;
-    MCK(ensure_zout(m), "inference buffers");
-    float *dX = m->xin;
-    cudaError_t e = cudaSuccess;
-    for (int s0 = 0; s0 < n && e == cudaSuccess; s0 += chunk) {
-        const int B = std::min(chunk, n - s0);
-        e = cudaMemcpyAsync(dX, X + (size_t)s0 * din, (size_t)B * din * sizeof(float), cudaMemcpyHostToDevice,
-                            m->stream);
-        if (e != cudaSuccess) break;
-        const bf16 *x0 = nullptr;
-        e = forward_infer(m, B, dX, &x0, m->zout, m->ldz, 1.0f, true);
-        if (e != cudaSuccess) break;
-        e = copy_out(m->zout, m->ldz, m->Z[m->L - 1], B, dout, Y + (size_t)s0 * dout, cudaMemcpyDeviceToHost,
-                     m->stream);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-    MCK(e, "predict");
-    return umma_check(m);
+    return pt_mlp_predict_ensemble(&m, 1, X, n, Y);
 }
 
 pt_status pt_mlp_set_tcgen05(pt_mlp *m, int enabled)
@@ -1699,67 +2091,40 @@ pt_status pt_mlp_set_tcgen05(pt_mlp *m, int enabled)
 pt_status pt_mlp_predict_ensemble(pt_mlp *const *members, int count, const float *X, int n, float *Y)
 {
     if (!members || count < 1 || !X || !Y || n < 0) return PT_ERR_ARG;
+    int chunk = 0;
+    pt_status st = ensemble_check(members, count, &chunk);
+    if (st != PT_OK) return st;
     pt_mlp *m = members[0];
-    if (!m) return PT_ERR_ARG;
-    int chunk = m->max_batch;
-    for (int j = 0; j < count; j++) {
-        pt_mlp *q = members[j];
-        if (!q) return PT_ERR_ARG;
-        if (q->L != m->L) return mfail(m, PT_ERR_ARG, "ensemble members differ in depth");
-        for (int l = 0; l <= m->L; l++)
-            if (q->width[l] != m->width[l]) return mfail(m, PT_ERR_ARG, "ensemble members differ in widths");
-        chunk = std::min(chunk, q->max_batch);
-    }
     const int din = m->width[0], dout = m->width[m->L];
     const cudaStream_t s = m->stream;
-    // every member runs on the first member's stream: finish what is queued on its own
-    for (int j = 1; j < count; j++)
-        if (members[j]->stream != s) MCK(cudaStreamSynchronize(members[j]->stream), "ensemble member stream");
-    // the members' mean accumulates in the first member's padded output buffer
-    MCK(ensure_zout(m), "inference buffers");
-    float *dX = m->xin, *acc = m->zout;   // chunk <= m->max_batch rows
+    if (!m->xin) MCK(dalloc(m, &m->xin, (size_t)m->max_batch * din), "inference input");
+    float *dX = m->xin, *dY = m->Z[m->L - 1];   // chunk <= m->max_batch rows
     cudaError_t e = cudaSuccess;
     for (int s0 = 0; s0 < n && e == cudaSuccess; s0 += chunk) {
         const int B = std::min(chunk, n - s0);
         e = cudaMemcpyAsync(dX, X + (size_t)s0 * din, (size_t)B * din * sizeof(float), cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = ensemble_chunk(members, count, B, dX, acc, m->ldz, s);
+        if (e == cudaSuccess) e = ensemble_chunk(members, count, B, dX, dY, s);
         if (e == cudaSuccess)
-            e = copy_out(acc, m->ldz, m->Z[m->L - 1], B, dout, Y + (size_t)s0 * dout, cudaMemcpyDeviceToHost, s);
+            e = cudaMemcpyAsync(Y + (size_t)s0 * dout, dY, (size_t)B * dout * sizeof(float), cudaMemcpyDeviceToHost, s);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    MCK(e, "ensemble predict");
-    for (int j = 0; j < count; j++) {
-        const pt_status st = umma_check(members[j]);
-        if (st != PT_OK) return st;
-    }
-    return PT_OK;
+    MCK(e, "predict");
+    for (int j = 0; j < count && st == PT_OK; j++) st = umma_check(members[j]);
+    return st;
 }
 
 pt_status pt_mlp_predict_ensemble_device(pt_mlp *const *members, int count, const float *X, int n, float *Y)
 {
     if (!members || count < 1 || !X || !Y || n < 0) return PT_ERR_ARG;
+    int chunk = 0;
+    pt_status st = ensemble_check(members, count, &chunk);
+    if (st != PT_OK) return st;
     pt_mlp *m = members[0];
-    if (!m) return PT_ERR_ARG;
-    int chunk = m->max_batch;
-    for (int j = 0; j < count; j++) {
-        pt_mlp *q = members[j];
-        if (!q) return PT_ERR_ARG;
-        if (q->L != m->L) return mfail(m, PT_ERR_ARG, "ensemble members differ in depth");
-        for (int l = 0; l <= m->L; l++)
-            if (q->width[l] != m->width[l]) return mfail(m, PT_ERR_ARG, "ensemble members differ in widths");
-        chunk = std::min(chunk, q->max_batch);
-    }
     const int din = m->width[0], dout = m->width[m->L];
-    const cudaStream_t s = m->stream;
-    for (int j = 1; j < count; j++)
-        if (members[j]->stream != s) MCK(cudaStreamSynchronize(members[j]->stream), "ensemble member stream");
-    MCK(ensure_zout(m), "inference output");
     for (int s0 = 0; s0 < n; s0 += chunk) {
         const int B = std::min(chunk, n - s0);
-        MCK(ensemble_chunk(members, count, B, X + (size_t)s0 * din, m->zout, m->ldz, s), "ensemble predict (device)");
-        // the mean, from the padded accumulator into y's rows
-        MCK(copy_out(m->zout, m->ldz, nullptr, B, dout, Y + (size_t)s0 * dout, cudaMemcpyDeviceToDevice, s),
-            "ensemble mean");
+        MCK(ensemble_chunk(members, count, B, X + (size_t)s0 * din, Y + (size_t)s0 * dout, m->stream),
+            "ensemble predict (device)");
     }
     return PT_OK;
 }
@@ -1770,6 +2135,7 @@ void pt_mlp_destroy(pt_mlp *m)
     if (m->stream) cudaStreamSynchronize(m->stream);
     else cudaDeviceSynchronize();
     for (void *p : m->allocs) cudaFree(p);
+    if (m->umma_err) cudaFreeHost(m->umma_err);
     delete m;
 }
 
