@@ -346,14 +346,16 @@ struct RadixPass {
     int E, pass, passes, dbits;
     const int *digit_base;
     RadixSegments sg;
-    unsigned long long *status;
-    int *ctl, *error;
+    unsigned long long *status, *ctl;
+    int *error;
     const int *skip;
 };
 
 // The tile a block works on: its ticket, its segment and what it reads there.
 struct RadixTile {
-    int tile, seg, stile;   // ticket, segment, tile within the segment
+    int tile;               // ticket
+    unsigned epoch;         // the launch's
+    int seg, stile;         // segment, tile within the segment
     int base, count;        // the segment's first entry slot and entries
     int dense;              // day's first pass: the segment reads the schedule keys
     int nk, pb, bb;         // dense: the instance's persons, first person; bb: its first bucket
@@ -396,7 +398,13 @@ __device__ __forceinline__ int radix_look_back(volatile unsigned long long *st, 
 // One stable pass over dbits bits of the keys.  Persistent blocks take tiles from a
 // ticket in order until the entries run out, so a short input costs no idle blocks.
 // Look-back words carry the launch epoch (see lb_word), so they need no reset between
-// passes.
+// passes; ticket and epoch are one word, which a block draws from when it starts and,
+// while it works on a tile, for its next one.  Every block that takes part draws until
+// a ticket is past the last tile, so the draw number tiles + blocks is the launch's last,
+// and it sets the ticket back and the epoch on.
+//
+// A short input is a chain of latencies: 200,000 entries take 10 us, 17 with the ticket
+// drawn between tiles, a finish count and an entry's region looked up just before its load.
 //
 // Segmented sorts (sg.tile_prefix set): segment k's entries lie at
 // [ic[k].kbase, ic[k].kbase + is[k].marked) and are ordered within the segment only,
@@ -407,7 +415,13 @@ __device__ __forceinline__ int radix_look_back(volatile unsigned long long *st, 
 template <int IN, int OUT>
 __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass(RadixPass a)
 {
-    if (a.skip && *(volatile const int *)a.skip) return;
+    const RadixSegments &sg = a.sg;
+    const int *const tprefix = IN == kInDay ? sg.tile_prefix0 : sg.tile_prefix;
+    const int skip = a.skip ? *(volatile const int *)a.skip : 0;
+    const int tiles = sg.tile_prefix ? *(volatile const int *)&tprefix[sg.segments] : (a.E + kRadixTile - 1) / kRadixTile;
+    // only as many blocks as there are tiles take part
+    const int active = min(tiles, (int)gridDim.x);
+    if (skip || (int)blockIdx.x >= active) return;
     extern __shared__ __align__(16) uint8_t radix_smem[];
     uint2 *const s_pair = reinterpret_cast<uint2 *>(radix_smem);                              // kRadixTile
     unsigned *const s_peers = reinterpret_cast<unsigned *>(radix_smem + kRadixTile * 8);      // kRadixWarps x 256
@@ -415,13 +429,6 @@ __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass
     uint16_t (*const s_hist)[256] = reinterpret_cast<uint16_t (*)[256]>(radix_smem + kRadixTile * 8 + kRadixWarps * 1024);
     __shared__ RadixTile s_t;
     __shared__ int s_base[256];   // global position of digit d's entries, less its tile-local start
-    const RadixSegments &sg = a.sg;
-    const int *const tprefix = IN == kInDay ? sg.tile_prefix0 : sg.tile_prefix;
-    const int tiles = sg.tile_prefix ? *(volatile const int *)&tprefix[sg.segments] : (a.E + kRadixTile - 1) / kRadixTile;
-    // only as many blocks as there are tiles take part (ticket, finish count)
-    const int active = min(tiles, (int)gridDim.x);
-    if ((int)blockIdx.x >= active) return;
-    const unsigned epoch = (unsigned)(*(volatile int *)&a.ctl[2]) & 0x3FFFFFFFu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned bit = 1u << lane, lt = bit - 1u, dmask = (1u << a.dbits) - 1u;
     const int shift = a.dbits * a.pass;
@@ -431,12 +438,13 @@ __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass
         (&s_hist[0][0])[i] = 0;
         s_peers[i] = 0u;
     }
+    unsigned long long drawn = 0;   // warp 0's lane 0: epoch (high half) and next ticket
+    if (threadIdx.x == 0) drawn = atomicAdd(a.ctl, 1ull);
     for (;;) {
         if (warp == 0) {
-            int t = 0;
-            if (lane == 0) t = atomicAdd(&a.ctl[0], 1);
-            t = __shfl_sync(0xffffffffu, t, 0);
-            RadixTile r = {t, 0, t, 0, a.E, 0, 0, 0, 0, 0};
+            drawn = __shfl_sync(0xffffffffu, drawn, 0);
+            const int t = (int)(unsigned)drawn;
+            RadixTile r = {t, (unsigned)(drawn >> 32) & 0x3FFFFFFFu, 0, t, 0, a.E, 0, 0, 0, 0, 0};
             if (sg.tile_prefix && t < tiles) {
                 // the segment owning tile t: the last k with tprefix[k] <= t, 32 probes a step
                 int lo = 0, hi = sg.segments;   // in [lo, hi)
@@ -467,7 +475,9 @@ __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass
         __syncthreads();   // (also ends the last tile's use of shared memory)
         const int tile = s_t.tile, stile = s_t.stile, sbase = s_t.base, scount = s_t.count, table_base = s_t.bb;
         const int rlast = s_t.rlast;
+        const unsigned epoch = s_t.epoch;
         if (tile >= tiles) break;
+        if (threadIdx.x == 0) drawn = atomicAdd(a.ctl, 1ull);
         const int first = stile * kRadixTile + warp * kRadixWarpItems + lane;   // index within the segment
         const bool full = (stile + 1) * kRadixTile <= scount;
         bool whole = full;   // every entry of the tile takes part
@@ -501,6 +511,7 @@ __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass
             for (int q = 0; q < kChunks; q++)
                 rec[q] = c0 + q * kRegionChunk < scount ? sg.chunk_region[(sbase + c0) / kRegionChunk + q]
                                                         : make_int4(0, 0, INT_MAX, INT_MAX);
+            // where each entry lies first, then all loads together
 #pragma unroll
             for (int j = 0; j < kRadixItems; j++) {
                 const int i = first + 32 * j;
@@ -520,9 +531,12 @@ __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass
                             } while (i >= next);
                         }
                     }
-                    kv[j] = a.in[3 * (size_t)r * sg.region_persons + (i - at)];
+                    kv[j].x = 3u * (unsigned)r * (unsigned)sg.region_persons + (unsigned)(i - at);
                 }
             }
+#pragma unroll
+            for (int j = 0; j < kRadixItems; j++)
+                if (full || first + 32 * j < scount) kv[j] = a.in[kv[j].x];
         } else {
 #pragma unroll
             for (int j = 0; j < kRadixItems; j++) {
@@ -631,16 +645,8 @@ __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass
             for (int i = d; i < valid; i += kRadixThreads) write(i);
         }
     }
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const int fin = atomicAdd(&a.ctl[1], 1);
-        if (fin == active - 1) {
-            a.ctl[0] = 0;
-            a.ctl[1] = 0;
-            atomicAdd(&a.ctl[2], 1);
-            __threadfence();
-        }
-    }
+    if (threadIdx.x == 0 && (int)(unsigned)drawn == tiles + active - 1)
+        atomicAdd(a.ctl, (1ull << 32) - (unsigned long long)(tiles + active));
 }
 
 static int key_bits(int buckets)

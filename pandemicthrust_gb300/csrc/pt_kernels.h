@@ -119,7 +119,7 @@ struct DevArrays {
     int32_t *bkt_people;      // 3P person ids bucket by bucket, ascending in each
     uint2 *rp0, *rp1;         // 3P each: radix ping-pong (key, value) pairs
     unsigned long long *radix_status;  // ceil(3P/4096) x 256 epoch-tagged look-back words
-    int *radix_ctl;           // ticket, finished
+    unsigned long long *radix_ctl;   // epoch (high half) and ticket
     int *digit_hist;          // K x kDigitStripes x 4 x 256 (the first 4 x 256 also serve the setup sorts)
     int *digit_base;          // K x 4 x 256
     int32_t *tile_prefix;     // K + 1: radix tiles of the instances' segments
@@ -230,7 +230,7 @@ struct RadixArgs {
     const int *digit_base;        // [segment][pass][256]
     RadixSegments seg;
     unsigned long long *status;   // look-back words, ceil(E/4096) x 256, epoch-tagged
-    int *ctl;                     // ticket, finished, epoch
+    unsigned long long *ctl;      // epoch (high half) and ticket
     int *error;
     const int *skip;
     int blocks_per_sm = 4;        // persistent blocks per SM, at most what fits

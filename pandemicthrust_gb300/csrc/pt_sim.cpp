@@ -427,7 +427,7 @@ static pt_status engine_setup(Engine *s)
     bytes += round256(3 * n * 8) * 2;           // radix pairs p0, p1
     bytes += round256((size_t)Bmax * 4);        // bkt_count (also the workplace histogram)
     bytes += round256(radix_tiles * 256 * 8);   // radix look-back words
-    bytes += round256(8 * 4);                                                      // radix ctl
+    bytes += round256(8);                                                          // radix ctl
     bytes += round256((size_t)K * ptk::kDigitStripes * 4 * 256 * 4);               // digit histograms
     bytes += round256((size_t)K * 4 * 256 * 4) + 2 * round256(((size_t)K + 1) * 4);  // digit bases, tile prefixes
     const size_t nregions = n / ptk::kSchedMinRegion, nchunks = 3 * n / ptk::kRegionChunk + 1;
@@ -458,7 +458,7 @@ static pt_status engine_setup(Engine *s)
     d.rp1 = a.take<uint2>(3 * n);
     d.bkt_count = a.take<int32_t>((size_t)Bmax);
     d.radix_status = a.take<unsigned long long>(radix_tiles * 256);
-    d.radix_ctl = a.take<int>(8);
+    d.radix_ctl = a.take<unsigned long long>(1);
     d.digit_hist = a.take<int>((size_t)K * ptk::kDigitStripes * 4 * 256);
     d.digit_base = a.take<int>((size_t)K * 4 * 256);
     d.tile_prefix = a.take<int32_t>((size_t)K + 1);
@@ -488,7 +488,7 @@ static pt_status engine_setup(Engine *s)
         CK(cudaStreamSynchronize(s->stream), "tile map sync");
     }
     CK(cudaMemsetAsync(d.bkt_count, 0, (size_t)Bmax * 4, s->stream), "memset counts");
-    CK(cudaMemsetAsync(d.radix_ctl, 0, 8 * 4, s->stream), "memset radix ctl");
+    CK(cudaMemsetAsync(d.radix_ctl, 0, 8, s->stream), "memset radix ctl");
     CK(cudaMemsetAsync(d.radix_status, 0, radix_tiles * 256 * 8, s->stream), "memset radix words");
     CK(cudaMemsetAsync(d.digit_hist, 0, (size_t)K * ptk::kDigitStripes * 4 * 256 * 4, s->stream), "memset digit hist");
 

@@ -124,7 +124,7 @@ extern "C" pt_status pt_bucket_table_static(const int32_t *keys, int n, int buck
     r.out = (uint32_t *)table;
     r.digit_base = (const int *)(base + kOffDigitBase);
     r.status = (unsigned long long *)(base + kOffStatus);
-    r.ctl = (int *)(base + kOffRadixCtl);
+    r.ctl = (unsigned long long *)(base + kOffRadixCtl);
     r.error = error;
     r.skip = nullptr;
     if (n == 0) {
