@@ -1733,22 +1733,44 @@ cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, cudaStream_t s)
 
 // ------------------------------------------------------------------ infection
 // device_selectRandomPersonFromLocation (PandemicSim.cu:2028-2071).  A location with
-// at most one person gives victim = count and type NONE (kappa 0).
-__device__ __forceinline__ int select_victim(int self, int off, int count, uint32_t r, bool home,
-                                             const int32_t *table, int &victim)
+// at most one person gives victim = count and type NONE (kappa 0).  Without a table the
+// location's persons are off, off + 1, ... (a household).
+__device__ __forceinline__ int select_victim(int self, int off, int count, uint32_t r, int &victim,
+                                             const int32_t *table = nullptr)
 {
     if (count <= 1) {
         victim = count;
         return 0;
     }
     int o = (int)(r % (uint32_t)count);
-    int v = home ? off + o : table[off + o];
+    int v = table ? table[off + o] : off + o;
     if (v == self) {
         o = (o + 1) % count;
-        v = home ? off + o : table[off + o];
+        v = table ? table[off + o] : off + o;
     }
     victim = v;
     return 1;
+}
+
+// The same for NC locations with tables, the tables' loads together.
+template <int NC>
+__device__ __forceinline__ void select_victims(int self, const int (&off)[NC], const int (&cnt)[NC],
+                                               const int32_t *const (&table)[NC], const uint32_t *r, int *victim,
+                                               int *kv)
+{
+    int o[NC];
+#pragma unroll
+    for (int j = 0; j < NC; j++) {
+        kv[j] = cnt[j] > 1 ? 1 : 0;
+        victim[j] = cnt[j];
+        if (kv[j]) {
+            o[j] = (int)(r[j] % (uint32_t)cnt[j]);
+            victim[j] = table[j][off[j] + o[j]];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NC; j++)
+        if (kv[j] && victim[j] == self) victim[j] = table[j][off[j] + (o[j] + 1) % cnt[j]];
 }
 
 // First claims of the day, collected per warp in shared memory and appended to the
@@ -1811,6 +1833,9 @@ struct Infector {
 // the day claims (victim, strain) with key (position, slot); the smallest key wins.
 // A victim is only ever drawn by infectors of its own instance, whose list positions
 // keep the instance's order.
+//
+// The draws come first, then the loads of every victim drawn, then a strain's claims:
+// one after the other, each waits for its own load and its own atomic.
 template <int NC>
 __device__ __forceinline__ void process_contacts(const SimConst &c, const TfKey &key, const Infector &inf,
                                                  unsigned long long ctr, const int (&victims)[NC],
@@ -1822,45 +1847,60 @@ __device__ __forceinline__ void process_contacts(const SimConst &c, const TfKey 
     tf2x64(key, ctr + 1, w + 4);
     tf2x64(key, ctr + 2, w + 8);
     tf2x64(key, ctr + 3, w + 12);
+    unsigned hits = 0;   // bit 2 j + strain
 #pragma unroll
     for (int j = 0; j < NC; j++) {
         const float kf = __int2float_rn(kv[j]);
 #pragma unroll
-        for (int strain = 0; strain < 2; strain++) {
+        for (int strain = 0; strain < 2; strain++)
+            if (to_unit(w[2 * j + strain]) < __fmul_rn(inf.prob[strain], kf)) hits |= 1u << (2 * j + strain);
+    }
+    uint32_t st[NC];
+#pragma unroll
+    for (int j = 0; j < NC; j++) {
+        st[j] = 0u;
+        if ((hits >> (2 * j)) & 3u) st[j] = state[victims[j]];
+    }
+#pragma unroll
+    for (int strain = 0; strain < 2; strain++) {
+        unsigned long long old[NC];
+#pragma unroll
+        for (int j = 0; j < NC; j++) {
             const int u = 2 * j + strain;
-            const float y = to_unit(w[u]);
-            const bool hit = y < __fmul_rn(inf.prob[strain], kf);
-            if (hit) {
-                const int v = victims[j];
-                const uint32_t st = state[v];
-                const uint32_t vstatus = strain ? ((st >> 8) & 0xFFu) : (st & 0xFFu);
-                if (vstatus == 1u) {
-                    const int profile = infection_profile(c, w[u] ^ w[(u + 1) & 15]);
-                    unsigned long long k = ((unsigned long long)((long long)inf.pos * 8 + j) << 16) |
-                                           ((unsigned long long)profile << 8) | (unsigned long long)(inf.gen[strain] & 0xFF);
-                    unsigned long long old = atomicMin(&claim[2 * (size_t)v + strain], k);
-                    if (old == ~0ull) queue.push(2 * v + strain);
-                }
+            old[j] = 0ull;
+            if (((hits >> u) & 1u) && ((st[j] >> (8 * strain)) & 0xFFu) == 1u) {
+                const int profile = infection_profile(c, w[u] ^ w[(u + 1) & 15]);
+                const unsigned long long k =
+                    ((unsigned long long)((long long)inf.pos * 8 + j) << 16) | ((unsigned long long)profile << 8) |
+                    (unsigned long long)(inf.gen[strain] & 0xFF);
+                old[j] = atomicMin(&claim[2 * (size_t)victims[j] + strain], k);
             }
         }
+#pragma unroll
+        for (int j = 0; j < NC; j++)
+            if (old[j] == ~0ull) queue.push(2 * victims[j] + strain);
     }
 }
 
-__device__ __forceinline__ void infector_state(const SimConst &c, Infector &inf, uint32_t st, const uint8_t *gen_p,
-                                               const uint8_t *gen_s, int day, int ksum)
+// The generation of its victims, of each strain the infector (status word st) has.
+__device__ __forceinline__ void infector_gens(Infector &inf, uint32_t st, const uint8_t *gen_p, const uint8_t *gen_s)
+{
+    inf.gen[0] = (st & 0xFFu) >= 2u ? gen_p[inf.me] + 1 : 0xFF;
+    inf.gen[1] = ((st >> 8) & 0xFFu) >= 2u ? gen_s[inf.me] + 1 : 0xFF;
+}
+
+// Infection probability of each strain (device_calculateInfectionProbability); -1
+// when the strain is not infectious today.
+__device__ __forceinline__ void infector_probs(const SimConst &c, uint32_t st, int day, int ksum, float prob[2])
 {
 #pragma unroll
     for (int strain = 0; strain < 2; strain++) {
-        uint32_t status = strain ? ((st >> 8) & 0xFFu) : (st & 0xFFu);
-        uint32_t dday = strain ? (st >> 24) : ((st >> 16) & 0xFFu);
-        inf.prob[strain] = -1.f;
-        inf.gen[strain] = 0xFF;
+        const uint32_t status = strain ? ((st >> 8) & 0xFFu) : (st & 0xFFu);
+        const uint32_t dday = strain ? (st >> 24) : ((st >> 16) & 0xFFu);
+        prob[strain] = -1.f;
         if (status >= 2u) {
-            int pd = day - (int)dday;
-            if (pd >= 0 && pd < 10) {
-                inf.prob[strain] = infection_probability(c, (int)status - 2, pd, strain, ksum);
-                inf.gen[strain] = ((strain ? gen_s[inf.me] : gen_p[inf.me]) + 1) & 0xFF;
-            }
+            const int pd = day - (int)dday;
+            if (pd >= 0 && pd < 10) prob[strain] = infection_probability(c, (int)status - 2, pd, strain, ksum);
         }
     }
 }
@@ -1883,7 +1923,10 @@ struct InfectArgs {
 __device__ __forceinline__ uint4 load_record(const uint4 *prec, int me) { return __ldg(&prec[me]); }
 
 // kernel_doWeekday + device_makeContacts_weekday (PandemicSim.cu:3236-3308, :1669-1829),
-// one thread per infector.
+// one thread per infector.  Bound by random 32-byte sectors (record, keys, bucket
+// slots, tables, victims, claims) and by how many a warp has in flight, so each kind is
+// loaded for all contacts together: 36 ms of a 48-instance run's weekdays on a GB300, 42
+// with every contact's loads after the last one's.
 __global__ void __launch_bounds__(128) k_infect_weekday(InfectArgs a, int day)
 {
     Scalars *sc = a.sc;
@@ -1911,22 +1954,12 @@ __global__ void __launch_bounds__(128) k_infect_weekday(InfectArgs a, int day)
         tf2x64(key, ctr, w);
         tf2x64(key, ctr + 1, w + 4);
         const bool adult = prec_age(rec.w) == 5;
-        int victims[8], kv[8];
-        int ksum = 0;
-        // household: offset + r % count, the household table is the identity
-        const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            kv[j] = select_victim(me, hoff, hcnt, w[j], true, nullptr, victims[j]);
-            ksum += kv[j];
-        }
-        // workplace or school: max-contacts of its type
-        const int woff = (int)rec.y, wcnt = (int)rec.z;
-        const int desired = prec_desired(rec.w);
-        // errands / afterschool: destinations from today's keys; the adult
-        // profile is regenerated from the schedule counter (:3667-3705)
+        const uint32_t mine = a.state[me];
+        // errands / afterschool: destinations from today's keys
         const int32_t *kk = a.keys + ik.kbase;
-        const int dest[2] = {kk[lme], kk[c.N + lme]};
+        const uint2 slot0 = a.bkt[kk[lme]], slot1 = a.bkt[kk[c.N + lme]];
+        infector_gens(inf, mine, a.gen_p, a.gen_s);
+        // the adult profile is regenerated from the schedule counter (:3667-3705)
         int prof = 3;
         if (adult) {
             uint32_t e[4];
@@ -1934,21 +1967,29 @@ __global__ void __launch_bounds__(128) k_infect_weekday(InfectArgs a, int day)
             const int slot = 2 * (lme % 2);
             prof = (int)((e[slot] ^ e[slot + 1]) % 3u);
         }
-        int made = 3;
-        uint32_t wvoid = 0;  // contact slots voided by interventions
+        int victims[8], kv[8];
+        // household: offset + r % count, the household table is the identity
+        const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
 #pragma unroll
-        for (int j = 3; j < 8; j++) {
-            victims[j] = -1;
-            kv[j] = 0;
-        }
+        for (int j = 0; j < 3; j++) kv[j] = select_victim(me, hoff, hcnt, w[j], victims[j]);
+        // then the workplace's or school's max-contacts, then each errand hour's
+        const int desired = prec_desired(rec.w);
+        const int want0 = c_weekday_assign[prof][0], want = want0 + c_weekday_assign[prof][1];
+        int off[5], cnt[5];
+        const int32_t *table[5];
 #pragma unroll
-        for (int j = 3; j < 6; j++) {
-            if (j - 3 < desired) {
-                kv[j] = select_victim(me, woff, wcnt, w[j], false, a.wp_people, victims[j]);
-                ksum += kv[j];
-            }
+        for (int j = 0; j < 5; j++) {
+            const int e = j - desired;
+            const uint2 slot = e < want0 ? slot0 : slot1;
+            off[j] = e < 0 ? (int)rec.y : bucket_start(slot);
+            cnt[j] = e < 0 ? (int)rec.z : (e < want ? bucket_count(slot) : 0);
+            table[j] = e < 0 ? a.wp_people : a.bkt_people;
         }
-        made += desired;
+        select_victims<5>(me, off, cnt, table, w + 3, victims + 3, kv + 3);
+        int ksum = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) ksum += kv[j];
+        infector_probs(c, mine, day, ksum, inf.prob);
         // interventions: a closed school or an absent adult voids the workplace / school
         // contacts; they keep their share of ksum, so the contact does not happen
         // rather than passing its weight to the others
@@ -1956,36 +1997,19 @@ __global__ void __launch_bounds__(128) k_infect_weekday(InfectArgs a, int day)
             const bool closed = day >= ik.closure_start && day < ik.closure_end && prec_school(rec.w);
             const bool me_absent =
                 adult && intervention_hash(c.key0, c.key1, kTagAbsent, day, lme) < ik.absent_thr;
+            int age[3];
 #pragma unroll
-            for (int j = 3; j < 6; j++) {
-                if (j - 3 < desired && kv[j] != 0) {
-                    const int v = victims[j];
-                    const bool v_absent = ik.absent_thr != 0 && a.age[v] == 5 &&
-                                          intervention_hash(c.key0, c.key1, kTagAbsent, day, v - ik.pbase) <
-                                              ik.absent_thr;
-                    if (closed || me_absent || v_absent) wvoid |= 1u << j;
-                }
+            for (int j = 0; j < 3; j++) {
+                age[j] = 0;
+                if (j < desired && kv[3 + j] != 0 && ik.absent_thr != 0) age[j] = a.age[victims[3 + j]];
+            }
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const bool v_absent = age[j] == 5 && intervention_hash(c.key0, c.key1, kTagAbsent, day,
+                                                                       victims[3 + j] - ik.pbase) < ik.absent_thr;
+                if (j < desired && (closed || me_absent || v_absent)) kv[3 + j] = 0;
             }
         }
-#pragma unroll
-        for (int hour = 0; hour < 2; hour++) {
-            int want = c_weekday_assign[prof][hour];
-            const uint2 slot = a.bkt[dest[hour]];
-            const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
-#pragma unroll
-            for (int j = 3; j < 8; j++) {
-                if (j == made && want > 0) {
-                    kv[j] = select_victim(me, eoff, ecnt, w[j], false, a.bkt_people, victims[j]);
-                    ksum += kv[j];
-                    want--;
-                    made++;
-                }
-            }
-        }
-        infector_state(c, inf, a.state[me], a.gen_p, a.gen_s, day, ksum);
-#pragma unroll
-        for (int j = 3; j < 6; j++)
-            if ((wvoid >> j) & 1u) kv[j] = 0;
         process_contacts<8>(c, key, inf, ctr + 2, victims, kv, a.state, a.claim, queue);
     }
     queue.flush(1, lane);
@@ -2015,30 +2039,25 @@ __global__ void __launch_bounds__(128) k_infect_weekend(InfectArgs a, int day)
         const int lme = me - ik.pbase;
         const unsigned long long ctr = s.infect_offset + 6ull * (unsigned long long)(pos - s.start);
         const uint4 rec = load_record(a.prec, me);
+        const uint32_t mine = a.state[me];
         uint32_t w[4];
         tf2x64(key, ctr, w);
-        int victims[5], kv[5];
-        int ksum = 0;
-        const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            kv[j] = select_victim(me, hoff, hcnt, w[j], true, nullptr, victims[j]);
-            ksum += kv[j];
-        }
         const int prof = (int)(w[3] % 6u);
+        const int32_t *k3 = a.keys + ik.kbase + 3 * (size_t)lme;
+        const uint2 slot0 = a.bkt[k3[c_weekend_assign[prof][0]]], slot1 = a.bkt[k3[c_weekend_assign[prof][1]]];
+        infector_gens(inf, mine, a.gen_p, a.gen_s);
         // Threefry-2x32 on the low seed words with counter (u32)(ctr + 1) (:1895-1901)
         uint32_t v2[2];
         tf2x32(key, (uint32_t)(ctr + 1), v2);
-        const int32_t *k3 = a.keys + ik.kbase + 3 * (size_t)lme;
+        int victims[5], kv[5];
+        const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int loc = k3[c_weekend_assign[prof][j]];
-            const uint2 slot = a.bkt[loc];
-            const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
-            kv[3 + j] = select_victim(me, eoff, ecnt, v2[j], false, a.bkt_people, victims[3 + j]);
-            ksum += kv[3 + j];
-        }
-        infector_state(c, inf, a.state[me], a.gen_p, a.gen_s, day, ksum);
+        for (int j = 0; j < 3; j++) kv[j] = select_victim(me, hoff, hcnt, w[j], victims[j]);
+        const int off[2] = {bucket_start(slot0), bucket_start(slot1)};
+        const int cnt[2] = {bucket_count(slot0), bucket_count(slot1)};
+        const int32_t *const table[2] = {a.bkt_people, a.bkt_people};
+        select_victims<2>(me, off, cnt, table, v2, victims + 3, kv + 3);
+        infector_probs(c, mine, day, kv[0] + kv[1] + kv[2] + kv[3] + kv[4], inf.prob);
         process_contacts<5>(c, key, inf, ctr + 2, victims, kv, a.state, a.claim, queue);
     }
     queue.flush(1, lane);
@@ -2101,22 +2120,6 @@ __device__ __forceinline__ void claim_slot(const SimConst &c, const InfectArgs &
     }
 }
 
-// Infection probability of each strain (device_calculateInfectionProbability); -1
-// when the strain is not infectious today.
-__device__ __forceinline__ void infector_probs(const SimConst &c, uint32_t st, int day, int ksum, float prob[2])
-{
-#pragma unroll
-    for (int strain = 0; strain < 2; strain++) {
-        const uint32_t status = strain ? ((st >> 8) & 0xFFu) : (st & 0xFFu);
-        const uint32_t dday = strain ? (st >> 24) : ((st >> 16) & 0xFFu);
-        prob[strain] = -1.f;
-        if (status >= 2u) {
-            const int pd = day - (int)dday;
-            if (pd >= 0 && pd < 10) prob[strain] = infection_probability(c, (int)status - 2, pd, strain, ksum);
-        }
-    }
-}
-
 template <bool WEEKEND>
 __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
 {
@@ -2159,12 +2162,12 @@ __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
             const int prof = (int)(q3 % 6u);   // word 3 of block R (:1892)
             const uint32_t v0 = __shfl_sync(kFull, blk[0], gl + 1), v1 = __shfl_sync(kFull, blk[1], gl + 1);
             if (j < 3) {
-                kv = select_victim(me, hoff, hcnt, wc, true, nullptr, victim);
+                kv = select_victim(me, hoff, hcnt, wc, victim);
             } else if (j < 5) {
                 const int loc = a.keys[ik.kbase + 3 * (size_t)lme + c_weekend_assign[prof][j - 3]];
                 const uint2 slot = a.bkt[loc];
                 const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
-                kv = select_victim(me, eoff, ecnt, j == 3 ? v0 : v1, false, a.bkt_people, victim);
+                kv = select_victim(me, eoff, ecnt, j == 3 ? v0 : v1, victim, a.bkt_people);
             }
         } else {
             const bool adult = prec_age(rec.w) == 5;
@@ -2174,9 +2177,9 @@ __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
             const int pv6 = __shfl_sync(kFull, pv, gl + 6);   // every lane takes part in the shuffle
             const int prof = adult ? pv6 : 3;
             if (j < 3) {
-                kv = select_victim(me, hoff, hcnt, wc, true, nullptr, victim);
+                kv = select_victim(me, hoff, hcnt, wc, victim);
             } else if (j < 3 + desired) {
-                kv = select_victim(me, (int)rec.y, (int)rec.z, wc, false, a.wp_people, victim);
+                kv = select_victim(me, (int)rec.y, (int)rec.z, wc, victim, a.wp_people);
             } else {
                 const int e = j - 3 - desired, want0 = c_weekday_assign[prof][0], want1 = c_weekday_assign[prof][1];
                 const int hour = e < want0 ? 0 : (e < want0 + want1 ? 1 : -1);
@@ -2184,7 +2187,7 @@ __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
                     const int dest = a.keys[ik.kbase + (size_t)hour * c.N + lme];
                     const uint2 slot = a.bkt[dest];
                     const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
-                    kv = select_victim(me, eoff, ecnt, wc, false, a.bkt_people, victim);
+                    kv = select_victim(me, eoff, ecnt, wc, victim, a.bkt_people);
                 }
             }
         }
