@@ -186,7 +186,7 @@ pt_status pt_get_day_stage_ms(pt_sim *sim, int day, float ms[8]);
  * run time, by the caller or by pt_autotune.  Every choice gives bit-identical
  * results; only the speed differs. */
 typedef struct pt_tuning {
-    int infect_coop;            /* 0: one thread per infector; 1: eight lanes per infector */
+    int infect_coop;            /* 1: eight lanes per infector on every day; 0: on days of few infectors only */
     int infect_blocks_per_sm;   /* infection grid, 256-thread blocks per SM: 1..32 */
     int radix_blocks_per_sm;    /* persistent blocks of a day's radix pass per SM: 1..4
                                    (three fit; 4 runs as 3) */

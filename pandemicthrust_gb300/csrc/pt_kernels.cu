@@ -1917,151 +1917,11 @@ struct InfectArgs {
     unsigned long long *claim;
     int32_t *new_list;
     Scalars *sc;
+    int coop_most;   // up to this many infectors, eight lanes work on one
 };
 
 // An infector's packed record: one 128-bit read-only load.
 __device__ __forceinline__ uint4 load_record(const uint4 *prec, int me) { return __ldg(&prec[me]); }
-
-// kernel_doWeekday + device_makeContacts_weekday (PandemicSim.cu:3236-3308, :1669-1829),
-// one thread per infector.  Bound by random 32-byte sectors (record, keys, bucket
-// slots, tables, victims, claims) and by how many a warp has in flight, so each kind is
-// loaded for all contacts together: 36 ms of a 48-instance run's weekdays on a GB300, 42
-// with every contact's loads after the last one's.
-__global__ void __launch_bounds__(128) k_infect_weekday(InfectArgs a, int day)
-{
-    Scalars *sc = a.sc;
-    if (sc->done) return;
-    const int I = sc->infected;
-    const ClaimQueue queue = claim_queue<4>(a.new_list, sc);
-    const int lane = threadIdx.x & 31;
-    for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < I; base += gridDim.x * blockDim.x) {
-        queue.flush(kQueueRun, lane);
-        const int pos = base + lane;
-        if (pos >= I) continue;   // (the last round; the warp meets again at the flush)
-        const int inst = a.infected_inst[pos];
-        const InstConst &ik = a.ic[inst];
-        const SimConst &c = ik.c;
-        const InstState &s = a.is[inst];
-        const TfKey key = make_key(c);
-        Infector inf;
-        inf.pos = pos;
-        inf.me = a.infected[pos];
-        const int me = inf.me;
-        const int lme = me - ik.pbase;  // the instance's person number
-        const unsigned long long ctr = s.infect_offset + 6ull * (unsigned long long)(pos - s.start);
-        const uint4 rec = load_record(a.prec, me);
-        uint32_t w[8];
-        tf2x64(key, ctr, w);
-        tf2x64(key, ctr + 1, w + 4);
-        const bool adult = prec_age(rec.w) == 5;
-        const uint32_t mine = a.state[me];
-        // errands / afterschool: destinations from today's keys
-        const int32_t *kk = a.keys + ik.kbase;
-        const uint2 slot0 = a.bkt[kk[lme]], slot1 = a.bkt[kk[c.N + lme]];
-        infector_gens(inf, mine, a.gen_p, a.gen_s);
-        // the adult profile is regenerated from the schedule counter (:3667-3705)
-        int prof = 3;
-        if (adult) {
-            uint32_t e[4];
-            tf2x64(key, s.errand_offset + (uint64_t)(lme / 2), e);
-            const int slot = 2 * (lme % 2);
-            prof = (int)((e[slot] ^ e[slot + 1]) % 3u);
-        }
-        int victims[8], kv[8];
-        // household: offset + r % count, the household table is the identity
-        const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
-#pragma unroll
-        for (int j = 0; j < 3; j++) kv[j] = select_victim(me, hoff, hcnt, w[j], victims[j]);
-        // then the workplace's or school's max-contacts, then each errand hour's
-        const int desired = prec_desired(rec.w);
-        const int want0 = c_weekday_assign[prof][0], want = want0 + c_weekday_assign[prof][1];
-        int off[5], cnt[5];
-        const int32_t *table[5];
-#pragma unroll
-        for (int j = 0; j < 5; j++) {
-            const int e = j - desired;
-            const uint2 slot = e < want0 ? slot0 : slot1;
-            off[j] = e < 0 ? (int)rec.y : bucket_start(slot);
-            cnt[j] = e < 0 ? (int)rec.z : (e < want ? bucket_count(slot) : 0);
-            table[j] = e < 0 ? a.wp_people : a.bkt_people;
-        }
-        select_victims<5>(me, off, cnt, table, w + 3, victims + 3, kv + 3);
-        int ksum = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) ksum += kv[j];
-        infector_probs(c, mine, day, ksum, inf.prob);
-        // interventions: a closed school or an absent adult voids the workplace / school
-        // contacts; they keep their share of ksum, so the contact does not happen
-        // rather than passing its weight to the others
-        if (desired > 0 && (ik.absent_thr != 0 || (day >= ik.closure_start && day < ik.closure_end))) {
-            const bool closed = day >= ik.closure_start && day < ik.closure_end && prec_school(rec.w);
-            const bool me_absent =
-                adult && intervention_hash(c.key0, c.key1, kTagAbsent, day, lme) < ik.absent_thr;
-            int age[3];
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                age[j] = 0;
-                if (j < desired && kv[3 + j] != 0 && ik.absent_thr != 0) age[j] = a.age[victims[3 + j]];
-            }
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                const bool v_absent = age[j] == 5 && intervention_hash(c.key0, c.key1, kTagAbsent, day,
-                                                                       victims[3 + j] - ik.pbase) < ik.absent_thr;
-                if (j < desired && (closed || me_absent || v_absent)) kv[3 + j] = 0;
-            }
-        }
-        process_contacts<8>(c, key, inf, ctr + 2, victims, kv, a.state, a.claim, queue);
-    }
-    queue.flush(1, lane);
-}
-
-// kernel_doWeekend + device_makeContacts_weekend (PandemicSim.cu:3311-3379, :1833-1950)
-__global__ void __launch_bounds__(128) k_infect_weekend(InfectArgs a, int day)
-{
-    Scalars *sc = a.sc;
-    if (sc->done) return;
-    const int I = sc->infected;
-    const ClaimQueue queue = claim_queue<4>(a.new_list, sc);
-    const int lane = threadIdx.x & 31;
-    for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < I; base += gridDim.x * blockDim.x) {
-        queue.flush(kQueueRun, lane);
-        const int pos = base + lane;
-        if (pos >= I) continue;   // (the last round; the warp meets again at the flush)
-        const int inst = a.infected_inst[pos];
-        const InstConst &ik = a.ic[inst];
-        const SimConst &c = ik.c;
-        const InstState &s = a.is[inst];
-        const TfKey key = make_key(c);
-        Infector inf;
-        inf.pos = pos;
-        inf.me = a.infected[pos];
-        const int me = inf.me;
-        const int lme = me - ik.pbase;
-        const unsigned long long ctr = s.infect_offset + 6ull * (unsigned long long)(pos - s.start);
-        const uint4 rec = load_record(a.prec, me);
-        const uint32_t mine = a.state[me];
-        uint32_t w[4];
-        tf2x64(key, ctr, w);
-        const int prof = (int)(w[3] % 6u);
-        const int32_t *k3 = a.keys + ik.kbase + 3 * (size_t)lme;
-        const uint2 slot0 = a.bkt[k3[c_weekend_assign[prof][0]]], slot1 = a.bkt[k3[c_weekend_assign[prof][1]]];
-        infector_gens(inf, mine, a.gen_p, a.gen_s);
-        // Threefry-2x32 on the low seed words with counter (u32)(ctr + 1) (:1895-1901)
-        uint32_t v2[2];
-        tf2x32(key, (uint32_t)(ctr + 1), v2);
-        int victims[5], kv[5];
-        const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
-#pragma unroll
-        for (int j = 0; j < 3; j++) kv[j] = select_victim(me, hoff, hcnt, w[j], victims[j]);
-        const int off[2] = {bucket_start(slot0), bucket_start(slot1)};
-        const int cnt[2] = {bucket_count(slot0), bucket_count(slot1)};
-        const int32_t *const table[2] = {a.bkt_people, a.bkt_people};
-        select_victims<2>(me, off, cnt, table, v2, victims + 3, kv + 3);
-        infector_probs(c, mine, day, kv[0] + kv[1] + kv[2] + kv[3] + kv[4], inf.prob);
-        process_contacts<5>(c, key, inf, ctr + 2, victims, kv, a.state, a.claim, queue);
-    }
-    queue.flush(1, lane);
-}
 
 // ---------------------------------------------------- warp-cooperative contacts
 // The same draws with eight lanes per infector (four infectors per warp round).  Lane
@@ -2076,6 +1936,12 @@ __global__ void __launch_bounds__(128) k_infect_weekend(InfectArgs a, int day)
 // is a shuffle reduction over the group.  Every draw, victim and claim key equals the
 // one-thread-per-infector kernels' (same counters, same words, same slots).
 constexpr unsigned kFull = 0xffffffffu;
+// The thread-per-infector kernels work this way themselves on a day of at most
+// kCoopPerSm infectors an SM, where a thread's seven Threefry blocks in a row take longer
+// than the chip is busy: 10 us instead of 13 for a weekday of 100,000 persons, 1.12 ms
+// instead of 1.31 for the weekdays of a 1M run (64, 192 and 320 an SM: 1.19, 1.18, 1.23);
+// on larger days one thread an infector is faster (12M: 10 ms, 17.5 this way).
+constexpr int kCoopPerSm = 128;
 
 __device__ __forceinline__ uint32_t pick4(int i, uint32_t q0, uint32_t q1, uint32_t q2, uint32_t q3)
 {
@@ -2121,12 +1987,8 @@ __device__ __forceinline__ void claim_slot(const SimConst &c, const InfectArgs &
 }
 
 template <bool WEEKEND>
-__global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
+__device__ __forceinline__ void infect_coop(const InfectArgs &a, int day, int I, const ClaimQueue &queue)
 {
-    Scalars *sc = a.sc;
-    if (sc->done) return;
-    const int I = sc->infected;
-    const ClaimQueue queue = claim_queue<8>(a.new_list, sc);
     const int lane = threadIdx.x & 31, j = lane & 7, gl = lane & ~7;
     const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
@@ -2218,6 +2080,164 @@ __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
     queue.flush(1, lane);
 }
 
+template <bool WEEKEND>
+__global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
+{
+    Scalars *sc = a.sc;
+    if (sc->done) return;
+    infect_coop<WEEKEND>(a, day, sc->infected, claim_queue<8>(a.new_list, sc));
+}
+
+// kernel_doWeekday + device_makeContacts_weekday (PandemicSim.cu:3236-3308, :1669-1829),
+// one thread per infector.  Bound by random 32-byte sectors (record, keys, bucket
+// slots, tables, victims, claims) and by how many a warp has in flight, so each kind is
+// loaded for all contacts together: 36 ms of a 48-instance run's weekdays on a GB300, 42
+// with every contact's loads after the last one's.  Eight blocks an SM (64 registers) are
+// as good as six (80) there and better than ten (38 ms) or twelve (43).
+__global__ void __launch_bounds__(128, 8) k_infect_weekday(InfectArgs a, int day)
+{
+    Scalars *sc = a.sc;
+    if (sc->done) return;
+    const int I = sc->infected;
+    const ClaimQueue queue = claim_queue<4>(a.new_list, sc);
+    if (I <= a.coop_most) {
+        infect_coop<false>(a, day, I, queue);
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < I; base += gridDim.x * blockDim.x) {
+        queue.flush(kQueueRun, lane);
+        const int pos = base + lane;
+        if (pos >= I) continue;   // (the last round; the warp meets again at the flush)
+        const int inst = a.infected_inst[pos];
+        const InstConst &ik = a.ic[inst];
+        const SimConst &c = ik.c;
+        const InstState &s = a.is[inst];
+        const TfKey key = make_key(c);
+        Infector inf;
+        inf.pos = pos;
+        inf.me = a.infected[pos];
+        const int me = inf.me;
+        const int lme = me - ik.pbase;  // the instance's person number
+        const unsigned long long ctr = s.infect_offset + 6ull * (unsigned long long)(pos - s.start);
+        const uint4 rec = load_record(a.prec, me);
+        uint32_t w[8];
+        tf2x64(key, ctr, w);
+        tf2x64(key, ctr + 1, w + 4);
+        const bool adult = prec_age(rec.w) == 5;
+        const uint32_t mine = a.state[me];
+        // errands / afterschool: destinations from today's keys
+        const int32_t *kk = a.keys + ik.kbase;
+        const uint2 slot0 = a.bkt[kk[lme]], slot1 = a.bkt[kk[c.N + lme]];
+        infector_gens(inf, mine, a.gen_p, a.gen_s);
+        // the adult profile is regenerated from the schedule counter (:3667-3705)
+        int prof = 3;
+        if (adult) {
+            uint32_t e[4];
+            tf2x64(key, s.errand_offset + (uint64_t)(lme / 2), e);
+            const int slot = 2 * (lme % 2);
+            prof = (int)((e[slot] ^ e[slot + 1]) % 3u);
+        }
+        int victims[8], kv[8];
+        // household: offset + r % count, the household table is the identity
+        const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
+#pragma unroll
+        for (int j = 0; j < 3; j++) kv[j] = select_victim(me, hoff, hcnt, w[j], victims[j]);
+        // then the workplace's or school's max-contacts, then each errand hour's
+        const int desired = prec_desired(rec.w);
+        const int want0 = c_weekday_assign[prof][0], want = want0 + c_weekday_assign[prof][1];
+        int off[5], cnt[5];
+        const int32_t *table[5];
+#pragma unroll
+        for (int j = 0; j < 5; j++) {
+            const int e = j - desired;
+            const uint2 slot = e < want0 ? slot0 : slot1;
+            off[j] = e < 0 ? (int)rec.y : bucket_start(slot);
+            cnt[j] = e < 0 ? (int)rec.z : (e < want ? bucket_count(slot) : 0);
+            table[j] = e < 0 ? a.wp_people : a.bkt_people;
+        }
+        select_victims<5>(me, off, cnt, table, w + 3, victims + 3, kv + 3);
+        int ksum = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) ksum += kv[j];
+        infector_probs(c, mine, day, ksum, inf.prob);
+        // interventions: a closed school or an absent adult voids the workplace / school
+        // contacts; they keep their share of ksum, so the contact does not happen
+        // rather than passing its weight to the others
+        if (desired > 0 && (ik.absent_thr != 0 || (day >= ik.closure_start && day < ik.closure_end))) {
+            const bool closed = day >= ik.closure_start && day < ik.closure_end && prec_school(rec.w);
+            const bool me_absent =
+                adult && intervention_hash(c.key0, c.key1, kTagAbsent, day, lme) < ik.absent_thr;
+            int age[3];
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                age[j] = 0;
+                if (j < desired && kv[3 + j] != 0 && ik.absent_thr != 0) age[j] = a.age[victims[3 + j]];
+            }
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const bool v_absent = age[j] == 5 && intervention_hash(c.key0, c.key1, kTagAbsent, day,
+                                                                       victims[3 + j] - ik.pbase) < ik.absent_thr;
+                if (j < desired && (closed || me_absent || v_absent)) kv[3 + j] = 0;
+            }
+        }
+        process_contacts<8>(c, key, inf, ctr + 2, victims, kv, a.state, a.claim, queue);
+    }
+    queue.flush(1, lane);
+}
+
+// kernel_doWeekend + device_makeContacts_weekend (PandemicSim.cu:3311-3379, :1833-1950)
+__global__ void __launch_bounds__(128, 8) k_infect_weekend(InfectArgs a, int day)
+{
+    Scalars *sc = a.sc;
+    if (sc->done) return;
+    const int I = sc->infected;
+    const ClaimQueue queue = claim_queue<4>(a.new_list, sc);
+    if (I <= a.coop_most) {
+        infect_coop<true>(a, day, I, queue);
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < I; base += gridDim.x * blockDim.x) {
+        queue.flush(kQueueRun, lane);
+        const int pos = base + lane;
+        if (pos >= I) continue;   // (the last round; the warp meets again at the flush)
+        const int inst = a.infected_inst[pos];
+        const InstConst &ik = a.ic[inst];
+        const SimConst &c = ik.c;
+        const InstState &s = a.is[inst];
+        const TfKey key = make_key(c);
+        Infector inf;
+        inf.pos = pos;
+        inf.me = a.infected[pos];
+        const int me = inf.me;
+        const int lme = me - ik.pbase;
+        const unsigned long long ctr = s.infect_offset + 6ull * (unsigned long long)(pos - s.start);
+        const uint4 rec = load_record(a.prec, me);
+        const uint32_t mine = a.state[me];
+        uint32_t w[4];
+        tf2x64(key, ctr, w);
+        const int prof = (int)(w[3] % 6u);
+        const int32_t *k3 = a.keys + ik.kbase + 3 * (size_t)lme;
+        const uint2 slot0 = a.bkt[k3[c_weekend_assign[prof][0]]], slot1 = a.bkt[k3[c_weekend_assign[prof][1]]];
+        infector_gens(inf, mine, a.gen_p, a.gen_s);
+        // Threefry-2x32 on the low seed words with counter (u32)(ctr + 1) (:1895-1901)
+        uint32_t v2[2];
+        tf2x32(key, (uint32_t)(ctr + 1), v2);
+        int victims[5], kv[5];
+        const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
+#pragma unroll
+        for (int j = 0; j < 3; j++) kv[j] = select_victim(me, hoff, hcnt, w[j], victims[j]);
+        const int off[2] = {bucket_start(slot0), bucket_start(slot1)};
+        const int cnt[2] = {bucket_count(slot0), bucket_count(slot1)};
+        const int32_t *const table[2] = {a.bkt_people, a.bkt_people};
+        select_victims<2>(me, off, cnt, table, v2, victims + 3, kv + 3);
+        infector_probs(c, mine, day, kv[0] + kv[1] + kv[2] + kv[3] + kv[4], inf.prob);
+        process_contacts<5>(c, key, inf, ctr + 2, victims, kv, a.state, a.claim, queue);
+    }
+    queue.flush(1, lane);
+}
+
 cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_t s)
 {
     InfectArgs a;
@@ -2229,6 +2249,7 @@ cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_
     a.infected_inst = d.infected_inst;
     a.claim = d.claim; a.new_list = d.new_list; a.sc = d.sc;
     const Tuning &t = d.tune;
+    a.coop_most = kCoopPerSm * sm_count();
     if (t.infect_coop) {
         const int blocks = sm_count() * t.infect_blocks_per_sm;
         if (weekend) k_infect_coop<true><<<blocks, 256, 0, s>>>(a, day);

@@ -88,7 +88,7 @@ struct Scalars {
 // Launch shapes chosen at run time (the engine's tuner picks them per engine; every
 // choice gives bit-identical results, only the speed differs).
 struct Tuning {
-    int infect_coop = 0;            // 1: warp-cooperative contacts (8 lanes per infector)
+    int infect_coop = 0;            // 1: eight lanes per infector on every day, 0: on days of few
     int infect_blocks_per_sm = 8;   // infection grid: 256-thread blocks per SM (twice as
                                     // many 128-thread blocks for the thread-per-infector kernels)
     int radix_blocks_per_sm = 4;    // persistent blocks of a day's radix pass per SM (1..4;
