@@ -762,7 +762,8 @@ __global__ void k_reset_instances(const InstConst *ic, InstState *is, int K)
     for (int i = threadIdx.x; i < (int)(sizeof(InstState) / 4); i += blockDim.x) w[i] = 0;
     __syncthreads();
     if (threadIdx.x == 0)
-        is[k].rand_offset = (unsigned long long)(ic[k].c.H / 4) + (unsigned long long)(ic[k].c.N / 4);
+        is[k].rand_offset = is[k].next_offset[0] =
+            (unsigned long long)(ic[k].c.H / 4) + (unsigned long long)(ic[k].c.N / 4);
 }
 
 cudaError_t launch_reset_instances(const DevArrays &d, cudaStream_t s)
@@ -864,6 +865,13 @@ __device__ __forceinline__ bool instance_running(const InstConst &c, const InstS
     return !s.done && day < c.max_days;
 }
 
+// R0 of a day whose schedule starts at counter E0.
+__device__ __forceinline__ unsigned long long contact_offset(const InstConst &c, unsigned long long E0, bool weekend)
+{
+    const unsigned long long N = (unsigned long long)c.c.N;
+    return E0 + (weekend ? 2ull * N : N / 2ull);
+}
+
 // Sweep: one tile of 4096 persons per block; each thread holds 4 rounds of 4
 // persons (one 16-byte load per round).  Output order is (round, thread, item),
 // which is ascending person order within the tile.
@@ -937,9 +945,12 @@ __device__ __forceinline__ void sweep_flush_bins(InstState *is, int k, int day, 
 __global__ void __launch_bounds__(kSweepThreads, 8) k_sweep_count(const InstConst *ic, InstState *is,
                                                                   const int32_t *tile_inst, int tiles, int per_block,
                                                                   uint32_t *state, uint16_t *flags_out,
-                                                                  int32_t *tile_count, const Scalars *sc, int day)
+                                                                  int32_t *tile_count, uint2 *clear, int clear_n,
+                                                                  const Scalars *sc, int day)
 {
     if (*(volatile const int *)&sc->done) return;
+    for (int i = blockIdx.x * kSweepThreads + threadIdx.x; i < clear_n; i += gridDim.x * kSweepThreads)
+        clear[i] = make_uint2(0u, 0u);
     const int t0 = blockIdx.x * per_block;
     const int t1 = t0 + per_block < tiles ? t0 + per_block : tiles;
     const int d2r = day - 10;
@@ -965,17 +976,17 @@ __global__ void __launch_bounds__(kSweepThreads, 8) k_sweep_count(const InstCons
         // end of the tile's persons: none when the instance no longer runs
         const long long N = instance_running(ic[k], is[k], day) ? (long long)ic[k].pbase + ic[k].c.N : tile_base;
         uint32_t flags = 0;  // bit (4*round + item)
+        auto load = [&](int r) {
+            const long long p0 = tile_base + ((long long)r * kSweepThreads + threadIdx.x) * 4;
+            if (p0 < N) return *reinterpret_cast<const uint4 *>(state + p0);   // (padding persons follow)
+            return make_uint4(0u, 0u, 0u, 0u);
+        };
+        uint4 next = load(0);   // a round's load goes before the last round's stores
 #pragma unroll
         for (int r = 0; r < kSweepRounds; r++) {
             long long p0 = tile_base + ((long long)r * kSweepThreads + threadIdx.x) * 4;
-            uint32_t st[4];
-            if (p0 + 3 < N) {
-                uint4 v = *reinterpret_cast<const uint4 *>(state + p0);
-                st[0] = v.x; st[1] = v.y; st[2] = v.z; st[3] = v.w;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) st[j] = (p0 + j < N) ? state[p0 + j] : 0u;
-            }
+            const uint32_t st[4] = {next.x, next.y, next.z, next.w};
+            if (r + 1 < kSweepRounds) next = load(r + 1);
             bool any_changed = false;
             uint32_t out[4];
 #pragma unroll
@@ -1017,6 +1028,54 @@ __global__ void __launch_bounds__(kSweepThreads, 8) k_sweep_count(const InstCons
 
 constexpr int kSweepScanThreads = 1024;
 
+// A running instance's day (runToCompletion, PandemicSim.cu:891-937): its run
+// [start, end) of the infected list, the statistics row, the stop on zero infected, the
+// counter offsets E0 / R0 of the schedule and the contacts.  The day's first counter is
+// next_offset[day & 1], which nothing writes that day (k_sweep_list's blocks read it
+// while one of them is here).
+__device__ __forceinline__ void begin_instance_day(const InstConst &c, InstState &s, int start, int end, int day,
+                                                   int dense_level)
+{
+    const bool weekend = (day % 7) >= 5;  // PandemicSim.h:283-284
+    s.start = start;
+    s.list_end = end;
+    s.marked = 0;
+    s.dense = 0;
+    if (!instance_running(c, s, day)) {
+        s.infected = 0;
+        return;
+    }
+    const int I = end - start;
+    s.infected = I;
+    // When the infected (each marks one or two buckets) are many against the
+    // buckets, most buckets will be read, and the sort can read the schedule keys
+    // directly: dense_level 1, 2, 3 take I >= B / 4, I >= B, I >= 2 B; 0 never.
+    // Either way the tables are the same.
+    const long long B = c.bcount[weekend ? 1 : 0];
+    s.dense = dense_level > 0 && 4ll * I >= B * (dense_level == 1 ? 1 : (dense_level == 2 ? 4 : 8)) ? 1 : 0;
+    s.infected_per_day[day] = I;
+    s.day = day;
+    s.days_run = day + 1;
+    if (I == 0) {
+        s.done = 1;
+        return;
+    }
+    const unsigned long long E0 = s.next_offset[day & 1], R0 = contact_offset(c, E0, weekend);
+    s.errand_offset = E0;
+    s.infect_offset = R0;
+    s.rand_offset = s.next_offset[(day + 1) & 1] = R0 + 6ull * (unsigned long long)I;
+}
+
+// The batch's day; done holds the number of days run (so that a block of the launch that
+// sets it can tell the day's own end from an earlier one).
+__device__ __forceinline__ void begin_day(Scalars *sc, int total, int day)
+{
+    sc->infected = total;
+    sc->day = day;
+    sc->new_count = 0;
+    if (total == 0) sc->done = day + 1;
+}
+
 __global__ void __launch_bounds__(kSweepScanThreads) k_sweep_scan(const InstConst *ic, InstState *is, int K,
                                                                   int32_t *tile_count, int tiles, Scalars *sc,
                                                                   int day, int dense_level)
@@ -1036,49 +1095,10 @@ __global__ void __launch_bounds__(kSweepScanThreads) k_sweep_scan(const InstCons
     }
     if (threadIdx.x == 0) tile_count[tiles] = total;
     __syncthreads();
-    // each running instance's day (runToCompletion, PandemicSim.cu:891-937: the
-    // statistics row, the stop on zero infected, the counter offsets E0 / R0 of the
-    // schedule and the contacts)
-    const bool weekend = (day % 7) >= 5;  // PandemicSim.h:283-284
-    for (int k = threadIdx.x; k < K; k += kSweepScanThreads) {
-        InstState &s = is[k];
-        const int start = tile_count[ic[k].pbase / kSweepTile], end = tile_count[ic[k].pend / kSweepTile];
-        s.start = start;
-        s.list_end = end;
-        s.marked = 0;
-        s.dense = 0;
-        if (!instance_running(ic[k], s, day)) {
-            s.infected = 0;
-            continue;
-        }
-        const int I = end - start;
-        s.infected = I;
-        // When the infected (each marks one or two buckets) are many against the
-        // buckets, most buckets will be read, and the sort can read the schedule keys
-        // directly: dense_level 1, 2, 3 take I >= B / 4, I >= B, I >= 2 B; 0 never.
-        // Either way the tables are the same.
-        const long long B = ic[k].bcount[weekend ? 1 : 0];
-        s.dense = dense_level > 0 && 4ll * I >= B * (dense_level == 1 ? 1 : (dense_level == 2 ? 4 : 8)) ? 1 : 0;
-        s.infected_per_day[day] = I;
-        s.day = day;
-        s.days_run = day + 1;
-        if (I == 0) {
-            s.done = 1;
-        } else {
-            const unsigned long long N = (unsigned long long)ic[k].c.N;
-            const unsigned long long E0 = s.rand_offset;
-            const unsigned long long R0 = E0 + (weekend ? 2ull * N : N / 2ull);
-            s.errand_offset = E0;
-            s.infect_offset = R0;
-            s.rand_offset = R0 + 6ull * (unsigned long long)I;
-        }
-    }
-    if (threadIdx.x == 0) {
-        sc->infected = total;
-        sc->day = day;
-        sc->new_count = 0;
-        if (total == 0) sc->done = 1;
-    }
+    for (int k = threadIdx.x; k < K; k += kSweepScanThreads)
+        begin_instance_day(ic[k], is[k], tile_count[ic[k].pbase / kSweepTile], tile_count[ic[k].pend / kSweepTile], day,
+                           dense_level);
+    if (threadIdx.x == 0) begin_day(sc, total, day);
 }
 
 // Emit for small runs: a block per person tile, a block scan of the threads' packed
@@ -1164,35 +1184,6 @@ __global__ void __launch_bounds__(kEmitWarps * 32) k_sweep_emit(const int32_t *t
     }
 }
 
-cudaError_t launch_sweep(const DevArrays &d, int day, cudaStream_t s)
-{
-    const int tiles = d.P / kSweepTile;
-    // several tiles per block only where the grid still fills every SM eight times over
-    // (a small simulation keeps one tile per block and all its parallelism)
-    const int per_block = tiles >= kSweepTilesPerBlock * 8 * sm_count() ? kSweepTilesPerBlock : 1;
-    k_sweep_count<<<div_up(tiles, per_block), kSweepThreads, 0, s>>>(d.ic, d.is, d.tile_inst, tiles, per_block, d.state,
-                                                                    d.sweep_flags, d.sweep_tiles, d.sc, day);
-    count_launch();
-    k_sweep_scan<<<1, kSweepScanThreads, 0, s>>>(d.ic, d.is, d.K, d.sweep_tiles, tiles, d.sc, day,
-                                                 d.tune.dense_level);
-    count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_infected_list(const DevArrays &d, cudaStream_t s)
-{
-    const int tiles = d.P / kSweepTile;
-    if (tiles >= kSweepTilesPerBlock * 8 * sm_count())
-        k_sweep_emit<<<div_up(tiles, kEmitWarps), kEmitWarps * 32, 0, s>>>(d.tile_inst, tiles, d.sweep_flags,
-                                                                           d.sweep_tiles, d.infected, d.infected_inst,
-                                                                           d.sc);
-    else
-        k_sweep_emit_block<<<tiles, kSweepThreads, 0, s>>>(d.tile_inst, d.sweep_flags, d.sweep_tiles, d.infected,
-                                                           d.infected_inst, d.sc);
-    count_launch();
-    return cudaGetLastError();
-}
-
 // ------------------------------------------------------------------ schedules
 // Weekday schedule (kernel_assignWeekdayAfterschoolAndErrands, PandemicSim.cu:2972-3022):
 // counter E0 + g -> the instance's persons 2g, 2g+1.  Hour-0 keys at [0,N), hour-1
@@ -1238,6 +1229,34 @@ __device__ __forceinline__ void mark_bucket_shared(uint32_t *s_mark, int b)
     if (!(*(volatile uint32_t *)&s_mark[b >> 5] & bit)) atomicOr(&s_mark[b >> 5], bit);
 }
 
+// The buckets (global) that today's contact draws of an infected person read, -1 for
+// none: `person` global, lpos its place in its instance's infected list.
+__device__ __forceinline__ int2 read_buckets(const InstConst &ik, const uint8_t *age, int weekend, unsigned long long E0,
+                                             unsigned long long R0, int person, int lpos)
+{
+    const SimConst &c = ik.c;
+    const TfKey key = make_key(c);
+    const int me = person - ik.pbase;   // the instance's person number
+    uint32_t w[4];
+    if (weekend) {
+        const int lo = c.type_offset[9], R = c.L - lo;
+        int d[3];
+        weekend_errands(c, key, E0 + 2ull * (unsigned long long)me, lo, R, d);
+        tf2x64(key, R0 + 6ull * (unsigned long long)lpos, w);
+        const int prof = (int)(w[3] % 6u);
+        return make_int2(ik.bbase[1] + d[c_weekend_assign[prof][0]], ik.bbase[1] + d[c_weekend_assign[prof][1]]);
+    }
+    const int lo = c.type_offset[8], R = c.L - lo;
+    tf2x64(key, E0 + (uint64_t)(me / 2), w);
+    const bool adult = age[person] == 5;
+    const int slot = 2 * (me & 1);
+    int k1, k2;
+    weekday_pair_keys(c, w, me & 1, adult, lo, R, k1, k2);
+    const int prof = adult ? (int)((w[slot] ^ w[slot + 1]) % 3u) : 3;
+    return make_int2(c_weekday_assign[prof][0] > 0 ? ik.bbase[0] + k1 : -1,
+                     c_weekday_assign[prof][1] > 0 ? ik.bbase[0] + k2 : -1);
+}
+
 // Marks the errand buckets today's contact draws will read: the only buckets that
 // must be materialised.  Destinations are regenerated from the schedule counter, as
 // the reference's device_recalc_* functions do (PandemicSim.cu:3667-3705,
@@ -1270,44 +1289,14 @@ __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *
     }
     for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < I; pos += gridDim.x * blockDim.x) {
         const int k = infected_inst[pos];
-        const InstConst &ik = ic[k];
-        const SimConst &c = ik.c;
         const InstState &s = is[k];
-        const TfKey key = make_key(c);
-        const int me = infected[pos] - ik.pbase;   // the instance's person number
-        const int lpos = pos - s.start;            // the instance's list position
-        if (weekend) {
-            const int lo = c.type_offset[9], R = c.L - lo;
-            int d[3];
-            weekend_errands(c, key, s.errand_offset + 2ull * (unsigned long long)me, lo, R, d);
-            uint32_t w[4];
-            tf2x64(key, s.infect_offset + 6ull * (unsigned long long)lpos, w);
-            const int prof = (int)(w[3] % 6u);
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const int b = ik.bbase[1] + d[c_weekend_assign[prof][j]];
-                if (shared) mark_bucket_shared(s_mark, b);
-                else mark_bucket(mark, b);
-            }
+        const int2 b = read_buckets(ic[k], age, weekend, s.errand_offset, s.infect_offset, infected[pos], pos - s.start);
+        if (shared) {
+            if (b.x >= 0) mark_bucket_shared(s_mark, b.x);
+            if (b.y >= 0) mark_bucket_shared(s_mark, b.y);
         } else {
-            const int lo = c.type_offset[8], R = c.L - lo;
-            uint32_t w[4];
-            tf2x64(key, s.errand_offset + (uint64_t)(me / 2), w);
-            const bool adult = age[infected[pos]] == 5;
-            const int slot = 2 * (me & 1);
-            int k1, k2;
-            weekday_pair_keys(c, w, me & 1, adult, lo, R, k1, k2);
-            k1 += ik.bbase[0];
-            k2 += ik.bbase[0];
-            const int prof = adult ? (int)((w[slot] ^ w[slot + 1]) % 3u) : 3;
-            if (c_weekday_assign[prof][0] > 0) {
-                if (shared) mark_bucket_shared(s_mark, k1);
-                else mark_bucket(mark, k1);
-            }
-            if (c_weekday_assign[prof][1] > 0) {
-                if (shared) mark_bucket_shared(s_mark, k2);
-                else mark_bucket(mark, k2);
-            }
+            if (b.x >= 0) mark_bucket(mark, b.x);
+            if (b.y >= 0) mark_bucket(mark, b.y);
         }
     }
     if (shared) {
@@ -1319,6 +1308,161 @@ __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *
             if (s_mark[w]) red_or(&mark[w], s_mark[w]);
         }
     }
+}
+
+// A small run's list and marks in one launch instead of three (scan, emit, mark): a block
+// per person tile sums the counts of the tiles itself, emits its part of the list and
+// marks its persons' buckets.  The block of an instance's first tile begins the
+// instance's day, the last tile's block the batch's; no block waits for another.  Small
+// runs are bound by their launches: a day of 100,000 persons has seven of 3 to 10 us.
+// Up to kListTiles tiles (4M persons) the sums are four loads a thread.
+constexpr int kListTiles = 4 * kSweepThreads;
+constexpr int kListMarkWords = 2048;   // a bitmap this small is marked in shared memory and merged once a block
+
+__global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *ic, InstState *is, const int32_t *tile_inst,
+                                                              int tiles, const uint16_t *flags_in,
+                                                              const int32_t *tile_count, int32_t *infected,
+                                                              int32_t *infected_inst, const uint8_t *age, uint32_t *mark,
+                                                              int words, int mark_all, Scalars *sc, int day,
+                                                              int dense_level)
+{
+    const int ended = *(volatile const int *)&sc->done;
+    if (ended != 0 && ended != day + 1) return;
+    const bool weekend = (day % 7) >= 5;
+    const int tile = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t f = flags_in[(size_t)tile * kSweepThreads + t];
+    const int k = tile_inst[tile], n = tile_count[tile];
+    const InstConst &ik = ic[k];
+    const unsigned long long E0 = is[k].next_offset[day & 1];
+    const int first = ik.pbase / kSweepTile, end = ik.pend / kSweepTile;
+    // infected before the instance, in it before the tile, in it from the tile on, behind it
+    int sum[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int q = 0; q < kListTiles / kSweepThreads; q++) {
+        const int i = t + q * kSweepThreads;
+        const int c = i < tiles ? tile_count[i] : 0;
+        if (i < first) sum[0] += c;
+        else if (i < tile) sum[1] += c;
+        else if (i < end) sum[2] += c;
+        else sum[3] += c;
+    }
+    __shared__ int s_sum[kSweepThreads / 32][4];
+    __shared__ uint16_t s_list[kSweepTile];
+    __shared__ uint32_t s_mark[kListMarkWords];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int v = __reduce_add_sync(0xffffffffu, sum[q]);
+        if (lane == 0) s_sum[warp][q] = v;
+    }
+    const bool shared = words <= kListMarkWords;
+    if (n > 0 && shared && !mark_all)
+        for (int i = t; i < words; i += kSweepThreads) s_mark[i] = 0u;
+    __syncthreads();
+    int start = 0, prefix = 0, list_end = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kSweepThreads / 32; w++) {
+        start += s_sum[w][0];
+        prefix += s_sum[w][1];
+        list_end += s_sum[w][2];
+        total += s_sum[w][3];
+    }
+    prefix += start;
+    list_end += prefix;
+    total += list_end;
+    if (t == 0 && tile == first) begin_instance_day(ik, is[k], start, list_end, day, dense_level);
+    if (t == 0 && tile == tiles - 1) begin_day(sc, total, day);
+    if (n == 0) return;
+    unsigned long long packed = 0;
+#pragma unroll
+    for (int r = 0; r < kSweepRounds; r++) packed |= (unsigned long long)__popc((f >> (4 * r)) & 0xFu) << (16 * r);
+    // positions in person order: scan the four per-round counts at once (16-bit fields)
+    unsigned long long round_tot;
+    const unsigned long long excl = block_exclusive_scan<kSweepThreads, unsigned long long>(packed, round_tot);
+    int round_base = 0;
+#pragma unroll
+    for (int r = 0; r < kSweepRounds; r++) {
+        int at = round_base + (int)((excl >> (16 * r)) & 0xFFFF);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (f & (1u << (4 * r + j))) s_list[at++] = (uint16_t)((r * kSweepThreads + t) * 4 + j);
+        round_base += (int)((round_tot >> (16 * r)) & 0xFFFF);
+    }
+    __syncthreads();
+    const unsigned long long R0 = contact_offset(ik, E0, weekend);
+    for (int i = t; i < n; i += kSweepThreads) {
+        const int person = tile * kSweepTile + s_list[i];
+        infected[prefix + i] = person;
+        infected_inst[prefix + i] = k;
+        if (mark_all) continue;
+        const int2 b = read_buckets(ik, age, weekend, E0, R0, person, prefix + i - start);
+        if (shared) {
+            if (b.x >= 0) mark_bucket_shared(s_mark, b.x);
+            if (b.y >= 0) mark_bucket_shared(s_mark, b.y);
+        } else {
+            if (b.x >= 0) mark_bucket(mark, b.x);
+            if (b.y >= 0) mark_bucket(mark, b.y);
+        }
+    }
+    if (mark_all || !shared) return;
+    __syncthreads();
+    for (int i = t; i < words; i += kSweepThreads)
+        if (s_mark[i]) red_or(&mark[i], s_mark[i]);
+}
+
+// Bytes from the marks over the day's bucket slots, which lie behind them.
+static size_t day_clear_bytes(const DevArrays &d, bool weekend)
+{
+    return (size_t)(reinterpret_cast<char *>(d.bkt + d.buckets[weekend ? 1 : 0]) - reinterpret_cast<char *>(d.mark));
+}
+
+cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t s)
+{
+    const int tiles = d.P / kSweepTile;
+    // several tiles per block only where the grid still fills every SM eight times over
+    // (a small simulation keeps one tile per block and all its parallelism)
+    const int per_block = tiles >= kSweepTilesPerBlock * 8 * sm_count() ? kSweepTilesPerBlock : 1;
+    const bool small = tiles <= kListTiles;
+    k_sweep_count<<<div_up(tiles, per_block), kSweepThreads, 0, s>>>(
+        d.ic, d.is, d.tile_inst, tiles, per_block, d.state, d.sweep_flags, d.sweep_tiles,
+        reinterpret_cast<uint2 *>(d.mark), small ? (int)(day_clear_bytes(d, weekend) / sizeof(uint2)) : 0, d.sc, day);
+    count_launch();
+    if (!small) {
+        k_sweep_scan<<<1, kSweepScanThreads, 0, s>>>(d.ic, d.is, d.K, d.sweep_tiles, tiles, d.sc, day, d.tune.dense_level);
+        count_launch();
+    }
+    return cudaGetLastError();
+}
+
+// The infected list and the marks of the buckets that its persons read (every bucket's
+// for complete tables).
+cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables, cudaStream_t s)
+{
+    const int tiles = d.P / kSweepTile, B = d.buckets[weekend ? 1 : 0], words = B / 32 + 1;
+    cudaError_t e = cudaSuccess;
+    if (tiles <= kListTiles) {
+        if (full_tables) e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
+        if (e != cudaSuccess) return e;
+        k_sweep_list<<<tiles, kSweepThreads, 0, s>>>(d.ic, d.is, d.tile_inst, tiles, d.sweep_flags, d.sweep_tiles,
+                                                     d.infected, d.infected_inst, d.age, d.mark, words,
+                                                     full_tables ? 1 : 0, d.sc, day, d.tune.dense_level);
+        count_launch();
+        return cudaGetLastError();
+    }
+    if (tiles >= kSweepTilesPerBlock * 8 * sm_count())
+        k_sweep_emit<<<div_up(tiles, kEmitWarps), kEmitWarps * 32, 0, s>>>(d.tile_inst, tiles, d.sweep_flags,
+                                                                           d.sweep_tiles, d.infected, d.infected_inst,
+                                                                           d.sc);
+    else
+        k_sweep_emit_block<<<tiles, kSweepThreads, 0, s>>>(d.tile_inst, d.sweep_flags, d.sweep_tiles, d.infected,
+                                                           d.infected_inst, d.sc);
+    count_launch();
+    e = cudaMemsetAsync(d.mark, 0, day_clear_bytes(d, weekend), s);
+    if (e == cudaSuccess && full_tables) e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
+    if (e != cudaSuccess || full_tables) return e;
+    k_mark_buckets<<<sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, s>>>(
+        d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.mark, words, d.sc);
+    count_launch();
+    return cudaGetLastError();
 }
 
 // Schedule kernel.  The persons are cut into regions of C consecutive ones (64 to 1024,
@@ -1560,22 +1704,8 @@ static int sched_region_persons(long long P)
     return C;
 }
 
-// mark (or mark everything for complete tables), then the schedule kernel
-cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, bool full_tables, cudaStream_t s)
+cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, cudaStream_t s)
 {
-    const int B = d.buckets[weekend ? 1 : 0];
-    // the marks and, behind them, the day's bucket slots: one clear
-    cudaError_t e = cudaMemsetAsync(d.mark, 0, (size_t)(reinterpret_cast<char *>(d.bkt + B) -
-                                                        reinterpret_cast<char *>(d.mark)), s);
-    if (e == cudaSuccess && full_tables) e = cudaMemsetAsync(d.mark, 0xFF, ((size_t)B / 32 + 1) * 4, s);
-    if (e != cudaSuccess) return e;
-    if (!full_tables) {
-        k_mark_buckets<<<sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, s>>>(
-            d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.mark, B / 32 + 1, d.sc);
-        count_launch();
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
     const int C = sched_region_persons(d.P), regions = d.P / C;
     const int blocks = std::min(div_up(regions, kSchedWarps), kSchedBlocksPerSm * sm_count());
     const int passes = radix_passes(d.bucket_max[weekend ? 1 : 0]), dbits = radix_digit_bits(d.bucket_max[weekend ? 1 : 0]);
@@ -1625,17 +1755,21 @@ static RadixArgs day_radix_args(const DevArrays &d, bool weekend)
     return r;
 }
 
-// The day's sort tables, a row of blocks per instance (blockIdx.y).
-//  * Block 0 of the row: the digit bases of the instance's segment from the digit
-//    histograms the schedule kernel accumulated (summing the stripes, clearing them).
-//  * Every block: its 4096 regions of the instance.  Their place in the segment is an
+// The day's sort tables, a row of blocks per instance (blockIdx.y), every block with one
+// task and no wait for another.
+//  * Block 0: the digit bases of the instance's segment from the digit histograms the
+//    schedule kernel accumulated (summing the stripes, clearing them).  Every entry has
+//    a digit in every pass, so the passes' totals are equal and one scan over all
+//    passes' digits gives every pass's.
+//  * Block 1, of the first row: the numbers of the segments' radix tiles (tile_prefix),
+//    and the day's materialised entries added to the running total.
+//  * The others: 4096 regions of the instance each.  Their place in the segment is an
 //    exclusive scan of the regions' entry counts; a block sums the counts before its
 //    own itself (at most a few hundred KB from L2) rather than wait for the others.
 //    Output: region_prefix, and for every kRegionChunk entries of the segment the region
 //    the first of them lies in, its prefix, its end and the next one's (chunk_region).
-//  * The first block also numbers the segments' radix tiles (tile_prefix) and adds the
-//    day's materialised entries to the running total.
-constexpr int kBasesThreads = 1024, kBasesRegions = 4 * kBasesThreads;
+constexpr int kBasesThreads = 1024, kBasesRegions = 4 * kBasesThreads, kBasesTasks = 2;
+static_assert(kBasesThreads == kMaxRadixPasses * 256, "a thread per digit of every pass");
 
 __global__ void __launch_bounds__(kBasesThreads) k_day_digit_bases(int *digit_hist, int *digit_base, int passes,
                                                                    const InstConst *ic, const InstState *is, int K,
@@ -1645,10 +1779,11 @@ __global__ void __launch_bounds__(kBasesThreads) k_day_digit_bases(int *digit_hi
                                                                    Scalars *sc)
 {
     if (*(volatile const int *)&sc->done) return;
-    const int k = blockIdx.y, t = threadIdx.x;
-    // regions of the block (an instance starts on a person tile, and 4 C persons divide one)
-    const int r0 = ic[k].pbase / C, r1 = ic[k].pend / C, rb = r0 + (int)blockIdx.x * kBasesRegions;
-    if (rb < r1 && is[k].marked > 0 && !is[k].dense) {
+    const int k = blockIdx.y, t = threadIdx.x, task = (int)blockIdx.x - kBasesTasks;
+    if (task >= 0) {
+        // regions of the block (an instance starts on a person tile, and 4 C persons divide one)
+        const int r0 = ic[k].pbase / C, r1 = ic[k].pend / C, rb = r0 + task * kBasesRegions;
+        if (rb >= r1 || is[k].marked == 0 || is[k].dense) return;
         int before = 0;
         for (int r = r0 + 4 * t; r < rb; r += kBasesRegions) {
             const int4 c = *reinterpret_cast<const int4 *>(region_count + r);
@@ -1657,8 +1792,8 @@ __global__ void __launch_bounds__(kBasesThreads) k_day_digit_bases(int *digit_hi
         int4 c = make_int4(0, 0, 0, 0);
         const int r = rb + 4 * t;
         if (r < r1) c = *reinterpret_cast<const int4 *>(region_count + r);
-        int carry, total;
-        block_exclusive_scan<kBasesThreads, int>(before, carry);
+        int carry = 0, total;
+        if (task > 0) block_exclusive_scan<kBasesThreads, int>(before, carry);
         int at = carry + block_exclusive_scan<kBasesThreads, int>(c.x + c.y + c.z + c.w, total);
         if (r < r1) {
             int4 *const chunks = chunk_region + ic[k].kbase / kRegionChunk;
@@ -1673,19 +1808,28 @@ __global__ void __launch_bounds__(kBasesThreads) k_day_digit_bases(int *digit_hi
             }
             *reinterpret_cast<int4 *>(region_prefix + r) = make_int4(pre[0], pre[1], pre[2], pre[3]);
         }
+        return;
     }
-    if (blockIdx.x != 0) return;
-    for (int p = 0; p < passes; p++) {
-        int v = 0;
-        if (t < 256)
+    if (task == -kBasesTasks) {
+        const int p = t / 256;
+        unsigned v = 0;
+        if (p < passes) {
+            int *const h = digit_hist + (size_t)k * kDigitStripes * kMaxRadixPasses * 256 + t;
+            int x[kDigitStripes];   // all loads before the first store
+#pragma unroll
+            for (int st = 0; st < kDigitStripes; st++) x[st] = h[st * kMaxRadixPasses * 256];
+#pragma unroll
             for (int st = 0; st < kDigitStripes; st++) {
-                int *h = &digit_hist[(((size_t)k * kDigitStripes + st) * kMaxRadixPasses + p) * 256 + t];
-                v += *h;
-                *h = 0;
+                v += (unsigned)x[st];
+                h[st * kMaxRadixPasses * 256] = 0;
             }
-        int total;
-        const int excl = block_exclusive_scan<kBasesThreads, int>(v, total);
-        if (t < 256) digit_base[((size_t)k * passes + p) * 256 + t] = excl;
+        }
+        unsigned total;
+        const unsigned excl = block_exclusive_scan<kBasesThreads, unsigned>(v, total);
+        // (modulo 2^32, like the scan)
+        if (p < passes)
+            digit_base[((size_t)k * passes + p) * 256 + t % 256] = (int)(excl - (unsigned)is[k].marked * (unsigned)p);
+        return;
     }
     if (k != 0) return;
     int carry = 0, carry0 = 0;
@@ -1718,7 +1862,7 @@ cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s)
 {
     const int P = radix_passes(d.bucket_max[weekend ? 1 : 0]);
     const int C = sched_region_persons(d.P);
-    const dim3 grid(std::max(1, div_up(d.persons_max / C, kBasesRegions)), d.K);
+    const dim3 grid(kBasesTasks + std::max(1, div_up(d.persons_max / C, kBasesRegions)), d.K);
     k_day_digit_bases<<<grid, kBasesThreads, 0, s>>>(d.digit_hist, d.digit_base, P, d.ic, d.is, d.K, weekend ? 1 : 0,
                                                     C, d.region_count, d.region_prefix,
                                                     d.chunk_region, d.tile_prefix, d.tile_prefix0, d.sc);
@@ -2270,22 +2414,18 @@ __global__ void k_apply(uint32_t *state, uint8_t *gen_p, uint8_t *gen_s, unsigne
 {
     if (sc->done) return;
     const int n = sc->new_count;
-    const uint32_t dset = (uint32_t)((day + 1) & 0xFF);
+    const uint8_t dset = (uint8_t)(day + 1);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int e = new_list[i];
         const int v = e >> 1, strain = e & 1;
         unsigned long long *cp = &claim[2 * (size_t)v + strain];
         const unsigned long long cl = *cp;
         *cp = ~0ull;
-        const uint32_t profile = (uint32_t)(cl >> 8) & 0xFFu;
-        const uint8_t gen = (uint8_t)(cl & 0xFFu);
-        const uint32_t sshift = strain ? 8 : 0, dshift = strain ? 24 : 16;
-        uint32_t old = state[v], assumed;
-        do {
-            assumed = old;
-            uint32_t nw = (assumed & ~((0xFFu << sshift) | (0xFFu << dshift))) | (profile << sshift) | (dset << dshift);
-            old = atomicCAS(&state[v], assumed, nw);
-        } while (old != assumed);
+        const uint8_t profile = (uint8_t)(cl >> 8), gen = (uint8_t)cl;
+        // the strain's two bytes of the status word; the other strain's may be written now too
+        uint8_t *const st = reinterpret_cast<uint8_t *>(state + v) + strain;
+        st[0] = profile;
+        st[2] = dset;
         if (strain) gen_s[v] = gen;
         else gen_p[v] = gen;
     }

@@ -58,6 +58,7 @@ constexpr uint64_t kTagAbsent = 1, kTagVaccinated = 2;
 // the device, so a whole run needs no host round trip.
 struct InstState {
     unsigned long long rand_offset;     // next free Random123 counter
+    unsigned long long next_offset[2];  // the same, of an even and an odd day's start
     unsigned long long errand_offset;   // E0 of the current day's schedule
     unsigned long long infect_offset;   // R0 of the current day's contacts
     int infected;                       // infected count of the current day
@@ -77,7 +78,7 @@ struct InstState {
 struct Scalars {
     unsigned long long materialised_sum;  // schedule entries written to bucket tables, all days
     int infected;                         // length of today's infected list (all instances)
-    int done;                             // set once a day finds no instance with infected
+    int done;                             // the number of days once a day finds no instance with infected
     int day;                              // current day index
     int new_count;                        // entries in the new-infection list
     int error;                            // nonzero: a bounded device wait gave up
@@ -255,9 +256,10 @@ cudaError_t launch_seed_infected(const int32_t *seeds, int P, int S, uint32_t *s
 cudaError_t launch_person_records(const DevArrays &d, cudaStream_t s);
 
 // ---- day (every instance of the batch in each launch)
-cudaError_t launch_sweep(const DevArrays &d, int day, cudaStream_t s);          // recover, count, scan, bookkeeping
-cudaError_t launch_infected_list(const DevArrays &d, cudaStream_t s);           // the ordered infected list
-cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, bool full_tables, cudaStream_t s);
+cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t s);   // recover, count, bookkeeping
+cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables,
+                                 cudaStream_t s);                                     // the ordered list, the marks
+cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, cudaStream_t s);
 cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s);
 cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, cudaStream_t s);
 cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_t s);

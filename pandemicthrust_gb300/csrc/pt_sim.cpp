@@ -586,11 +586,11 @@ static pt_status enqueue_day(Engine *s, int day)
     cudaStream_t st = s->stream;
     const bool t = s->timing;
     if (t) cudaEventRecord(stage_event(s, day, kStSweep), st);
-    CK(ptk::launch_sweep(d, day, st), "sweep");
+    CK(ptk::launch_sweep(d, weekend, day, st), "sweep");
     if (t) cudaEventRecord(stage_event(s, day, kStInfectedList), st);
-    CK(ptk::launch_infected_list(d, st), "infected list");
+    CK(ptk::launch_infected_list(d, weekend, day, s->full_tables, st), "infected list");
     if (t) cudaEventRecord(stage_event(s, day, kStSchedule), st);
-    CK(ptk::launch_schedule(d, weekend, day, s->full_tables, st), "schedule");
+    CK(ptk::launch_schedule(d, weekend, day, st), "schedule");
     if (t) cudaEventRecord(stage_event(s, day, kStDigits), st);
     CK(ptk::launch_bucket_scan(d, weekend, st), "digit bases");
     if (t) cudaEventRecord(stage_event(s, day, kStRadix), st);
