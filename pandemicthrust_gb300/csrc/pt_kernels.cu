@@ -2438,6 +2438,27 @@ cudaError_t launch_apply(const DevArrays &d, int day, cudaStream_t s)
     return cudaGetLastError();
 }
 
+__global__ void k_day_rows(const InstState *is, int K, int day, const Scalars *sc, int *out)
+{
+    const int n = K * kDayRow;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
+        if (i == n) {
+            out[0] = sc->error;
+            continue;
+        }
+        const InstState &s = is[i / kDayRow];
+        const int f = i % kDayRow;
+        out[1 + i] = f < 16 ? s.counts[day][f] : (f == 16 ? s.infected_per_day[day] : s.days_run);
+    }
+}
+
+cudaError_t launch_day_rows(const DevArrays &d, int day, int *out, cudaStream_t s)
+{
+    k_day_rows<<<std::min(div_up(d.K * kDayRow + 1, 256), sm_count()), 256, 0, s>>>(d.is, d.K, day, d.sc, out);
+    count_launch();
+    return cudaGetLastError();
+}
+
 // ================================================================== bounded-wait probe
 // The look-back wait above, in isolation: one warp plays tile 1 of a fresh look-back
 // (epoch 1, words zeroed by the host) and waits for tile 0.  With publish_first the

@@ -264,6 +264,10 @@ cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s)
 cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, cudaStream_t s);
 cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_t s);
 cudaError_t launch_apply(const DevArrays &d, int day, cudaStream_t s);
+// A day's rows of every instance to mapped host memory: out[0] the device error word, then
+// per instance its 16 counts, infected and days run.
+constexpr int kDayRow = 18;
+cudaError_t launch_day_rows(const DevArrays &d, int day, int *out, cudaStream_t s);
 // weekday / weekend buckets of one instance (compact keys hour * R + dest - lo)
 int day_buckets(const SimConst &c, bool weekend);
 
