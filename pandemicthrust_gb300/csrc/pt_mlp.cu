@@ -139,7 +139,7 @@ struct GemmOp {
     int ldw;
 };
 
-constexpr int kMaxOps = 4;
+constexpr int kMaxOps = 16;
 struct GemmLaunch {
     GemmOp op[kMaxOps];
     AdamArgs adam;
@@ -813,6 +813,265 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
 
+// ---------------------------------------------------------------- training chain
+// The forward pass, the loss and the data gradients of a batch in one launch: a row
+// needs nothing of another row until the parameters' gradients are summed.  Sixteen rows
+// are one m16 tile, and a cluster of four CTAs takes them through all layers, each CTA
+// 64 of a layer's columns (8 a warp): a batch of 512 fills 128 SMs, and an SM reads a
+// quarter of the weights.  The activations (then the dZ) of the rows lie in every CTA's
+// shared memory, twice: a step's epilogue sends its columns to all four CTAs with
+// st.async, whose bytes complete the mbarrier that the next step waits for.  Whoever has
+// a step's rows complete knows that every warp is done with the step before, so nothing
+// else guards the two copies, nor the ring of the CTA's weights (forward: its 64 rows of
+// W; back: its 64 columns; loaded two steps ahead).  What the parameter gradients
+// read (activations, dZ) goes to global memory on the side, and so does Z, which the
+// thread that wrote it reads again on the way back.
+//
+// Bound by the chain itself: per step 16 dependent MMAs, an epilogue and the way to the
+// other CTAs.  With the parameter gradients of all layers in a second launch, a step of
+// the 11-4x256-222 network at batch 512 takes 34 us on a GB300, 17 of them here; layer by
+// layer it was ten launches, 82 us.  (With cluster barriers and without the four loader
+// warps 42: a barrier's release waits 0.5 us for what was stored, and queueing a step's
+// weights takes as long.)  Products, their order and the epilogues are k_gemm's, and so
+// are the results.  Every wait is bounded.
+constexpr int kChainCtas = 4, kChainRows = 16, kChainThreads = 256, kChainLoaders = 128, kChainStages = 3, kChainLayers = 8;
+constexpr int kChainWidth = 256, kChainCols = kChainWidth / kChainCtas;
+constexpr int kChainPitchK = (kChainWidth + 8) * 2, kChainPitchN = (kChainCols + 8) * 2;   // bytes; odd multiples of 16
+constexpr int kChainStage = kChainWidth * kChainPitchN, kChainAct = kChainRows * kChainPitchK;
+static_assert(kChainCols * kChainPitchK <= kChainStage, "a stage holds a CTA's part of a layer in both orders");
+static_assert(kChainThreads / 32 * 8 == kChainCols, "eight columns a warp");
+static_assert(2 * kChainLayers <= kMaxOps, "the parameter gradients of all layers are one launch");
+constexpr int kChainBars = 8 * 2;   // each copy of the rows is complete
+constexpr int kChainSmem = 2 * kChainAct + kChainStages * kChainStage + kChainBars;
+static_assert(kChainSmem <= 227 * 1024, "the chain needs more shared memory than a CTA has");
+
+struct ChainLayer {
+    const bf16 *w;        // ldn x ldk, zero outside N x (the layer before's N)
+    const float *bias;
+    float *Z, *dZf;       // row stride ldn
+    bf16 *H, *dZb;        // the layer's activations and dZ, row stride ldn
+    int N, ldn, ldk;
+};
+
+struct ChainArgs {
+    ChainLayer layer[kChainLayers];
+    int L, B;
+    const bf16 *x;        // inputs, row stride layer[0].ldk
+    const float *Y;       // targets, rows by `rows` (nullptr: in order)
+    const int *rows;
+    float *loss;
+    int *error;
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+// Queues loader t's share of CTA q's part of step c's weights: c < L the rows of layer c, then layers L - 1 to 1
+// column by column.  (As bulk copies of a row each, 64 or 256 a step, a training step took
+// 70 us: the copy engine takes them one after another.)
+__device__ __forceinline__ void chain_load(const ChainArgs &a, int c, int q, uint32_t dst, int t)
+{
+    const bool fwd = c < a.L;
+    const ChainLayer &w = a.layer[fwd ? c : 2 * a.L - 1 - c];
+    const int first = q * kChainCols;
+    if (fwd) {   // a row a warp
+        const int k = t % 32 * 8, rows = k < w.ldk ? min(kChainCols, w.ldn - first) : 0;
+#pragma unroll
+        for (int i = 0; i < kChainCols * 32 / kChainLoaders; i++) {
+            const int r = t / 32 + i * (kChainLoaders / 32);
+            if (r < rows) cp_async16(dst + r * kChainPitchK + k * 2, w.w + (first + r) * w.ldk + k, true);
+        }
+    } else {     // four rows a warp
+        const int k = t % (kChainCols / 8) * 8, rows = first + k < w.ldk ? w.ldn : 0;
+#pragma unroll
+        for (int i = 0; i < kChainWidth * (kChainCols / 8) / kChainLoaders; i++) {
+            const int r = t / (kChainCols / 8) + i * (kChainLoaders * 8 / kChainCols);
+            if (r < rows) cp_async16(dst + r * kChainPitchN + k * 2, w.w + r * w.ldk + first + k, true);
+        }
+    }
+}
+
+__global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThreads + kChainLoaders, 1)
+    k_chain(const __grid_constant__ ChainArgs a)
+{
+    extern __shared__ __align__(16) uint8_t chain_smem[];
+    __shared__ int s_fail;
+    const uint32_t s_act = smem_u32(chain_smem), s_w = s_act + 2 * kChainAct;
+    const uint32_t b_act = s_w + kChainStages * kChainStage;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q = (int)blockIdx.x % kChainCtas, r0 = (int)blockIdx.x / kChainCtas * kChainRows;
+    const int steps = 2 * a.L - 1;
+    const int ldx = a.layer[0].ldk;
+    if (threadIdx.x == 0) {
+        mbar_init(b_act, 1);
+        mbar_init(b_act + 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_fail = 0;
+    }
+    if (threadIdx.x >= kChainThreads) {
+        // the loaders: step 0's rows and weights, then a step's weights two steps ahead
+        const int t = threadIdx.x - kChainThreads;
+        cluster_arrive();
+        for (int e = t; e < kChainRows * (ldx / 8); e += kChainLoaders) {
+            const int r = e / (ldx / 8), k = e % (ldx / 8) * 8;
+            const bool in = r0 + r < a.B;
+            cp_async16(s_act + r * kChainPitchK + k * 2, in ? a.x + (long long)(r0 + r) * ldx + k : a.x, in);
+        }
+        chain_load(a, 0, q, s_w, t);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (steps > 1) chain_load(a, 1, q, s_w + kChainStage, t);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        cluster_wait();
+        for (int c = 0; c < steps; c++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kChainStages - 2) : "memory");
+            if (!__syncthreads_and(1)) break;   // step c's weights have landed; step c - 1's are used up
+            if (c + kChainStages - 1 < steps)
+                chain_load(a, c + kChainStages - 1, q, s_w + (c + kChainStages - 1) % kChainStages * kChainStage, t);
+            asm volatile("cp.async.commit_group;" ::: "memory");   // (empty past the end, so the waits count alike)
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+        cluster_wait();
+        return;
+    }
+    const int l7 = lane & 7, l8 = (lane >> 3) & 1, l16 = lane >> 4;
+    const int row = lane >> 2, j = q * kChainCols + 8 * warp + 2 * (lane & 3);   // outputs (row + 8h, j + 0..1)
+    const float count = (float)((long long)a.B * a.layer[a.L - 1].N), scale = 2.f / count;
+    // what step c's epilogue reads, loaded while the step before runs: biases (forward) or
+    // Z (back), and the targets (outside the rows and columns: the last ones', not used)
+    const int i0 = min(r0 + row, a.B - 1), i1 = min(r0 + row + 8, a.B - 1);
+    float x0[4], x1[4], y0[4], y1[4];
+    auto fetch = [&](int c) {
+        if (c < a.L) {
+            const ChainLayer &o = a.layer[c];
+            const int j0 = min(j, o.N - 1), j1 = min(j + 1, o.N - 1);
+            y0[0] = y0[2] = o.bias[j0];
+            y0[1] = y0[3] = o.bias[j1];
+            if (c == a.L - 1) {
+                const float *const t0 = a.Y + (long long)(a.rows ? a.rows[i0] : i0) * o.N;
+                const float *const t1 = a.Y + (long long)(a.rows ? a.rows[i1] : i1) * o.N;
+                y1[0] = t0[j0];
+                y1[1] = t0[j1];
+                y1[2] = t1[j0];
+                y1[3] = t1[j1];
+            }
+        } else {
+            const ChainLayer &o = a.layer[2 * a.L - 2 - c];
+            const int jj = min(j, o.ldn - 2);   // (even, and so is the stride)
+            const float2 z0 = *reinterpret_cast<const float2 *>(o.Z + (long long)i0 * o.ldn + jj);
+            const float2 z1 = *reinterpret_cast<const float2 *>(o.Z + (long long)i1 * o.ldn + jj);
+            y0[0] = z0.x;
+            y0[1] = z0.y;
+            y0[2] = z1.x;
+            y0[3] = z1.y;
+        }
+    };
+    cluster_arrive();   // every CTA of the cluster is here before one sends to it
+    fetch(0);
+    cluster_wait();
+    float part = 0.f;
+    bool ok = true;
+    int c = 0;
+    for (; c < steps; c++) {
+        const bool fwd = c < a.L, last = c == a.L - 1;
+        const ChainLayer &w = a.layer[fwd ? c : 2 * a.L - 1 - c], &o = fwd ? w : a.layer[2 * a.L - 2 - c];   // o: the outputs'
+        const bool active = j - 2 * (lane & 3) < o.ldn;   // (of the whole warp)
+        const uint32_t sa = s_act + (c & 1) * kChainAct, sw = s_w + (c % kChainStages) * kChainStage;
+        const uint32_t next_act = b_act + 8 * ((c + 1) & 1);
+        if (threadIdx.x == 0 && c + 1 < steps) mbar_expect_tx(next_act, kChainRows * o.ldn * 2);
+        ok = c == 0 || mbar_wait(b_act + 8 * (c & 1), ((c - 1) >> 1) & 1, &s_fail);
+        ok = __syncthreads_and(ok);   // (step c's weights have landed for every thread)
+        if (!ok) break;
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            x0[e] = y0[e];
+            x1[e] = y1[e];
+        }
+        if (c + 1 < steps) fetch(c + 1);
+        float f[4];
+        bf16 b[4];
+        if (active) {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            const int n = (fwd ? w.ldk : w.ldn) / 16;
+            const uint32_t pa = sa + (l7 + 8 * l8) * kChainPitchK + 16 * l16;
+            // B of two steps: four 8 x 8 matrices along the reduction
+            const uint32_t pb = fwd ? sw + (8 * warp + l7) * kChainPitchK + 16 * (l8 + 2 * l16)
+                                    : sw + (l7 + 8 * (l8 + 2 * l16)) * kChainPitchN + 16 * warp;
+            // all fragments first (those past n lie in the buffers and are not used)
+            constexpr int kSteps = kChainWidth / 16;
+            uint32_t fa[kSteps][4], fb[kSteps / 2][4];
+#pragma unroll
+            for (int k = 0; k < kSteps; k += 2) {
+                if (fwd) ldmatrix4<false>(fb[k / 2], pb + 32 * k);
+                else ldmatrix4<true>(fb[k / 2], pb + 16 * k * kChainPitchN);
+                ldmatrix4<false>(fa[k], pa + 32 * k);
+                ldmatrix4<false>(fa[k + 1], pa + 32 * (k + 1));
+            }
+#pragma unroll
+            for (int k = 0; k < kSteps; k++)
+                if (k < n) mma_bf16(acc, fa[k], fb[k / 2][2 * (k & 1)], fb[k / 2][2 * (k & 1) + 1]);
+            // (output e: row + 8 (e / 2), column j + e % 2)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                if (fwd && !last) {
+                    f[e] = acc[e] + x0[e];
+                    b[e] = __float2bfloat16(gelu(f[e]));
+                } else if (last) {
+                    const float d = r0 + row + 8 * (e >> 1) < a.B && j + (e & 1) < o.N ? acc[e] + x0[e] - x1[e] : 0.f;
+                    part += d * d;
+                    f[e] = scale * d;
+                    b[e] = __float2bfloat16(f[e]);
+                } else {
+                    f[e] = acc[e] * gelu_grad(x0[e]);
+                    b[e] = __float2bfloat16(f[e]);
+                }
+                if (j + (e & 1) >= o.N) b[e] = __float2bfloat16(0.f);
+            }
+            if (c + 1 < steps) {
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    // a quad has a row's eight columns: its lane r sends them to CTA r
+                    const __nv_bfloat162 pair(b[2 * h], b[2 * h + 1]);
+                    const uint32_t word = *reinterpret_cast<const uint32_t *>(&pair);
+                    uint32_t v[4];
+#pragma unroll
+                    for (int r = 0; r < 4; r++) v[r] = __shfl_sync(0xffffffffu, word, (lane & ~3) + r);
+                    const uint32_t dst =
+                        s_act + ((c + 1) & 1) * kChainAct + (row + 8 * h) * kChainPitchK + (q * kChainCols + 8 * warp) * 2;
+                    asm volatile("{\n\t.reg .b32 ra, rb;\n\tmapa.shared::cluster.u32 ra, %0, %2;\n\t"
+                                 "mapa.shared::cluster.u32 rb, %1, %2;\n\t"
+                                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [ra], {%3, %4, %5, %6}, [rb];\n\t}"
+                                 ::"r"(dst), "r"(next_act), "r"(lane & 3), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                                 : "memory");
+                }
+            }
+        }
+        if (active) {
+            float *const out = fwd && !last ? o.Z : o.dZf;
+            bf16 *const outb = fwd && !last ? o.H : o.dZb;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int i = r0 + row + 8 * h;
+                const long long at = (long long)i * o.ldn + j;
+                if (i < a.B && j + 1 < o.N) {
+                    *reinterpret_cast<float2 *>(out + at) = make_float2(f[2 * h], f[2 * h + 1]);
+                    *reinterpret_cast<__nv_bfloat162 *>(outb + at) = __nv_bfloat162(b[2 * h], b[2 * h + 1]);
+                } else if (i < a.B && j < o.N) {
+                    out[at] = f[2 * h];
+                    outb[at] = b[2 * h];
+                }
+            }
+        }
+    }
+    if (!ok && threadIdx.x == 0) umma_fail(&s_fail, a.error);
+    // no CTA leaves while another may still send to it
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+    cluster_wait();
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) part += __shfl_xor_sync(0xffffffffu, part, s);
+    if (lane == 0 && part != 0.f) atomicAdd(a.loss, part / count);
+}
+
 // ---------------------------------------------------------------- fused hidden layers
 // All hidden layers of one or more networks of a shape, activations kept on chip.  A
 // layer-by-layer launch writes and reads 0.5 KB of activations per row and layer, which
@@ -1465,8 +1724,9 @@ static cudaError_t forward(pt_mlp *m, int B, const bf16 *h0, const float *Y = nu
 
 // gradients of every parameter for the B rows at h0 whose forward pass has run: into
 // `grad`, or (nullptr) straight into Adam's update.  Layer l's weights are updated one
-// launch after the last product that reads them.
-static cudaError_t backward(pt_mlp *m, int B, const bf16 *h0, float *grad, const AdamArgs &adam)
+// launch after the last product that reads them.  With `chained` every dZ is there
+// already, and all parameters are one launch.
+static cudaError_t backward(pt_mlp *m, int B, const bf16 *h0, float *grad, const AdamArgs &adam, bool chained)
 {
     auto weights = [&](GemmOp &g, int l) {   // dW_l[j][k] = sum_i dZ_l[i][j] H_l[i][k]
         g = GemmOp{};
@@ -1496,7 +1756,7 @@ static cudaError_t backward(pt_mlp *m, int B, const bf16 *h0, float *grad, const
     GemmLaunch gl = {};
     gl.adam = adam;
     const int last = m->L - 1;
-    for (int l = last; l >= 1; l--) {
+    for (int l = chained ? 0 : last; l >= 1; l--) {
         // dZ_{l-1}[i][k] = (sum_j dZ_l[i][j] W_l[j][k]) GELU'(Z_{l-1}[i][k])
         GemmOp &g = gl.op[0];
         g = GemmOp{};
@@ -1523,11 +1783,68 @@ static cudaError_t backward(pt_mlp *m, int B, const bf16 *h0, float *grad, const
         if (e != cudaSuccess) return e;
     }
     int ops = 0;
-    for (int l = std::min(1, last); l >= 0; l--) {
+    for (int l = chained ? last : std::min(1, last); l >= 0; l--) {
         weights(gl.op[ops++], l);
         bias(gl.op[ops++], l);
     }
     return gemm(m, gl, ops);
+}
+
+// Whether a network trains by k_chain: its layers and their widths fit one cluster.
+static bool chain_fits(const pt_mlp *m)
+{
+    bool ok = m->L <= kChainLayers;
+    for (int ld : m->ld) ok = ok && ld <= kChainWidth;
+    return ok;
+}
+
+// The word that a device wait writes when it gives up (host memory the device writes).
+static cudaError_t error_word(pt_mlp *m)
+{
+    if (m->umma_err) return cudaSuccess;
+    const cudaError_t e = cudaHostAlloc((void **)&m->umma_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess) *m->umma_err = 0;
+    return e;
+}
+
+static cudaError_t chain(pt_mlp *m, int B, const bf16 *h0, const float *Y, const int *rows, float *loss)
+{
+    static const cudaError_t attr = cudaFuncSetAttribute(k_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmem);
+    if (attr != cudaSuccess) return attr;
+    const cudaError_t e = error_word(m);
+    if (e != cudaSuccess) return e;
+    ChainArgs a = {};
+    a.error = m->umma_err;
+    a.L = m->L;
+    a.B = B;
+    a.x = h0;
+    a.Y = Y;
+    a.rows = rows;
+    a.loss = loss;
+    for (int l = 0; l < m->L; l++) {
+        ChainLayer &c = a.layer[l];
+        c.w = m->wpk[l];
+        c.bias = m->w + m->boff[l];
+        c.Z = m->Z[l];
+        c.dZf = m->dZf[l];
+        c.H = m->H[l + 1];
+        c.dZb = m->dZb[l];
+        c.N = m->width[l + 1];
+        c.ldn = m->ld[l + 1];
+        c.ldk = m->ld[l];
+    }
+    k_chain<<<(B + kChainRows - 1) / kChainRows * kChainCtas, kChainThreads + kChainLoaders, kChainSmem, m->stream>>>(a);
+    return cudaGetLastError();
+}
+
+// The loss (added to *loss) of the B rows at h0 against the targets Y, rows by `rows`, and
+// the gradients of every parameter: into `grad`, or (nullptr) into Adam's update.
+static cudaError_t training_pass(pt_mlp *m, int B, const bf16 *h0, const float *Y, const int *rows, float *loss,
+                                 float *grad, const AdamArgs &adam)
+{
+    const bool chained = chain_fits(m);
+    const cudaError_t e = chained ? chain(m, B, h0, Y, rows, loss) : forward(m, B, h0, Y, rows, loss);
+    return e == cudaSuccess ? backward(m, B, h0, grad, adam, chained) : e;
 }
 
 static int grid_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 4096); }
@@ -1625,6 +1942,8 @@ static cudaError_t ensure_zout(pt_mlp *m)
 static cudaError_t umma_prepare(pt_mlp *m)
 {
     if (m->h0p) return cudaSuccess;
+    cudaError_t e = error_word(m);
+    if (e != cudaSuccess) return e;
     static const cudaError_t attr = [] {
         cudaError_t a = cudaFuncSetAttribute(k_umma_layer<kUmmaEpiWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              kUmmaSmem);
@@ -1635,11 +1954,6 @@ static cudaError_t umma_prepare(pt_mlp *m)
         return a;
     }();
     if (attr != cudaSuccess) return attr;
-    if (!m->umma_err) {
-        cudaError_t e = cudaHostAlloc((void **)&m->umma_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
-        if (e != cudaSuccess) return e;
-        *m->umma_err = 0;
-    }
     return dalloc(m, &m->h0p, (size_t)m->max_batch * m->ld[0]);
 }
 
@@ -1852,13 +2166,13 @@ static cudaError_t ensemble_chunk(pt_mlp *const *members, int count, int B, cons
     return cudaGetLastError();
 }
 
-// A device wait of the tcgen05 path that gave up: reported once, then cleared.  The
+// A device wait of a kernel here that gave up: reported once, then cleared.  The
 // stream has been synchronised.
 static pt_status umma_check(pt_mlp *m)
 {
     if (!m->umma_err || *(volatile int *)m->umma_err == 0) return PT_OK;
     *(volatile int *)m->umma_err = 0;
-    return mfail(m, PT_ERR_TIMEOUT, "a tcgen05 MMA completion wait gave up");
+    return mfail(m, PT_ERR_TIMEOUT, "a device-side wait gave up");
 }
 
 // The checks of an ensemble call; the rows its networks take at a time.
@@ -2025,7 +2339,6 @@ pt_status pt_mlp_train(pt_mlp *m, int epochs, int batch, float lr, uint64_t shuf
         for (int s = 0; s < steps; s++) {
             const int s0 = s * batch, B = std::min(batch, m->n - s0);
             const bf16 *h0 = m->Xe + (size_t)s0 * m->ld[0];
-            MCK(forward(m, B, h0, m->Y, m->perm + s0, m->loss + s), "forward");
             m->step++;
             AdamArgs a;
             a.w = m->w;
@@ -2034,13 +2347,15 @@ pt_status pt_mlp_train(pt_mlp *m, int epochs, int batch, float lr, uint64_t shuf
             a.lr = lr;
             a.c1 = 1.f - std::pow(0.9f, (float)m->step);
             a.c2 = 1.f - std::pow(0.999f, (float)m->step);
-            MCK(backward(m, B, h0, nullptr, a), "backward");
+            MCK(training_pass(m, B, h0, m->Y, m->perm + s0, m->loss + s, nullptr, a), "training step");
         }
     }
     // the last epoch's losses
     std::vector<float> l(steps);
     MCK(cudaMemcpyAsync(l.data(), m->loss, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost, m->stream), "losses");
     MCK(cudaStreamSynchronize(m->stream), "sync");
+    const pt_status waits = umma_check(m);
+    if (waits != PT_OK) return waits;
     double sum = 0.0;
     for (int s = 0; s < steps; s++) sum += l[s] * std::min(batch, m->n - s * batch);
     if (epoch_loss) *epoch_loss = (float)(sum / m->n);
@@ -2061,8 +2376,7 @@ pt_status pt_mlp_gradients(pt_mlp *m, const float *X, const float *Y, int n, flo
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream);
-    if (e == cudaSuccess) e = forward(m, n, m->H[0], dY, nullptr, m->loss);
-    if (e == cudaSuccess) e = backward(m, n, m->H[0], m->grad, AdamArgs{});
+    if (e == cudaSuccess) e = training_pass(m, n, m->H[0], dY, nullptr, m->loss, m->grad, AdamArgs{});
     float l = 0.f;
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(grads, m->grad, (size_t)m->nparam * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
@@ -2072,7 +2386,7 @@ pt_status pt_mlp_gradients(pt_mlp *m, const float *X, const float *Y, int n, flo
     cudaFree(dY);
     MCK(e, "gradients");
     if (loss) *loss = l;
-    return PT_OK;
+    return umma_check(m);
 }
 
 pt_status pt_mlp_predict(pt_mlp *m, const float *X, int n, float *Y)
