@@ -1230,7 +1230,11 @@ __device__ __forceinline__ void mark_bucket_shared(uint32_t *s_mark, int b)
 }
 
 // The buckets (global) that today's contact draws of an infected person read, -1 for
-// none: `person` global, lpos its place in its instance's infected list.
+// none: `person` global, lpos its place in its instance's infected list.  They are kept in
+// list order (d.read) for the infection kernels, which would otherwise gather them from
+// every person's keys and draw the adults' profile again; so nobody's keys are written
+// unless the sort reads them (a dense instance).  Weekdays a person's two errand contacts
+// go to the first bucket, the second or one each; weekends one each, in slot order.
 __device__ __forceinline__ int2 read_buckets(const InstConst &ik, const uint8_t *age, int weekend, unsigned long long E0,
                                              unsigned long long R0, int person, int lpos)
 {
@@ -1277,7 +1281,7 @@ constexpr int kMarkThreads = 256, kMarkBlocksPerSm = 4;
 __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *ic, const InstState *is,
                                                                const uint8_t *age, const int32_t *infected,
                                                                const int32_t *infected_inst, int weekend,
-                                                               uint32_t *mark, int words, const Scalars *sc)
+                                                               int2 *read, uint32_t *mark, int words, const Scalars *sc)
 {
     if (sc->done) return;
     const int I = sc->infected;
@@ -1291,6 +1295,7 @@ __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *
         const int k = infected_inst[pos];
         const InstState &s = is[k];
         const int2 b = read_buckets(ic[k], age, weekend, s.errand_offset, s.infect_offset, infected[pos], pos - s.start);
+        read[pos] = b;
         if (shared) {
             if (b.x >= 0) mark_bucket_shared(s_mark, b.x);
             if (b.y >= 0) mark_bucket_shared(s_mark, b.y);
@@ -1322,7 +1327,8 @@ constexpr int kListMarkWords = 2048;   // a bitmap this small is marked in share
 __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *ic, InstState *is, const int32_t *tile_inst,
                                                               int tiles, const uint16_t *flags_in,
                                                               const int32_t *tile_count, int32_t *infected,
-                                                              int32_t *infected_inst, const uint8_t *age, uint32_t *mark,
+                                                              int32_t *infected_inst, int2 *read, const uint8_t *age,
+                                                              uint32_t *mark,
                                                               int words, int mark_all, Scalars *sc, int day,
                                                               int dense_level)
 {
@@ -1393,8 +1399,9 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
         const int person = tile * kSweepTile + s_list[i];
         infected[prefix + i] = person;
         infected_inst[prefix + i] = k;
-        if (mark_all) continue;
         const int2 b = read_buckets(ik, age, weekend, E0, R0, person, prefix + i - start);
+        read[prefix + i] = b;
+        if (mark_all) continue;
         if (shared) {
             if (b.x >= 0) mark_bucket_shared(s_mark, b.x);
             if (b.y >= 0) mark_bucket_shared(s_mark, b.y);
@@ -1443,7 +1450,7 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
         if (full_tables) e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
         if (e != cudaSuccess) return e;
         k_sweep_list<<<tiles, kSweepThreads, 0, s>>>(d.ic, d.is, d.tile_inst, tiles, d.sweep_flags, d.sweep_tiles,
-                                                     d.infected, d.infected_inst, d.age, d.mark, words,
+                                                     d.infected, d.infected_inst, d.read, d.age, d.mark, words,
                                                      full_tables ? 1 : 0, d.sc, day, d.tune.dense_level);
         count_launch();
         return cudaGetLastError();
@@ -1458,9 +1465,9 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
     count_launch();
     e = cudaMemsetAsync(d.mark, 0, day_clear_bytes(d, weekend), s);
     if (e == cudaSuccess && full_tables) e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
-    if (e != cudaSuccess || full_tables) return e;
+    if (e != cudaSuccess) return e;
     k_mark_buckets<<<sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, s>>>(
-        d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.mark, words, d.sc);
+        d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.read, d.mark, words, d.sc);
     count_launch();
     return cudaGetLastError();
 }
@@ -1469,11 +1476,11 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
 // launch_schedule), each inside one instance.  A persistent block owns a run of regions
 // and its warps take them one by one; a warp walks its region in rounds (weekday: 64
 // persons a round, a pair per lane, one Threefry block per pair; weekend: 32 persons a
-// round, one per lane).  The kernel writes every person's keys and keeps the entries of
-// marked buckets, compacted in ascending person order, in the warp's part of shared
-// memory; full parts are added to the block's radix digit histograms and copied, as
-// (instance-local key, person), to the region's slots of the entry array (3C from 3C
-// times the region's number).  The sort's first pass reads the regions of an instance
+// round, one per lane).  The kernel keeps the entries of marked buckets, compacted in
+// ascending person order, in the warp's part of shared memory; full parts are added to
+// the block's radix digit histograms and copied, as (instance-local key, person), to the
+// region's slots of the entry array (3C from 3C times the region's number), or, for a
+// dense instance, every person's keys are written instead.  The sort's first pass reads the regions of an instance
 // one after another (k_day_digit_bases scans their counts): the order its stability needs.
 //
 // No warp waits for another within an instance.  A form that placed the entries of
@@ -1594,18 +1601,21 @@ __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
 #pragma unroll
                     for (int k = 0; k < 3; k++)
                         kb[k] = (uint32_t)(errand_bucket<true>(s_row, w[3 + k], errand_p9<true>(true), 0) + h[k] * R);
-                    // the round's 96 key slots, written in whole 16-byte pieces through the
-                    // unused end of the warp's part (run <= 3 (p0 - part))
-                    uint32_t *const stage = my_key + 3 * (p0 - part);
+                    if (dense) {
+                        // the round's 96 key slots, written in whole 16-byte pieces through the
+                        // unused end of the warp's part (run <= 3 (p0 - part))
+                        uint32_t *const stage = my_key + 3 * (p0 - part);
 #pragma unroll
-                    for (int k = 0; k < 3; k++) stage[3 * lane + k] = kb[k];
-                    __syncwarp();
-                    if (p0 + 32 <= N) {
-                        if (lane < 24)
-                            *reinterpret_cast<uint4 *>(kk + 3 * (size_t)p0 + 4 * lane) =
-                                *reinterpret_cast<const uint4 *>(stage + 4 * lane);
-                    } else {
-                        for (int i = lane; i < 3 * (N - p0); i += 32) kk[3 * (size_t)p0 + i] = (int32_t)stage[i];
+                        for (int k = 0; k < 3; k++) stage[3 * lane + k] = kb[k];
+                        __syncwarp();
+                        if (p0 + 32 <= N) {
+                            if (lane < 24)
+                                *reinterpret_cast<uint4 *>(kk + 3 * (size_t)p0 + 4 * lane) =
+                                    *reinterpret_cast<const uint4 *>(stage + 4 * lane);
+                        } else {
+                            for (int i = lane; i < 3 * (N - p0); i += 32) kk[3 * (size_t)p0 + i] = (int32_t)stage[i];
+                        }
+                        __syncwarp();   // the stage is read before the entries below reach it
                     }
                     const uint32_t in = p < N ? 1u : 0u;
                     uint32_t mk[3];
@@ -1613,7 +1623,6 @@ __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
                     for (int k = 0; k < 3; k++) mk[k] = mark_bit(mark, kb[k]) & in;
                     const uint32_t cnt = mk[0] + mk[1] + mk[2];
                     const unsigned b0 = __ballot_sync(0xffffffffu, cnt & 1u), b1 = __ballot_sync(0xffffffffu, cnt & 2u);
-                    __syncwarp();   // the stage is read before the entries below reach it
                     if ((b0 | b1) == 0) continue;
                     int pos = run + __popc(b0 & lt) + 2 * __popc(b1 & lt);
 #pragma unroll
@@ -1646,7 +1655,7 @@ __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
                     uint32_t mk[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++) mk[k] = mark_bit(mark, kb[k]) & in[k >> 1];
-                    if (p + 1 < N) {
+                    if (dense && p + 1 < N) {
                         *reinterpret_cast<int2 *>(kk + p) = make_int2((int)kb[0], (int)kb[2]);
                         if ((N & 1) == 0) {   // hour 1's slots start 8-byte aligned
                             *reinterpret_cast<int2 *>(kk + (size_t)N + p) = make_int2((int)kb[1], (int)kb[3]);
@@ -1654,7 +1663,7 @@ __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
                             kk[(size_t)N + p] = (int)kb[1];
                             kk[(size_t)N + p + 1] = (int)kb[3];
                         }
-                    } else if (p < N) {
+                    } else if (dense && p < N) {
                         kk[p] = (int)kb[0];
                         kk[(size_t)N + p] = (int)kb[1];
                     }
@@ -1687,6 +1696,40 @@ __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
         __syncthreads();
         r = end;
     }
+}
+
+// Every person's schedule keys of the last day run, as the sort numbers them.
+__global__ void k_day_keys(const InstConst *ic, const InstState *is, const uint8_t *age, int weekend, int32_t *keys)
+{
+    const int k = blockIdx.y;
+    const InstConst &ik = ic[k];
+    const SimConst &c = ik.c;
+    const TfKey key = make_key(c);
+    const unsigned long long E0 = is[k].errand_offset;
+    int32_t *const kk = keys + ik.kbase;
+    const int lo = c.type_offset[weekend ? 9 : 8], R = c.L - lo, bb = ik.bbase[weekend ? 1 : 0];
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < c.N; p += gridDim.x * blockDim.x) {
+        if (weekend) {
+            int d[3];
+            weekend_errands(c, key, E0 + 2ull * (unsigned long long)p, lo, R, d);
+            for (int j = 0; j < 3; j++) kk[3 * (size_t)p + j] = bb + d[j];
+        } else {
+            uint32_t w[4];
+            tf2x64(key, E0 + (uint64_t)(p / 2), w);
+            int k1, k2;
+            weekday_pair_keys(c, w, p & 1, age[ik.pbase + p] == 5, lo, R, k1, k2);
+            kk[p] = bb + k1;
+            kk[(size_t)c.N + p] = bb + k2;
+        }
+    }
+}
+
+cudaError_t launch_day_keys(const DevArrays &d, bool weekend, cudaStream_t s)
+{
+    k_day_keys<<<dim3(std::min(div_up(d.persons_max, 256), 8 * sm_count()), d.K), 256, 0, s>>>(d.ic, d.is, d.age,
+                                                                                         weekend ? 1 : 0, d.keys);
+    count_launch();
+    return cudaGetLastError();
 }
 
 int day_buckets(const SimConst &c, bool weekend)
@@ -2057,12 +2100,16 @@ struct InfectArgs {
     const uint4 *prec;
     const int32_t *wp_people;
     const uint2 *bkt;
-    const int32_t *keys, *bkt_people, *infected, *infected_inst;
+    const int32_t *bkt_people, *infected, *infected_inst;
+    const int2 *read;   // the buckets an infector's contacts read (read_buckets)
     unsigned long long *claim;
     int32_t *new_list;
     Scalars *sc;
     int coop_most;   // up to this many infectors, eight lanes work on one
 };
+
+// Errand contacts of a weekday infector that go to its first bucket, of two.
+__device__ __forceinline__ int first_errands(int2 read) { return read.x < 0 ? 0 : (read.y < 0 ? 2 : 1); }
 
 // An infector's packed record: one 128-bit read-only load.
 __device__ __forceinline__ uint4 load_record(const uint4 *prec, int me) { return __ldg(&prec[me]); }
@@ -2072,7 +2119,7 @@ __device__ __forceinline__ uint4 load_record(const uint4 *prec, int me) { return
 // j of a group first computes one Threefry block of the infector's draws, all in
 // parallel:
 //   weekday  j = 0, 1: contact words (counters R + 6 pos, +1); j = 2..5: infection
-//            words (+2..+5); j = 6: the schedule block of the adult's errand profile
+//            words (+2..+5)
 //   weekend  j = 0: contact words; j = 1: the Threefry-2x32 errand block; j = 2..5:
 //            infection words
 // then picks contact slot j's victim (its own gather chain) and draws slot j's two
@@ -2149,13 +2196,13 @@ __device__ __forceinline__ void infect_coop(const InfectArgs &a, int day, int I,
         const unsigned long long ctr = s.infect_offset + 6ull * (unsigned long long)(pos - s.start);
         const TfKey key = make_key(c);
         const uint4 rec = load_record(a.prec, me);
+        const int2 read = a.read[pos];
         // one Threefry block per lane
         uint32_t blk[4] = {0u, 0u, 0u, 0u};
         if (WEEKEND && j == 1) {
             tf2x32(key, (uint32_t)(ctr + 1), blk);   // :1895-1901, counter truncated to 32 bits
         } else {
-            const uint64_t cc = (!WEEKEND && j >= 6) ? s.errand_offset + (uint64_t)(lme / 2) : ctr + (uint64_t)j;
-            tf2x64(key, cc, blk);
+            tf2x64(key, ctr + (uint64_t)j, blk);
         }
         // contact words: W[j] of blocks R, R + 1 (weekday), W[j] of block R (weekend)
         const int csrc = WEEKEND ? gl : gl + (j >> 2);
@@ -2165,33 +2212,24 @@ __device__ __forceinline__ void infect_coop(const InfectArgs &a, int day, int I,
         int victim = -1, kv = 0;
         const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
         if (WEEKEND) {
-            const int prof = (int)(q3 % 6u);   // word 3 of block R (:1892)
             const uint32_t v0 = __shfl_sync(kFull, blk[0], gl + 1), v1 = __shfl_sync(kFull, blk[1], gl + 1);
             if (j < 3) {
                 kv = select_victim(me, hoff, hcnt, wc, victim);
             } else if (j < 5) {
-                const int loc = a.keys[ik.kbase + 3 * (size_t)lme + c_weekend_assign[prof][j - 3]];
-                const uint2 slot = a.bkt[loc];
+                const uint2 slot = a.bkt[j == 3 ? read.x : read.y];
                 const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
                 kv = select_victim(me, eoff, ecnt, j == 3 ? v0 : v1, victim, a.bkt_people);
             }
         } else {
-            const bool adult = prec_age(rec.w) == 5;
             const int desired = prec_desired(rec.w);
-            // the adult's errand profile from the schedule block on lane 6 (:3697-3702)
-            const int pv = (j == 6) ? (int)(((lme & 1) ? (blk[2] ^ blk[3]) : (blk[0] ^ blk[1])) % 3u) : 0;
-            const int pv6 = __shfl_sync(kFull, pv, gl + 6);   // every lane takes part in the shuffle
-            const int prof = adult ? pv6 : 3;
             if (j < 3) {
                 kv = select_victim(me, hoff, hcnt, wc, victim);
             } else if (j < 3 + desired) {
                 kv = select_victim(me, (int)rec.y, (int)rec.z, wc, victim, a.wp_people);
             } else {
-                const int e = j - 3 - desired, want0 = c_weekday_assign[prof][0], want1 = c_weekday_assign[prof][1];
-                const int hour = e < want0 ? 0 : (e < want0 + want1 ? 1 : -1);
-                if (hour >= 0) {
-                    const int dest = a.keys[ik.kbase + (size_t)hour * c.N + lme];
-                    const uint2 slot = a.bkt[dest];
+                const int e = j - 3 - desired;   // the infector's e-th errand contact of two
+                if (e < 2) {
+                    const uint2 slot = a.bkt[e < first_errands(read) ? read.x : read.y];
                     const int eoff = bucket_start(slot), ecnt = bucket_count(slot);
                     kv = select_victim(me, eoff, ecnt, wc, victim, a.bkt_people);
                 }
@@ -2270,18 +2308,11 @@ __global__ void __launch_bounds__(128, 8) k_infect_weekday(InfectArgs a, int day
         tf2x64(key, ctr + 1, w + 4);
         const bool adult = prec_age(rec.w) == 5;
         const uint32_t mine = a.state[me];
-        // errands / afterschool: destinations from today's keys
-        const int32_t *kk = a.keys + ik.kbase;
-        const uint2 slot0 = a.bkt[kk[lme]], slot1 = a.bkt[kk[c.N + lme]];
+        // errands / afterschool
+        const int2 read = a.read[pos];
+        const uint2 none = make_uint2(0u, 0u);
+        const uint2 slot0 = read.x >= 0 ? a.bkt[read.x] : none, slot1 = read.y >= 0 ? a.bkt[read.y] : none;
         infector_gens(inf, mine, a.gen_p, a.gen_s);
-        // the adult profile is regenerated from the schedule counter (:3667-3705)
-        int prof = 3;
-        if (adult) {
-            uint32_t e[4];
-            tf2x64(key, s.errand_offset + (uint64_t)(lme / 2), e);
-            const int slot = 2 * (lme % 2);
-            prof = (int)((e[slot] ^ e[slot + 1]) % 3u);
-        }
         int victims[8], kv[8];
         // household: offset + r % count, the household table is the identity
         const int hoff = (int)rec.x, hcnt = prec_household_size(rec.w);
@@ -2289,7 +2320,7 @@ __global__ void __launch_bounds__(128, 8) k_infect_weekday(InfectArgs a, int day
         for (int j = 0; j < 3; j++) kv[j] = select_victim(me, hoff, hcnt, w[j], victims[j]);
         // then the workplace's or school's max-contacts, then each errand hour's
         const int desired = prec_desired(rec.w);
-        const int want0 = c_weekday_assign[prof][0], want = want0 + c_weekday_assign[prof][1];
+        const int want0 = first_errands(read);
         int off[5], cnt[5];
         const int32_t *table[5];
 #pragma unroll
@@ -2297,7 +2328,7 @@ __global__ void __launch_bounds__(128, 8) k_infect_weekday(InfectArgs a, int day
             const int e = j - desired;
             const uint2 slot = e < want0 ? slot0 : slot1;
             off[j] = e < 0 ? (int)rec.y : bucket_start(slot);
-            cnt[j] = e < 0 ? (int)rec.z : (e < want ? bucket_count(slot) : 0);
+            cnt[j] = e < 0 ? (int)rec.z : (e < 2 ? bucket_count(slot) : 0);
             table[j] = e < 0 ? a.wp_people : a.bkt_people;
         }
         select_victims<5>(me, off, cnt, table, w + 3, victims + 3, kv + 3);
@@ -2355,15 +2386,13 @@ __global__ void __launch_bounds__(128, 8) k_infect_weekend(InfectArgs a, int day
         inf.pos = pos;
         inf.me = a.infected[pos];
         const int me = inf.me;
-        const int lme = me - ik.pbase;
         const unsigned long long ctr = s.infect_offset + 6ull * (unsigned long long)(pos - s.start);
         const uint4 rec = load_record(a.prec, me);
         const uint32_t mine = a.state[me];
         uint32_t w[4];
         tf2x64(key, ctr, w);
-        const int prof = (int)(w[3] % 6u);
-        const int32_t *k3 = a.keys + ik.kbase + 3 * (size_t)lme;
-        const uint2 slot0 = a.bkt[k3[c_weekend_assign[prof][0]]], slot1 = a.bkt[k3[c_weekend_assign[prof][1]]];
+        const int2 read = a.read[pos];
+        const uint2 slot0 = a.bkt[read.x], slot1 = a.bkt[read.y];
         infector_gens(inf, mine, a.gen_p, a.gen_s);
         // Threefry-2x32 on the low seed words with counter (u32)(ctr + 1) (:1895-1901)
         uint32_t v2[2];
@@ -2388,7 +2417,7 @@ cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_
     a.ic = d.ic; a.is = d.is;
     a.state = d.state; a.gen_p = d.gen_p; a.gen_s = d.gen_s; a.age = d.age;
     a.prec = d.prec;
-    a.wp_people = d.wp_people; a.keys = d.keys;
+    a.wp_people = d.wp_people; a.read = d.read;
     a.bkt = d.bkt; a.bkt_people = d.bkt_people; a.infected = d.infected;
     a.infected_inst = d.infected_inst;
     a.claim = d.claim; a.new_list = d.new_list; a.sc = d.sc;

@@ -114,7 +114,7 @@ struct DevArrays {
     int32_t *wp_people;       // P (padding persons last, in the spare bucket)
     int32_t *wp_offset;       // locations + 2
     uint4 *prec;              // P packed per-person records for the contact draws (see PersonRec)
-    int32_t *keys;            // 3P schedule keys (global bucket indices)
+    int32_t *keys;            // 3P schedule keys (global bucket indices) of dense instances (launch_day_keys: of all)
     uint2 *bkt;               // today's buckets: start and size (BucketSlot below)
     int32_t *bkt_count;       // the workplace histogram of the setup, zero between uses
     int32_t *bkt_people;      // 3P person ids bucket by bucket, ascending in each
@@ -131,6 +131,7 @@ struct DevArrays {
     uint32_t *mark;           // bitmap over today's buckets: 1 = materialise
     int32_t *infected;        // P ascending infected ids
     int32_t *infected_inst;   // P: instance of each infected list position
+    int2 *read;               // P: the buckets that position's contacts read today, -1 for none
     uint16_t *sweep_flags;    // P / 16: the sweep's per-thread infected masks
     int32_t *sweep_tiles;     // P / kPersonTile + 1: infected per person tile, then their prefix
     unsigned long long *claim;// 2P (victim, strain) -> min attempt key
@@ -260,6 +261,7 @@ cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t
 cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables,
                                  cudaStream_t s);                                     // the ordered list, the marks
 cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, cudaStream_t s);
+cudaError_t launch_day_keys(const DevArrays &d, bool weekend, cudaStream_t s);        // for inspection
 cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s);
 cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, cudaStream_t s);
 cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_t s);

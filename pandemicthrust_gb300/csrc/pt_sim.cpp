@@ -436,7 +436,7 @@ static pt_status engine_setup(Engine *s)
     bytes += 2 * round256(nregions * 4) + round256(nchunks * sizeof(int4));   // schedule regions
     // the mark bitmap and, right behind it, the bucket slots of a day (cleared together)
     bytes += round256(((size_t)Bday + 1) * sizeof(uint2)) + round256(((size_t)Bday / 32 + 1) * 4);
-    bytes += round256(n * 4) * 2;               // infected, infected_inst
+    bytes += round256(n * 4) * 2 + round256(n * 8);   // infected, infected_inst, read
     bytes += round256(n / 16 * 2) + round256((ntiles + 1) * 4);  // sweep masks, sweep tile counts
     bytes += round256(2 * n * 8);               // claim
     bytes += round256(2 * n * 4);               // new_list
@@ -472,6 +472,7 @@ static pt_status engine_setup(Engine *s)
     d.bkt = a.take<uint2>((size_t)Bday + 1);
     d.infected = a.take<int32_t>(n);
     d.infected_inst = a.take<int32_t>(n);
+    d.read = a.take<int2>(n);
     d.sweep_flags = a.take<uint16_t>(n / 16);
     d.sweep_tiles = a.take<int32_t>(ntiles + 1);
     d.claim = a.take<unsigned long long>(2 * n);
@@ -1182,6 +1183,7 @@ pt_status pt_get_day_tables(pt_sim *s, int32_t *infected, int32_t *keys, int32_t
     if (infected && I > 0)
         CK(pt_memcpy_sync(s, infected, s->d.infected, (size_t)I * 4, cudaMemcpyDeviceToHost), "copy");
     if (keys) {
+        CK(ptk::launch_day_keys(s->d, weekend, s->stream), "keys");
         CK(pt_memcpy_sync(s, keys, s->d.keys, (size_t)E * 4, cudaMemcpyDeviceToHost), "copy");
         for (int i = 0; i < E; i++) {
             int h = keys[i] / R, loc = keys[i] % R + lo;
