@@ -1738,12 +1738,14 @@ int day_buckets(const SimConst &c, bool weekend)
 }
 
 // Persons per region of the schedule kernel: the largest power of two that still
-// leaves four regions for every resident warp (small simulations spread over the SMs,
-// large ones have fewer counts to scan and longer runs of entries per region).
+// leaves two regions for every resident warp (small simulations spread over the SMs,
+// large ones have fewer counts to scan and longer runs of entries per region: a run of
+// 24 instances of 1M persons, most of them with few infected, takes 72 ms, with four
+// regions a warp 76, because the sort looks up twice as many regions an entry).
 static int sched_region_persons(long long P)
 {
     int C = kSchedMaxRegion;
-    while (C > kSchedMinRegion && P / C < 4ll * kSchedWarps * kSchedBlocksPerSm * sm_count()) C /= 2;
+    while (C > kSchedMinRegion && P / C < 2ll * kSchedWarps * kSchedBlocksPerSm * sm_count()) C /= 2;
     return C;
 }
 
