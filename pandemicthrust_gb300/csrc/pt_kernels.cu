@@ -878,8 +878,6 @@ __device__ __forceinline__ unsigned long long contact_offset(const InstConst &c,
 constexpr int kSweepThreads = 256, kSweepRounds = 4, kSweepTile = kSweepThreads * 4 * kSweepRounds;
 static_assert(kSweepTile == kPersonTile, "a sweep tile is a person tile");
 
-constexpr uint32_t kNeverInfected = 0x01u | (0x01u << 8) | (0xFFu << 16) | (0xFFu << 24);
-
 __device__ __forceinline__ uint32_t recover_word(uint32_t st, int d2r, bool &changed)
 {
     uint32_t sp = st & 0xFFu, ss = (st >> 8) & 0xFFu, dp = (st >> 16) & 0xFFu, ds = st >> 24;
@@ -893,7 +891,7 @@ __device__ __forceinline__ uint32_t recover_word(uint32_t st, int d2r, bool &cha
 // The sweep: kernel_countInfectedStatusAndRecover (PandemicSim.cu:2097-2192), the
 // copy_if of the infected (:2207-2224) and runToCompletion's day bookkeeping
 // (:891-937) in three launches over every instance:
-//   count  four person tiles per block (one for small runs): recover, count the
+//   count  a run of person tiles per block (one for small runs): recover, count the
 //          instances' 16 status bins (reduced once per block and instance), and
 //          record each thread's infected persons as a 16-bit mask and each tile's
 //          infected count.  Thread t of a tile holds persons (r * 256 + t) * 4 + j,
@@ -903,17 +901,51 @@ __device__ __forceinline__ uint32_t recover_word(uint32_t st, int d2r, bool &cha
 //   emit   one person tile per warp (per block for small runs): the infected ids,
 //          in ascending order, at their list positions.
 // Each launch depends only on the one before, so no block waits for another.
-constexpr int kSweepTilesPerBlock = 4;   // at most, person tiles a count block sweeps one after another
+// Person tiles a count block sweeps one after another: as many as make the grid one wave
+// of the blocks that fit (kSweepBlocksPerSm), at most what 8-bit status counts hold.
+constexpr int kSweepBlocksPerSm = 8, kSweepTilesPerBlock = 255 / (4 * kSweepRounds);
+// From this many tiles an SM on, the emit kernel has a warp per tile instead of a block.
+constexpr int kSweepEmitTilesPerSm = 32;
 
-// Adds a thread's packed status bins (and its never-infected persons, bin S of both
-// strains) into instance k's row of the day: warp reductions, one shared atomic per
-// bin per warp, one global atomic per bin per block.  Block-uniform; clears the bins.
-__device__ __forceinline__ void sweep_flush_bins(InstState *is, int k, int day, unsigned long long &bp_lo,
-                                                 unsigned long long &bp_hi, unsigned long long &bs_lo,
-                                                 unsigned long long &bs_hi, int &nss, int *s_bins)
+// A thread's persons by status.  Most have neither strain now: those take a test and an
+// addition each (bytes 0 and 1 of `susceptible`: how many of them are susceptible, status 1
+// and not 0, to each strain); the others a byte a status and strain, statuses 0-3 and 4-7.
+// (With every person counted the second way the sweep of 24M persons with vaccinations
+// took 65 us, now 29, for 100 MB.)
+struct SweepBins {
+    uint32_t p[2], s[2];
+    uint32_t susceptible;
+    int healthy;   // persons counted in `susceptible`
+};
+
+// One more person of statuses sp, ss (0..7).  (shl gives 0 for shifts of 32 and more, and
+// the shift less 32 is such a one when it is negative.)
+__device__ __forceinline__ void sweep_count_person(SweepBins &b, uint32_t sp, uint32_t ss)
 {
-    bp_lo += (unsigned long long)nss << 16;  // bin 1 (S) of each strain
-    bs_lo += (unsigned long long)nss << 16;
+    uint32_t v[4];
+    asm("shl.b32 %0, 1, %1;" : "=r"(v[0]) : "r"(8u * sp));
+    asm("shl.b32 %0, 1, %1;" : "=r"(v[1]) : "r"(8u * sp - 32u));
+    asm("shl.b32 %0, 1, %1;" : "=r"(v[2]) : "r"(8u * ss));
+    asm("shl.b32 %0, 1, %1;" : "=r"(v[3]) : "r"(8u * ss - 32u));
+    b.p[0] += v[0];
+    b.p[1] += v[1];
+    b.s[0] += v[2];
+    b.s[1] += v[3];
+}
+
+// Adds a thread's bins into instance k's row of the day: warp reductions, one shared
+// atomic per bin per warp, one global atomic per bin per block.  Block-uniform; clears
+// the bins.
+__device__ __forceinline__ void sweep_flush_bins(InstState *is, int k, int day, SweepBins &bins, int *s_bins)
+{
+    // four 16-bit counts a word; a warp's sums stay below 2^13
+    auto spread = [](uint32_t v) {
+        return (unsigned long long)__byte_perm(v, 0u, 0x4140) | (unsigned long long)__byte_perm(v, 0u, 0x4342) << 32;
+    };
+    const uint32_t sus_p = bins.susceptible & 0xFFu, sus_s = (bins.susceptible >> 8) & 0xFFu;
+    unsigned long long bp_lo = spread(bins.p[0]) + (((uint32_t)bins.healthy - sus_p) | sus_p << 16);
+    unsigned long long bs_lo = spread(bins.s[0]) + (((uint32_t)bins.healthy - sus_s) | sus_s << 16);
+    unsigned long long bp_hi = spread(bins.p[1]), bs_hi = spread(bins.s[1]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         bp_lo += __shfl_xor_sync(0xffffffffu, bp_lo, o);
@@ -938,11 +970,10 @@ __device__ __forceinline__ void sweep_flush_bins(InstState *is, int k, int day, 
         s_bins[threadIdx.x] = 0;
     }
     __syncthreads();
-    bp_lo = bp_hi = bs_lo = bs_hi = 0;
-    nss = 0;
+    bins = SweepBins{};
 }
 
-__global__ void __launch_bounds__(kSweepThreads, 8) k_sweep_count(const InstConst *ic, InstState *is,
+__global__ void __launch_bounds__(kSweepThreads, kSweepBlocksPerSm) k_sweep_count(const InstConst *ic, InstState *is,
                                                                   const int32_t *tile_inst, int tiles, int per_block,
                                                                   uint32_t *state, uint16_t *flags_out,
                                                                   int32_t *tile_count, uint2 *clear, int clear_n,
@@ -959,62 +990,50 @@ __global__ void __launch_bounds__(kSweepThreads, 8) k_sweep_count(const InstCons
     if (threadIdx.x < 16) s_bins[threadIdx.x] = 0;
     if (threadIdx.x < kSweepTilesPerBlock) s_tc[threadIdx.x] = 0;
     __syncthreads();
-    // packed per-thread status bins of the current instance: 16-bit fields, bins 0-3 /
-    // 4-7 per strain
-    unsigned long long bp_lo = 0, bp_hi = 0, bs_lo = 0, bs_hi = 0;
-    int nss = 0;         // persons in the never-infected state (S, S, day 255, day 255)
+    SweepBins bins = {};   // of the current instance
     int cur = tile_inst[t0];
     for (int tile = t0;; tile++) {
         // after the last tile, or when the tiles move on to the next instance: the bins
         const int k = tile < t1 ? tile_inst[tile] : -1;
         if (k != cur) {
-            sweep_flush_bins(is, cur, day, bp_lo, bp_hi, bs_lo, bs_hi, nss, s_bins);  // (ends with a barrier)
+            sweep_flush_bins(is, cur, day, bins, s_bins);  // (ends with a barrier)
             cur = k;
         }
         if (k < 0) break;
-        const long long tile_base = (long long)tile * kSweepTile;
+        const int first = tile * kSweepTile + 4 * (int)threadIdx.x;
         // end of the tile's persons: none when the instance no longer runs
-        const long long N = instance_running(ic[k], is[k], day) ? (long long)ic[k].pbase + ic[k].c.N : tile_base;
+        const int N = instance_running(ic[k], is[k], day) ? ic[k].pbase + ic[k].c.N : 0;
         uint32_t flags = 0;  // bit (4*round + item)
         auto load = [&](int r) {
-            const long long p0 = tile_base + ((long long)r * kSweepThreads + threadIdx.x) * 4;
-            if (p0 < N) return *reinterpret_cast<const uint4 *>(state + p0);   // (padding persons follow)
-            return make_uint4(0u, 0u, 0u, 0u);
+            const int p0 = first + r * 4 * kSweepThreads, n = N - p0;   // persons from p0 on
+            if (n <= 0) return make_uint4(0u, 0u, 0u, 0u);
+            uint4 v = *reinterpret_cast<const uint4 *>(state + p0);     // (padding persons follow)
+            if (n < 4) {
+                v.w = 0u;
+                if (n < 3) v.z = 0u;
+                if (n < 2) v.y = 0u;
+            }
+            bins.healthy += min(n, 4);   // those with a strain are taken off below
+            return v;
         };
         uint4 next = load(0);   // a round's load goes before the last round's stores
 #pragma unroll
         for (int r = 0; r < kSweepRounds; r++) {
-            long long p0 = tile_base + ((long long)r * kSweepThreads + threadIdx.x) * 4;
             const uint32_t st[4] = {next.x, next.y, next.z, next.w};
             if (r + 1 < kSweepRounds) next = load(r + 1);
-            bool any_changed = false;
-            uint32_t out[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                // never infected by either strain: nothing to recover, bin S twice
-                if (st[j] == kNeverInfected && p0 + j < N) {
-                    out[j] = st[j];
-                    nss++;
+                if ((st[j] & 0xFEFEu) == 0u) {   // neither strain (or past the end): nothing to recover
+                    bins.susceptible += st[j] & 0x0101u;
                     continue;
                 }
-                bool ch;
-                out[j] = recover_word(st[j], d2r, ch);
-                if (p0 + j < N) {
-                    any_changed |= ch;
-                    uint32_t sp = out[j] & 0xFFu, ss = (out[j] >> 8) & 0xFFu;
-                    if (sp < 4) bp_lo += 1ull << (16 * sp); else bp_hi += 1ull << (16 * (sp - 4));
-                    if (ss < 4) bs_lo += 1ull << (16 * ss); else bs_hi += 1ull << (16 * (ss - 4));
-                    if (sp >= 2u || ss >= 2u) flags |= 1u << (4 * r + j);
-                }
-            }
-            if (any_changed) {
-                if (p0 + 3 < N) {
-                    *reinterpret_cast<uint4 *>(state + p0) = make_uint4(out[0], out[1], out[2], out[3]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        if (p0 + j < N) state[p0 + j] = out[j];
-                }
+                bins.healthy--;
+                bool changed;
+                const uint32_t out = recover_word(st[j], d2r, changed);
+                const uint32_t sp = out & 0xFFu, ss = (out >> 8) & 0xFFu;
+                sweep_count_person(bins, sp, ss);
+                if (sp >= 2u || ss >= 2u) flags |= 1u << (4 * r + j);
+                if (changed) state[first + r * 4 * kSweepThreads + j] = out;
             }
         }
         flags_out[(size_t)tile * kSweepThreads + threadIdx.x] = (uint16_t)flags;
@@ -1425,9 +1444,7 @@ static size_t day_clear_bytes(const DevArrays &d, bool weekend)
 cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t s)
 {
     const int tiles = d.P / kSweepTile;
-    // several tiles per block only where the grid still fills every SM eight times over
-    // (a small simulation keeps one tile per block and all its parallelism)
-    const int per_block = tiles >= kSweepTilesPerBlock * 8 * sm_count() ? kSweepTilesPerBlock : 1;
+    const int per_block = std::min(div_up(tiles, kSweepBlocksPerSm * sm_count()), kSweepTilesPerBlock);
     const bool small = tiles <= kListTiles;
     k_sweep_count<<<div_up(tiles, per_block), kSweepThreads, 0, s>>>(
         d.ic, d.is, d.tile_inst, tiles, per_block, d.state, d.sweep_flags, d.sweep_tiles,
@@ -1455,7 +1472,7 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
         count_launch();
         return cudaGetLastError();
     }
-    if (tiles >= kSweepTilesPerBlock * 8 * sm_count())
+    if (tiles >= kSweepEmitTilesPerSm * sm_count())
         k_sweep_emit<<<div_up(tiles, kEmitWarps), kEmitWarps * 32, 0, s>>>(d.tile_inst, tiles, d.sweep_flags,
                                                                            d.sweep_tiles, d.infected, d.infected_inst,
                                                                            d.sc);
