@@ -93,9 +93,12 @@ struct Engine {
     int stage_days[2] = {0, 0};
     std::vector<float> day_stage_ms;      // kMaxDays x kStages: the last timed run of each day
     mutable uint64_t h2d_bytes = 0, d2h_bytes = 0;  // host<->device copies issued
-    // The whole day loop (days 0..max_days-1) captured once and replayed by run().
-    // Every per-day decision (early stop, counters, offsets) reads device state, so
-    // the same graph serves every run after a reset.
+    // The whole day loop (days 0..max_days-1), captured once and replayed by later runs.
+    // Every per-day decision (early stop, counters, offsets) reads device state, so the
+    // same graph serves every run after a reset.  The run that captures it queues its own
+    // launches one by one first (2 us each, faster than the device takes them) and
+    // captures while the device works: capturing and instantiating the 900 launches of
+    // 100 days before the first one starts cost 2.5 ms.
     cudaGraphExec_t run_graph = nullptr;
     uint64_t graph_kernels = 0;
     int *day_rows = nullptr;              // mapped host memory of a stepped day's rows (launch_day_rows)
@@ -751,31 +754,36 @@ static pt_status engine_step(Engine *s, int *running)
     return all_zero_stopped(s) ? PT_DONE : PT_OK;
 }
 
+// Captures the whole day loop for later runs.
+static pt_status capture_run(Engine *s)
+{
+    const uint64_t before = ptk::launches();
+    CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+    pt_status st = PT_OK;
+    for (int day = 0; day < s->max_days && st == PT_OK; day++) st = enqueue_day(s, day);
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    s->graph_kernels = ptk::launches() - before;
+    ptk::add_launches(-(int64_t)s->graph_kernels);  // counted when the graph runs
+    if (st != PT_OK) {
+        if (g) cudaGraphDestroy(g);
+        return st;
+    }
+    CK(e, "end capture");
+    e = cudaGraphInstantiate(&s->run_graph, g, 0);
+    cudaGraphDestroy(g);
+    CK(e, "graph instantiate");
+    return PT_OK;
+}
+
 // The remaining days of every instance on the device, then one copy of the rows.
 static pt_status engine_run(Engine *s)
 {
     if (!s->setup_done) return fail(s, PT_ERR_STATE, "run before setup");
     const int first = s->next_day, M = s->max_days;
     if (instances_running(s) > 0 && first < M) {
-        if (first == 0 && !s->timing) {
-            if (!s->run_graph) {
-                const uint64_t before = ptk::launches();
-                CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-                pt_status st = PT_OK;
-                for (int day = 0; day < M && st == PT_OK; day++) st = enqueue_day(s, day);
-                cudaGraph_t g = nullptr;
-                cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-                if (st != PT_OK) {
-                    if (g) cudaGraphDestroy(g);
-                    return st;
-                }
-                CK(e, "end capture");
-                e = cudaGraphInstantiate(&s->run_graph, g, 0);
-                cudaGraphDestroy(g);
-                CK(e, "graph instantiate");
-                s->graph_kernels = ptk::launches() - before;
-                ptk::add_launches(-(int64_t)s->graph_kernels);  // counted when the graph runs
-            }
+        const bool replay = first == 0 && !s->timing && s->run_graph;
+        if (replay) {
             CK(cudaGraphLaunch(s->run_graph, s->stream), "graph launch");
             ptk::add_launches((int64_t)s->graph_kernels);
         } else {
@@ -783,6 +791,10 @@ static pt_status engine_run(Engine *s)
                 pt_status st = enqueue_day(s, day);
                 if (st != PT_OK) return st;
             }
+        }
+        if (first == 0 && !s->timing && !s->run_graph) {
+            const pt_status st = capture_run(s);
+            if (st != PT_OK) return st;
         }
         s->next_day = M;
     }
