@@ -54,11 +54,11 @@ FALLBACK_HBM_GBS = 6800.0
 # use (2 hours x locations of types 8-13 weekday, 10 hours x types 9-13 weekend).
 #   sweep          4N read (status + day, both strains)
 #   infected_list  4I written (the ascending infected ids)
-#   schedule       weekday 1N age read + 4E keys written; weekend 4E keys written
+#   schedule       weekday 1N age read; 8E' entries (bucket, person) written, E' = entries of
+#                  the buckets that the day's infected visit (the only ones materialised)
 #   digit_bases    (no compulsory traffic: the radix bookkeeping of the sort)
-#   bucket_sort    4E schedule read + 4E' bucket entries written, E' = entries of the
-#                  buckets that the day's infected visit (the only ones materialised)
-#   bucket_offsets 4(Bc+1) offsets written (the reference's lower_bound output)
+#   bucket_sort    8E' entries read + 4E' persons written + 8Bc bucket starts and sizes
+#   bucket_offsets (empty: the sort's last pass writes the buckets)
 #   infect         79 B per infected weekday, 52 B weekend
 #   apply          claim 8 B read + 8 B reset + state 4 B + generation 1 B per new infection
 def stage_bytes(stage, weekend, N, Bc, I_mean, new_mean=0.0, mat_frac=1.0):
@@ -66,10 +66,10 @@ def stage_bytes(stage, weekend, N, Bc, I_mean, new_mean=0.0, mat_frac=1.0):
     return {
         "sweep": 4 * N,
         "infected_list": 4 * I_mean,
-        "schedule": (4 * E) if weekend else (N + 4 * E),
+        "schedule": 8 * E * mat_frac + (0 if weekend else N),
         "digit_bases": 0,
-        "bucket_sort": 4 * E + 4 * E * mat_frac,
-        "bucket_offsets": 4 * (Bc + 1),
+        "bucket_sort": 12 * E * mat_frac + 8 * Bc,
+        "bucket_offsets": 0,
         "infect": (52 if weekend else 79) * I_mean,
         "apply": 21 * new_mean,
     }[stage]
@@ -903,7 +903,7 @@ def main():
             "roofline": {"bound": "hbm", "kernel": dominant, "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                          "traffic_source": ("mean DRAM bytes per launch over one 100-day run of this workload, "
-                                            "one-pass ncu capture (profiles/ncu_schedule_traffic_50M.md, "
+                                            "one-pass ncu capture (profiles/ncu_schedule_regions.md, "
                                             "profiles/ncu_traffic.txt)") if traffic else None},
             "int_roofline": int_roof(dominant, nwd, nwe),
             "day_roofline": {"achieved": day_achieved, "peak": peak, "unit": "GB/s", "frac": day_achieved / peak,
