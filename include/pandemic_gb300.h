@@ -118,7 +118,7 @@ pt_status pt_setup(pt_sim *sim);
 pt_status pt_step_day(pt_sim *sim, int counts16[16], int *infected_count);
 
 /* PandemicSim::runToCompletion without per-day host synchronisation: runs the
- * remaining days on the device (captured as one CUDA graph) and copies back, per
+ * remaining days on the device (queued at once; later runs replay one CUDA graph) and copies back, per
  * day, the 16 status bins (counts, max_days*16 ints, may be NULL) and the
  * infected count (infected, max_days ints, may be NULL).  days_run receives the
  * number of statistics rows, as the reference's output_infected_stats.csv. */
@@ -169,8 +169,8 @@ pt_status pt_set_full_tables(pt_sim *sim, int enabled);
 /* Device time per stage, from CUDA events recorded on the simulation's stream
  * around each stage of every day run while timing is enabled (pt_set_timing).
  * ms[0..7] sum the weekday stages, ms[8..15] the weekend stages, in the order:
- * sweep (recover, count), infected list, schedule, digit bases, bucket radix sort,
- * bucket offsets, infection, apply.
+ * sweep (recover, count), infected list and marks, schedule, digit bases, bucket radix
+ * sort (which writes the buckets), bucket offsets (empty), infection, apply.
  * days[0], days[1] receive the number of weekdays and weekend days timed.  The sums
  * reset after each call.  With timing enabled, a day run by pt_step_day or pt_run
  * records events but adds no host synchronisation. */
@@ -329,7 +329,7 @@ const char *pt_last_error(const pt_sim *sim);
 /* ------------------------------------------------------------------ batches
  * A batch runs many independent simulations (replicates, scenarios, uneven sizes)
  * together: every day is one set of kernel launches over all of them, and the whole
- * day loop is one CUDA graph.  The reference runs one simulation per process; its
+ * day loop is one CUDA graph from the second run on.  The reference runs one simulation per process; its
  * PythonBatcher scripts (write_gpu_constants.py) start one process per scenario and
  * seed.  Instance k of a batch gives exactly the results of pt_create(&params[k],
  * core_seeds[k]) run alone: statistics rows, generation counts and per-person state.
