@@ -1631,6 +1631,7 @@ struct pt_mlp {
     // tcgen05 inference: the padded input batch and a wait error word (host memory the
     // device writes)
     int use_umma = 1;
+    bool chain_ready = false;   // training: k_chain may be launched
     bf16 *h0p = nullptr;
     int *umma_err = nullptr;
     // inference input (FP32 rows copied from the host), and the accumulator of last layers
@@ -1809,10 +1810,12 @@ static cudaError_t error_word(pt_mlp *m)
 
 static cudaError_t chain(pt_mlp *m, int B, const bf16 *h0, const float *Y, const int *rows, float *loss)
 {
-    static const cudaError_t attr = cudaFuncSetAttribute(k_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmem);
-    if (attr != cudaSuccess) return attr;
-    const cudaError_t e = error_word(m);
-    if (e != cudaSuccess) return e;
+    if (!m->chain_ready) {   // (a kernel's attributes are those of the network's device)
+        cudaError_t e = cudaFuncSetAttribute(k_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmem);
+        if (e == cudaSuccess) e = error_word(m);
+        if (e != cudaSuccess) return e;
+        m->chain_ready = true;
+    }
     ChainArgs a = {};
     a.error = m->umma_err;
     a.L = m->L;
@@ -1944,16 +1947,12 @@ static cudaError_t umma_prepare(pt_mlp *m)
     if (m->h0p) return cudaSuccess;
     cudaError_t e = error_word(m);
     if (e != cudaSuccess) return e;
-    static const cudaError_t attr = [] {
-        cudaError_t a = cudaFuncSetAttribute(k_umma_layer<kUmmaEpiWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             kUmmaSmem);
-        if (a == cudaSuccess)
-            a = cudaFuncSetAttribute(k_umma_mean_layer, cudaFuncAttributeMaxDynamicSharedMemorySize, kMeanSmem);
-        if (a == cudaSuccess)
-            a = cudaFuncSetAttribute(k_umma_hidden, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmem);
-        return a;
-    }();
-    if (attr != cudaSuccess) return attr;
+    // once a network: a kernel's attributes are those of its device
+    e = cudaFuncSetAttribute(k_umma_layer<kUmmaEpiWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_umma_mean_layer, cudaFuncAttributeMaxDynamicSharedMemorySize, kMeanSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_umma_hidden, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmem);
+    if (e != cudaSuccess) return e;
     return dalloc(m, &m->h0p, (size_t)m->max_batch * m->ld[0]);
 }
 
