@@ -318,8 +318,9 @@ cudaError_t launch_count_keys(const int32_t *keys, int n, int32_t *count, cudaSt
 // What bounds it (24M pairs on a GB300, each part left out in turn): reading and
 // writing 16 bytes an entry 64 us, ranking 50, look-back one tile a step 45, scattered
 // instead of linear writes 12.  So the look-back reads four predecessors a step, and
-// after the tile is placed, when more of them are ready (143 us instead of 171); and
-// three blocks of 256 threads an SM (80 registers) do better than four (64, 163 us),
+// after the tile is placed, when more of them are ready (143 us instead of 171), and only
+// the digits a pass has publish and look (128 of 256 where it sorts 7 bits: weekdays of 48
+// instances 77.5 -> 75.2 ms a run); and three blocks of 256 threads an SM (80 registers) do better than four (64, 163 us),
 // 16 x 384 or 512 threads (154, 170) or 12 entries a thread (187).  Ranking by ballots
 // (160), match (208) or one warp barrier a round with three word sets (160) is slower.
 constexpr int kRadixThreads = 256, kRadixItems = 16, kRadixWarps = kRadixThreads / 32;
@@ -601,7 +602,8 @@ __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass
             run += s_hist[w][d];
         }
         volatile unsigned long long *const st = a.status;
-        st[(size_t)tile * 256 + d] = lb_word(epoch, stile == 0 ? 2 : 1, (unsigned)run);
+        const bool digit = d <= (int)dmask;   // (the others have no entries)
+        if (digit) st[(size_t)tile * 256 + d] = lb_word(epoch, stile == 0 ? 2 : 1, (unsigned)run);
         int valid;
         const int toff = block_exclusive_scan<kRadixThreads, int>(run, valid);
 #pragma unroll
@@ -612,11 +614,11 @@ __global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm) k_radix_pass
         for (int j = 0; j < kRadixItems; j++)
             if (whole || kv[j].y != kDropped) s_pair[hist[(kv[j].x >> shift) & dmask] + place[j]] = kv[j];
         int excl = 0;
-        if (stile != 0) {
+        if (digit && stile != 0) {
             excl = radix_look_back(st, epoch, tile, tile - stile, d, a.error);
             st[(size_t)tile * 256 + d] = lb_word(epoch, 2, (unsigned)(excl + run));
         }
-        s_base[d] = sbase + a.digit_base[((size_t)s_t.seg * a.passes + a.pass) * 256 + d] + excl - toff;
+        if (digit) s_base[d] = sbase + a.digit_base[((size_t)s_t.seg * a.passes + a.pass) * 256 + d] + excl - toff;
         __syncthreads();
 #pragma unroll
         for (int w = 0; w < kRadixWarps; w++) s_hist[w][d] = 0;   // for the next tile (whose barrier follows)
