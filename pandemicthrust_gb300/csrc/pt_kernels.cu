@@ -867,6 +867,13 @@ __device__ __forceinline__ bool instance_running(const InstConst &c, const InstS
     return !s.done && day < c.max_days;
 }
 
+// The day of a launch: its own, or (-1, a launch of a graph that serves every stepped
+// day of its kind) the next one to step.
+__device__ __forceinline__ int launch_day(int day, const Scalars *sc)
+{
+    return day >= 0 ? day : *(volatile const int *)&sc->step_day;
+}
+
 // R0 of a day whose schedule starts at counter E0.
 __device__ __forceinline__ unsigned long long contact_offset(const InstConst &c, unsigned long long E0, bool weekend)
 {
@@ -981,6 +988,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepBlocksPerSm) k_sweep_coun
                                                                   int32_t *tile_count, uint2 *clear, int clear_n,
                                                                   const Scalars *sc, int day)
 {
+    day = launch_day(day, sc);
     if (*(volatile const int *)&sc->done) return;
     for (int i = blockIdx.x * kSweepThreads + threadIdx.x; i < clear_n; i += gridDim.x * kSweepThreads)
         clear[i] = make_uint2(0u, 0u);
@@ -1101,6 +1109,7 @@ __global__ void __launch_bounds__(kSweepScanThreads) k_sweep_scan(const InstCons
                                                                   int32_t *tile_count, int tiles, Scalars *sc,
                                                                   int day, int dense_level)
 {
+    day = launch_day(day, sc);
     if (*(volatile const int *)&sc->done) return;
     // exclusive scan in place, a contiguous chunk per thread; entry `tiles` = total
     const int per = (tiles + kSweepScanThreads - 1) / kSweepScanThreads;
@@ -1358,6 +1367,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
                                                               int words, int mark_all, Scalars *sc, int day,
                                                               int dense_level)
 {
+    day = launch_day(day, sc);
     const int ended = *(volatile const int *)&sc->done;
     if (ended != 0 && ended != day + 1) return;
     const bool weekend = (day % 7) >= 5;
@@ -1557,6 +1567,7 @@ __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
             const uint32_t *mark, int32_t *keys, int *digit_hist, int passes, int dbits, uint2 *entries,
             int32_t *region_count, const Scalars *sc, int day)
 {
+    day = launch_day(day, sc);
     if (*(volatile const int *)&sc->done) return;
     static_assert(kSchedThreads == 256, "one thread per digit in sched_flush_digits");
     constexpr int kPer = WEEKEND ? 3 : 2;                       // keys per person
@@ -2292,6 +2303,7 @@ template <bool WEEKEND>
 __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
 {
     Scalars *sc = a.sc;
+    day = launch_day(day, sc);
     if (sc->done) return;
     infect_coop<WEEKEND>(a, day, sc->infected, claim_queue<8>(a.new_list, sc));
 }
@@ -2305,6 +2317,7 @@ __global__ void __launch_bounds__(256) k_infect_coop(InfectArgs a, int day)
 __global__ void __launch_bounds__(128, 8) k_infect_weekday(InfectArgs a, int day)
 {
     Scalars *sc = a.sc;
+    day = launch_day(day, sc);
     if (sc->done) return;
     const int I = sc->infected;
     const ClaimQueue queue = claim_queue<4>(a.new_list, sc);
@@ -2391,6 +2404,7 @@ __global__ void __launch_bounds__(128, 8) k_infect_weekday(InfectArgs a, int day
 __global__ void __launch_bounds__(128, 8) k_infect_weekend(InfectArgs a, int day)
 {
     Scalars *sc = a.sc;
+    day = launch_day(day, sc);
     if (sc->done) return;
     const int I = sc->infected;
     const ClaimQueue queue = claim_queue<4>(a.new_list, sc);
@@ -2467,6 +2481,7 @@ cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_
 __global__ void k_apply(uint32_t *state, uint8_t *gen_p, uint8_t *gen_s, unsigned long long *claim,
                         const int32_t *new_list, Scalars *sc, int day)
 {
+    day = launch_day(day, sc);
     if (sc->done) return;
     const int n = sc->new_count;
     const uint8_t dset = (uint8_t)(day + 1);
@@ -2493,23 +2508,25 @@ cudaError_t launch_apply(const DevArrays &d, int day, cudaStream_t s)
     return cudaGetLastError();
 }
 
-__global__ void k_day_rows(const InstState *is, int K, int day, const Scalars *sc, int *out)
+// (one block: it also moves the next stepped day on)
+__global__ void __launch_bounds__(1024) k_day_rows(const InstState *is, int K, int day, Scalars *sc, int *out)
 {
-    const int n = K * kDayRow;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-        if (i == n) {
-            out[0] = sc->error;
-            continue;
-        }
+    day = launch_day(day, sc);
+    for (int i = threadIdx.x; i < K * kDayRow; i += blockDim.x) {
         const InstState &s = is[i / kDayRow];
         const int f = i % kDayRow;
         out[1 + i] = f < 16 ? s.counts[day][f] : (f == 16 ? s.infected_per_day[day] : s.days_run);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        out[0] = sc->error;
+        sc->step_day = day + 1;
     }
 }
 
 cudaError_t launch_day_rows(const DevArrays &d, int day, int *out, cudaStream_t s)
 {
-    k_day_rows<<<std::min(div_up(d.K * kDayRow + 1, 256), sm_count()), 256, 0, s>>>(d.is, d.K, day, d.sc, out);
+    k_day_rows<<<1, std::min(1024, div_up(d.K * kDayRow, 32) * 32), 0, s>>>(d.is, d.K, day, d.sc, out);
     count_launch();
     return cudaGetLastError();
 }

@@ -83,7 +83,7 @@ struct Scalars {
     int new_count;                        // entries in the new-infection list
     int error;                            // nonzero: a bounded device wait gave up
     int error_site;
-    int pad;
+    int step_day;                         // next day to step (launches with day -1 read it)
 };
 
 // Launch shapes chosen at run time (the engine's tuner picks them per engine; every

@@ -102,8 +102,21 @@ struct Engine {
     cudaGraphExec_t run_graph = nullptr;
     uint64_t graph_kernels = 0;
     int *day_rows = nullptr;              // mapped host memory of a stepped day's rows (launch_day_rows)
+    // A stepped weekday's and weekend day's launches: the first of each kind is queued and
+    // then captured while the device works; the later ones replay it and read their day on
+    // the device.  (Ten launches take 35 us of a step's 90 on an Arm host, a replay 8.)
+    cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
+    uint64_t step_kernels[2] = {0, 0};
+    bool no_step_graph = false;           // the stream cannot be captured
 
     int K() const { return (int)inst.size(); }
+    void drop_graphs()   // what was captured depends on the settings
+    {
+        for (cudaGraphExec_t *g : {&run_graph, &step_graph[0], &step_graph[1]}) {
+            if (*g) cudaGraphExecDestroy(*g);
+            *g = nullptr;
+        }
+    }
     ~Engine();
 };
 
@@ -196,7 +209,7 @@ static pt_status cuda_fail(Engine *s, cudaError_t e, const char *where)
 Engine::~Engine()
 {
     if (stream) cudaStreamSynchronize(stream);
-    if (run_graph) cudaGraphExecDestroy(run_graph);
+    drop_graphs();
     // back to the pool, in stream order
     if (arena_mem) cudaFreeAsync(arena_mem, stream);
     if (setup_mem) cudaFreeAsync(setup_mem, stream);
@@ -585,18 +598,21 @@ static cudaEvent_t stage_event(Engine *s, int day, int k)
 // Enqueues one day of every instance: sweep, schedule, bucket build (scan, radix
 // sort), infection, apply.  Every kernel after the sweep skips an instance that
 // counted no infected, and skips itself once no instance has infected left.
-static pt_status enqueue_day(Engine *s, int day)
+// `launch` is the day the launches are told, the day or -1 (see launch_day).
+static bool is_weekend(int day) { return (day % 7) >= 5; }  // PandemicSim.h:283-284
+
+static pt_status enqueue_day(Engine *s, int day, int launch)
 {
-    const bool weekend = (day % 7) >= 5;  // PandemicSim.h:283-284
+    const bool weekend = is_weekend(day);
     const ptk::DevArrays &d = s->d;
     cudaStream_t st = s->stream;
     const bool t = s->timing;
     if (t) cudaEventRecord(stage_event(s, day, kStSweep), st);
-    CK(ptk::launch_sweep(d, weekend, day, st), "sweep");
+    CK(ptk::launch_sweep(d, weekend, launch, st), "sweep");
     if (t) cudaEventRecord(stage_event(s, day, kStInfectedList), st);
-    CK(ptk::launch_infected_list(d, weekend, day, s->full_tables, st), "infected list");
+    CK(ptk::launch_infected_list(d, weekend, launch, s->full_tables, st), "infected list");
     if (t) cudaEventRecord(stage_event(s, day, kStSchedule), st);
-    CK(ptk::launch_schedule(d, weekend, day, st), "schedule");
+    CK(ptk::launch_schedule(d, weekend, launch, st), "schedule");
     if (t) cudaEventRecord(stage_event(s, day, kStDigits), st);
     CK(ptk::launch_bucket_scan(d, weekend, st), "digit bases");
     if (t) cudaEventRecord(stage_event(s, day, kStRadix), st);
@@ -604,9 +620,9 @@ static pt_status enqueue_day(Engine *s, int day)
     // (the sort's last pass writes the bucket slots: the offsets stage is empty)
     if (t) cudaEventRecord(stage_event(s, day, kStOffsets), st);
     if (t) cudaEventRecord(stage_event(s, day, kStInfect), st);
-    CK(ptk::launch_infect(d, weekend, day, st), "infect");
+    CK(ptk::launch_infect(d, weekend, launch, st), "infect");
     if (t) cudaEventRecord(stage_event(s, day, kStApply), st);
-    CK(ptk::launch_apply(d, day, st), "apply");
+    CK(ptk::launch_apply(d, launch, st), "apply");
     if (t) cudaEventRecord(stage_event(s, day, kStages), st);
     if (t) s->timed_days.push_back(day);
     return PT_OK;
@@ -700,16 +716,57 @@ static pt_status fetch_rows(Engine *s, int lo, int hi)
     return PT_OK;
 }
 
-// The same for one day that has just been queued.  A caller that steps waits for this
-// every day, so a kernel writes the rows to mapped host memory: four copies to pageable
-// memory took 40 us of a 120 us step (24,000 persons, GB300).
-static pt_status fetch_day(Engine *s, int day)
+// Queues a stepped day and the copy of its rows; `launch` as for enqueue_day.
+static pt_status queue_step(Engine *s, int day, int launch)
 {
-    const int K = s->K();
+    const pt_status st = enqueue_day(s, day, launch);
+    if (st != PT_OK) return st;
+    CK(ptk::launch_day_rows(s->d, launch, s->day_rows, s->stream), "day rows");
+    return PT_OK;
+}
+
+// Captures a stepped day of the kind of `day` for later ones.  A stream that cannot be
+// captured goes on without.
+static pt_status capture_step(Engine *s, int day)
+{
+    const int kind = is_weekend(day) ? 1 : 0;
+    if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        cudaGetLastError();
+        s->no_step_graph = true;
+        return PT_OK;
+    }
+    const uint64_t before = ptk::launches();
+    const pt_status st = queue_step(s, day, -1);
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    s->step_kernels[kind] = ptk::launches() - before;
+    ptk::add_launches(-(int64_t)s->step_kernels[kind]);  // counted when the graph runs
+    if (st == PT_OK && e == cudaSuccess) cudaGraphInstantiate(&s->step_graph[kind], g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (st != PT_OK) return st;
+    CK(e, "end capture");
+    CK(cudaGetLastError(), "graph instantiate");
+    return PT_OK;
+}
+
+// One stepped day and its rows.  A caller that steps waits for them every day, so a
+// kernel writes them to mapped host memory: four copies to pageable memory took 40 us of
+// a 120 us step (24,000 persons, GB300).
+static pt_status step_day(Engine *s, int day)
+{
+    const int K = s->K(), kind = is_weekend(day) ? 1 : 0;
     const size_t bytes = ((size_t)K * ptk::kDayRow + 1) * sizeof(int);
     if (!s->day_rows)
         CK(cudaHostAlloc((void **)&s->day_rows, bytes, cudaHostAllocMapped | cudaHostAllocPortable), "day rows");
-    CK(ptk::launch_day_rows(s->d, day, s->day_rows, s->stream), "day rows");
+    pt_status st = PT_OK;
+    if (!s->timing && s->step_graph[kind]) {
+        CK(cudaGraphLaunch(s->step_graph[kind], s->stream), "graph launch");
+        ptk::add_launches((int64_t)s->step_kernels[kind]);
+    } else {
+        st = queue_step(s, day, day);
+        if (st == PT_OK && !s->timing && !s->no_step_graph) st = capture_step(s, day);
+    }
+    if (st != PT_OK) return st;
     s->d2h_bytes += bytes;
     CK(cudaStreamSynchronize(s->stream), "sync");
     if (s->day_rows[0]) return fail(s, PT_ERR_TIMEOUT, "a device-side wait gave up (look-back ordering)");
@@ -745,10 +802,8 @@ static pt_status engine_step(Engine *s, int *running)
     if (!s->setup_done) return fail(s, PT_ERR_STATE, "step before setup");
     if (instances_running(s) == 0) return all_zero_stopped(s) ? PT_DONE : PT_FINISHED;
     const int day = s->next_day;
-    pt_status st = enqueue_day(s, day);
-    if (st != PT_OK) return st;
     s->next_day = day + 1;
-    st = fetch_day(s, day);
+    const pt_status st = step_day(s, day);
     if (st != PT_OK) return st;
     if (running) *running = instances_running(s);
     return all_zero_stopped(s) ? PT_DONE : PT_OK;
@@ -760,7 +815,7 @@ static pt_status capture_run(Engine *s)
     const uint64_t before = ptk::launches();
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     pt_status st = PT_OK;
-    for (int day = 0; day < s->max_days && st == PT_OK; day++) st = enqueue_day(s, day);
+    for (int day = 0; day < s->max_days && st == PT_OK; day++) st = enqueue_day(s, day, day);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
     s->graph_kernels = ptk::launches() - before;
@@ -788,7 +843,7 @@ static pt_status engine_run(Engine *s)
             ptk::add_launches((int64_t)s->graph_kernels);
         } else {
             for (int day = first; day < M; day++) {
-                pt_status st = enqueue_day(s, day);
+                pt_status st = enqueue_day(s, day, day);
                 if (st != PT_OK) return st;
             }
         }
@@ -972,8 +1027,7 @@ static pt_status engine_set_tuning(Engine *s, const pt_tuning *t)
         n.dense_level != s->d.tune.dense_level || n.radix_threads != s->d.tune.radix_threads) {
         // the captured day loop holds the old launch shapes
         if (s->stream) cudaStreamSynchronize(s->stream);
-        if (s->run_graph) cudaGraphExecDestroy(s->run_graph);
-        s->run_graph = nullptr;
+        s->drop_graphs();
     }
     s->d.tune = n;
     return PT_OK;
@@ -1230,11 +1284,8 @@ pt_status pt_set_full_tables(pt_sim *s, int enabled)
 {
     if (!s) return PT_ERR_ARG;
     const bool v = enabled != 0;
-    if (v != s->full_tables && s->run_graph) {
-        // the captured day loop bakes this choice in; capture again on the next run
-        cudaGraphExecDestroy(s->run_graph);
-        s->run_graph = nullptr;
-    }
+    // the captured launches bake this choice in; they are captured again when needed
+    if (v != s->full_tables) s->drop_graphs();
     s->full_tables = v;
     return PT_OK;
 }
