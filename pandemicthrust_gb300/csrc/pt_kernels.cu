@@ -2508,6 +2508,29 @@ cudaError_t launch_apply(const DevArrays &d, int day, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// Four persons a thread; the persons up to the next multiple of four are padding.
+__global__ void k_unpack_state(const uint32_t *state, int n, size_t plane, uint8_t *out)
+{
+    const int i = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    const uint4 v = *reinterpret_cast<const uint4 *>(state + i);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t lo = __byte_perm(v.x, v.y, k | (4 + k) << 4), hi = __byte_perm(v.z, v.w, k | (4 + k) << 4);
+        *reinterpret_cast<uint32_t *>(out + k * plane + i) = __byte_perm(lo, hi, 0x5410);
+    }
+}
+
+uint8_t *state_planes(const DevArrays &d) { return reinterpret_cast<uint8_t *>(d.new_list); }
+
+cudaError_t launch_unpack_state(const DevArrays &d, int first, int n, cudaStream_t s)
+{
+    if (n <= 0) return cudaSuccess;
+    k_unpack_state<<<div_up(n, 4 * 256), 256, 0, s>>>(d.state + first, n, state_plane((size_t)n), state_planes(d));
+    count_launch();
+    return cudaGetLastError();
+}
+
 // (one block: it also moves the next stepped day on)
 __global__ void __launch_bounds__(1024) k_day_rows(const InstState *is, int K, int day, Scalars *sc, int *out)
 {

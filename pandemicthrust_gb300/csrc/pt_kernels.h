@@ -269,6 +269,11 @@ cudaError_t launch_apply(const DevArrays &d, int day, cudaStream_t s);
 // A day's rows of every instance to mapped host memory: out[0] the device error word, then
 // per instance its 16 counts, infected and days run.
 constexpr int kDayRow = 18;
+// The state words of n persons from `first` on (a tile boundary) as four planes of bytes, each
+// state_plane(n) long, in the day's claim list (free between days): status_p, status_s, day_p, day_s.
+inline size_t state_plane(size_t n) { return (n + 15) / 16 * 16; }
+uint8_t *state_planes(const DevArrays &d);
+cudaError_t launch_unpack_state(const DevArrays &d, int first, int n, cudaStream_t s);
 cudaError_t launch_day_rows(const DevArrays &d, int day, int *out, cudaStream_t s);
 // weekday / weekend buckets of one instance (compact keys hour * R + dest - lo)
 int day_buckets(const SimConst &c, bool weekend);
