@@ -716,6 +716,15 @@ static pt_status fetch_rows(Engine *s, int lo, int hi)
     return PT_OK;
 }
 
+// A run or a step waits for its rows, so it cannot be part of a caller's capture.
+static pt_status refuse_capture(Engine *s)
+{
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s->stream, &capture), "stream");
+    if (capture != cudaStreamCaptureStatusNone) CK(cudaErrorStreamCaptureUnsupported, "days in a capture");
+    return PT_OK;
+}
+
 // Queues a stepped day and the copy of its rows; `launch` as for enqueue_day.
 static pt_status queue_step(Engine *s, int day, int launch)
 {
@@ -801,6 +810,8 @@ static pt_status engine_step(Engine *s, int *running)
 {
     if (!s->setup_done) return fail(s, PT_ERR_STATE, "step before setup");
     if (instances_running(s) == 0) return all_zero_stopped(s) ? PT_DONE : PT_FINISHED;
+    const pt_status captured = refuse_capture(s);
+    if (captured != PT_OK) return captured;
     const int day = s->next_day;
     s->next_day = day + 1;
     const pt_status st = step_day(s, day);
@@ -837,6 +848,8 @@ static pt_status engine_run(Engine *s)
     if (!s->setup_done) return fail(s, PT_ERR_STATE, "run before setup");
     const int first = s->next_day, M = s->max_days;
     if (instances_running(s) > 0 && first < M) {
+        const pt_status captured = refuse_capture(s);
+        if (captured != PT_OK) return captured;
         const bool replay = first == 0 && !s->timing && s->run_graph;
         if (replay) {
             CK(cudaGraphLaunch(s->run_graph, s->stream), "graph launch");

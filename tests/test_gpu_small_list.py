@@ -49,3 +49,25 @@ def test_instances_that_end_on_different_days(native_lib):
         assert np.array_equal(counts, bc) and np.array_equal(infected, bi)
         sim.close()
     batch.close()
+
+
+def test_a_run_inside_a_capture_is_refused(native_lib):
+    torch = pytest.importorskip("torch")
+    stream = torch.cuda.Stream()
+    p = make_params(max_days=4, r_pandemic=1.5, r_seasonal=1.5, initial_pandemic=5, initial_seasonal=5,
+                    people_scaling=0.002, location_scaling=0.002)
+    sim = pt.PandemicSim(p, 3, stream=stream.cuda_stream)
+    sim.setupSim()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        with pytest.raises(pt.PtError):
+            sim.runToCompletion()
+        with pytest.raises(pt.PtError):
+            sim.step_day()
+    counts, infected = sim.runToCompletion()
+    other = pt.PandemicSim(p, 3)
+    other.setupSim()
+    c, i = other.runToCompletion()
+    assert np.array_equal(counts, c) and np.array_equal(infected, i)
+    sim.close()
+    other.close()
