@@ -1092,8 +1092,9 @@ __global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThrea
 // Every wait is bounded, as in k_umma_layer.  The order of the MMAs into an accumulator is
 // that of k_umma_layer, and so are the results, bit for bit.  262,144 rows through 11-256-
 // 256-256-222 take 764 us with it, 607 of them here, against 1,031 layer by layer (GB300);
-// 32 rows 65 us instead of 220.  Bound by the weight slices, 27 bytes a clock and SM from
-// L2 with every SM reading, and then by the epilogue's GELUs.
+// 32 rows 65 us instead of 220.  No unit is near its limit (tensor pipe 29% busy, issue
+// 42%, shared-memory banks 13%; with half of each weight slice copied 752 us, so L2 is not
+// it): a slice's two MMAs take 500 to 650 cycles beside the other item's epilogue, 256 alone.
 constexpr int kNetStages = 6, kNetK = 32, kNetStageBytes = kUmmaMaxN * kNetK * 2, kNetTileBytes = kUmmaM * kUmmaMaxK * 2;
 constexpr int kNetBarBytes = 1024;
 constexpr int kNetSmem = kNetBarBytes + 2 * kNetTileBytes + kNetStages * kNetStageBytes;
