@@ -1088,7 +1088,11 @@ __global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThrea
 //   warps 2-17  epilogue: bias, GELU, the next layer's activations (to shared memory in
 //               the operand layout; the last layer's to global memory)
 // Barriers: full / empty per stage; per item slot (X, Y) x: the inputs have landed, acc: the
-// layer's MMAs are done, a: its epilogue is (activations stored, accumulator drained).
+// layer's MMAs are done, a: its epilogue is (activations stored, accumulator drained), free:
+// the item's last MMAs are done.  The producer waits for `free`, one phase an item, before an
+// item's inputs go into a slot.  (acc has a phase a layer: a wait by parity on it is only
+// right for one who has seen the phase before, and at 64 hidden columns the ring holds more
+// slices than an item has.)
 // Every wait is bounded, as in k_umma_layer.  The order of the MMAs into an accumulator is
 // that of k_umma_layer, and so are the results, bit for bit.  262,144 rows through 11-256-
 // 256-256-222 take 764 us with it, 607 of them here, against 1,031 layer by layer (GB300);
@@ -1117,7 +1121,7 @@ __global__ void __launch_bounds__(kNetThreads, 1)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t b_full = smem_u32(smem), b_empty = b_full + 8 * kNetStages, b_x = b_empty + 8 * kNetStages,
-                   b_acc = b_x + 16, b_a = b_acc + 16, b_drain = b_a + 16;
+                   b_acc = b_x + 16, b_a = b_acc + 16, b_free = b_a + 16, b_drain = b_free + 16;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 512);
     volatile int *fail = reinterpret_cast<volatile int *>(smem + 576);
     const uint32_t sA_u = smem_u32(smem + kNetBarBytes), sW_u = sA_u + 2 * kNetTileBytes;
@@ -1135,6 +1139,7 @@ __global__ void __launch_bounds__(kNetThreads, 1)
             mbar_init(b_x + 8 * i, 1);
             mbar_init(b_acc + 8 * i, 1);
             mbar_init(b_a + 8 * i, kNetEpiWarps);
+            mbar_init(b_free + 8 * i, 1);
         }
         mbar_init(b_drain, 1);
         *fail = 0;
@@ -1157,7 +1162,7 @@ __global__ void __launch_bounds__(kNetThreads, 1)
                         const int m = (i0 + t) % n.members;
                         if (l == 0) {
                             // the slot's buffer is free once its last item's last MMAs have read it
-                            if (seen[t] > 0 && !mbar_wait(b_acc + 8 * t, (seen[t] * n.layers - 1) & 1, fail)) {
+                            if (seen[t] > 0 && !mbar_wait(b_free + 8 * t, (seen[t] - 1) & 1, fail)) {
                                 ok = false;
                                 break;
                             }
@@ -1232,7 +1237,10 @@ __global__ void __launch_bounds__(kNetThreads, 1)
                                 umma_bf16(d, ad, wd, idesc, g != 0);
                             }
                             umma_commit(b_empty + 8 * st);   // the stage is free once these MMAs complete
-                            if (k0 + kNetK >= K) umma_commit(b_acc + 8 * t);
+                            if (k0 + kNetK >= K) {
+                                umma_commit(b_acc + 8 * t);
+                                if (l + 1 == n.layers) umma_commit(b_free + 8 * t);
+                            }
                         }
                         __syncwarp();
                     }
