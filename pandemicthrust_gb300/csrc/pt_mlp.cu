@@ -820,9 +820,11 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
 // 64 of a layer's columns (8 a warp): a batch of 512 fills 128 SMs, and an SM reads a
 // quarter of the weights.  The activations (then the dZ) of the rows lie in every CTA's
 // shared memory, twice: a step's epilogue sends its columns to all four CTAs with
-// st.async, whose bytes complete the mbarrier that the next step waits for.  Whoever has
-// a step's rows complete knows that every warp is done with the step before, so nothing
-// else guards the two copies, nor the ring of the CTA's weights (forward: its 64 rows of
+// st.async, whose bytes complete the mbarrier that the next step waits for.  A CTA with no
+// columns in a layer (they all lie past its padded width) sends 16 bytes instead, which no
+// product reads.  So whoever has a step's rows complete knows that every CTA has the rows of
+// the step before and that every warp has read them, and nothing else guards the two copies
+// and their barriers, nor the ring of the CTA's weights (forward: its 64 rows of
 // W; back: its 64 columns; loaded two steps ahead).  What the parameter gradients
 // read (activations, dZ) goes to global memory on the side, and so does Z, which the
 // thread that wrote it reads again on the way back.
@@ -851,6 +853,7 @@ struct ChainLayer {
     float *Z, *dZf;       // row stride ldn
     bf16 *H, *dZb;        // the layer's activations and dZ, row stride ldn
     int N, ldn, ldk;
+    int bytes;            // of the rows' ldn columns and of the tokens of the CTAs that have none of them
 };
 
 struct ChainArgs {
@@ -891,6 +894,17 @@ __device__ __forceinline__ void chain_load(const ChainArgs &a, int c, int q, uin
     }
 }
 
+// 16 bytes to shared address dst of CTA `cta`, counted by its barrier at bar.
+constexpr int kChainToken = 16;
+__device__ __forceinline__ void chain_send(uint32_t dst, uint32_t bar, int cta, const uint32_t v[4])
+{
+    asm volatile("{\n\t.reg .b32 ra, rb;\n\tmapa.shared::cluster.u32 ra, %0, %2;\n\t"
+                 "mapa.shared::cluster.u32 rb, %1, %2;\n\t"
+                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [ra], {%3, %4, %5, %6}, [rb];\n\t}"
+                 ::"r"(dst), "r"(bar), "r"(cta), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+
 __global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThreads + kChainLoaders, 1)
     k_chain(const __grid_constant__ ChainArgs a)
 {
@@ -928,6 +942,12 @@ __global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThrea
             if (c + kChainStages - 1 < steps)
                 chain_load(a, c + kChainStages - 1, q, s_w + (c + kChainStages - 1) % kChainStages * kChainStage, t);
             asm volatile("cp.async.commit_group;" ::: "memory");   // (empty past the end, so the waits count alike)
+            // a CTA with no columns in this step's outputs says to each that it has come here
+            const int ldn = a.layer[c < a.L ? c : 2 * a.L - 2 - c].ldn;
+            if (q * kChainCols >= ldn && t < kChainCtas && c + 1 < steps) {
+                const uint32_t none[4] = {0u, 0u, 0u, 0u};
+                chain_send(s_act + ((c + 1) & 1) * kChainAct + q * kChainCols * 2, b_act + 8 * ((c + 1) & 1), t, none);
+            }
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
@@ -978,7 +998,7 @@ __global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThrea
         const bool active = j - 2 * (lane & 3) < o.ldn;   // (of the whole warp)
         const uint32_t sa = s_act + (c & 1) * kChainAct, sw = s_w + (c % kChainStages) * kChainStage;
         const uint32_t next_act = b_act + 8 * ((c + 1) & 1);
-        if (threadIdx.x == 0 && c + 1 < steps) mbar_expect_tx(next_act, kChainRows * o.ldn * 2);
+        if (threadIdx.x == 0 && c + 1 < steps) mbar_expect_tx(next_act, o.bytes);
         ok = c == 0 || mbar_wait(b_act + 8 * (c & 1), ((c - 1) >> 1) & 1, &s_fail);
         ok = __syncthreads_and(ok);   // (step c's weights have landed for every thread)
         if (!ok) break;
@@ -1036,13 +1056,8 @@ __global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThrea
                     uint32_t v[4];
 #pragma unroll
                     for (int r = 0; r < 4; r++) v[r] = __shfl_sync(0xffffffffu, word, (lane & ~3) + r);
-                    const uint32_t dst =
-                        s_act + ((c + 1) & 1) * kChainAct + (row + 8 * h) * kChainPitchK + (q * kChainCols + 8 * warp) * 2;
-                    asm volatile("{\n\t.reg .b32 ra, rb;\n\tmapa.shared::cluster.u32 ra, %0, %2;\n\t"
-                                 "mapa.shared::cluster.u32 rb, %1, %2;\n\t"
-                                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [ra], {%3, %4, %5, %6}, [rb];\n\t}"
-                                 ::"r"(dst), "r"(next_act), "r"(lane & 3), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
-                                 : "memory");
+                    chain_send(s_act + ((c + 1) & 1) * kChainAct + (row + 8 * h) * kChainPitchK +
+                                   (q * kChainCols + 8 * warp) * 2, next_act, lane & 3, v);
                 }
             }
         }
@@ -1844,6 +1859,7 @@ static cudaError_t chain(pt_mlp *m, int B, const bf16 *h0, const float *Y, const
         c.N = m->width[l + 1];
         c.ldn = m->ld[l + 1];
         c.ldk = m->ld[l];
+        c.bytes = kChainRows * c.ldn * 2 + kChainToken * (kChainCtas - (c.ldn + kChainCols - 1) / kChainCols);
     }
     k_chain<<<(B + kChainRows - 1) / kChainRows * kChainCtas, kChainThreads + kChainLoaders, kChainSmem, m->stream>>>(a);
     return cudaGetLastError();
