@@ -716,12 +716,18 @@ static pt_status fetch_rows(Engine *s, int lo, int hi)
     return PT_OK;
 }
 
-// A run or a step waits for its rows, so it cannot be part of a caller's capture.
+// A run or a step waits for its rows, so it cannot be part of a caller's capture, nor run
+// while a capture of another stream forbids this thread to wait (the query is forbidden
+// then too).  Asked before anything is queued: days whose rows cannot be fetched would
+// leave the device ahead of the host.
 static pt_status refuse_capture(Engine *s)
 {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s->stream, &capture), "stream");
     if (capture != cudaStreamCaptureStatusNone) CK(cudaErrorStreamCaptureUnsupported, "days in a capture");
+    const cudaError_t e = cudaStreamQuery(s->stream);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e != cudaErrorNotReady) CK(e, "days beside a capture");
     return PT_OK;
 }
 
@@ -776,6 +782,7 @@ static pt_status step_day(Engine *s, int day)
         if (st == PT_OK && !s->timing && !s->no_step_graph) st = capture_step(s, day);
     }
     if (st != PT_OK) return st;
+    s->next_day = day + 1;
     s->d2h_bytes += bytes;
     CK(cudaStreamSynchronize(s->stream), "sync");
     if (s->day_rows[0]) return fail(s, PT_ERR_TIMEOUT, "a device-side wait gave up (look-back ordering)");
@@ -812,9 +819,7 @@ static pt_status engine_step(Engine *s, int *running)
     if (instances_running(s) == 0) return all_zero_stopped(s) ? PT_DONE : PT_FINISHED;
     const pt_status captured = refuse_capture(s);
     if (captured != PT_OK) return captured;
-    const int day = s->next_day;
-    s->next_day = day + 1;
-    const pt_status st = step_day(s, day);
+    const pt_status st = step_day(s, s->next_day);
     if (st != PT_OK) return st;
     if (running) *running = instances_running(s);
     return all_zero_stopped(s) ? PT_DONE : PT_OK;
