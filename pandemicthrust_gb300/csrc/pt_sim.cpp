@@ -107,7 +107,7 @@ struct Engine {
     // the device.  (Ten launches take 35 us of a step's 90 on an Arm host, a replay 8.)
     cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
     uint64_t step_kernels[2] = {0, 0};
-    bool no_step_graph = false;           // the stream cannot be captured
+    bool no_graphs = false;               // a capture has failed: days are queued one by one
 
     int K() const { return (int)inst.size(); }
     void drop_graphs()   // what was captured depends on the settings
@@ -740,28 +740,30 @@ static pt_status queue_step(Engine *s, int day, int launch)
     return PT_OK;
 }
 
-// Captures a stepped day of the kind of `day` for later ones.  A stream that cannot be
-// captured goes on without.
-static pt_status capture_step(Engine *s, int day)
+// Captures what `queue` queues as a graph for later calls, which counts its kernels.  The
+// days themselves have been queued before, so a capture that fails (the legacy default
+// stream cannot be captured) costs no call: the engine goes on without graphs.
+template <class Queue>
+static void capture_days(Engine *s, cudaGraphExec_t *graph, uint64_t *kernels, Queue queue)
 {
-    const int kind = is_weekend(day) ? 1 : 0;
-    if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        cudaGetLastError();
-        s->no_step_graph = true;
-        return PT_OK;
-    }
+    if (s->no_graphs) return;
     const uint64_t before = ptk::launches();
-    const pt_status st = queue_step(s, day, -1);
+    const std::string err = s->err;
     cudaGraph_t g = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-    s->step_kernels[kind] = ptk::launches() - before;
-    ptk::add_launches(-(int64_t)s->step_kernels[kind]);  // counted when the graph runs
-    if (st == PT_OK && e == cudaSuccess) cudaGraphInstantiate(&s->step_graph[kind], g, 0);
+    bool ok = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    if (ok) {
+        ok = queue() == PT_OK;
+        ok = cudaStreamEndCapture(s->stream, &g) == cudaSuccess && ok;
+    }
+    *kernels = ptk::launches() - before;
+    ptk::add_launches(-(int64_t)*kernels);  // counted when the graph runs
+    if (!ok || cudaGraphInstantiate(graph, g, 0) != cudaSuccess) {
+        *graph = nullptr;
+        s->no_graphs = true;
+        s->err = err;
+        cudaGetLastError();
+    }
     if (g) cudaGraphDestroy(g);
-    if (st != PT_OK) return st;
-    CK(e, "end capture");
-    CK(cudaGetLastError(), "graph instantiate");
-    return PT_OK;
 }
 
 // One stepped day and its rows.  A caller that steps waits for them every day, so a
@@ -779,7 +781,8 @@ static pt_status step_day(Engine *s, int day)
         ptk::add_launches((int64_t)s->step_kernels[kind]);
     } else {
         st = queue_step(s, day, day);
-        if (st == PT_OK && !s->timing && !s->no_step_graph) st = capture_step(s, day);
+        if (st == PT_OK && !s->timing)   // for later days of its kind
+            capture_days(s, &s->step_graph[kind], &s->step_kernels[kind], [&] { return queue_step(s, day, -1); });
     }
     if (st != PT_OK) return st;
     s->next_day = day + 1;
@@ -825,28 +828,6 @@ static pt_status engine_step(Engine *s, int *running)
     return all_zero_stopped(s) ? PT_DONE : PT_OK;
 }
 
-// Captures the whole day loop for later runs.
-static pt_status capture_run(Engine *s)
-{
-    const uint64_t before = ptk::launches();
-    CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-    pt_status st = PT_OK;
-    for (int day = 0; day < s->max_days && st == PT_OK; day++) st = enqueue_day(s, day, day);
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-    s->graph_kernels = ptk::launches() - before;
-    ptk::add_launches(-(int64_t)s->graph_kernels);  // counted when the graph runs
-    if (st != PT_OK) {
-        if (g) cudaGraphDestroy(g);
-        return st;
-    }
-    CK(e, "end capture");
-    e = cudaGraphInstantiate(&s->run_graph, g, 0);
-    cudaGraphDestroy(g);
-    CK(e, "graph instantiate");
-    return PT_OK;
-}
-
 // The remaining days of every instance on the device, then one copy of the rows.
 static pt_status engine_run(Engine *s)
 {
@@ -865,11 +846,13 @@ static pt_status engine_run(Engine *s)
                 if (st != PT_OK) return st;
             }
         }
-        if (first == 0 && !s->timing && !s->run_graph) {
-            const pt_status st = capture_run(s);
-            if (st != PT_OK) return st;
-        }
         s->next_day = M;
+        if (first == 0 && !s->timing && !s->run_graph)   // for later runs
+            capture_days(s, &s->run_graph, &s->graph_kernels, [&] {
+                pt_status st = PT_OK;
+                for (int day = 0; day < M && st == PT_OK; day++) st = enqueue_day(s, day, day);
+                return st;
+            });
     }
     return fetch_rows(s, first, std::max(first, M));
 }
