@@ -82,7 +82,10 @@ struct Engine {
     int *d_hist = nullptr;            // K x 512
     int64_t persons = 0;              // real persons over all instances
     bool setup_done = false;
-    int next_day = 0;                 // next global day to run
+    int next_day = 0;                 // next global day to queue
+    int rows_day = 0;                 // first global day whose rows the host has not: next_day between calls, but
+                                      // for a stepped day whose call was not allowed to wait for it (beside
+                                      // another stream's capture); the next call fetches its rows
     int max_days = 0;                 // longest max_days of the instances
     std::string err;
     bool timing = false;
@@ -107,7 +110,7 @@ struct Engine {
     // the device.  (Ten launches take 35 us of a step's 90 on an Arm host, a replay 8.)
     cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
     uint64_t step_kernels[2] = {0, 0};
-    bool no_graphs = false;               // a capture has failed: days are queued one by one
+    bool no_graphs = false;               // the stream cannot be captured
 
     int K() const { return (int)inst.size(); }
     void drop_graphs()   // what was captured depends on the settings
@@ -577,7 +580,7 @@ static pt_status engine_reset(Engine *s)
     CK(cudaMemsetAsync(d.sc, 0, sizeof(ptk::Scalars), s->stream), "memset scalars");
     CK(ptk::launch_reset_instances(d, s->stream), "reset instances");
     CK(cudaStreamSynchronize(s->stream), "reset sync");
-    s->next_day = 0;
+    s->next_day = s->rows_day = 0;
     for (Instance &in : s->inst) {
         in.day = 0;
         in.stopped = false;
@@ -682,11 +685,33 @@ static void update_mirrors(Engine *s, int lo, int hi, Row row, Run run)
     }
 }
 
-// Copies every instance's rows of days [lo, hi) (strided copies out of the device
-// state records), checks the device error word and updates the host mirrors.
-static pt_status fetch_rows(Engine *s, int lo, int hi)
+// A run or a step waits for its rows, so it cannot be part of a caller's capture.
+static pt_status refuse_capture(Engine *s)
 {
-    const int K = s->K();
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s->stream, &capture), "stream");
+    if (capture != cudaStreamCaptureStatusNone) CK(cudaErrorStreamCaptureUnsupported, "days in a capture");
+    return PT_OK;
+}
+
+// Nor can a run's rows be fetched while a capture of another stream forbids this thread to
+// wait (the query is forbidden then too): asked before anything is queued.  (A stepped day
+// does not ask, the query's 1.5 us are 2% of a small one; see Engine::rows_day.)
+static pt_status refuse_beside_capture(Engine *s)
+{
+    const cudaError_t e = cudaStreamQuery(s->stream);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e != cudaErrorNotReady) CK(e, "days beside a capture");
+    return PT_OK;
+}
+
+// Copies every instance's rows of the days queued since the last fetch (strided copies out
+// of the device state records), checks the device error word and updates the host mirrors.
+static pt_status fetch_rows(Engine *s)
+{
+    const pt_status waits = refuse_beside_capture(s);
+    if (waits != PT_OK) return waits;
+    const int K = s->K(), lo = s->rows_day, hi = s->next_day;
     const size_t pitch = sizeof(ptk::InstState);
     const int days = std::max(0, hi - lo);
     std::vector<int> hc((size_t)K * 16 * std::max(days, 1)), hi_((size_t)K * std::max(days, 1)), rows(K);
@@ -713,21 +738,7 @@ static pt_status fetch_rows(Engine *s, int lo, int hi)
                        return std::make_pair((const int *)&hc[r * 16], hi_[r]);
                    },
                    [&](int k) { return rows[k]; });
-    return PT_OK;
-}
-
-// A run or a step waits for its rows, so it cannot be part of a caller's capture, nor run
-// while a capture of another stream forbids this thread to wait (the query is forbidden
-// then too).  Asked before anything is queued: days whose rows cannot be fetched would
-// leave the device ahead of the host.
-static pt_status refuse_capture(Engine *s)
-{
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(s->stream, &capture), "stream");
-    if (capture != cudaStreamCaptureStatusNone) CK(cudaErrorStreamCaptureUnsupported, "days in a capture");
-    const cudaError_t e = cudaStreamQuery(s->stream);
-    if (e != cudaSuccess) cudaGetLastError();
-    if (e != cudaErrorNotReady) CK(e, "days beside a capture");
+    s->rows_day = hi;
     return PT_OK;
 }
 
@@ -741,8 +752,9 @@ static pt_status queue_step(Engine *s, int day, int launch)
 }
 
 // Captures what `queue` queues as a graph for later calls, which counts its kernels.  The
-// days themselves have been queued before, so a capture that fails (the legacy default
-// stream cannot be captured) costs no call: the engine goes on without graphs.
+// days themselves have been queued before, so a capture that fails costs no call: the
+// engine goes on without the graph, on a stream that cannot be captured (the legacy default
+// one) without any.
 template <class Queue>
 static void capture_days(Engine *s, cudaGraphExec_t *graph, uint64_t *kernels, Queue queue)
 {
@@ -751,6 +763,7 @@ static void capture_days(Engine *s, cudaGraphExec_t *graph, uint64_t *kernels, Q
     const std::string err = s->err;
     cudaGraph_t g = nullptr;
     bool ok = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    s->no_graphs = !ok;
     if (ok) {
         ok = queue() == PT_OK;
         ok = cudaStreamEndCapture(s->stream, &g) == cudaSuccess && ok;
@@ -759,7 +772,6 @@ static void capture_days(Engine *s, cudaGraphExec_t *graph, uint64_t *kernels, Q
     ptk::add_launches(-(int64_t)*kernels);  // counted when the graph runs
     if (!ok || cudaGraphInstantiate(graph, g, 0) != cudaSuccess) {
         *graph = nullptr;
-        s->no_graphs = true;
         s->err = err;
         cudaGetLastError();
     }
@@ -797,6 +809,7 @@ static pt_status step_day(Engine *s, int day)
                        return std::make_pair(r, r[16]);
                    },
                    [&](int k) { return rows[(size_t)k * ptk::kDayRow + 17]; });
+    s->rows_day = day + 1;
     return PT_OK;
 }
 
@@ -822,7 +835,7 @@ static pt_status engine_step(Engine *s, int *running)
     if (instances_running(s) == 0) return all_zero_stopped(s) ? PT_DONE : PT_FINISHED;
     const pt_status captured = refuse_capture(s);
     if (captured != PT_OK) return captured;
-    const pt_status st = step_day(s, s->next_day);
+    const pt_status st = s->rows_day < s->next_day ? fetch_rows(s) : step_day(s, s->next_day);
     if (st != PT_OK) return st;
     if (running) *running = instances_running(s);
     return all_zero_stopped(s) ? PT_DONE : PT_OK;
@@ -834,15 +847,16 @@ static pt_status engine_run(Engine *s)
     if (!s->setup_done) return fail(s, PT_ERR_STATE, "run before setup");
     const int first = s->next_day, M = s->max_days;
     if (instances_running(s) > 0 && first < M) {
-        const pt_status captured = refuse_capture(s);
-        if (captured != PT_OK) return captured;
+        pt_status st = refuse_capture(s);
+        if (st == PT_OK) st = refuse_beside_capture(s);
+        if (st != PT_OK) return st;
         const bool replay = first == 0 && !s->timing && s->run_graph;
         if (replay) {
             CK(cudaGraphLaunch(s->run_graph, s->stream), "graph launch");
             ptk::add_launches((int64_t)s->graph_kernels);
         } else {
             for (int day = first; day < M; day++) {
-                pt_status st = enqueue_day(s, day, day);
+                st = enqueue_day(s, day, day);
                 if (st != PT_OK) return st;
             }
         }
@@ -854,7 +868,7 @@ static pt_status engine_run(Engine *s)
                 return st;
             });
     }
-    return fetch_rows(s, first, std::max(first, M));
+    return fetch_rows(s);
 }
 
 static pt_status engine_gen_counts(Engine *s, int *gen_p, int *gen_s)
