@@ -690,7 +690,7 @@ static pt_status refuse_capture(Engine *s)
 {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s->stream, &capture), "stream");
-    if (capture != cudaStreamCaptureStatusNone) CK(cudaErrorStreamCaptureUnsupported, "days in a capture");
+    if (capture != cudaStreamCaptureStatusNone) CK(cudaErrorStreamCaptureUnsupported, "a call that waits in a capture");
     return PT_OK;
 }
 
@@ -701,7 +701,7 @@ static pt_status refuse_beside_capture(Engine *s)
 {
     const cudaError_t e = cudaStreamQuery(s->stream);
     if (e != cudaSuccess) cudaGetLastError();
-    if (e != cudaErrorNotReady) CK(e, "days beside a capture");
+    if (e != cudaErrorNotReady) CK(e, "a call that waits beside a capture");
     return PT_OK;
 }
 
@@ -927,6 +927,10 @@ static pt_status engine_person_state(Engine *s, int k, uint8_t *status_p, uint8_
                                      uint8_t *day_s, uint8_t *gen_p, uint8_t *gen_s, uint8_t *age)
 {
     if (!s->setup_done) return fail(s, PT_ERR_STATE, "state before setup");
+    // (before the caller's arrays are touched)
+    pt_status st = refuse_capture(s);
+    if (st == PT_OK) st = refuse_beside_capture(s);
+    if (st != PT_OK) return st;
     const size_t N = (size_t)s->inst[k].c.N, pb = (size_t)s->ic[k].pbase;
     uint8_t *const planes[4] = {status_p, status_s, day_p, day_s};
     // A copy to pages that nobody has touched yet runs at 1.4 GB/s (a fresh array of a
