@@ -1315,9 +1315,12 @@ constexpr int kMarkThreads = 256, kMarkBlocksPerSm = 4;
 __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *ic, const InstState *is,
                                                                const uint8_t *age, const int32_t *infected,
                                                                const int32_t *infected_inst, int weekend,
-                                                               int2 *read, uint32_t *mark, int words, const Scalars *sc)
+                                                               int2 *read, uint32_t *mark, int words, uint2 *slot,
+                                                               int slots, const Scalars *sc)
 {
-    if (sc->done) return;
+    if (sc->done) return;   // (the tables of the last day with infected stay)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x)
+        slot[i] = make_uint2(0u, 0u);
     const int I = sc->infected;
     __shared__ uint32_t s_mark[kMarkSharedWords];
     const bool shared = words <= kMarkSharedWords && I >= kMarkSharedPerWord * words;
@@ -1351,10 +1354,11 @@ __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *
 }
 
 // A small run's list and marks in one launch instead of three (scan, emit, mark): a block
-// per person tile sums the counts of the tiles itself, emits its part of the list and
-// marks its persons' buckets.  The block of an instance's first tile begins the
-// instance's day, the last tile's block the batch's; no block waits for another.  Small
-// runs are bound by their launches: a day of 100,000 persons has seven of 3 to 10 us.
+// per person tile sums the counts of the tiles itself, clears its part of the day's bucket
+// slots, emits its part of the list and marks its persons' buckets.  The block of an
+// instance's first tile begins the instance's day, the last tile's block the batch's; no
+// block waits for another.  Small runs are bound by their launches: a day of 100,000
+// persons has seven of 3 to 10 us.
 // Up to kListTiles tiles (4M persons) the sums are four loads a thread.
 constexpr int kListTiles = 4 * kSweepThreads;
 constexpr int kListMarkWords = 2048;   // a bitmap this small is marked in shared memory and merged once a block
@@ -1364,8 +1368,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
                                                               const int32_t *tile_count, int32_t *infected,
                                                               int32_t *infected_inst, int2 *read, const uint8_t *age,
                                                               uint32_t *mark,
-                                                              int words, int mark_all, Scalars *sc, int day,
-                                                              int dense_level)
+                                                              int words, int mark_all, uint2 *slot, int slots,
+                                                              Scalars *sc, int day, int dense_level)
 {
     day = launch_day(day, sc);
     const int ended = *(volatile const int *)&sc->done;
@@ -1413,6 +1417,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
     total += list_end;
     if (t == 0 && tile == first) begin_instance_day(ik, is[k], start, list_end, day, dense_level);
     if (t == 0 && tile == tiles - 1) begin_day(sc, total, day);
+    if (total > 0)   // (the tables of the last day with infected stay)
+        for (int i = tile * kSweepThreads + t; i < slots; i += tiles * kSweepThreads) slot[i] = make_uint2(0u, 0u);
     if (n == 0) return;
     unsigned long long packed = 0;
 #pragma unroll
@@ -1452,11 +1458,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
         if (s_mark[i]) red_or(&mark[i], s_mark[i]);
 }
 
-// Bytes from the marks over the day's bucket slots, which lie behind them.
-static size_t day_clear_bytes(const DevArrays &d, bool weekend)
-{
-    return (size_t)(reinterpret_cast<char *>(d.bkt + d.buckets[weekend ? 1 : 0]) - reinterpret_cast<char *>(d.mark));
-}
+// Words of the day's mark bitmap.
+static int mark_words(const DevArrays &d, bool weekend) { return d.buckets[weekend ? 1 : 0] / 32 + 1; }
 
 cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t s)
 {
@@ -1465,7 +1468,7 @@ cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t
     const bool small = tiles <= kListTiles;
     k_sweep_count<<<div_up(tiles, per_block), kSweepThreads, 0, s>>>(
         d.ic, d.is, d.tile_inst, tiles, per_block, d.state, d.sweep_flags, d.sweep_tiles,
-        reinterpret_cast<uint2 *>(d.mark), small ? (int)(day_clear_bytes(d, weekend) / sizeof(uint2)) : 0, d.sc, day);
+        reinterpret_cast<uint2 *>(d.mark), small ? (mark_words(d, weekend) + 1) / 2 : 0, d.sc, day);
     count_launch();
     if (!small) {
         k_sweep_scan<<<1, kSweepScanThreads, 0, s>>>(d.ic, d.is, d.K, d.sweep_tiles, tiles, d.sc, day, d.tune.dense_level);
@@ -1478,14 +1481,14 @@ cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t
 // for complete tables).
 cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables, cudaStream_t s)
 {
-    const int tiles = d.P / kSweepTile, B = d.buckets[weekend ? 1 : 0], words = B / 32 + 1;
+    const int tiles = d.P / kSweepTile, B = d.buckets[weekend ? 1 : 0], words = mark_words(d, weekend);
     cudaError_t e = cudaSuccess;
     if (tiles <= kListTiles) {
         if (full_tables) e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
         if (e != cudaSuccess) return e;
         k_sweep_list<<<tiles, kSweepThreads, 0, s>>>(d.ic, d.is, d.tile_inst, tiles, d.sweep_flags, d.sweep_tiles,
                                                      d.infected, d.infected_inst, d.read, d.age, d.mark, words,
-                                                     full_tables ? 1 : 0, d.sc, day, d.tune.dense_level);
+                                                     full_tables ? 1 : 0, d.bkt, B, d.sc, day, d.tune.dense_level);
         count_launch();
         return cudaGetLastError();
     }
@@ -1497,11 +1500,10 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
         k_sweep_emit_block<<<tiles, kSweepThreads, 0, s>>>(d.tile_inst, d.sweep_flags, d.sweep_tiles, d.infected,
                                                            d.infected_inst, d.sc);
     count_launch();
-    e = cudaMemsetAsync(d.mark, 0, day_clear_bytes(d, weekend), s);
-    if (e == cudaSuccess && full_tables) e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
+    e = cudaMemsetAsync(d.mark, full_tables ? 0xFF : 0, (size_t)words * 4, s);
     if (e != cudaSuccess) return e;
     k_mark_buckets<<<sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, s>>>(
-        d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.read, d.mark, words, d.sc);
+        d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.read, d.mark, words, d.bkt, B, d.sc);
     count_launch();
     return cudaGetLastError();
 }

@@ -153,7 +153,7 @@ struct DevArrays {
 
 // BucketSlot: a bucket of the day's errand table, one 8-byte load.  x: kMaxStart less the
 // place of its first person in bkt_people (0: no entries); y: its persons.  Cleared to
-// zero each day; the sort's last pass raises x to the largest offer (the smallest
+// zero each day that finds infected; the sort's last pass raises x to the largest offer (the smallest
 // place) and adds up y.
 constexpr uint32_t kMaxStart = 0x7FFFFFFFu;   // above every place, so a bucket with entries has x > 0
 __host__ __device__ inline int bucket_start(uint2 slot) { return (int)(kMaxStart - slot.x); }

@@ -453,7 +453,7 @@ static pt_status engine_setup(Engine *s)
     bytes += round256((size_t)K * 4 * 256 * 4) + 2 * round256(((size_t)K + 1) * 4);  // digit bases, tile prefixes
     const size_t nregions = n / ptk::kSchedMinRegion, nchunks = 3 * n / ptk::kRegionChunk + 1;
     bytes += 2 * round256(nregions * 4) + round256(nchunks * sizeof(int4));   // schedule regions
-    // the mark bitmap and, right behind it, the bucket slots of a day (cleared together)
+    // the mark bitmap and the bucket slots of a day
     bytes += round256(((size_t)Bday + 1) * sizeof(uint2)) + round256(((size_t)Bday / 32 + 1) * 4);
     bytes += round256(n * 4) * 2 + round256(n * 8);   // infected, infected_inst, read
     bytes += round256(n / 16 * 2) + round256((ntiles + 1) * 4);  // sweep masks, sweep tile counts
@@ -1285,10 +1285,10 @@ pt_status pt_get_day_tables(pt_sim *s, int32_t *infected, int32_t *keys, int32_t
         // starts of the buckets with entries; an empty one starts where the next one does
         std::vector<uint2> slots((size_t)Bc);
         CK(pt_memcpy_sync(s, slots.data(), s->d.bkt, (size_t)Bc * sizeof(uint2), cudaMemcpyDeviceToHost), "copy");
-        int marked = 0;
-        CK(pt_memcpy_sync(s, &marked, &s->d.is[0].marked, sizeof(int), cudaMemcpyDeviceToHost), "marked");
         std::vector<int32_t> co((size_t)Bc + 1);
-        co[Bc] = marked;
+        co[Bc] = 0;
+        for (const uint2 &b : slots)
+            if (ptk::bucket_count(b) > 0) co[Bc] = std::max(co[Bc], ptk::bucket_start(b) + ptk::bucket_count(b));
         for (int b = Bc - 1; b >= 0; b--) co[b] = ptk::bucket_count(slots[b]) > 0 ? ptk::bucket_start(slots[b]) : co[b + 1];
         for (int h = 0; h < hours; h++)
             for (int loc = 0; loc < L; loc++)
