@@ -28,7 +28,13 @@ namespace ptk {
 static std::atomic<uint64_t> g_launches{0};
 uint64_t launches() { return g_launches.load(); }
 void add_launches(int64_t n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
-static inline void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+static thread_local uint64_t t_launches = 0;
+uint64_t thread_launches() { return t_launches; }
+static inline void count_launch()
+{
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    t_launches++;
+}
 
 int sm_count()
 {

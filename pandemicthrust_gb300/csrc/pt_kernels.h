@@ -289,6 +289,7 @@ cudaError_t launch_errand_selftest(unsigned long long *counts, cudaStream_t s);
 long long max_spin_limit();   // the polls every wait of the simulation allows
 
 uint64_t launches();
+uint64_t thread_launches();    // the calling thread's own (what a capture records)
 void add_launches(int64_t n);  // kernels run by a replayed graph
 
 }  // namespace ptk

@@ -759,7 +759,7 @@ template <class Queue>
 static void capture_days(Engine *s, cudaGraphExec_t *graph, uint64_t *kernels, Queue queue)
 {
     if (s->no_graphs) return;
-    const uint64_t before = ptk::launches();
+    const uint64_t before = ptk::thread_launches();
     const std::string err = s->err;
     cudaGraph_t g = nullptr;
     bool ok = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
@@ -768,7 +768,7 @@ static void capture_days(Engine *s, cudaGraphExec_t *graph, uint64_t *kernels, Q
         ok = queue() == PT_OK;
         ok = cudaStreamEndCapture(s->stream, &g) == cudaSuccess && ok;
     }
-    *kernels = ptk::launches() - before;
+    *kernels = ptk::thread_launches() - before;
     ptk::add_launches(-(int64_t)*kernels);  // counted when the graph runs
     if (!ok || cudaGraphInstantiate(graph, g, 0) != cudaSuccess) {
         *graph = nullptr;
