@@ -915,6 +915,7 @@ __device__ __forceinline__ uint32_t recover_word(uint32_t st, int d2r, bool &cha
 //          [start, list_end) of the infected list and its day bookkeeping.
 //   emit   one person tile per warp (per block for small runs): the infected ids,
 //          in ascending order, at their list positions.
+// The count kernel also clears the day's marks and the emit kernel its bucket slots.
 // Each launch depends only on the one before, so no block waits for another.
 // Person tiles a count block sweeps one after another: as many as make the grid one wave
 // of the blocks that fit (kSweepBlocksPerSm), at most what 8-bit status counts hold.
@@ -1137,13 +1138,23 @@ __global__ void __launch_bounds__(kSweepScanThreads) k_sweep_scan(const InstCons
     if (threadIdx.x == 0) begin_day(sc, total, day);
 }
 
+// The grid's threads clear the day's bucket slots.  Only on a day that goes on: the tables
+// of the last day with infected stay.
+__device__ __forceinline__ void clear_slots(uint2 *slot, int slots)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x)
+        slot[i] = make_uint2(0u, 0u);
+}
+
 // Emit for small runs: a block per person tile, a block scan of the threads' packed
 // per-round counts (a warp per tile would leave most SMs idle).
 __global__ void __launch_bounds__(kSweepThreads) k_sweep_emit_block(const int32_t *tile_inst, const uint16_t *flags_in,
                                                                     const int32_t *tile_prefix, int32_t *infected,
-                                                                    int32_t *infected_inst, const Scalars *sc)
+                                                                    int32_t *infected_inst, uint2 *slot, int slots,
+                                                                    const Scalars *sc)
 {
     if (*(volatile const int *)&sc->done) return;
+    clear_slots(slot, slots);
     const int tile = blockIdx.x;
     const int prefix = tile_prefix[tile];
     if (tile_prefix[tile + 1] == prefix) return;  // no infected in this tile
@@ -1181,9 +1192,11 @@ constexpr int kEmitWarps = 8;   // person tiles per emit block, one warp each
 __global__ void __launch_bounds__(kEmitWarps * 32) k_sweep_emit(const int32_t *tile_inst, int tiles,
                                                                 const uint16_t *flags_in,
                                                                 const int32_t *tile_prefix, int32_t *infected,
-                                                                int32_t *infected_inst, const Scalars *sc)
+                                                                int32_t *infected_inst, uint2 *slot, int slots,
+                                                                const Scalars *sc)
 {
     if (*(volatile const int *)&sc->done) return;
+    clear_slots(slot, slots);
     const int lane = threadIdx.x & 31;
     const int tile = blockIdx.x * kEmitWarps + (threadIdx.x >> 5);
     if (tile >= tiles) return;
@@ -1321,12 +1334,9 @@ constexpr int kMarkThreads = 256, kMarkBlocksPerSm = 4;
 __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *ic, const InstState *is,
                                                                const uint8_t *age, const int32_t *infected,
                                                                const int32_t *infected_inst, int weekend,
-                                                               int2 *read, uint32_t *mark, int words, uint2 *slot,
-                                                               int slots, const Scalars *sc)
+                                                               int2 *read, uint32_t *mark, int words, const Scalars *sc)
 {
-    if (sc->done) return;   // (the tables of the last day with infected stay)
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x)
-        slot[i] = make_uint2(0u, 0u);
+    if (sc->done) return;
     const int I = sc->infected;
     __shared__ uint32_t s_mark[kMarkSharedWords];
     const bool shared = words <= kMarkSharedWords && I >= kMarkSharedPerWord * words;
@@ -1423,8 +1433,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
     total += list_end;
     if (t == 0 && tile == first) begin_instance_day(ik, is[k], start, list_end, day, dense_level);
     if (t == 0 && tile == tiles - 1) begin_day(sc, total, day);
-    if (total > 0)   // (the tables of the last day with infected stay)
-        for (int i = tile * kSweepThreads + t; i < slots; i += tiles * kSweepThreads) slot[i] = make_uint2(0u, 0u);
+    if (total > 0) clear_slots(slot, slots);
     if (n == 0) return;
     unsigned long long packed = 0;
 #pragma unroll
@@ -1471,12 +1480,11 @@ cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t
 {
     const int tiles = d.P / kSweepTile;
     const int per_block = std::min(div_up(tiles, kSweepBlocksPerSm * sm_count()), kSweepTilesPerBlock);
-    const bool small = tiles <= kListTiles;
     k_sweep_count<<<div_up(tiles, per_block), kSweepThreads, 0, s>>>(
         d.ic, d.is, d.tile_inst, tiles, per_block, d.state, d.sweep_flags, d.sweep_tiles,
-        reinterpret_cast<uint2 *>(d.mark), small ? (mark_words(d, weekend) + 1) / 2 : 0, d.sc, day);
+        reinterpret_cast<uint2 *>(d.mark), (mark_words(d, weekend) + 1) / 2, d.sc, day);
     count_launch();
-    if (!small) {
+    if (tiles > kListTiles) {
         k_sweep_scan<<<1, kSweepScanThreads, 0, s>>>(d.ic, d.is, d.K, d.sweep_tiles, tiles, d.sc, day, d.tune.dense_level);
         count_launch();
     }
@@ -1488,10 +1496,11 @@ cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t
 cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables, cudaStream_t s)
 {
     const int tiles = d.P / kSweepTile, B = d.buckets[weekend ? 1 : 0], words = mark_words(d, weekend);
-    cudaError_t e = cudaSuccess;
-    if (tiles <= kListTiles) {
-        if (full_tables) e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
+    if (full_tables) {
+        const cudaError_t e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
         if (e != cudaSuccess) return e;
+    }
+    if (tiles <= kListTiles) {
         k_sweep_list<<<tiles, kSweepThreads, 0, s>>>(d.ic, d.is, d.tile_inst, tiles, d.sweep_flags, d.sweep_tiles,
                                                      d.infected, d.infected_inst, d.read, d.age, d.mark, words,
                                                      full_tables ? 1 : 0, d.bkt, B, d.sc, day, d.tune.dense_level);
@@ -1501,15 +1510,13 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
     if (tiles >= kSweepEmitTilesPerSm * sm_count())
         k_sweep_emit<<<div_up(tiles, kEmitWarps), kEmitWarps * 32, 0, s>>>(d.tile_inst, tiles, d.sweep_flags,
                                                                            d.sweep_tiles, d.infected, d.infected_inst,
-                                                                           d.sc);
+                                                                           d.bkt, B, d.sc);
     else
         k_sweep_emit_block<<<tiles, kSweepThreads, 0, s>>>(d.tile_inst, d.sweep_flags, d.sweep_tiles, d.infected,
-                                                           d.infected_inst, d.sc);
+                                                           d.infected_inst, d.bkt, B, d.sc);
     count_launch();
-    e = cudaMemsetAsync(d.mark, full_tables ? 0xFF : 0, (size_t)words * 4, s);
-    if (e != cudaSuccess) return e;
     k_mark_buckets<<<sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, s>>>(
-        d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.read, d.mark, words, d.bkt, B, d.sc);
+        d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.read, d.mark, words, d.sc);
     count_launch();
     return cudaGetLastError();
 }
