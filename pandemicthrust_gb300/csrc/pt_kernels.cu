@@ -2546,25 +2546,27 @@ cudaError_t launch_unpack_state(const DevArrays &d, int first, int n, cudaStream
     return cudaGetLastError();
 }
 
-// (one block: it also moves the next stepped day on)
-__global__ void __launch_bounds__(1024) k_day_rows(const InstState *is, int K, int day, Scalars *sc, int *out)
+// Also moves the next stepped day on, which nothing here reads: the day is the one that the
+// list has begun.  As many blocks as there are rows for: with one block a step of 4,096
+// instances took 1,272 us, now 1,203.
+__global__ void __launch_bounds__(256) k_day_rows(const InstState *is, int K, Scalars *sc, int *out)
 {
-    day = launch_day(day, sc);
-    for (int i = threadIdx.x; i < K * kDayRow; i += blockDim.x) {
+    const int day = sc->day, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < K * kDayRow) {
         const InstState &s = is[i / kDayRow];
         const int f = i % kDayRow;
         out[1 + i] = f < 16 ? s.counts[day][f] : (f == 16 ? s.infected_per_day[day] : s.days_run);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    if (i == 0) {
         out[0] = sc->error;
         sc->step_day = day + 1;
     }
 }
 
-cudaError_t launch_day_rows(const DevArrays &d, int day, int *out, cudaStream_t s)
+cudaError_t launch_day_rows(const DevArrays &d, int *out, cudaStream_t s)
 {
-    k_day_rows<<<1, std::min(1024, div_up(d.K * kDayRow, 32) * 32), 0, s>>>(d.is, d.K, day, d.sc, out);
+    const int n = d.K * kDayRow, threads = std::min(256, div_up(n, 32) * 32);
+    k_day_rows<<<div_up(n, threads), threads, 0, s>>>(d.is, d.K, d.sc, out);
     count_launch();
     return cudaGetLastError();
 }

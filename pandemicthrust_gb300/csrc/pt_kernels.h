@@ -274,7 +274,7 @@ constexpr int kDayRow = 18;
 inline size_t state_plane(size_t n) { return (n + 15) / 16 * 16; }
 uint8_t *state_planes(const DevArrays &d);
 cudaError_t launch_unpack_state(const DevArrays &d, int first, int n, cudaStream_t s);
-cudaError_t launch_day_rows(const DevArrays &d, int day, int *out, cudaStream_t s);
+cudaError_t launch_day_rows(const DevArrays &d, int *out, cudaStream_t s);
 // weekday / weekend buckets of one instance (compact keys hour * R + dest - lo)
 int day_buckets(const SimConst &c, bool weekend);
 

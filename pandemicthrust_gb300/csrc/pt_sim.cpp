@@ -747,7 +747,7 @@ static pt_status queue_step(Engine *s, int day, int launch)
 {
     const pt_status st = enqueue_day(s, day, launch);
     if (st != PT_OK) return st;
-    CK(ptk::launch_day_rows(s->d, launch, s->day_rows, s->stream), "day rows");
+    CK(ptk::launch_day_rows(s->d, s->day_rows, s->stream), "day rows");
     return PT_OK;
 }
 
