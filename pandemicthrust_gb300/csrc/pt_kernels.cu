@@ -19,6 +19,7 @@
 #include <cstdio>
 #include <climits>
 #include <atomic>
+#include <tuple>
 #include "pt_kernels.h"
 #include "pt_device.cuh"
 #include "pt_lookback.cuh"
@@ -27,13 +28,58 @@ namespace ptk {
 
 static std::atomic<uint64_t> g_launches{0};
 uint64_t launches() { return g_launches.load(); }
-void add_launches(int64_t n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
-static thread_local uint64_t t_launches = 0;
-uint64_t thread_launches() { return t_launches; }
-static inline void count_launch()
+void add_launches(uint64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+static inline void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+
+// The next node of a graph's chain.
+template <class Add>
+static cudaError_t chain_node(DayQueue &q, Add add)
 {
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    t_launches++;
+    cudaGraphNode_t node = nullptr;
+    const cudaError_t e = add(&node, q.last ? &q.last : nullptr, q.last ? 1 : 0);
+    if (e == cudaSuccess) q.last = node;
+    return e;
+}
+
+// A kernel launch to the queue's stream, or its node.
+template <class... P, class... A>
+static cudaError_t queue_kernel(DayQueue &q, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, const A &...args)
+{
+    std::tuple<P...> values(args...);   // in the kernel's own types
+    return std::apply(
+        [&](P &...v) {
+            void *params[] = {(void *)&v...};
+            if (!q.graph) {
+                count_launch();
+                return cudaLaunchKernel((const void *)kernel, grid, block, params, smem, q.stream);
+            }
+            cudaKernelNodeParams n = {};
+            n.func = (void *)kernel;
+            n.gridDim = grid;
+            n.blockDim = block;
+            n.sharedMemBytes = (unsigned)smem;
+            n.kernelParams = params;
+            q.kernels++;
+            return chain_node(q, [&](cudaGraphNode_t *node, const cudaGraphNode_t *after, size_t count) {
+                return cudaGraphAddKernelNode(node, q.graph, after, count, &n);
+            });
+        },
+        values);
+}
+
+// `words` words of `value` at p.
+static cudaError_t queue_fill(DayQueue &q, uint32_t *p, uint32_t value, size_t words)
+{
+    if (!q.graph) return cudaMemsetAsync(p, (int)(value & 0xFFu), words * 4, q.stream);   // (its bytes are alike)
+    cudaMemsetParams m = {};
+    m.dst = p;
+    m.value = value;
+    m.elementSize = 4;
+    m.width = words;
+    m.height = 1;
+    return chain_node(q, [&](cudaGraphNode_t *node, const cudaGraphNode_t *after, size_t count) {
+        return cudaGraphAddMemsetNode(node, q.graph, after, count, &m);
+    });
 }
 
 int sm_count()
@@ -677,15 +723,13 @@ int radix_digit_bits(int buckets)
 constexpr int kRadixSmem = kRadixTile * 8 + kRadixWarps * 256 * (4 + 2);
 
 template <int IN, int OUT>
-static cudaError_t radix_launch(const RadixPass &a, int grid, cudaStream_t s)
+static cudaError_t radix_launch(const RadixPass &a, int grid, DayQueue &q)
 {
     static_assert(kRadixSmem <= 46 * 1024, "with the static part, no more than a launch may ask for without opt-in");
-    k_radix_pass<IN, OUT><<<grid, kRadixThreads, kRadixSmem, s>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    return queue_kernel(q, k_radix_pass<IN, OUT>, grid, kRadixThreads, kRadixSmem, a);
 }
 
-cudaError_t launch_radix_sort(const RadixArgs &r, cudaStream_t s)
+cudaError_t launch_radix_sort(const RadixArgs &r, DayQueue &q)
 {
     const int P = radix_passes(r.buckets);
     const int tiles = std::max(1, div_up(r.E, kRadixTile));
@@ -710,10 +754,10 @@ cudaError_t launch_radix_sort(const RadixArgs &r, cudaStream_t s)
         a.pass = p;
         a.out_pairs = (p & 1) ? r.p1 : r.p0;
         cudaError_t e;
-        if (first && day) e = last ? radix_launch<kInDay, kOutTable>(a, grid, s) : radix_launch<kInDay, kOutPairs>(a, grid, s);
-        else if (first) e = last ? radix_launch<kInKeys, kOutValues>(a, grid, s) : radix_launch<kInKeys, kOutPairs>(a, grid, s);
-        else if (!last) e = radix_launch<kInPairs, kOutPairs>(a, grid, s);
-        else e = day ? radix_launch<kInPairs, kOutTable>(a, grid, s) : radix_launch<kInPairs, kOutValues>(a, grid, s);
+        if (first && day) e = last ? radix_launch<kInDay, kOutTable>(a, grid, q) : radix_launch<kInDay, kOutPairs>(a, grid, q);
+        else if (first) e = last ? radix_launch<kInKeys, kOutValues>(a, grid, q) : radix_launch<kInKeys, kOutPairs>(a, grid, q);
+        else if (!last) e = radix_launch<kInPairs, kOutPairs>(a, grid, q);
+        else e = day ? radix_launch<kInPairs, kOutTable>(a, grid, q) : radix_launch<kInPairs, kOutValues>(a, grid, q);
         if (e != cudaSuccess) return e;
         a.in = a.out_pairs;
     }
@@ -737,7 +781,8 @@ cudaError_t launch_bucket_table(const RadixArgs &r, int32_t *counts, bool count_
     count_launch();
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return launch_radix_sort(r, s);
+    DayQueue q{s};
+    return launch_radix_sort(r, q);
 }
 
 // setup_initializeStatusArrays (PandemicSim.cu:3654-3664): S/S, day 255/255, gen 255.
@@ -1476,49 +1521,40 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
 // Words of the day's mark bitmap.
 static int mark_words(const DevArrays &d, bool weekend) { return d.buckets[weekend ? 1 : 0] / 32 + 1; }
 
-cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t s)
+cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, DayQueue &q)
 {
     const int tiles = d.P / kSweepTile;
     const int per_block = std::min(div_up(tiles, kSweepBlocksPerSm * sm_count()), kSweepTilesPerBlock);
-    k_sweep_count<<<div_up(tiles, per_block), kSweepThreads, 0, s>>>(
-        d.ic, d.is, d.tile_inst, tiles, per_block, d.state, d.sweep_flags, d.sweep_tiles,
-        reinterpret_cast<uint2 *>(d.mark), (mark_words(d, weekend) + 1) / 2, d.sc, day);
-    count_launch();
-    if (tiles > kListTiles) {
-        k_sweep_scan<<<1, kSweepScanThreads, 0, s>>>(d.ic, d.is, d.K, d.sweep_tiles, tiles, d.sc, day, d.tune.dense_level);
-        count_launch();
-    }
-    return cudaGetLastError();
+    const cudaError_t e = queue_kernel(q, k_sweep_count, div_up(tiles, per_block), kSweepThreads, 0, d.ic, d.is, d.tile_inst,
+                                       tiles, per_block, d.state, d.sweep_flags, d.sweep_tiles,
+                                       reinterpret_cast<uint2 *>(d.mark), (mark_words(d, weekend) + 1) / 2, d.sc, day);
+    if (e != cudaSuccess || tiles <= kListTiles) return e;
+    return queue_kernel(q, k_sweep_scan, 1, kSweepScanThreads, 0, d.ic, d.is, d.K, d.sweep_tiles, tiles, d.sc, day,
+                        d.tune.dense_level);
 }
 
 // The infected list and the marks of the buckets that its persons read (every bucket's
 // for complete tables).
-cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables, cudaStream_t s)
+cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables, DayQueue &q)
 {
     const int tiles = d.P / kSweepTile, B = d.buckets[weekend ? 1 : 0], words = mark_words(d, weekend);
     if (full_tables) {
-        const cudaError_t e = cudaMemsetAsync(d.mark, 0xFF, (size_t)words * 4, s);
+        const cudaError_t e = queue_fill(q, d.mark, 0xFFFFFFFFu, (size_t)words);
         if (e != cudaSuccess) return e;
     }
-    if (tiles <= kListTiles) {
-        k_sweep_list<<<tiles, kSweepThreads, 0, s>>>(d.ic, d.is, d.tile_inst, tiles, d.sweep_flags, d.sweep_tiles,
-                                                     d.infected, d.infected_inst, d.read, d.age, d.mark, words,
-                                                     full_tables ? 1 : 0, d.bkt, B, d.sc, day, d.tune.dense_level);
-        count_launch();
-        return cudaGetLastError();
-    }
-    if (tiles >= kSweepEmitTilesPerSm * sm_count())
-        k_sweep_emit<<<div_up(tiles, kEmitWarps), kEmitWarps * 32, 0, s>>>(d.tile_inst, tiles, d.sweep_flags,
-                                                                           d.sweep_tiles, d.infected, d.infected_inst,
-                                                                           d.bkt, B, d.sc);
-    else
-        k_sweep_emit_block<<<tiles, kSweepThreads, 0, s>>>(d.tile_inst, d.sweep_flags, d.sweep_tiles, d.infected,
-                                                           d.infected_inst, d.bkt, B, d.sc);
-    count_launch();
-    k_mark_buckets<<<sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, s>>>(
-        d.ic, d.is, d.age, d.infected, d.infected_inst, weekend ? 1 : 0, d.read, d.mark, words, d.sc);
-    count_launch();
-    return cudaGetLastError();
+    if (tiles <= kListTiles)
+        return queue_kernel(q, k_sweep_list, tiles, kSweepThreads, 0, d.ic, d.is, d.tile_inst, tiles, d.sweep_flags,
+                            d.sweep_tiles, d.infected, d.infected_inst, d.read, d.age, d.mark, words,
+                            full_tables ? 1 : 0, d.bkt, B, d.sc, day, d.tune.dense_level);
+    const cudaError_t e =
+        tiles >= kSweepEmitTilesPerSm * sm_count()
+            ? queue_kernel(q, k_sweep_emit, div_up(tiles, kEmitWarps), kEmitWarps * 32, 0, d.tile_inst, tiles,
+                           d.sweep_flags, d.sweep_tiles, d.infected, d.infected_inst, d.bkt, B, d.sc)
+            : queue_kernel(q, k_sweep_emit_block, tiles, kSweepThreads, 0, d.tile_inst, d.sweep_flags, d.sweep_tiles,
+                           d.infected, d.infected_inst, d.bkt, B, d.sc);
+    if (e != cudaSuccess) return e;
+    return queue_kernel(q, k_mark_buckets, sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, d.ic, d.is, d.age, d.infected,
+                        d.infected_inst, weekend ? 1 : 0, d.read, d.mark, words, d.sc);
 }
 
 // Schedule kernel.  The persons are cut into regions of C consecutive ones (64 to 1024,
@@ -1799,19 +1835,13 @@ static int sched_region_persons(long long P)
     return C;
 }
 
-cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, cudaStream_t s)
+cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, DayQueue &q)
 {
     const int C = sched_region_persons(d.P), regions = d.P / C;
     const int blocks = std::min(div_up(regions, kSchedWarps), kSchedBlocksPerSm * sm_count());
     const int passes = radix_passes(d.bucket_max[weekend ? 1 : 0]), dbits = radix_digit_bits(d.bucket_max[weekend ? 1 : 0]);
-#define PT_SCHED(W)                                                                                              \
-    k_sched<W><<<blocks, kSchedThreads, 0, s>>>(d.ic, d.is, d.tile_inst, regions, C, d.age, d.mark, d.keys,       \
-                                                d.digit_hist, passes, dbits, d.rp1, d.region_count, d.sc, day)
-    if (weekend) PT_SCHED(true);
-    else PT_SCHED(false);
-#undef PT_SCHED
-    count_launch();
-    return cudaGetLastError();
+    return queue_kernel(q, weekend ? k_sched<true> : k_sched<false>, blocks, kSchedThreads, 0, d.ic, d.is, d.tile_inst,
+                        regions, C, d.age, d.mark, d.keys, d.digit_hist, passes, dbits, d.rp1, d.region_count, d.sc, day);
 }
 
 // The day's radix sort: one sorted segment per instance, keys local to the instance,
@@ -1953,21 +1983,19 @@ __global__ void __launch_bounds__(kBasesThreads) k_day_digit_bases(int *digit_hi
     }
 }
 
-cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s)
+cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, DayQueue &q)
 {
     const int P = radix_passes(d.bucket_max[weekend ? 1 : 0]);
     const int C = sched_region_persons(d.P);
     const dim3 grid(kBasesTasks + std::max(1, div_up(d.persons_max / C, kBasesRegions)), d.K);
-    k_day_digit_bases<<<grid, kBasesThreads, 0, s>>>(d.digit_hist, d.digit_base, P, d.ic, d.is, d.K, weekend ? 1 : 0,
-                                                    C, d.region_count, d.region_prefix,
-                                                    d.chunk_region, d.tile_prefix, d.tile_prefix0, d.sc);
-    count_launch();
-    return cudaGetLastError();
+    return queue_kernel(q, k_day_digit_bases, grid, kBasesThreads, 0, d.digit_hist, d.digit_base, P, d.ic, d.is, d.K,
+                        weekend ? 1 : 0, C, d.region_count, d.region_prefix, d.chunk_region, d.tile_prefix,
+                        d.tile_prefix0, d.sc);
 }
 
-cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, cudaStream_t s)
+cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, DayQueue &q)
 {
-    return launch_radix_sort(day_radix_args(d, weekend), s);
+    return launch_radix_sort(day_radix_args(d, weekend), q);
 }
 
 // ------------------------------------------------------------------ infection
@@ -2466,7 +2494,7 @@ __global__ void __launch_bounds__(128, 8) k_infect_weekend(InfectArgs a, int day
     queue.flush(1, lane);
 }
 
-cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_t s)
+cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, DayQueue &q)
 {
     InfectArgs a;
     a.ic = d.ic; a.is = d.is;
@@ -2478,17 +2506,9 @@ cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_
     a.claim = d.claim; a.new_list = d.new_list; a.sc = d.sc;
     const Tuning &t = d.tune;
     a.coop_most = kCoopPerSm * sm_count();
-    if (t.infect_coop) {
-        const int blocks = sm_count() * t.infect_blocks_per_sm;
-        if (weekend) k_infect_coop<true><<<blocks, 256, 0, s>>>(a, day);
-        else k_infect_coop<false><<<blocks, 256, 0, s>>>(a, day);
-    } else {
-        const int blocks = sm_count() * t.infect_blocks_per_sm * 2;   // blocks of 128 threads
-        if (weekend) k_infect_weekend<<<blocks, 128, 0, s>>>(a, day);
-        else k_infect_weekday<<<blocks, 128, 0, s>>>(a, day);
-    }
-    count_launch();
-    return cudaGetLastError();
+    const int blocks = sm_count() * t.infect_blocks_per_sm;
+    if (t.infect_coop) return queue_kernel(q, weekend ? k_infect_coop<true> : k_infect_coop<false>, blocks, 256, 0, a, day);
+    return queue_kernel(q, weekend ? k_infect_weekend : k_infect_weekday, 2 * blocks, 128, 0, a, day);
 }
 
 // device_setInfectionStatus (PandemicSim.cu:3048-3067) for the winning claims:
@@ -2516,11 +2536,9 @@ __global__ void k_apply(uint32_t *state, uint8_t *gen_p, uint8_t *gen_s, unsigne
     }
 }
 
-cudaError_t launch_apply(const DevArrays &d, int day, cudaStream_t s)
+cudaError_t launch_apply(const DevArrays &d, int day, DayQueue &q)
 {
-    k_apply<<<sm_count() * 8, 256, 0, s>>>(d.state, d.gen_p, d.gen_s, d.claim, d.new_list, d.sc, day);
-    count_launch();
-    return cudaGetLastError();
+    return queue_kernel(q, k_apply, sm_count() * 8, 256, 0, d.state, d.gen_p, d.gen_s, d.claim, d.new_list, d.sc, day);
 }
 
 // Four persons a thread; the persons up to the next multiple of four are padding.
@@ -2563,12 +2581,10 @@ __global__ void __launch_bounds__(256) k_day_rows(const InstState *is, int K, Sc
     }
 }
 
-cudaError_t launch_day_rows(const DevArrays &d, int *out, cudaStream_t s)
+cudaError_t launch_day_rows(const DevArrays &d, int *out, DayQueue &q)
 {
     const int n = d.K * kDayRow, threads = std::min(256, div_up(n, 32) * 32);
-    k_day_rows<<<div_up(n, threads), threads, 0, s>>>(d.is, d.K, d.sc, out);
-    count_launch();
-    return cudaGetLastError();
+    return queue_kernel(q, k_day_rows, div_up(n, threads), threads, 0, d.is, d.K, d.sc, out);
 }
 
 // ================================================================== bounded-wait probe

@@ -176,6 +176,16 @@ __host__ __device__ inline bool prec_school(uint32_t w) { return ((w >> 10) & 1u
 // Launch configuration helpers
 int sm_count();
 
+// Where a day's launches go: to a stream, or (graph set) to a graph, as nodes one behind
+// the other.  (Not by capturing the stream: while a stream is captured, a thread that waits
+// for the device is refused and ends the capture.)
+struct DayQueue {
+    cudaStream_t stream = nullptr;
+    cudaGraph_t graph = nullptr;
+    cudaGraphNode_t last = nullptr;   // the graph's last node
+    uint64_t kernels = 0;             // kernel nodes
+};
+
 // ---- setup
 cudaError_t launch_household_types(const SimConst &c, uint8_t *types, int32_t *sizes, int *adults,
                                    int *persons, cudaStream_t s);
@@ -239,7 +249,7 @@ struct RadixArgs {
 };
 int radix_passes(int buckets);
 int radix_digit_bits(int buckets);   // bits of a pass's digit
-cudaError_t launch_radix_sort(const RadixArgs &r, cudaStream_t s);
+cudaError_t launch_radix_sort(const RadixArgs &r, DayQueue &q);
 // count (optional) + scan + digit bases + radix passes: a complete bucket table
 cudaError_t launch_bucket_table(const RadixArgs &r, int32_t *counts, bool count_keys, int32_t *offset,
                                 unsigned long long *tiles, int *lb_ctl, int *digit_hist, cudaStream_t s);
@@ -257,15 +267,15 @@ cudaError_t launch_seed_infected(const int32_t *seeds, int P, int S, uint32_t *s
 cudaError_t launch_person_records(const DevArrays &d, cudaStream_t s);
 
 // ---- day (every instance of the batch in each launch)
-cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, cudaStream_t s);   // recover, count, bookkeeping
+cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, DayQueue &q);   // recover, count, bookkeeping
 cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables,
-                                 cudaStream_t s);                                     // the ordered list, the marks
-cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, cudaStream_t s);
+                                 DayQueue &q);                                        // the ordered list, the marks
+cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, DayQueue &q);
 cudaError_t launch_day_keys(const DevArrays &d, bool weekend, cudaStream_t s);        // for inspection
-cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, cudaStream_t s);
-cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, cudaStream_t s);
-cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, cudaStream_t s);
-cudaError_t launch_apply(const DevArrays &d, int day, cudaStream_t s);
+cudaError_t launch_bucket_scan(const DevArrays &d, bool weekend, DayQueue &q);
+cudaError_t launch_bucket_sort(const DevArrays &d, bool weekend, DayQueue &q);
+cudaError_t launch_infect(const DevArrays &d, bool weekend, int day, DayQueue &q);
+cudaError_t launch_apply(const DevArrays &d, int day, DayQueue &q);
 // A day's rows of every instance to mapped host memory: out[0] the device error word, then
 // per instance its 16 counts, infected and days run.
 constexpr int kDayRow = 18;
@@ -274,7 +284,7 @@ constexpr int kDayRow = 18;
 inline size_t state_plane(size_t n) { return (n + 15) / 16 * 16; }
 uint8_t *state_planes(const DevArrays &d);
 cudaError_t launch_unpack_state(const DevArrays &d, int first, int n, cudaStream_t s);
-cudaError_t launch_day_rows(const DevArrays &d, int *out, cudaStream_t s);
+cudaError_t launch_day_rows(const DevArrays &d, int *out, DayQueue &q);
 // weekday / weekend buckets of one instance (compact keys hour * R + dest - lo)
 int day_buckets(const SimConst &c, bool weekend);
 
@@ -289,7 +299,6 @@ cudaError_t launch_errand_selftest(unsigned long long *counts, cudaStream_t s);
 long long max_spin_limit();   // the polls every wait of the simulation allows
 
 uint64_t launches();
-uint64_t thread_launches();    // the calling thread's own (what a capture records)
-void add_launches(int64_t n);  // kernels run by a replayed graph
+void add_launches(uint64_t n);  // kernels run by a replayed graph
 
 }  // namespace ptk

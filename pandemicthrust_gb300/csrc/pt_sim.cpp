@@ -63,6 +63,12 @@ struct Instance {
 enum { kStSweep, kStInfectedList, kStSchedule, kStDigits, kStRadix, kStOffsets, kStInfect, kStApply, kStages };
 static_assert(kStages == 8, "eight stages per day type in pt_get_stage_ms");
 
+// A graph of days and the kernels that a launch of it runs.
+struct DayGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint64_t kernels = 0;
+};
+
 }  // namespace
 
 struct Engine {
@@ -84,8 +90,8 @@ struct Engine {
     bool setup_done = false;
     int next_day = 0;                 // next global day to queue
     int rows_day = 0;                 // first global day whose rows the host has not: next_day between calls, but
-                                      // for a stepped day whose call was not allowed to wait for it (beside
-                                      // another stream's capture); the next call fetches its rows
+                                      // for days whose call was not allowed to wait for them (beside another
+                                      // stream's capture); the next call fetches their rows
     int max_days = 0;                 // longest max_days of the instances
     std::string err;
     bool timing = false;
@@ -96,28 +102,25 @@ struct Engine {
     int stage_days[2] = {0, 0};
     std::vector<float> day_stage_ms;      // kMaxDays x kStages: the last timed run of each day
     mutable uint64_t h2d_bytes = 0, d2h_bytes = 0;  // host<->device copies issued
-    // The whole day loop (days 0..max_days-1), captured once and replayed by later runs.
+    // The whole day loop (days 0..max_days-1), made a graph once and replayed by later runs.
     // Every per-day decision (early stop, counters, offsets) reads device state, so the
-    // same graph serves every run after a reset.  The run that captures it queues its own
+    // same graph serves every run after a reset.  The run that makes it queues its own
     // launches one by one first (2 us each, faster than the device takes them) and
-    // captures while the device works: capturing and instantiating the 900 launches of
-    // 100 days before the first one starts cost 2.5 ms.
-    cudaGraphExec_t run_graph = nullptr;
-    uint64_t graph_kernels = 0;
+    // makes it while the device works: making a graph of the 900 launches of 100 days
+    // before the first one starts cost 2.5 ms.
+    DayGraph run_graph;
     int *day_rows = nullptr;              // mapped host memory of a stepped day's rows (launch_day_rows)
     // A stepped weekday's and weekend day's launches: the first of each kind is queued and
-    // then captured while the device works; the later ones replay it and read their day on
-    // the device.  (Ten launches take 35 us of a step's 90 on an Arm host, a replay 8.)
-    cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
-    uint64_t step_kernels[2] = {0, 0};
-    bool no_graphs = false;               // the stream cannot be captured
+    // then made a graph while the device works; the later ones replay it and read their day
+    // on the device.  (Ten launches take 35 us of a step's 90 on an Arm host, a replay 8.)
+    DayGraph step_graph[2];
 
     int K() const { return (int)inst.size(); }
-    void drop_graphs()   // what was captured depends on the settings
+    void drop_graphs()   // they depend on the settings
     {
-        for (cudaGraphExec_t *g : {&run_graph, &step_graph[0], &step_graph[1]}) {
-            if (*g) cudaGraphExecDestroy(*g);
-            *g = nullptr;
+        for (DayGraph *g : {&run_graph, &step_graph[0], &step_graph[1]}) {
+            if (g->exec) cudaGraphExecDestroy(g->exec);
+            *g = DayGraph{};
         }
     }
     ~Engine();
@@ -604,28 +607,28 @@ static cudaEvent_t stage_event(Engine *s, int day, int k)
 // `launch` is the day the launches are told, the day or -1 (see launch_day).
 static bool is_weekend(int day) { return (day % 7) >= 5; }  // PandemicSim.h:283-284
 
-static pt_status enqueue_day(Engine *s, int day, int launch)
+static pt_status enqueue_day(Engine *s, int day, int launch, ptk::DayQueue &q)
 {
     const bool weekend = is_weekend(day);
     const ptk::DevArrays &d = s->d;
     cudaStream_t st = s->stream;
-    const bool t = s->timing;
+    const bool t = s->timing && !q.graph;
     if (t) cudaEventRecord(stage_event(s, day, kStSweep), st);
-    CK(ptk::launch_sweep(d, weekend, launch, st), "sweep");
+    CK(ptk::launch_sweep(d, weekend, launch, q), "sweep");
     if (t) cudaEventRecord(stage_event(s, day, kStInfectedList), st);
-    CK(ptk::launch_infected_list(d, weekend, launch, s->full_tables, st), "infected list");
+    CK(ptk::launch_infected_list(d, weekend, launch, s->full_tables, q), "infected list");
     if (t) cudaEventRecord(stage_event(s, day, kStSchedule), st);
-    CK(ptk::launch_schedule(d, weekend, launch, st), "schedule");
+    CK(ptk::launch_schedule(d, weekend, launch, q), "schedule");
     if (t) cudaEventRecord(stage_event(s, day, kStDigits), st);
-    CK(ptk::launch_bucket_scan(d, weekend, st), "digit bases");
+    CK(ptk::launch_bucket_scan(d, weekend, q), "digit bases");
     if (t) cudaEventRecord(stage_event(s, day, kStRadix), st);
-    CK(ptk::launch_bucket_sort(d, weekend, st), "bucket sort");
+    CK(ptk::launch_bucket_sort(d, weekend, q), "bucket sort");
     // (the sort's last pass writes the bucket slots: the offsets stage is empty)
     if (t) cudaEventRecord(stage_event(s, day, kStOffsets), st);
     if (t) cudaEventRecord(stage_event(s, day, kStInfect), st);
-    CK(ptk::launch_infect(d, weekend, launch, st), "infect");
+    CK(ptk::launch_infect(d, weekend, launch, q), "infect");
     if (t) cudaEventRecord(stage_event(s, day, kStApply), st);
-    CK(ptk::launch_apply(d, launch, st), "apply");
+    CK(ptk::launch_apply(d, launch, q), "apply");
     if (t) cudaEventRecord(stage_event(s, day, kStages), st);
     if (t) s->timed_days.push_back(day);
     return PT_OK;
@@ -694,9 +697,10 @@ static pt_status refuse_capture(Engine *s)
     return PT_OK;
 }
 
-// Nor can a run's rows be fetched while a capture of another stream forbids this thread to
-// wait (the query is forbidden then too): asked before anything is queued.  (A stepped day
-// does not ask, the query's 1.5 us are 2% of a small one; see Engine::rows_day.)
+// Nor can it wait while a capture of another stream forbids that to this thread (a query is
+// forbidden then, too).  Asked before copies to memory that would be gone if the wait
+// behind them were refused.  What has been queued by then stays: see Engine::rows_day.
+// (Not asked before: the query's 1.5 us are 2% of a small stepped day.)
 static pt_status refuse_beside_capture(Engine *s)
 {
     const cudaError_t e = cudaStreamQuery(s->stream);
@@ -743,39 +747,37 @@ static pt_status fetch_rows(Engine *s)
 }
 
 // Queues a stepped day and the copy of its rows; `launch` as for enqueue_day.
-static pt_status queue_step(Engine *s, int day, int launch)
+static pt_status queue_step(Engine *s, int day, int launch, ptk::DayQueue &q)
 {
-    const pt_status st = enqueue_day(s, day, launch);
+    const pt_status st = enqueue_day(s, day, launch, q);
     if (st != PT_OK) return st;
-    CK(ptk::launch_day_rows(s->d, s->day_rows, s->stream), "day rows");
+    CK(ptk::launch_day_rows(s->d, s->day_rows, q), "day rows");
     return PT_OK;
 }
 
-// Captures what `queue` queues as a graph for later calls, which counts its kernels.  The
-// days themselves have been queued before, so a capture that fails costs no call: the
-// engine goes on without the graph, on a stream that cannot be captured (the legacy default
-// one) without any.
+// Makes a graph of what `queue` queues, for later calls.  The days themselves have been
+// queued before, so a graph that cannot be made costs no call: the engine goes on without it.
 template <class Queue>
-static void capture_days(Engine *s, cudaGraphExec_t *graph, uint64_t *kernels, Queue queue)
+static void make_graph(Engine *s, DayGraph &g, Queue queue)
 {
-    if (s->no_graphs) return;
-    const uint64_t before = ptk::thread_launches();
     const std::string err = s->err;
-    cudaGraph_t g = nullptr;
-    bool ok = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-    s->no_graphs = !ok;
-    if (ok) {
-        ok = queue() == PT_OK;
-        ok = cudaStreamEndCapture(s->stream, &g) == cudaSuccess && ok;
-    }
-    *kernels = ptk::thread_launches() - before;
-    ptk::add_launches(-(int64_t)*kernels);  // counted when the graph runs
-    if (!ok || cudaGraphInstantiate(graph, g, 0) != cudaSuccess) {
-        *graph = nullptr;
+    ptk::DayQueue q;
+    bool ok = cudaGraphCreate(&q.graph, 0) == cudaSuccess;
+    ok = ok && queue(q) == PT_OK && cudaGraphInstantiate(&g.exec, q.graph, 0) == cudaSuccess;
+    if (q.graph) cudaGraphDestroy(q.graph);
+    g.kernels = q.kernels;
+    if (!ok) {
+        g.exec = nullptr;
         s->err = err;
         cudaGetLastError();
     }
-    if (g) cudaGraphDestroy(g);
+}
+
+static pt_status launch_graph(Engine *s, const DayGraph &g)
+{
+    CK(cudaGraphLaunch(g.exec, s->stream), "graph launch");
+    ptk::add_launches(g.kernels);
+    return PT_OK;
 }
 
 // One stepped day and its rows.  A caller that steps waits for them every day, so a
@@ -788,13 +790,13 @@ static pt_status step_day(Engine *s, int day)
     if (!s->day_rows)
         CK(cudaHostAlloc((void **)&s->day_rows, bytes, cudaHostAllocMapped | cudaHostAllocPortable), "day rows");
     pt_status st = PT_OK;
-    if (!s->timing && s->step_graph[kind]) {
-        CK(cudaGraphLaunch(s->step_graph[kind], s->stream), "graph launch");
-        ptk::add_launches((int64_t)s->step_kernels[kind]);
+    if (!s->timing && s->step_graph[kind].exec) {
+        st = launch_graph(s, s->step_graph[kind]);
     } else {
-        st = queue_step(s, day, day);
+        ptk::DayQueue now{s->stream};
+        st = queue_step(s, day, day, now);
         if (st == PT_OK && !s->timing)   // for later days of its kind
-            capture_days(s, &s->step_graph[kind], &s->step_kernels[kind], [&] { return queue_step(s, day, -1); });
+            make_graph(s, s->step_graph[kind], [&](ptk::DayQueue &q) { return queue_step(s, day, -1, q); });
     }
     if (st != PT_OK) return st;
     s->next_day = day + 1;
@@ -848,25 +850,18 @@ static pt_status engine_run(Engine *s)
     const int first = s->next_day, M = s->max_days;
     if (instances_running(s) > 0 && first < M) {
         pt_status st = refuse_capture(s);
-        if (st == PT_OK) st = refuse_beside_capture(s);
         if (st != PT_OK) return st;
-        const bool replay = first == 0 && !s->timing && s->run_graph;
-        if (replay) {
-            CK(cudaGraphLaunch(s->run_graph, s->stream), "graph launch");
-            ptk::add_launches((int64_t)s->graph_kernels);
-        } else {
-            for (int day = first; day < M; day++) {
-                st = enqueue_day(s, day, day);
-                if (st != PT_OK) return st;
-            }
-        }
+        auto days = [&](ptk::DayQueue &q) {
+            pt_status st = PT_OK;
+            for (int day = first; day < M && st == PT_OK; day++) st = enqueue_day(s, day, day, q);
+            return st;
+        };
+        const bool whole = first == 0 && !s->timing;
+        ptk::DayQueue now{s->stream};
+        st = whole && s->run_graph.exec ? launch_graph(s, s->run_graph) : days(now);
+        if (st != PT_OK) return st;
         s->next_day = M;
-        if (first == 0 && !s->timing && !s->run_graph)   // for later runs
-            capture_days(s, &s->run_graph, &s->graph_kernels, [&] {
-                pt_status st = PT_OK;
-                for (int day = 0; day < M && st == PT_OK; day++) st = enqueue_day(s, day, day);
-                return st;
-            });
+        if (whole && !s->run_graph.exec) make_graph(s, s->run_graph, days);   // for later runs
     }
     return fetch_rows(s);
 }
@@ -1061,7 +1056,7 @@ static pt_status engine_set_tuning(Engine *s, const pt_tuning *t)
     if (n.infect_coop != s->d.tune.infect_coop || n.infect_blocks_per_sm != s->d.tune.infect_blocks_per_sm ||
         n.radix_blocks_per_sm != s->d.tune.radix_blocks_per_sm || n.sched_tf != s->d.tune.sched_tf ||
         n.dense_level != s->d.tune.dense_level || n.radix_threads != s->d.tune.radix_threads) {
-        // the captured day loop holds the old launch shapes
+        // the graphs hold the old launch shapes
         if (s->stream) cudaStreamSynchronize(s->stream);
         s->drop_graphs();
     }
@@ -1320,7 +1315,7 @@ pt_status pt_set_full_tables(pt_sim *s, int enabled)
 {
     if (!s) return PT_ERR_ARG;
     const bool v = enabled != 0;
-    // the captured launches bake this choice in; they are captured again when needed
+    // the graphs bake this choice in; they are made again when needed
     if (v != s->full_tables) s->drop_graphs();
     s->full_tables = v;
     return PT_OK;
