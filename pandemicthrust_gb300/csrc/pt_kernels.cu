@@ -5,7 +5,7 @@
 //           workplace buckets                         (setupSim, :146-208)
 //   sweep   recover + 16 status bins + ordered infected list, one pass
 //           (kernel_countInfectedStatusAndRecover :2097-2192 + copy_if :2207-2224)
-//   sched   schedule keys + bucket histogram          (:2972-3022 / :2082-2094)
+//   sched   schedule keys + digit histograms          (:2972-3022 / :2082-2094)
 //   bucket  a stable LSD radix sort of the (key, person) entries, whose last pass also
 //           writes each bucket's start and size (CUB sort + lower_bound, :1212-1248,
 //           :1313-1354)
@@ -960,7 +960,7 @@ __device__ __forceinline__ uint32_t recover_word(uint32_t st, int d2r, bool &cha
 //          [start, list_end) of the infected list and its day bookkeeping.
 //   emit   one person tile per warp (per block for small runs): the infected ids,
 //          in ascending order, at their list positions.
-// The count kernel also clears the day's marks and the emit kernel its bucket slots.
+// The count kernel also clears the day's marks.
 // Each launch depends only on the one before, so no block waits for another.
 // Person tiles a count block sweeps one after another: as many as make the grid one wave
 // of the blocks that fit (kSweepBlocksPerSm), at most what 8-bit status counts hold.
@@ -1183,23 +1183,13 @@ __global__ void __launch_bounds__(kSweepScanThreads) k_sweep_scan(const InstCons
     if (threadIdx.x == 0) begin_day(sc, total, day);
 }
 
-// The grid's threads clear the day's bucket slots.  Only on a day that goes on: the tables
-// of the last day with infected stay.
-__device__ __forceinline__ void clear_slots(uint2 *slot, int slots)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x)
-        slot[i] = make_uint2(0u, 0u);
-}
-
 // Emit for small runs: a block per person tile, a block scan of the threads' packed
 // per-round counts (a warp per tile would leave most SMs idle).
 __global__ void __launch_bounds__(kSweepThreads) k_sweep_emit_block(const int32_t *tile_inst, const uint16_t *flags_in,
                                                                     const int32_t *tile_prefix, int32_t *infected,
-                                                                    int32_t *infected_inst, uint2 *slot, int slots,
-                                                                    const Scalars *sc)
+                                                                    int32_t *infected_inst, const Scalars *sc)
 {
     if (*(volatile const int *)&sc->done) return;
-    clear_slots(slot, slots);
     const int tile = blockIdx.x;
     const int prefix = tile_prefix[tile];
     if (tile_prefix[tile + 1] == prefix) return;  // no infected in this tile
@@ -1237,11 +1227,9 @@ constexpr int kEmitWarps = 8;   // person tiles per emit block, one warp each
 __global__ void __launch_bounds__(kEmitWarps * 32) k_sweep_emit(const int32_t *tile_inst, int tiles,
                                                                 const uint16_t *flags_in,
                                                                 const int32_t *tile_prefix, int32_t *infected,
-                                                                int32_t *infected_inst, uint2 *slot, int slots,
-                                                                const Scalars *sc)
+                                                                int32_t *infected_inst, const Scalars *sc)
 {
     if (*(volatile const int *)&sc->done) return;
-    clear_slots(slot, slots);
     const int lane = threadIdx.x & 31;
     const int tile = blockIdx.x * kEmitWarps + (threadIdx.x >> 5);
     if (tile >= tiles) return;
@@ -1415,11 +1403,10 @@ __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *
 }
 
 // A small run's list and marks in one launch instead of three (scan, emit, mark): a block
-// per person tile sums the counts of the tiles itself, clears its part of the day's bucket
-// slots, emits its part of the list and marks its persons' buckets.  The block of an
-// instance's first tile begins the instance's day, the last tile's block the batch's; no
-// block waits for another.  Small runs are bound by their launches: a day of 100,000
-// persons has seven of 3 to 10 us.
+// per person tile sums the counts of the tiles itself, emits its part of the list and
+// marks its persons' buckets.  The block of an instance's first tile begins the
+// instance's day, the last tile's block the batch's; no block waits for another.  Small
+// runs are bound by their launches: a day of 100,000 persons has seven of 3 to 10 us.
 // Up to kListTiles tiles (4M persons) the sums are four loads a thread.
 constexpr int kListTiles = 4 * kSweepThreads;
 constexpr int kListMarkWords = 2048;   // a bitmap this small is marked in shared memory and merged once a block
@@ -1429,8 +1416,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
                                                               const int32_t *tile_count, int32_t *infected,
                                                               int32_t *infected_inst, int2 *read, const uint8_t *age,
                                                               uint32_t *mark,
-                                                              int words, int mark_all, uint2 *slot, int slots,
-                                                              Scalars *sc, int day, int dense_level)
+                                                              int words, int mark_all, Scalars *sc, int day,
+                                                              int dense_level)
 {
     day = launch_day(day, sc);
     const int ended = *(volatile const int *)&sc->done;
@@ -1478,7 +1465,6 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep_list(const InstConst *i
     total += list_end;
     if (t == 0 && tile == first) begin_instance_day(ik, is[k], start, list_end, day, dense_level);
     if (t == 0 && tile == tiles - 1) begin_day(sc, total, day);
-    if (total > 0) clear_slots(slot, slots);
     if (n == 0) return;
     unsigned long long packed = 0;
 #pragma unroll
@@ -1537,7 +1523,7 @@ cudaError_t launch_sweep(const DevArrays &d, bool weekend, int day, DayQueue &q)
 // for complete tables).
 cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool full_tables, DayQueue &q)
 {
-    const int tiles = d.P / kSweepTile, B = d.buckets[weekend ? 1 : 0], words = mark_words(d, weekend);
+    const int tiles = d.P / kSweepTile, words = mark_words(d, weekend);
     if (full_tables) {
         const cudaError_t e = queue_fill(q, d.mark, 0xFFFFFFFFu, (size_t)words);
         if (e != cudaSuccess) return e;
@@ -1545,13 +1531,13 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
     if (tiles <= kListTiles)
         return queue_kernel(q, k_sweep_list, tiles, kSweepThreads, 0, d.ic, d.is, d.tile_inst, tiles, d.sweep_flags,
                             d.sweep_tiles, d.infected, d.infected_inst, d.read, d.age, d.mark, words,
-                            full_tables ? 1 : 0, d.bkt, B, d.sc, day, d.tune.dense_level);
+                            full_tables ? 1 : 0, d.sc, day, d.tune.dense_level);
     const cudaError_t e =
         tiles >= kSweepEmitTilesPerSm * sm_count()
             ? queue_kernel(q, k_sweep_emit, div_up(tiles, kEmitWarps), kEmitWarps * 32, 0, d.tile_inst, tiles,
-                           d.sweep_flags, d.sweep_tiles, d.infected, d.infected_inst, d.bkt, B, d.sc)
+                           d.sweep_flags, d.sweep_tiles, d.infected, d.infected_inst, d.sc)
             : queue_kernel(q, k_sweep_emit_block, tiles, kSweepThreads, 0, d.tile_inst, d.sweep_flags, d.sweep_tiles,
-                           d.infected, d.infected_inst, d.bkt, B, d.sc);
+                           d.infected, d.infected_inst, d.sc);
     if (e != cudaSuccess) return e;
     return queue_kernel(q, k_mark_buckets, sm_count() * kMarkBlocksPerSm, kMarkThreads, 0, d.ic, d.is, d.age, d.infected,
                         d.infected_inst, weekend ? 1 : 0, d.read, d.mark, words, d.sc);
@@ -1579,7 +1565,7 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
 // with marking, 620 and 1,250 before (look-back, selects, add / add-with-carry Threefry).
 constexpr int kSchedThreads = 256, kSchedWarps = kSchedThreads / 32;
 constexpr int kSchedPart = 256;       // persons whose entries a warp's part holds (a person's place fits a byte)
-constexpr int kSchedBlocksPerSm = 5;  // 47 registers; 6 (40) and 7 (32, spills) cost 15% and 21% more on weekends
+constexpr int kSchedBlocksPerSm = 5;  // 48 registers; 6 (40) and 7 (32, spills) cost 15% and 21% more on weekends
                                       // and 5% and 55% more on weekdays at 50M persons
 
 // Adds the block's histograms to instance k's stripe of the day's digit histograms
@@ -1616,10 +1602,14 @@ template <bool WEEKEND>
 __global__ void __launch_bounds__(kSchedThreads, kSchedBlocksPerSm)
     k_sched(const InstConst *ic, InstState *is, const int32_t *tile_inst, int regions, int C, const uint8_t *age,
             const uint32_t *mark, int32_t *keys, int *digit_hist, int passes, int dbits, uint2 *entries,
-            int32_t *region_count, const Scalars *sc, int day)
+            int32_t *region_count, uint2 *slot, int slots, const Scalars *sc, int day)
 {
     day = launch_day(day, sc);
     if (*(volatile const int *)&sc->done) return;
+    // the day's bucket slots, for the sort (only on a day that goes on: the tables of the
+    // last day with infected stay)
+    for (int i = blockIdx.x * kSchedThreads + threadIdx.x; i < slots; i += gridDim.x * kSchedThreads)
+        slot[i] = make_uint2(0u, 0u);
     static_assert(kSchedThreads == 256, "one thread per digit in sched_flush_digits");
     constexpr int kPer = WEEKEND ? 3 : 2;                       // keys per person
     constexpr int kCap = kPer * kSchedPart;                     // entries of a warp's part at most
@@ -1841,7 +1831,8 @@ cudaError_t launch_schedule(const DevArrays &d, bool weekend, int day, DayQueue 
     const int blocks = std::min(div_up(regions, kSchedWarps), kSchedBlocksPerSm * sm_count());
     const int passes = radix_passes(d.bucket_max[weekend ? 1 : 0]), dbits = radix_digit_bits(d.bucket_max[weekend ? 1 : 0]);
     return queue_kernel(q, weekend ? k_sched<true> : k_sched<false>, blocks, kSchedThreads, 0, d.ic, d.is, d.tile_inst,
-                        regions, C, d.age, d.mark, d.keys, d.digit_hist, passes, dbits, d.rp1, d.region_count, d.sc, day);
+                        regions, C, d.age, d.mark, d.keys, d.digit_hist, passes, dbits, d.rp1, d.region_count, d.bkt,
+                        d.buckets[weekend ? 1 : 0], d.sc, day);
 }
 
 // The day's radix sort: one sorted segment per instance, keys local to the instance,
