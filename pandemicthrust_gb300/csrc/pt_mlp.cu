@@ -2470,8 +2470,7 @@ pt_status pt_mlp_predict_ensemble_device(pt_mlp *const *members, int count, cons
 void pt_mlp_destroy(pt_mlp *m)
 {
     if (!m) return;
-    if (m->stream) cudaStreamSynchronize(m->stream);
-    else cudaDeviceSynchronize();
+    cudaStreamSynchronize(m->stream);   // (not the device, which is forbidden while any stream is being captured)
     for (void *p : m->allocs) cudaFree(p);
     if (m->umma_err) cudaFreeHost(m->umma_err);
     delete m;
