@@ -319,7 +319,8 @@ const char *pt_mlp_last_error(const pt_mlp *mlp);
 void pt_destroy(pt_sim *sim);
 
 /* Hands the memory the pool of the current GPU keeps, and no simulation uses, back to
- * the device (cudaMemPoolTrimTo).  Call it before allocating elsewhere what the
+ * the device (cudaMemPoolTrimTo), and the few small mapped host buffers that destroyed
+ * simulations and networks leave for the next ones.  Call it before allocating elsewhere what the
  * library no longer needs. */
 pt_status pt_trim_device_memory(void);
 

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "pandemic_gb300.h"
+#include "pt_mapped.h"
 
 namespace {
 
@@ -1657,7 +1658,8 @@ struct pt_mlp {
     int use_umma = 1;
     bool chain_ready = false;   // training: k_chain may be launched
     bf16 *h0p = nullptr;
-    int *umma_err = nullptr;
+    ptm::Mapped err_word;
+    int *umma_err = nullptr;    // err_word's
     // inference input (FP32 rows copied from the host), and the accumulator of last layers
     // that run one by one (rows padded to a multiple of 32), max_batch rows each
     float *xin = nullptr;
@@ -1827,9 +1829,11 @@ static bool chain_fits(const pt_mlp *m)
 static cudaError_t error_word(pt_mlp *m)
 {
     if (m->umma_err) return cudaSuccess;
-    const cudaError_t e = cudaHostAlloc((void **)&m->umma_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
-    if (e == cudaSuccess) *m->umma_err = 0;
-    return e;
+    const cudaError_t e = ptm::mapped_take(sizeof(int), &m->err_word);
+    if (e != cudaSuccess) return e;
+    m->umma_err = (int *)m->err_word.ptr;
+    *m->umma_err = 0;
+    return cudaSuccess;
 }
 
 static cudaError_t chain(pt_mlp *m, int B, const bf16 *h0, const float *Y, const int *rows, float *loss)
@@ -2470,9 +2474,10 @@ pt_status pt_mlp_predict_ensemble_device(pt_mlp *const *members, int count, cons
 void pt_mlp_destroy(pt_mlp *m)
 {
     if (!m) return;
-    cudaStreamSynchronize(m->stream);   // (not the device, which is forbidden while any stream is being captured)
-    for (void *p : m->allocs) cudaFree(p);
-    if (m->umma_err) cudaFreeHost(m->umma_err);
+    // (not the device, which is forbidden while any stream is being captured)
+    bool idle = cudaStreamSynchronize(m->stream) == cudaSuccess;
+    for (void *p : m->allocs) idle = cudaFree(p) == cudaSuccess && idle;   // (waits for other streams' use, too)
+    ptm::mapped_give(m->err_word, idle);
     delete m;
 }
 

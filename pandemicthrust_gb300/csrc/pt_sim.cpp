@@ -20,6 +20,7 @@
 #include "pandemic_gb300.h"
 #include "pt_host.h"
 #include "pt_kernels.h"
+#include "pt_mapped.h"
 
 namespace {
 
@@ -109,7 +110,7 @@ struct Engine {
     // makes it while the device works: making a graph of the 900 launches of 100 days
     // before the first one starts cost 2.5 ms.
     DayGraph run_graph;
-    int *day_rows = nullptr;              // mapped host memory of a stepped day's rows (launch_day_rows)
+    ptm::Mapped day_rows;                 // a stepped day's rows (launch_day_rows)
     // A stepped weekday's and weekend day's launches: the first of each kind is queued and
     // then made a graph while the device works; the later ones replay it and read their day
     // on the device.  (Ten launches take 35 us of a step's 90 on an Arm host, a replay 8.)
@@ -220,8 +221,8 @@ Engine::~Engine()
     if (arena_mem) cudaFreeAsync(arena_mem, stream);
     if (setup_mem) cudaFreeAsync(setup_mem, stream);
     if (small_mem) cudaFreeAsync(small_mem, stream);
-    if (stream) cudaStreamSynchronize(stream);
-    if (day_rows) cudaFreeHost(day_rows);
+    const bool idle = stream && cudaStreamSynchronize(stream) == cudaSuccess;
+    ptm::mapped_give(day_rows, idle);
     for (auto &e : day_events)
         if (e) cudaEventDestroy(e);
     if (own_stream && stream) cudaStreamDestroy(stream);
@@ -751,7 +752,7 @@ static pt_status queue_step(Engine *s, int day, int launch, ptk::DayQueue &q)
 {
     const pt_status st = enqueue_day(s, day, launch, q);
     if (st != PT_OK) return st;
-    CK(ptk::launch_day_rows(s->d, s->day_rows, q), "day rows");
+    CK(ptk::launch_day_rows(s->d, (int *)s->day_rows.ptr, q), "day rows");
     return PT_OK;
 }
 
@@ -787,8 +788,7 @@ static pt_status step_day(Engine *s, int day)
 {
     const int K = s->K(), kind = is_weekend(day) ? 1 : 0;
     const size_t bytes = ((size_t)K * ptk::kDayRow + 1) * sizeof(int);
-    if (!s->day_rows)
-        CK(cudaHostAlloc((void **)&s->day_rows, bytes, cudaHostAllocMapped | cudaHostAllocPortable), "day rows");
+    if (!s->day_rows.ptr) CK(ptm::mapped_take(bytes, &s->day_rows), "day rows");
     pt_status st = PT_OK;
     if (!s->timing && s->step_graph[kind].exec) {
         st = launch_graph(s, s->step_graph[kind]);
@@ -802,9 +802,9 @@ static pt_status step_day(Engine *s, int day)
     s->next_day = day + 1;
     s->d2h_bytes += bytes;
     CK(cudaStreamSynchronize(s->stream), "sync");
-    if (s->day_rows[0]) return fail(s, PT_ERR_TIMEOUT, "a device-side wait gave up (look-back ordering)");
+    const int *const rows = (const int *)s->day_rows.ptr + 1;
+    if (rows[-1]) return fail(s, PT_ERR_TIMEOUT, "a device-side wait gave up (look-back ordering)");
     accumulate_timing(s);
-    const int *rows = s->day_rows + 1;
     update_mirrors(s, day, day + 1,
                    [&](int k, int) {
                        const int *r = rows + (size_t)k * ptk::kDayRow;
@@ -1421,6 +1421,7 @@ pt_status pt_trim_device_memory(void)
     cudaMemPool_t pool = nullptr;
     cudaError_t e = engine_pool(&pool);
     if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool, 0);
+    ptm::mapped_trim();
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "trim device memory");
     return PT_OK;
 }
