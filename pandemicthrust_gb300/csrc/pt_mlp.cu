@@ -2259,21 +2259,24 @@ pt_status pt_mlp_create(int layers, const int *widths, int max_batch, uint64_t s
         return PT_ERR_CUDA;
     m->loss_cap = 1;
     // The BF16 buffers' padding columns (and the weights' padding rows) stay zero: they
-    // are cleared here and never written.
+    // are cleared here and never written.  A buffer without any is left as it is (clearing
+    // the 1.3 GB of a 262,144-row network takes 200 us).
     m->wpk.resize(layers);
     m->H.resize(layers + 1);
     m->Z.resize(layers);
     m->dZf.resize(layers);
     m->dZb.resize(layers);
-    auto zeroed = [&](bf16 **p, size_t n, const char *what) {
-        return bad(dalloc(m, p, n), what) || bad(cudaMemsetAsync(*p, 0, n * sizeof(bf16), m->stream), what);
+    auto zeroed = [&](bf16 **p, size_t n, const char *what, bool padded = true) {
+        return bad(dalloc(m, p, n), what) ||
+               (padded && bad(cudaMemsetAsync(*p, 0, n * sizeof(bf16), m->stream), what));
     };
+    auto padded = [&](int l) { return m->ld[l] != widths[l]; };
     for (int l = 0; l <= layers; l++)
-        if (zeroed(&m->H[l], (size_t)max_batch * m->ld[l], "activations")) return PT_ERR_CUDA;
+        if (zeroed(&m->H[l], (size_t)max_batch * m->ld[l], "activations", padded(l))) return PT_ERR_CUDA;
     for (int l = 0; l < layers; l++) {
         const size_t n = (size_t)max_batch * m->ld[l + 1];
         if (bad(dalloc(m, &m->Z[l], n), "pre-activations") || bad(dalloc(m, &m->dZf[l], n), "gradients") ||
-            zeroed(&m->dZb[l], n, "gradients") ||
+            zeroed(&m->dZb[l], n, "gradients", padded(l + 1)) ||
             zeroed(&m->wpk[l], (size_t)m->ld[l + 1] * m->ld[l], "bf16 weights"))
             return PT_ERR_CUDA;
     }
