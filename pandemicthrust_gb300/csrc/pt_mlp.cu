@@ -739,13 +739,13 @@ __global__ void __launch_bounds__(32 * (2 + EPI), 1)
         __syncwarp();
     } else if (warp == 1) {
         // MMA issuer (every lane; elect_one issues)
-        bool ok = mbar_wait(b_w, 0, fail);
+        bool ok = __all_sync(0xffffffffu, mbar_wait(b_w, 0, fail));   // (the lanes decide together)
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t idesc = umma_idesc(kUmmaM, Np);
         int it = 0, tc = 0;
         for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, tc++) {
             const int b = tc & 1, use = tc >> 1;
-            ok = __all_sync(0xffffffffu, ok && (use == 0 || mbar_wait(b_acce + 8 * b, (use - 1) & 1, fail)));
+            ok = __all_sync(0xffffffffu, use == 0 || mbar_wait(b_acce + 8 * b, (use - 1) & 1, fail));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
             const uint32_t d = tmem + 256u * b;
