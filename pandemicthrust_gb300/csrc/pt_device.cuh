@@ -325,9 +325,6 @@ __device__ __forceinline__ int errand_step(float w, float p9, int base, float &x
 template <bool WEEKEND>
 __device__ __forceinline__ float errand_p9(bool adult) { return adult ? kTwo32 * ErrandPdf<WEEKEND>::p9 : kNoRow; }
 
-// x / d of a table row, rounded to nearest (div_rn_recip on the scaled values)
-__device__ __forceinline__ float errand_quotient(const ErrandRow &e, float x) { return div_rn_recip(x, e.d, e.r); }
-
 // The bucket draw r falls into: business_in_type's rounding and clamp on the table.
 template <bool WEEKEND>
 __device__ __forceinline__ int errand_bucket(const ErrandRow *rows, uint32_t r, float p9, int base)

@@ -1407,7 +1407,10 @@ __global__ void __launch_bounds__(kMarkThreads) k_mark_buckets(const InstConst *
 // marks its persons' buckets.  The block of an instance's first tile begins the
 // instance's day, the last tile's block the batch's; no block waits for another.  Small
 // runs are bound by their launches: a day of 100,000 persons has seven of 3 to 10 us.
-// Up to kListTiles tiles (4M persons) the sums are four loads a thread.
+// Up to kListTiles tiles (4M persons) the sums are four loads a thread: 30 days of 1.2M and
+// 3.9M persons 2.60 and 3.41 ms, 2.87 and 3.71 with the three launches.  With sixteen loads
+// (to 16M persons) everything below 4M is 1% slower and 4 to 9M 3 to 0.5% faster; at 16M
+// the three launches are faster by 1%.
 constexpr int kListTiles = 4 * kSweepThreads;
 constexpr int kListMarkWords = 2048;   // a bitmap this small is marked in shared memory and merged once a block
 
@@ -1565,7 +1568,7 @@ cudaError_t launch_infected_list(const DevArrays &d, bool weekend, int day, bool
 // with marking, 620 and 1,250 before (look-back, selects, add / add-with-carry Threefry).
 constexpr int kSchedThreads = 256, kSchedWarps = kSchedThreads / 32;
 constexpr int kSchedPart = 256;       // persons whose entries a warp's part holds (a person's place fits a byte)
-constexpr int kSchedBlocksPerSm = 5;  // 48 registers; 6 (40) and 7 (32, spills) cost 15% and 21% more on weekends
+constexpr int kSchedBlocksPerSm = 5;  // 47 and 48 registers; 6 (40) and 7 (32, spills) cost 15% and 21% more on weekends
                                       // and 5% and 55% more on weekdays at 50M persons
 
 // Adds the block's histograms to instance k's stripe of the day's digit histograms

@@ -1964,12 +1964,6 @@ static cudaError_t ensure_zout(pt_mlp *m)
     return dalloc(m, &m->zout, (size_t)m->max_batch * m->ldz);
 }
 
-// forward pass for inference over B rows of x (device, B x width[0] FP32), its outputs
-// z accumulated into y (row stride ldy): y = scale z when `first`, else y + scale z.
-// tcgen05 layers when the shapes fit (hidden H[l] receive the activations, the last
-// layer accumulates in its epilogue), else forward() and k_accumulate.  *x0 caches the
-// zero-padded BF16 copy of x that the tcgen05 layers read: the first network of an
-// ensemble makes it (into its h0p), the others reuse it.
 // The tcgen05 path's per-network state: the padded input buffer and the wait error word.
 static cudaError_t umma_prepare(pt_mlp *m)
 {
@@ -1985,6 +1979,12 @@ static cudaError_t umma_prepare(pt_mlp *m)
     return dalloc(m, &m->h0p, (size_t)m->max_batch * m->ld[0]);
 }
 
+// forward pass for inference over B rows of x (device, B x width[0] FP32), its outputs
+// z accumulated into y (row stride ldy): y = scale z when `first`, else y + scale z.
+// tcgen05 layers when the shapes fit (hidden H[l] receive the activations, the last
+// layer accumulates in its epilogue), else forward() and k_accumulate.  *x0 caches the
+// zero-padded BF16 copy of x that the tcgen05 layers read: the first network of an
+// ensemble makes it (into its h0p), the others reuse it.
 // With hidden_only, the tcgen05 path stops after the last hidden layer (H[L-1] holds
 // its activations) and y is not written.
 static cudaError_t forward_infer(pt_mlp *m, int B, const float *x, const bf16 **x0, float *y, long long ldy,

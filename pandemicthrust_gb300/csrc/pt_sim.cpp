@@ -602,12 +602,12 @@ static cudaEvent_t stage_event(Engine *s, int day, int k)
     return s->day_events[(size_t)day * (kStages + 1) + k];
 }
 
+static bool is_weekend(int day) { return (day % 7) >= 5; }  // PandemicSim.h:283-284
+
 // Enqueues one day of every instance: sweep, schedule, bucket build (scan, radix
 // sort), infection, apply.  Every kernel after the sweep skips an instance that
 // counted no infected, and skips itself once no instance has infected left.
 // `launch` is the day the launches are told, the day or -1 (see launch_day).
-static bool is_weekend(int day) { return (day % 7) >= 5; }  // PandemicSim.h:283-284
-
 static pt_status enqueue_day(Engine *s, int day, int launch, ptk::DayQueue &q)
 {
     const bool weekend = is_weekend(day);
@@ -1054,9 +1054,8 @@ static pt_status engine_set_tuning(Engine *s, const pt_tuning *t)
     n.dense_level = t->dense_level;
     n.radix_threads = t->radix_threads;
     if (n.infect_coop != s->d.tune.infect_coop || n.infect_blocks_per_sm != s->d.tune.infect_blocks_per_sm ||
-        n.radix_blocks_per_sm != s->d.tune.radix_blocks_per_sm || n.sched_tf != s->d.tune.sched_tf ||
-        n.dense_level != s->d.tune.dense_level || n.radix_threads != s->d.tune.radix_threads) {
-        // the graphs hold the old launch shapes
+        n.radix_blocks_per_sm != s->d.tune.radix_blocks_per_sm || n.dense_level != s->d.tune.dense_level) {
+        // the graphs hold the old launch shapes (sched_tf and radix_threads have no effect)
         if (s->stream) cudaStreamSynchronize(s->stream);
         s->drop_graphs();
     }
@@ -1092,7 +1091,7 @@ static pt_status engine_autotune(Engine *s, int days, pt_tuning *chosen)
         }
     }
     struct Cand { int coop, bps; };
-    // thread-per-infector kernel: 9 resident 128-thread blocks per SM at 56 registers;
+    // thread-per-infector kernel: 8 resident 128-thread blocks per SM at 64 registers;
     // warp-cooperative kernel: 6 resident 256-thread blocks per SM at 40 registers
     const Cand infect[] = {{0, 8}, {0, 4}, {1, 6}, {1, 12}, {1, 3}, {0, 16}};
     const int runs = (int)(sizeof(infect) / sizeof(infect[0]));
