@@ -118,10 +118,14 @@ pt_status pt_setup(pt_sim *sim);
 pt_status pt_step_day(pt_sim *sim, int counts16[16], int *infected_count);
 
 /* PandemicSim::runToCompletion without per-day host synchronisation: runs the
- * remaining days on the device (queued at once; later runs replay one CUDA graph) and copies back, per
- * day, the 16 status bins (counts, max_days*16 ints, may be NULL) and the
- * infected count (infected, max_days ints, may be NULL).  days_run receives the
- * number of statistics rows, as the reference's output_infected_stats.csv. */
+ * remaining days on the device (queued at once; later runs replay one CUDA graph) and
+ * copies back, per day, the 16 status bins (counts, max_days*16 ints, may be NULL) and
+ * the infected count (infected, max_days ints, may be NULL).  days_run receives the
+ * number of statistics rows, as the reference's output_infected_stats.csv.
+ * Inside a capture of the simulation's stream, pt_run and pt_step_day are refused with
+ * nothing queued (PT_ERR_CUDA).  Beside a capture of another stream that forbids the
+ * calling thread to wait, the days may have been queued when the call fails; the next
+ * call fetches their rows. */
 pt_status pt_run(pt_sim *sim, int *counts, int *infected, int *days_run);
 
 /* final_countReproduction (PandemicSim.cu:2227-2304): the number of persons per
@@ -152,7 +156,9 @@ pt_status pt_get_population(pt_sim *sim, int32_t *household, int32_t *household_
  * entries and buckets receive the sizes.  By default a day materialises only the
  * buckets that its infected persons visit (the only ones the contact draws read), so
  * the person table and the offsets of the other buckets are complete only after
- * pt_set_full_tables(sim, 1). */
+ * pt_set_full_tables(sim, 1).  A day that finds nobody infected builds no tables: keys,
+ * person table and offsets stay those of the day before (in the layout of the last day's
+ * type; where the two days' types differ, only infected, entries and buckets mean anything). */
 pt_status pt_get_day_tables(pt_sim *sim, int32_t *infected, int32_t *keys, int32_t *people,
                             int32_t *offsets, int *entries, int *buckets);
 
