@@ -672,7 +672,7 @@ static void update_mirrors(Engine *s, int lo, int hi, Row row, Run run)
     for (int k = 0; k < s->K(); k++) {
         Instance &in = s->inst[k];
         if (in.stopped) continue;
-        const int rows = run(k);
+        const int rows = std::min(run(k), hi);   // (the device may have run more, see Engine::rows_day)
         for (int day = in.days_run; day < rows; day++) {
             if (day < lo || day >= hi) continue;  // outside the rows copied
             const std::pair<const int *, int> r = row(k, day);
@@ -710,13 +710,13 @@ static pt_status refuse_beside_capture(Engine *s)
     return PT_OK;
 }
 
-// Copies every instance's rows of the days queued since the last fetch (strided copies out
-// of the device state records), checks the device error word and updates the host mirrors.
-static pt_status fetch_rows(Engine *s)
+// Copies every instance's rows from the last fetch to day hi (strided copies out of the
+// device state records), checks the device error word and updates the host mirrors.
+static pt_status fetch_rows(Engine *s, int hi)
 {
     const pt_status waits = refuse_beside_capture(s);
     if (waits != PT_OK) return waits;
-    const int K = s->K(), lo = s->rows_day, hi = s->next_day;
+    const int K = s->K(), lo = s->rows_day;
     const size_t pitch = sizeof(ptk::InstState);
     const int days = std::max(0, hi - lo);
     std::vector<int> hc((size_t)K * 16 * std::max(days, 1)), hi_((size_t)K * std::max(days, 1)), rows(K);
@@ -837,7 +837,7 @@ static pt_status engine_step(Engine *s, int *running)
     if (instances_running(s) == 0) return all_zero_stopped(s) ? PT_DONE : PT_FINISHED;
     const pt_status captured = refuse_capture(s);
     if (captured != PT_OK) return captured;
-    const pt_status st = s->rows_day < s->next_day ? fetch_rows(s) : step_day(s, s->next_day);
+    const pt_status st = s->rows_day < s->next_day ? fetch_rows(s, s->rows_day + 1) : step_day(s, s->next_day);
     if (st != PT_OK) return st;
     if (running) *running = instances_running(s);
     return all_zero_stopped(s) ? PT_DONE : PT_OK;
@@ -863,7 +863,7 @@ static pt_status engine_run(Engine *s)
         s->next_day = M;
         if (whole && !s->run_graph.exec) make_graph(s, s->run_graph, days);   // for later runs
     }
-    return fetch_rows(s);
+    return fetch_rows(s, s->next_day);
 }
 
 static pt_status engine_gen_counts(Engine *s, int *gen_p, int *gen_s)
