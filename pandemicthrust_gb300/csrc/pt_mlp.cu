@@ -1685,9 +1685,11 @@ static pt_status mfail(pt_mlp *m, pt_status st, const std::string &msg)
 #define MCK(expr, where)                                                                                       \
     do {                                                                                                       \
         cudaError_t _e = (expr);                                                                               \
-        if (_e != cudaSuccess)                                                                                 \
+        if (_e != cudaSuccess) {                                                                               \
+            cudaGetLastError(); /* reported here; the next launch would report it again */                     \
             return mfail(m, _e == cudaErrorMemoryAllocation ? PT_ERR_OOM : PT_ERR_CUDA,                        \
                          std::string(where) + ": " + cudaGetErrorString(_e));                                  \
+        }                                                                                                      \
     } while (0)
 
 template <typename T>

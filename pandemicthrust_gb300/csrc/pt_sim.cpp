@@ -204,6 +204,7 @@ static pt_status fail(Engine *s, pt_status st, const std::string &msg)
 static pt_status cuda_fail(Engine *s, cudaError_t e, const char *where)
 {
     std::string m = std::string(where) + ": " + cudaGetErrorString(e);
+    cudaGetLastError();   // reported here; the next launch would report it again
     return fail(s, e == cudaErrorMemoryAllocation ? PT_ERR_OOM : PT_ERR_CUDA, m);
 }
 
